@@ -23,14 +23,16 @@
 #include "ocomath.h"
 #include "oco_consts.h"
 #include "oco_internal.h"
+#include "recip_div.h"
 
 namespace oco {
 using namespace k;
 
 /* ---- pillars ------------------------------------------------------------------------ */
-/* The record of one (column, z) cell from its rho and T. */
+/* The record of one (column, z) cell from its rho and T; same_T: the level below it in the column
+ * has the same temperature, bit for bit. */
 __device__ __forceinline__ void pillar_record(const double r, const double t, double fully_ionized_T, int grey,
-                                              double *__restrict__ o) {
+                                              bool same_T, double *__restrict__ o) {
   if (grey) { /* grey_parameters, continuous_opacity.f90:383-384 */
     double t2 = t * t;
     o[G_RHO] = r;
@@ -83,7 +85,7 @@ __device__ __forceinline__ void pillar_record(const double r, const double t, do
   o[F_ESCAT] = escat;
   o[F_ESCM] = escat * mp1;
   o[F_HMBF] = hmbf;
-  o[F_NEUTRAL] = ((1.0 - x) > switch_ionfraction) ? 1.0 : 0.0;
+  o[F_FLAGS] = __hiloint2double(0, (((1.0 - x) > switch_ionfraction) ? FLAG_NEUTRAL : 0) | (same_T ? FLAG_SAME_T : 0));
 #pragma unroll
   for (int q = 0; q < 6; q++) o[F_E1 + q] = E[q];
   o[F_UNSOLD] = unsold;
@@ -136,7 +138,7 @@ struct LamR {
   __device__ __forceinline__ double gff() const { return L.gff; }
   __device__ __forceinline__ double wa3() const { return L.wa3; }
   __device__ __forceinline__ double s() const { return L.s; }
-  __device__ __forceinline__ double hmon() const { return L.hmon; }
+  __device__ __forceinline__ bool hmon() const { return L.hmon != 0.0; }
   __device__ __forceinline__ double f1() const { return L.f1; }
   __device__ __forceinline__ double f2() const { return L.f2; }
   __device__ __forceinline__ double f3() const { return L.f3; }
@@ -149,14 +151,16 @@ struct LamR {
 };
 struct LamS {
   const double *p; /* &table[0][lane] */
-  template <class IT> __device__ __forceinline__ LamS(const IT &, const double *col, bool = true) : p(col) {}
+  bool hm;
+  template <class IT>
+  __device__ __forceinline__ LamS(const IT &, const double *col, bool load = true) : p(col), hm(load && col[5 * 32] != 0.0) {}
   __device__ __forceinline__ double f(int k) const { return p[k * 32]; }
   __device__ __forceinline__ double chi() const { return f(0); }
   __device__ __forceinline__ double chi1() const { return f(1); }
   __device__ __forceinline__ double gff() const { return f(2); }
   __device__ __forceinline__ double wa3() const { return f(3); }
   __device__ __forceinline__ double s() const { return f(4); }
-  __device__ __forceinline__ double hmon() const { return f(5); }
+  __device__ __forceinline__ bool hmon() const { return hm; }
   __device__ __forceinline__ double f1() const { return f(6); }
   __device__ __forceinline__ double f2() const { return f(7); }
   __device__ __forceinline__ double f3() const { return f(8); }
@@ -185,9 +189,50 @@ struct SharedRec {
   __device__ __forceinline__ double operator[](int f) const { return p[f]; }
 };
 
+/* Opacity and source function of one (z, lambda), and the absorption fraction w = 1 - albedo
+ * (stable form: the ratio of the absorption terms to the sum, no cancellation).  w comes from the
+ * quotient num/kr by recip_div.h: where ok is 0 its operands failed the checks and settle_opac
+ * divides with the operator. */
 struct Opac {
-  double op, alb, S;
-  double oma; /* stable form: 1 - albedo from the absorption terms (no cancellation) */
+  double op, w, S;
+  double num, kr;
+  int ok;
+};
+template <bool STABLE>
+__device__ __forceinline__ void settle_opac(Opac &o) {
+  if (!o.ok) {
+    const double q = o.num / o.kr;
+    o.w = STABLE ? q : 1.0 - q;
+    o.ok = 1;
+  }
+}
+
+/* The factors of a (z, lambda) point that depend on (T, lambda) alone.  A disk's temperature
+ * falls to its floor a few scale heights from the midplane (floorTemp of the decks; 85% of the
+ * levels of the AGN and Athena-style grids), so the lane keeps the last level's factors and takes
+ * them again while the record says that T has not changed by a bit: three exponentials, a
+ * division, the level sum and the free-free Gaunt factor less per point, the same bits.
+ * AGN grid, 3072 columns x 512 levels x 256 wavelengths, plain: 11.05 -> 7.2 ms; ragged turbulent
+ * batch of 400 columns 5.2 -> 3.6 ms; a disk without a floor unchanged (13.7 ms). */
+struct TFac {
+  double stim, p10f, S, lev, gff;
+};
+enum { NTC = 5 };
+struct TCacheR { /* in registers (lanes of a warp in different columns) */
+  TFac v;
+  __device__ __forceinline__ TFac get() const { return v; }
+  __device__ __forceinline__ void put(const TFac &t) { v = t; }
+};
+struct TCacheS { /* the lane's column of the warp's shared table [NTC][32] */
+  double *p;
+  __device__ __forceinline__ TFac get() const { return TFac{p[0], p[32], p[64], p[96], p[128]}; }
+  __device__ __forceinline__ void put(const TFac &t) {
+    p[0] = t.stim;
+    p[32] = t.p10f;
+    p[64] = t.S;
+    p[96] = t.lev;
+    p[128] = t.gff;
+  }
 };
 
 /* calc_opacity_and_albedo for one (z, lambda), continuous_opacity.f90:175-201 with
@@ -212,29 +257,37 @@ __device__ __forceinline__ void pow10_pow10_exp(double y1, double y2, double x3,
   r3 = f3;
 }
 
-template <bool STABLE, class R, class LM>
-__device__ __forceinline__ Opac opacity_at(const R P, const LM &L) {
-  double damping = P[F_DFT1] * L.wcm1();
-  if (damping > log_overflow_limit) damping = log_overflow_limit;
-  double p10_stim, p10_flam, e_planck;
-  pow10_pow10_exp(-(L.chi() * P[F_THETA]), ((L.f1() + L.f2() * P[F_LGT]) + L.f3() * P[F_LGT2]) - 26.0, damping,
-                  p10_stim, p10_flam, e_planck);
-  /* read after the exponentials: one register fewer across them (the batch kernels spill less) */
-  const double ionf = P[F_IONF];
-  const double stim = 1.0 - p10_stim;
-  double sm = 0.0;
+template <bool STABLE, class R, class LM, class TC>
+__device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc) {
+  const int flags = __double2loint(P[F_FLAGS]);
+  TFac t;
+  if (flags & FLAG_SAME_T) {
+    t = tc.get();
+  } else {
+    double damping = P[F_DFT1] * L.wcm1();
+    if (damping > log_overflow_limit) damping = log_overflow_limit;
+    double p10_stim, e_planck;
+    pow10_pow10_exp(-(L.chi() * P[F_THETA]), ((L.f1() + L.f2() * P[F_LGT]) + L.f3() * P[F_LGT2]) - 26.0, damping,
+                    p10_stim, t.p10f, e_planck); /* p10f = 10^(f1 + f2 lgt + f3 lgt^2 - 26) */
+    t.stim = 1.0 - p10_stim;
+    double sm = 0.0;
 #pragma unroll
-  for (int q = 0; q < 6; q++) sm = sm + L.gn(q) * P[F_E1 + q];
-  double kHbf = (((AHbf * stim) * ionf) * L.wa3()) * (P[F_UNSOLD] + sm);
-  double kHmbf = (L.hmon() != 0.0) ? ((P[F_HMBF] * stim) * ionf) * L.s() : 0.0;
-  double kHmff = P[F_AFF] * p10_flam; /* 10^(f1 + f2 lgt + f3 lgt^2 - 26) */
+    for (int q = 0; q < 6; q++) sm = sm + L.gn(q) * P[F_E1 + q];
+    t.lev = P[F_UNSOLD] + sm;
+    t.gff = 1.0 + L.gff() * ((P[F_TH1L] * L.chi1()) + 0.5);
+    t.S = L.sw5() / (e_planck - 1.0);
+    tc.put(t);
+  }
+  const double ionf = P[F_IONF];
+  double kHbf = (((AHbf * t.stim) * ionf) * L.wa3()) * t.lev;
+  double kHmbf = L.hmon() ? ((P[F_HMBF] * t.stim) * ionf) * L.s() : 0.0;
+  double kHmff = P[F_AFF] * t.p10f;
   double kr = (((kHbf + kHmbf) + kHmff) + P[F_ESCAT]) * mp1;
   double kabs = STABLE ? ((kHbf + kHmbf) + kHmff) * mp1 : 0.0;
   const double rho = P[F_RHO];
   double op = kr * rho;
-  if (P[F_NEUTRAL] != 0.0) {
-    double g_ff = 1.0 + L.gff() * ((P[F_TH1L] * L.chi1()) + 0.5);
-    double kHff = ((((stim * ionf) * alpha0) * L.wa3()) * g_ff) * P[F_EF];
+  if (flags & FLAG_NEUTRAL) {
+    double kHff = ((((t.stim * ionf) * alpha0) * L.wa3()) * t.gff) * P[F_EF];
     kr = kr + kHff * mp1;
     op = op + kr * rho;
     if (STABLE) kabs = kabs + kHff * mp1;
@@ -248,21 +301,25 @@ __device__ __forceinline__ Opac opacity_at(const R P, const LM &L) {
   }
   Opac o;
   o.op = op;
-  o.alb = P[F_ESCM] / kr;
-  o.oma = STABLE ? kabs / kr : 0.0;
-  o.S = L.sw5() / (e_planck - 1.0);
+  o.S = t.S;
+  o.kr = kr;
+  o.num = STABLE ? kabs : P[F_ESCM];
+  const double q = div_quot(o.num, kr, div_recip(kr));
+  o.w = STABLE ? q : 1.0 - q;
+  o.ok = div_b_ok(kr) & div_a_ok(o.num);
   return o;
 }
 
 /* grey_parameters, continuous_opacity.f90:377-390 */
-template <class R>
+template <bool STABLE, class R>
 __device__ __forceinline__ Opac opacity_grey(const R P, double sg) {
   double alpha = P[G_ALPHA];
   Opac o;
   o.op = (alpha + sg) * P[G_RHO];
-  o.alb = sg / (alpha + sg);
-  o.oma = alpha / (alpha + sg);
+  o.w = STABLE ? alpha / (alpha + sg) : 1.0 - sg / (alpha + sg);
   o.S = P[G_S];
+  o.ok = 1;
+  o.num = o.kr = 0.0;
   return o;
 }
 
@@ -458,80 +515,191 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
   if (double *p = it.vbot()) __stcs(p, vbot);
 }
 
-template <int FORM, bool GREY, class IT, class PA, class LMT = LamR>
+/* State of the forward elimination between two rows, and the operand checks of the quotients that
+ * the next row forms with it (recip_div.h). */
+struct Elim {
+  double c;      /* c of the row */
+  double h;      /* stable form: h of the row */
+  double d;      /* divisor of the next row's quotients: bet (plain) or c + h = -bet (stable) */
+  double u;      /* u of the row */
+  double kh;     /* mean opacity between the row and the next */
+  double yd, yk; /* 1/d, 1/kh */
+  int ok;        /* d, c, (h) and kh pass the checks */
+};
+/* What a row leaves in the scratch: gamma, u, 1/kappa and (stable) q of the row below. */
+struct RowOut {
+  double g, q, o1;
+};
+
+/* Opacities whose squares, means and ratios stay in the quotients' range. */
+__device__ __forceinline__ int op_ok(double op) { return div_in_range(op, 159, 159) & div_b_frac_ok(op); }
+
+template <int FORM>
+__device__ __forceinline__ void elim_checks(Elim &e) {
+  e.yd = div_recip(e.d);
+  e.yk = div_recip(e.kh);
+  e.ok = div_b_ok(e.d) & div_a_ok(e.c) & op_ok(e.kh);
+  if (FORM == 1) e.ok &= div_a_ok(e.h);
+}
+
+/* Centre row (fill_center_coeffs :159-165; tridag :34-40 or its difference form
+ * bet = -(c + h), h = e + a h_prev/(c_prev + h_prev)) from the row below's state, with every
+ * quotient from a shared reciprocal: 1/kappa, c and a share the mean opacities' reciprocals with
+ * the neighbouring rows; gamma and u the pivot's (plain); gamma, q, a h and u the same divisor's
+ * (stable; -bet of a row is the next row's c + h).  ok: every operand passed its check. */
+template <int FORM>
+__device__ __forceinline__ int center_fast(const Elim &e, const Opac &cur, double op_next, double dz2, Elim &n,
+                                           RowOut &r) {
+  const double op = cur.op, o2 = op * op;
+  r.o1 = div_recip(op);
+  n.kh = 0.5 * (op_next + op);
+  n.yk = div_recip(n.kh);
+  const double aa = div_quot(o2, e.kh, e.yk), cc = div_quot(o2, n.kh, n.yk);
+  const double z3 = (dz2 * (op * (op * op))) * cur.w;
+  const double dd = -(cur.S * z3);
+  const double num = dd - aa * e.u;
+  int ok = e.ok & op_ok(op) & op_ok(n.kh) & div_a_ok(num);
+  n.c = cc;
+  if (FORM == 0) {
+    const double bb = -((aa + cc) + z3);
+    r.g = div_quot(e.c, e.d, e.yd);
+    r.q = 0.0;
+    n.h = 0.0;
+    n.d = bb - aa * r.g;
+    n.yd = div_recip(n.d);
+    n.u = div_quot(num, n.d, n.yd);
+    n.ok = div_b_ok(n.d);
+  } else {
+    const double ah = aa * e.h;
+    r.g = -div_quot(e.c, e.d, e.yd);
+    r.q = div_quot(e.h, e.d, e.yd);
+    n.h = z3 + div_quot(ah, e.d, e.yd);
+    n.d = cc + n.h;
+    n.yd = div_recip(n.d);
+    n.u = -div_quot(num, n.d, n.yd);
+    n.ok = div_b_ok(n.d) & div_a_ok(n.h);
+    ok &= div_a_ok(ah);
+  }
+  /* cc passes div_a_ok: o2 in [2^-320, 2^320] over kh in [2^-160, 2^160] */
+  return ok & n.ok;
+}
+
+/* The same row with the division operator. */
+template <int FORM>
+__device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, double op_next, double dz2, Elim &n,
+                                            RowOut &r, bool &bad) {
+  const double op = cur.op, o2 = op * op;
+  r.o1 = 1.0 / op;
+  n.kh = 0.5 * (op_next + op);
+  const double aa = o2 / e.kh, cc = o2 / n.kh;
+  const double z3 = (dz2 * (op * (op * op))) * cur.w;
+  const double dd = -(cur.S * z3);
+  n.c = cc;
+  double bet;
+  if (FORM == 0) {
+    const double bb = -((aa + cc) + z3);
+    r.g = e.c / e.d;
+    r.q = 0.0;
+    n.h = 0.0;
+    n.d = bet = bb - aa * r.g;
+  } else {
+    r.g = -(e.c / e.d);
+    r.q = e.h / e.d;
+    n.h = z3 + (aa * e.h) / e.d;
+    n.d = cc + n.h;
+    bet = -n.d;
+  }
+  if (bet == 0.0) bad = true;
+  n.u = (dd - aa * e.u) / bet;
+  elim_checks<FORM>(n);
+}
+
+/* Levels are bound by dependent FP64 latency, not by a pipe: a warp alone on its SM needed as long
+ * per level (~3900 cycles) as sixteen.  So the sweep keeps its chains short and in one basic
+ * block: factors of an unchanged temperature are kept (TFac), and a row's seven (plain) or ten
+ * (stable) quotients come from four reciprocals without branches, with one check per row
+ * (without the kept factors: AGN grid plain 11.84 -> 11.05 ms, 16 columns x 500 x 250 stable
+ * 1.03 -> 0.80 ms; with them 7.2 and 0.49 ms).  Five blocks per SM (96 registers, 100 bytes of
+ * spills) are slower: 8.1 and 0.66 ms. */
+template <int FORM, bool GREY, class IT, class PA, class LMT, class TC>
 __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, double *__restrict__ gam,
                                            double *__restrict__ uu, double *__restrict__ o1s,
-                                           double *__restrict__ qs, const double *lam_col = nullptr) {
+                                           double *__restrict__ qs, const double *lam_col, TC tc) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
   const LMT L(it, lam_col, !GREY);
   double *Kb = active ? it.K() : nullptr;
   const double dz = it.dz(), dz2 = it.dz2();
+  const int64_t kz = it.kz();
   bool bad = false;
+  auto opac = [&](int z) -> Opac {
+    if (GREY) return opacity_grey<FORM == 1>(pa.at(z), it.sigma_grey());
+    return opacity_at<FORM == 1>(pa.at(z), L, tc);
+  };
 
   /* forward sweep: row 0 (fill_boundary_coeffs :187-191) */
-  Opac cur = GREY ? opacity_grey(pa.at(0), it.sigma_grey()) : opacity_at<FORM == 1>(pa.at(0), L);
-  Opac nxt = GREY ? opacity_grey(pa.at(1), it.sigma_grey()) : opacity_at<FORM == 1>(pa.at(1), L);
-  double o1 = 1.0 / cur.op, o2 = cur.op * cur.op;
-  double zeta = ((cur.op * dz2) * (FORM == 1 ? cur.oma : (1.0 - cur.alb))) * 0.25;
-  double bet, h = 0.0;
-  if (FORM == 0) {
-    bet = -(((o1 + dz) + zeta) * o2);
-  } else {
-    h = (dz + zeta) * o2;
-    bet = -(cur.op + h);
-  }
-  if (bet == 0.0) bad = true;
-  double u = (-((cur.S * zeta) * o2)) / bet;
-  uu[0] = u;
-  o1s[0] = o1;
-  if (Kb) __stcs(&Kb[0], cur.op);
-  double c_prev = cur.op;
-  double kh_prev = 0.5 * (nxt.op + cur.op); /* kappa_p(1) = kappa_m(2), :147-154 */
-  cur = nxt;
-  for (int j = 1; j < nz; j++) {
-    const double op = cur.op;
-    o1 = 1.0 / op;
-    o2 = op * op;
-    double aa, bb, cc, dd, ee;
-    if (j < nz - 1) { /* fill_center_coeffs :159-165 */
-      nxt = GREY ? opacity_grey(pa.at(j + 1), it.sigma_grey()) : opacity_at<FORM == 1>(pa.at(j + 1), L);
-      aa = o2 / kh_prev;
-      double kh = 0.5 * (nxt.op + op);
-      cc = o2 / kh;
-      double z3 = (dz2 * (op * (op * op))) * (FORM == 1 ? cur.oma : (1.0 - cur.alb));
-      bb = -((aa + cc) + z3);
-      dd = -(cur.S * z3);
-      ee = z3;
-      kh_prev = kh;
-    } else { /* fill_boundary_coeffs :193-197 */
-      aa = op;
-      double zt = ((op * dz2) * (FORM == 1 ? cur.oma : (1.0 - cur.alb))) * 0.25;
-      bb = -(((o1 + dz) + zt) * o2);
-      cc = 0.0;
-      dd = -((cur.S * zt) * o2);
-      ee = (dz + zt) * o2;
-    }
-    double g;
-    if (FORM == 0) { /* tridag :34-35 */
-      g = c_prev / bet;
-      bet = bb - aa * g;
-    } else { /* difference form: bet = -(c + h), h = e + a*h_prev/(c_prev + h_prev) */
-      double den = c_prev + h;
-      g = -(c_prev / den);
-      qs[(j - 1) * ss] = h / den; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
-      h = ee + (aa * h) / den;
-      bet = -(cc + h);
-      (void)bb;
+  Opac cur = opac(0);
+  settle_opac<FORM == 1>(cur);
+  Opac nxt = opac(1);
+  settle_opac<FORM == 1>(nxt);
+  Elim e;
+  {
+    const double o1 = 1.0 / cur.op, o2 = cur.op * cur.op;
+    const double zeta = ((cur.op * dz2) * cur.w) * 0.25;
+    double bet;
+    e.c = cur.op;
+    if (FORM == 0) {
+      e.h = 0.0;
+      e.d = bet = -(((o1 + dz) + zeta) * o2);
+    } else {
+      e.h = (dz + zeta) * o2;
+      e.d = cur.op + e.h;
+      bet = -e.d;
     }
     if (bet == 0.0) bad = true;
-    u = (dd - aa * u) / bet; /* tridag :40 */
-    gam[j * ss] = g;
-    uu[j * ss] = u;
-    o1s[j * ss] = o1;
-    if (Kb) __stcs(&Kb[j * it.kz()], op);
-    c_prev = cc;
+    e.u = (-((cur.S * zeta) * o2)) / bet;
+    e.kh = 0.5 * (nxt.op + cur.op); /* kappa_p(1) = kappa_m(2), :147-154 */
+    elim_checks<FORM>(e);
+    uu[0] = e.u;
+    o1s[0] = o1;
+    if (Kb) __stcs(&Kb[0], cur.op);
+  }
+  for (int j = 1; j < nz - 1; j++) {
     cur = nxt;
+    nxt = opac(j + 1);
+    Elim n;
+    RowOut r;
+    if (!(center_fast<FORM>(e, cur, nxt.op, dz2, n, r) & nxt.ok)) {
+      settle_opac<FORM == 1>(nxt);
+      center_slow<FORM>(e, cur, nxt.op, dz2, n, r, bad);
+    }
+    gam[j * ss] = r.g;
+    uu[j * ss] = n.u;
+    o1s[j * ss] = r.o1;
+    if (FORM == 1) qs[(j - 1) * ss] = r.q;
+    if (Kb) __stcs(&Kb[j * kz], cur.op);
+    e = n;
+  }
+  { /* fill_boundary_coeffs :193-197 */
+    const int j = nz - 1;
+    const double op = nxt.op, o1 = 1.0 / op, o2 = op * op;
+    const double zt = ((op * dz2) * nxt.w) * 0.25;
+    const double dd = -((nxt.S * zt) * o2);
+    double g, bet;
+    if (FORM == 0) {
+      g = e.c / e.d;
+      bet = -(((o1 + dz) + zt) * o2) - op * g;
+    } else {
+      g = -(e.c / e.d);
+      qs[(j - 1) * ss] = e.h / e.d; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
+      bet = -(0.0 + ((dz + zt) * o2 + (op * e.h) / e.d));
+    }
+    if (bet == 0.0) bad = true;
+    e.u = (dd - op * e.u) / bet;
+    gam[j * ss] = g;
+    uu[j * ss] = e.u;
+    o1s[j * ss] = o1;
+    if (Kb) __stcs(&Kb[j * kz], op);
   }
   if (!active) return;
   if (bad) {
@@ -539,7 +707,7 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
     atomicMin(&it.status()[1], it.id());
   }
 
-  solve_reverse<FORM>(it, u, gam, uu, o1s, qs);
+  solve_reverse<FORM>(it, e.u, gam, uu, o1s, qs);
 }
 
 }  // namespace oco

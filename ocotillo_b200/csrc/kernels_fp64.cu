@@ -56,8 +56,12 @@ __device__ __forceinline__ void store_pillars(const double *r, double *__restric
   }
 }
 
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
 __global__ void __launch_bounds__(PIL_THREADS) k_pillars(const double *__restrict__ rho,
-                                                         const double *__restrict__ T, int64_t n,
+                                                         const double *__restrict__ T, int64_t n, int nz,
                                                          double fully_ionized_T, int grey,
                                                          double *__restrict__ pil) {
   __shared__ double s_buf[PIL_THREADS / 32][32 * PIL_STRIDE];
@@ -67,7 +71,7 @@ __global__ void __launch_bounds__(PIL_THREADS) k_pillars(const double *__restric
   double r[NF];
 #pragma unroll
   for (int k = 0; k < NF; k++) r[k] = 0.0; /* grey records set three fields */
-  if (i < n) pillar_record(rho[i], T[i], fully_ionized_T, grey, r);
+  if (i < n) pillar_record(rho[i], T[i], fully_ionized_T, grey, i % nz != 0 && same_bits(T[i], T[i - 1]), r);
   store_pillars(r, s_buf[threadIdx.x >> 5], pil, i0, n);
 }
 
@@ -94,7 +98,7 @@ __global__ void __launch_bounds__(PIL_THREADS) k_pillars_batch(const double *__r
         hi = mid;
     }
     const int64_t src = cols[lo].in_off + (i - rec_pre[lo]);
-    pillar_record(rho[src], T[src], fully_ionized_T, 0, r);
+    pillar_record(rho[src], T[src], fully_ionized_T, 0, i != rec_pre[lo] && same_bits(T[src], T[src - 1]), r);
   } else {
 #pragma unroll
     for (int k = 0; k < NF; k++) r[k] = 0.0; /* not stored */
@@ -109,7 +113,7 @@ struct DirectPillars {
   __device__ __forceinline__ GlobalRec at(int z) { return GlobalRec{base + (int64_t)z * NF}; }
 };
 
-constexpr int ZC = 16;            /* z records per staged chunk */
+constexpr int ZC = 12;            /* z records per staged chunk (static shared memory up to 48 KB) */
 constexpr int WARPS_PER_BLOCK = 4; /* k_solve runs 128-thread blocks */
 constexpr long long kSpinLimit = 1ll << 26;
 
@@ -245,7 +249,8 @@ __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
       const int64_t cl = item / a.nw;
       const int iw = (int)(item - cl * a.nw);
       DirectPillars pa{a.pil + cl * (int64_t)a.nz * NF};
-      solve_item<FORM, GREY>(BlockItem{a, cl, iw}, true, pa, gam, uu, o1, qs);
+      solve_item<FORM, GREY, BlockItem, DirectPillars, LamR>(BlockItem{a, cl, iw}, true, pa, gam, uu, o1, qs, nullptr,
+                                                             TCacheR{});
     }
   }
 }
@@ -256,6 +261,7 @@ template <int FORM, bool GREY>
 __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
   __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
   __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
+  __shared__ double s_tc[WARPS_PER_BLOCK][NTC * 32]; /* the lanes' temperature factors */
   __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -293,7 +299,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
     if (!GREY) store_lam_shared(&s_lam[wib][lane], a.lam, iw, a.nw);
     __syncwarp();
     solve_item<FORM, GREY, BlockItem, StagedPillars, LamS>(BlockItem{a, cl, iw}, active, pa, gam, uu, o1, qs,
-                                                          &s_lam[wib][lane]);
+                                                          &s_lam[wib][lane], TCacheS{&s_tc[wib][lane]});
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
       /* let copies still in flight land (bounded) before the block's shared memory is released */
@@ -342,6 +348,7 @@ template <int FORM>
 __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArgs b) {
   __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
   __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
+  __shared__ double s_tc[WARPS_PER_BLOCK][NTC * 32]; /* the lanes' temperature factors */
   __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -378,7 +385,7 @@ __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArg
     store_lam_shared(&s_lam[wib][lane], b.lam + __ldg(&c->lam_off), iw, nw);
     __syncwarp();
     solve_item<FORM, false, BatchItem, StagedPillars, LamS>(BatchItem{b, c, (int64_t)t.x, iw}, active, pa, gam, uu, o1,
-                                                           qs, &s_lam[wib][lane]);
+                                                           qs, &s_lam[wib][lane], TCacheS{&s_tc[wib][lane]});
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
       pa.wait(0);
@@ -416,7 +423,7 @@ cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int
   int64_t n = ncol * nz;
   if (n == 0) return cudaSuccess;
   const int64_t blocks = (n + PIL_THREADS - 1) / PIL_THREADS;
-  k_pillars<<<(unsigned)blocks, PIL_THREADS, 0, s>>>(rho, T, n, fully_ionized_T, grey, pil);
+  k_pillars<<<(unsigned)blocks, PIL_THREADS, 0, s>>>(rho, T, n, nz, fully_ionized_T, grey, pil);
   return cudaGetLastError();
 }
 

@@ -138,10 +138,12 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
       const int z = z0 - 1 + k;
       if (z < 0 || z >= nz) continue;
       double rec[NF];
-      pillar_record(rho[z], T[z], fit, 0, rec);
-      const Opac o = opacity_at<true>(SharedRec{rec}, L);
+      pillar_record(rho[z], T[z], fit, 0, false, rec);
+      TCacheR tc;
+      Opac o = opacity_at<true>(SharedRec{rec}, L, tc);
+      settle_opac<true>(o);
       g.op[k] = o.op;
-      g.oma[k] = o.oma;
+      g.oma[k] = o.w;
       g.S[k] = o.S;
       if (Kb && k >= 1 && k <= n) Kb[z * kz] = o.op;
     }
@@ -242,8 +244,12 @@ __device__ __forceinline__ void coef_item(const IT &it, const double *rec, int z
                                           int64_t pos) {
   const int lane = threadIdx.x & 31;
   const LamR L(it, nullptr);
-  Opac o{0.0, 0.0, 0.0, 0.0};
-  if (valid) o = opacity_at<true>(SharedRec{rec}, L);
+  Opac o{};
+  if (valid) {
+    TCacheR tc;
+    o = opacity_at<true>(SharedRec{rec}, L, tc);
+    settle_opac<true>(o);
+  }
   const double op_lo = __shfl_up_sync(0xffffffffu, o.op, 1), op_hi = __shfl_down_sync(0xffffffffu, o.op, 1);
   if (!valid || lane == 0 || lane > CZ) return;
   const int nz = it.nz(), j = zl;
@@ -253,7 +259,7 @@ __device__ __forceinline__ void coef_item(const IT &it, const double *rec, int z
   S.o1[q] = 1.0 / op;
   if (double *Kb = it.K()) Kb[j * it.kz()] = op;
   if (j == 0) { /* fill_boundary_coeffs :187-191; h_0 in ee */
-    const double zeta = ((op * dz2) * o.oma) * 0.25;
+    const double zeta = ((op * dz2) * o.w) * 0.25;
     S.ee[q] = (dz + zeta) * o2;
     S.dd[q] = -((o.S * zeta) * o2);
     S.cc[q] = op;
@@ -262,12 +268,12 @@ __device__ __forceinline__ void coef_item(const IT &it, const double *rec, int z
     const double kh = 0.5 * (op_hi + op);
     S.aa[q] = o2 / kh_prev;
     S.cc[q] = o2 / kh;
-    const double z3 = (dz2 * (op * (op * op))) * o.oma;
+    const double z3 = (dz2 * (op * (op * op))) * o.w;
     S.dd[q] = -(o.S * z3);
     S.ee[q] = z3;
   } else { /* fill_boundary_coeffs :193-197 */
     S.aa[q] = op;
-    const double zt = ((op * dz2) * o.oma) * 0.25;
+    const double zt = ((op * dz2) * o.w) * 0.25;
     S.cc[q] = 0.0;
     S.dd[q] = -((o.S * zt) * o2);
     S.ee[q] = (dz + zt) * o2;
@@ -304,7 +310,7 @@ __global__ void __launch_bounds__(CWARPS * 32, 4) k_repair_coef(const RepairArgs
     const double *T = a.block ? a.T + col * a.nz : a.T + bc->in_off;
     const int zl = c * CZ - 1 + lane;
     const bool valid = zl >= 0 && zl < nz && lane <= CZ + 1;
-    if (valid) pillar_record(rho[zl], T[zl], a.fully_ionized_T, 0, rec);
+    if (valid) pillar_record(rho[zl], T[zl], a.fully_ionized_T, 0, false, rec);
     for (unsigned m = a.bits[w]; m; m &= m - 1) {
       const int b = __ffs(m) - 1;
       const int64_t pos = a.slot[w * 32 + b];

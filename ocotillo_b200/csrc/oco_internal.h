@@ -35,7 +35,7 @@ enum PillarField {
   F_ESCAT,     /* Thomson cross-section per H (c_o :149) */
   F_ESCM,      /* e_scatter*mp1 (albedo numerator, c_o :195) */
   F_HMBF,      /* H- bound-free factor (c_o :161) */
-  F_NEUTRAL,   /* 1 if (1 - NHII/N) > switch_ionfraction else 0 (c_o :262) */
+  F_FLAGS,     /* integer bits in the low word: FLAG_NEUTRAL, FLAG_SAME_T */
   F_E1,        /* exp(-chi_n(n)*k1*T1), n = 1..6 (c_o :238) */
   F_E2,
   F_E3,
@@ -51,6 +51,8 @@ enum PillarField {
   F_PAD,
   NF
 };
+constexpr int FLAG_NEUTRAL = 1; /* (1 - NHII/N) > switch_ionfraction (c_o :262) */
+constexpr int FLAG_SAME_T = 2;  /* T equals the level below's bit for bit (never set at z = 0) */
 /* Grey RT re-uses the slots (continuous_opacity.f90:377-390). */
 enum GreyField { G_RHO = F_RHO, G_S = F_RHO1, G_ALPHA = F_T1 };
 
