@@ -85,7 +85,8 @@ __device__ __forceinline__ void pillar_record(const double r, const double t, do
   o[F_ESCAT] = escat;
   o[F_ESCM] = escat * mp1;
   o[F_HMBF] = hmbf;
-  o[F_FLAGS] = __hiloint2double(0, (((1.0 - x) > switch_ionfraction) ? FLAG_NEUTRAL : 0) | (same_T ? FLAG_SAME_T : 0));
+  o[F_FLAGS] = __hiloint2double(0, (((1.0 - x) > switch_ionfraction) ? FLAG_NEUTRAL : 0) | (same_T ? FLAG_SAME_T : 0) |
+                                       (div_a_ok(o[F_ESCM]) ? FLAG_ESC_OK : 0));
 #pragma unroll
   for (int q = 0; q < 6; q++) o[F_E1 + q] = E[q];
   o[F_UNSOLD] = unsold;
@@ -93,8 +94,7 @@ __device__ __forceinline__ void pillar_record(const double r, const double t, do
   o[F_EF] = (((0.5 * log10e) * theta1) * Iev1) * oco_pow10(-(theta * Iev));   /* c_o :265 */
   o[F_TPOW] = oco_pow(t * 1e-4, -1.5);                                              /* c_o :290 */
   o[F_LZ] = (oco_log(ne * (nHI + nHII)) + 2.0 * oco_log(1.0)) - 0.5 * oco_log(t);   /* c_o :292-294 */
-  o[F_LNRHO] = oco_log(r);
-  o[F_PAD] = 0.0;
+  o[F_PAD0] = o[F_PAD1] = 0.0;
 }
 
 /* ---- per-wavelength constants ------------------------------------------------------- */
@@ -136,8 +136,7 @@ struct LamR {
   __device__ __forceinline__ double chi() const { return L.chi; }
   __device__ __forceinline__ double chi1() const { return L.chi1; }
   __device__ __forceinline__ double gff() const { return L.gff; }
-  __device__ __forceinline__ double wa3() const { return L.wa3; }
-  __device__ __forceinline__ double s() const { return L.s; }
+  __device__ __forceinline__ double2 wa3_s() const { return make_double2(L.wa3, L.s); }
   __device__ __forceinline__ bool hmon() const { return L.hmon != 0.0; }
   __device__ __forceinline__ double f1() const { return L.f1; }
   __device__ __forceinline__ double f2() const { return L.f2; }
@@ -150,61 +149,73 @@ struct LamR {
   __device__ __forceinline__ double sw5() const { return L.sw5; }
 };
 struct LamS {
-  const double *p; /* &table[0][lane] */
+  const double *p; /* &table[0][lane] past the pairs */
   bool hm;
   template <class IT>
-  __device__ __forceinline__ LamS(const IT &, const double *col, bool load = true) : p(col), hm(load && col[5 * 32] != 0.0) {}
+  __device__ __forceinline__ LamS(const IT &, const double *table, bool load = true)
+      : p(table + 64 + (threadIdx.x & 31)), hm(load && p[3 * 32] != 0.0) {}
   __device__ __forceinline__ double f(int k) const { return p[k * 32]; }
+  /* the lane's (wa3, s) pair: two of the constants that every point reads, in one load */
+  __device__ __forceinline__ double2 wa3_s() const {
+    return *reinterpret_cast<const double2 *>(p - 64 + (threadIdx.x & 31));
+  }
   __device__ __forceinline__ double chi() const { return f(0); }
   __device__ __forceinline__ double chi1() const { return f(1); }
   __device__ __forceinline__ double gff() const { return f(2); }
-  __device__ __forceinline__ double wa3() const { return f(3); }
-  __device__ __forceinline__ double s() const { return f(4); }
   __device__ __forceinline__ bool hmon() const { return hm; }
-  __device__ __forceinline__ double f1() const { return f(6); }
-  __device__ __forceinline__ double f2() const { return f(7); }
-  __device__ __forceinline__ double f3() const { return f(8); }
-  __device__ __forceinline__ double gn(int q) const { return f(9 + q); }
-  __device__ __forceinline__ double nu9() const { return f(15); }
-  __device__ __forceinline__ double l3nu() const { return f(16); }
-  __device__ __forceinline__ double hnuk() const { return f(17); }
-  __device__ __forceinline__ double wcm1() const { return f(18); }
-  __device__ __forceinline__ double sw5() const { return f(19); }
+  __device__ __forceinline__ double f1() const { return f(4); }
+  __device__ __forceinline__ double f2() const { return f(5); }
+  __device__ __forceinline__ double f3() const { return f(6); }
+  __device__ __forceinline__ double gn(int q) const { return f(7 + q); }
+  __device__ __forceinline__ double nu9() const { return f(13); }
+  __device__ __forceinline__ double l3nu() const { return f(14); }
+  __device__ __forceinline__ double hnuk() const { return f(15); }
+  __device__ __forceinline__ double wcm1() const { return f(16); }
+  __device__ __forceinline__ double sw5() const { return f(17); }
 };
-/* Lane's column of the warp's shared table (wavelength iw of the global table). */
-__device__ __forceinline__ void store_lam_shared(double *col, const double *__restrict__ lam, int iw, int nw) {
-  const int src[NLF] = {L_CHI, L_CHI1, L_GFF, L_WA3, L_SCOEF, L_HMON, L_F1, L_F2, L_F3, L_GN1, L_GN2, L_GN3,
-                        L_GN4, L_GN5, L_GN6, L_NU9, L_L3NU, L_HNUK, L_WCM1, L_SW5};
+/* Lane's constants in the warp's shared table: the 32 lanes' (wa3, s) pairs, then [field][32]
+ * (wavelength iw of the global table). */
+__device__ __forceinline__ void store_lam_shared(double *table, int lane, const double *__restrict__ lam, int iw, int nw) {
+  const int src[NLF - 2] = {L_CHI, L_CHI1, L_GFF, L_HMON, L_F1, L_F2, L_F3, L_GN1, L_GN2, L_GN3,
+                            L_GN4, L_GN5, L_GN6, L_NU9, L_L3NU, L_HNUK, L_WCM1, L_SW5};
+  table[2 * lane] = __ldg(lam + (int64_t)L_WA3 * nw + iw);
+  table[2 * lane + 1] = __ldg(lam + (int64_t)L_SCOEF * nw + iw);
 #pragma unroll
-  for (int k = 0; k < NLF; k++) col[k * 32] = __ldg(lam + (int64_t)src[k] * nw + iw);
+  for (int k = 0; k < NLF - 2; k++) table[64 + k * 32 + lane] = __ldg(lam + (int64_t)src[k] * nw + iw);
 }
 
 /* One pillar record, read through the read-only cache (global) or from shared memory. */
 struct GlobalRec {
   const double *p;
   __device__ __forceinline__ double operator[](int f) const { return __ldg(p + f); }
+  __device__ __forceinline__ double2 pair(int f) const { return __ldg(reinterpret_cast<const double2 *>(p + f)); }
 };
 struct SharedRec {
   const double *p;
   __device__ __forceinline__ double operator[](int f) const { return p[f]; }
+  __device__ __forceinline__ double2 pair(int f) const { return *reinterpret_cast<const double2 *>(p + f); }
 };
 
 /* Opacity and source function of one (z, lambda), and the absorption fraction w = 1 - albedo
  * (stable form: the ratio of the absorption terms to the sum, no cancellation).  w comes from the
- * quotient num/kr by recip_div.h: where ok is 0 its operands failed the checks and settle_opac
- * divides with the operator. */
+ * quotient num/kr by recip_div.h: where wok is 0 its operands failed the checks and settle_opac
+ * divides with the operator.  ook: op lies in the range of the rows' quotients. */
 struct Opac {
   double op, w, S;
   double num, kr;
-  int ok;
+  int wok, ook;
 };
 template <bool STABLE>
 __device__ __forceinline__ void settle_opac(Opac &o) {
-  if (!o.ok) {
+  if (!o.wok) {
     const double q = o.num / o.kr;
     o.w = STABLE ? q : 1.0 - q;
-    o.ok = 1;
+    o.wok = 1;
   }
+}
+/* Opacities (positive) whose squares, means and ratios stay in the quotients' range. */
+__device__ __forceinline__ int op_ok(double op) {
+  return ((div_hi(op) - ((uint32_t)(1023 - 159) << 20)) < ((uint32_t)318 << 20)) & div_b_frac_ok(op);
 }
 
 /* The factors of a (z, lambda) point that depend on (T, lambda) alone.  A disk's temperature
@@ -215,23 +226,24 @@ __device__ __forceinline__ void settle_opac(Opac &o) {
  * AGN grid, 3072 columns x 512 levels x 256 wavelengths, plain: 11.05 -> 7.2 ms; ragged turbulent
  * batch of 400 columns 5.2 -> 3.6 ms; a disk without a floor unchanged (13.7 ms). */
 struct TFac {
-  double stim, p10f, S, lev, gff;
+  double stim, astim, p10f, S, lev, gff; /* astim = AHbf*stim */
 };
-enum { NTC = 5 };
+enum { NTC = 6 };
 struct TCacheR { /* in registers (lanes of a warp in different columns) */
   TFac v;
   __device__ __forceinline__ TFac get() const { return v; }
   __device__ __forceinline__ void put(const TFac &t) { v = t; }
 };
-struct TCacheS { /* the lane's column of the warp's shared table [NTC][32] */
-  double *p;
-  __device__ __forceinline__ TFac get() const { return TFac{p[0], p[32], p[64], p[96], p[128]}; }
+struct TCacheS { /* the lane's pairs in the warp's shared table [NTC/2][32] */
+  double2 *p;
+  __device__ __forceinline__ TFac get() const {
+    const double2 a = p[0], b = p[32], c = p[64];
+    return TFac{a.x, a.y, b.x, b.y, c.x, c.y};
+  }
   __device__ __forceinline__ void put(const TFac &t) {
-    p[0] = t.stim;
-    p[32] = t.p10f;
-    p[64] = t.S;
-    p[96] = t.lev;
-    p[128] = t.gff;
+    p[0] = make_double2(t.stim, t.astim);
+    p[32] = make_double2(t.p10f, t.S);
+    p[64] = make_double2(t.lev, t.gff);
   }
 };
 
@@ -259,7 +271,9 @@ __device__ __forceinline__ void pow10_pow10_exp(double y1, double y2, double x3,
 
 template <bool STABLE, class R, class LM, class TC>
 __device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc) {
-  const int flags = __double2loint(P[F_FLAGS]);
+  const double2 em = P.pair(F_ESCM);
+  const int flags = __double2loint(em.y);
+  const bool neutral = flags & FLAG_NEUTRAL;
   TFac t;
   if (flags & FLAG_SAME_T) {
     t = tc.get();
@@ -270,6 +284,7 @@ __device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc) {
     pow10_pow10_exp(-(L.chi() * P[F_THETA]), ((L.f1() + L.f2() * P[F_LGT]) + L.f3() * P[F_LGT2]) - 26.0, damping,
                     p10_stim, t.p10f, e_planck); /* p10f = 10^(f1 + f2 lgt + f3 lgt^2 - 26) */
     t.stim = 1.0 - p10_stim;
+    t.astim = AHbf * t.stim;
     double sm = 0.0;
 #pragma unroll
     for (int q = 0; q < 6; q++) sm = sm + L.gn(q) * P[F_E1 + q];
@@ -278,35 +293,35 @@ __device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc) {
     t.S = L.sw5() / (e_planck - 1.0);
     tc.put(t);
   }
-  const double ionf = P[F_IONF];
-  double kHbf = (((AHbf * t.stim) * ionf) * L.wa3()) * t.lev;
-  double kHmbf = L.hmon() ? ((P[F_HMBF] * t.stim) * ionf) * L.s() : 0.0;
-  double kHmff = P[F_AFF] * t.p10f;
-  double kr = (((kHbf + kHmbf) + kHmff) + P[F_ESCAT]) * mp1;
-  double kabs = STABLE ? ((kHbf + kHmbf) + kHmff) * mp1 : 0.0;
-  const double rho = P[F_RHO];
-  double op = kr * rho;
-  if (flags & FLAG_NEUTRAL) {
-    double kHff = ((((t.stim * ionf) * alpha0) * L.wa3()) * t.gff) * P[F_EF];
-    kr = kr + kHff * mp1;
+  const double2 ih = P.pair(F_IONF), ae = P.pair(F_AFF), re = P.pair(F_RHO), ws = L.wa3_s();
+  const double ionf = ih.x, rho = re.x;
+  const double kHbf = ((t.astim * ionf) * ws.x) * t.lev;
+  const double kHm = ((ih.y * t.stim) * ionf) * ws.y;
+  const double kHmbf = L.hmon() ? kHm : 0.0;
+  const double kHmff = ae.x * t.p10f;
+  const double abs3 = (kHbf + kHmbf) + kHmff;
+  double kr = (abs3 + ae.y) * mp1, op = kr * rho, x;
+  if (neutral) {
+    x = (((((t.stim * ionf) * alpha0) * ws.x) * t.gff) * re.y) * mp1; /* kHff*mp1 */
+    kr = kr + x;
     op = op + kr * rho;
-    if (STABLE) kabs = kabs + kHff * mp1;
   } else {
     double gaunt = oco_log(oco_exp(5.960 - (sqrt3 * pi1) * oco_log(L.nu9() * P[F_TPOW])) + exp1);
     double lnq = (P[F_LZ] - L.l3nu()) + oco_log(1.0 - oco_exp(-(L.hnuk() * P[F_T1])));
     double krho = (bremsstrahlung_constant * oco_exp(lnq)) * gaunt;
     op = op + krho;
-    kr = kr + op * P[F_RHO1];
-    if (STABLE) kabs = kabs + op * P[F_RHO1];
+    x = op * P[F_RHO1];
+    kr = kr + x;
   }
   Opac o;
   o.op = op;
-  o.S = t.S;
   o.kr = kr;
-  o.num = STABLE ? kabs : P[F_ESCM];
-  const double q = div_quot(o.num, kr, div_recip(kr));
+  o.S = t.S;
+  o.num = STABLE ? abs3 * mp1 + x : em.x;
+  const double q = div_quot(o.num, o.kr, div_recip(o.kr));
   o.w = STABLE ? q : 1.0 - q;
-  o.ok = div_b_ok(kr) & div_a_ok(o.num);
+  o.wok = div_b_ok(o.kr) & (STABLE ? div_a_ok(o.num) : (flags & FLAG_ESC_OK) != 0);
+  o.ook = op_ok(o.op);
   return o;
 }
 
@@ -318,8 +333,9 @@ __device__ __forceinline__ Opac opacity_grey(const R P, double sg) {
   o.op = (alpha + sg) * P[G_RHO];
   o.w = STABLE ? alpha / (alpha + sg) : 1.0 - sg / (alpha + sg);
   o.S = P[G_S];
-  o.ok = 1;
   o.num = o.kr = 0.0;
+  o.wok = 1;
+  o.ook = op_ok(o.op);
   return o;
 }
 
@@ -333,6 +349,8 @@ __device__ __forceinline__ Opac opacity_grey(const R P, double sg) {
 __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }
+
+constexpr int RING = 6; /* levels of scratch that the stable form's reverse sweep keeps in registers */
 
 /* PF: the scratch was written long before (by another kernel) and few warps run, so its loads
  * are DRAM latency: 1/kappa is loaded with the other scratch arrays 8 levels ahead of the
@@ -393,10 +411,9 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
     };
     auto stepD = [&](int k, double uf, double qk, double gk1) { stepDo(k, uf, qk, gk1, o1s[(k + 3) * ss]); };
     int k = n - 5;
-    for (; k >= 7; k -= 8) { /* scratch loads of 8 steps hoisted off the serial chain */
-      double ub[8], qb[8], gb[8];
-      if (PF) {
-        double ob[8];
+    if (PF) {
+      for (; k >= 7; k -= 8) { /* scratch loads of 8 steps hoisted off the serial chain */
+        double ub[8], qb[8], gb[8], ob[8];
         for (int q = 16; q < 24 && k - q >= 0; q++) { /* the block after next */
           prefetch_l2(&uu[(k - q) * ss]);
           prefetch_l2(&qs[(k - q) * ss]);
@@ -412,16 +429,31 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
-      } else {
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          ub[q] = uu[(k - q) * ss];
-          qb[q] = qs[(k - q) * ss];
-          gb[q] = gam[(k - q + 1) * ss];
-        }
-#pragma unroll
-        for (int q = 0; q < 8; q++) stepD(k - q, ub[q], qb[q], gb[q]);
       }
+    } else if (k >= RING - 1) { /* the scratch of RING levels in registers, as the plain form below */
+      constexpr int R = RING;
+      double ub[R], qb[R], gb[R], ob[R];
+#pragma unroll
+      for (int q = 0; q < R; q++) {
+        ub[q] = uu[(k - q) * ss];
+        qb[q] = qs[(k - q) * ss];
+        gb[q] = gam[(k - q + 1) * ss];
+        ob[q] = o1s[(k - q + 3) * ss];
+      }
+      for (; k >= 2 * R - 1; k -= R) {
+#pragma unroll
+        for (int q = 0; q < R; q++) {
+          const int kn = k - R - q;
+          stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
+          ub[q] = uu[kn * ss];
+          qb[q] = qs[kn * ss];
+          gb[q] = gam[(kn + 1) * ss];
+          ob[q] = o1s[(kn + 3) * ss];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < R; q++) stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
+      k -= R;
     }
     for (; k >= 0; k--) stepD(k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss]);
     if (Ub) __stcs(&Ub[2 * uz], 2.0 * U0 - U1);
@@ -457,8 +489,9 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
     double w0 = u4, w1 = u3, w2 = u2, w3 = u1, w4 = g1, w5 = g2, w6 = g3;
     vtop = emitV(n - 1, o1s[(n - 1) * ss], w0, w1, w2, w4, w5, w6);
     int kk = n - 5;
-    /* blocks of 8 steps with the scratch loads hoisted off the serial U chain */
-    for (; kk >= 7; kk -= 8) {
+    /* the scratch of 8 levels in registers: a level's slot is reloaded for 8 levels further down
+     * as soon as it is used, so that loads stay in flight throughout */
+    if (kk >= 7) {
       double ub[8], gb[8], ob[8];
 #pragma unroll
       for (int q = 0; q < 8; q++) {
@@ -466,13 +499,25 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
         gb[q] = gam[(kk - q + 1) * ss];
         ob[q] = o1s[(kk - q + 3) * ss];
       }
-#pragma unroll
-      for (int q = 0; q < 8; q++) {
-        double Uk = ub[q] - gb[q] * w0;
-        if (Ub) __stcs(&Ub[(3 + kk - q) * uz], Uk);
+      auto step = [&](int k, double uk, double gk1, double o1k3) {
+        double Uk = uk - gk1 * w0;
+        if (Ub) __stcs(&Ub[(3 + k) * uz], Uk);
         w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = Uk;
-        emitV(kk - q + 3, ob[q], w0, w1, w2, w4, w5, w6);
+        emitV(k + 3, o1k3, w0, w1, w2, w4, w5, w6);
+      };
+      for (; kk >= 15; kk -= 8) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+          const int kn = kk - 8 - q;
+          step(kk - q, ub[q], gb[q], ob[q]);
+          ub[q] = uu[kn * ss];
+          gb[q] = gam[(kn + 1) * ss];
+          ob[q] = o1s[(kn + 3) * ss];
+        }
       }
+#pragma unroll
+      for (int q = 0; q < 8; q++) step(kk - q, ub[q], gb[q], ob[q]);
+      kk -= 8;
     }
     for (; kk >= 0; kk--) {
       double Uk = uu[kk * ss] - gam[(kk + 1) * ss] * w0;
@@ -531,14 +576,12 @@ struct RowOut {
   double g, q, o1;
 };
 
-/* Opacities whose squares, means and ratios stay in the quotients' range. */
-__device__ __forceinline__ int op_ok(double op) { return div_in_range(op, 159, 159) & div_b_frac_ok(op); }
-
+/* ook: the opacities on both sides of kh pass op_ok. */
 template <int FORM>
-__device__ __forceinline__ void elim_checks(Elim &e) {
+__device__ __forceinline__ void elim_checks(Elim &e, int ook) {
   e.yd = div_recip(e.d);
   e.yk = div_recip(e.kh);
-  e.ok = div_b_ok(e.d) & div_a_ok(e.c) & op_ok(e.kh);
+  e.ok = ook & div_b_ok(e.d) & div_a_ok(e.c) & div_b_frac_ok(e.kh);
   if (FORM == 1) e.ok &= div_a_ok(e.h);
 }
 
@@ -546,19 +589,21 @@ __device__ __forceinline__ void elim_checks(Elim &e) {
  * bet = -(c + h), h = e + a h_prev/(c_prev + h_prev)) from the row below's state, with every
  * quotient from a shared reciprocal: 1/kappa, c and a share the mean opacities' reciprocals with
  * the neighbouring rows; gamma and u the pivot's (plain); gamma, q, a h and u the same divisor's
- * (stable; -bet of a row is the next row's c + h).  ok: every operand passed its check. */
+ * (stable; -bet of a row is the next row's c + h).  Returns whether every operand passed its
+ * check (kh lies between two opacities that did; c, an opacity squared over a mean, is then in
+ * range). */
 template <int FORM>
-__device__ __forceinline__ int center_fast(const Elim &e, const Opac &cur, double op_next, double dz2, Elim &n,
+__device__ __forceinline__ int center_fast(const Elim &e, const Opac &cur, const Opac &nxt, double dz2, Elim &n,
                                            RowOut &r) {
   const double op = cur.op, o2 = op * op;
   r.o1 = div_recip(op);
-  n.kh = 0.5 * (op_next + op);
+  n.kh = 0.5 * (nxt.op + op);
   n.yk = div_recip(n.kh);
   const double aa = div_quot(o2, e.kh, e.yk), cc = div_quot(o2, n.kh, n.yk);
   const double z3 = (dz2 * (op * (op * op))) * cur.w;
   const double dd = -(cur.S * z3);
   const double num = dd - aa * e.u;
-  int ok = e.ok & op_ok(op) & op_ok(n.kh) & div_a_ok(num);
+  int ok = e.ok & div_a_ok(num);
   n.c = cc;
   if (FORM == 0) {
     const double bb = -((aa + cc) + z3);
@@ -580,17 +625,17 @@ __device__ __forceinline__ int center_fast(const Elim &e, const Opac &cur, doubl
     n.ok = div_b_ok(n.d) & div_a_ok(n.h);
     ok &= div_a_ok(ah);
   }
-  /* cc passes div_a_ok: o2 in [2^-320, 2^320] over kh in [2^-160, 2^160] */
+  n.ok &= nxt.ook & div_b_frac_ok(n.kh);
   return ok & n.ok;
 }
 
 /* The same row with the division operator. */
 template <int FORM>
-__device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, double op_next, double dz2, Elim &n,
+__device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, const Opac &nxt, double dz2, Elim &n,
                                             RowOut &r, bool &bad) {
   const double op = cur.op, o2 = op * op;
   r.o1 = 1.0 / op;
-  n.kh = 0.5 * (op_next + op);
+  n.kh = 0.5 * (nxt.op + op);
   const double aa = o2 / e.kh, cc = o2 / n.kh;
   const double z3 = (dz2 * (op * (op * op))) * cur.w;
   const double dd = -(cur.S * z3);
@@ -611,23 +656,28 @@ __device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, doub
   }
   if (bet == 0.0) bad = true;
   n.u = (dd - aa * e.u) / bet;
-  elim_checks<FORM>(n);
+  elim_checks<FORM>(n, cur.ook & nxt.ook);
 }
 
 /* Levels are bound by dependent FP64 latency, not by a pipe: a warp alone on its SM needed as long
- * per level (~3900 cycles) as sixteen.  So the sweep keeps its chains short and in one basic
- * block: factors of an unchanged temperature are kept (TFac), and a row's seven (plain) or ten
- * (stable) quotients come from four reciprocals without branches, with one check per row
+ * per level (~3900 cycles) as sixteen.  So the sweep keeps its chains short and side by side:
+ * factors of an unchanged temperature are kept (TFac), a row's seven (plain) or ten (stable)
+ * quotients come from four reciprocals without branches, with one check per row
  * (without the kept factors: AGN grid plain 11.84 -> 11.05 ms, 16 columns x 500 x 250 stable
- * 1.03 -> 0.80 ms; with them 7.2 and 0.49 ms).  Five blocks per SM (96 registers, 100 bytes of
- * spills) are slower: 8.1 and 0.66 ms. */
+ * 1.03 -> 0.80 ms; with them 7.2 and 0.49 ms).  The GPU then runs this kernel at its 1000 W limit
+ * (1.82 GHz), so what counts is instructions per point: records, kept factors and constants are
+ * read in 16-byte pairs, the record pointer is advanced instead of computed, and the reverse
+ * sweep's loads never pause (ring of levels): 7.48 -> 7.37 ms, 0.49 -> 0.41 ms, batch of 400
+ * columns 3.67 -> 3.53 ms.  Not faster: row j's elimination beside the opacity of level j + 2
+ * (7.53 ms; 0.39 ms), the exponentials and logarithms behind calls (7.45; 14.5 for 13.6 ms on the
+ * warm disk), five blocks per SM at 96 registers (7.8 ms). */
 template <int FORM, bool GREY, class IT, class PA, class LMT, class TC>
 __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, double *__restrict__ gam,
                                            double *__restrict__ uu, double *__restrict__ o1s,
-                                           double *__restrict__ qs, const double *lam_col, TC tc) {
+                                           double *__restrict__ qs, const double *lam_table, TC tc) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
-  const LMT L(it, lam_col, !GREY);
+  const LMT L(it, lam_table, !GREY);
   double *Kb = active ? it.K() : nullptr;
   const double dz = it.dz(), dz2 = it.dz2();
   const int64_t kz = it.kz();
@@ -638,9 +688,8 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
   };
 
   /* forward sweep: row 0 (fill_boundary_coeffs :187-191) */
-  Opac cur = opac(0);
+  Opac cur = opac(0), nxt = opac(1);
   settle_opac<FORM == 1>(cur);
-  Opac nxt = opac(1);
   settle_opac<FORM == 1>(nxt);
   Elim e;
   {
@@ -659,47 +708,49 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
     if (bet == 0.0) bad = true;
     e.u = (-((cur.S * zeta) * o2)) / bet;
     e.kh = 0.5 * (nxt.op + cur.op); /* kappa_p(1) = kappa_m(2), :147-154 */
-    elim_checks<FORM>(e);
+    elim_checks<FORM>(e, cur.ook & nxt.ook);
     uu[0] = e.u;
     o1s[0] = o1;
     if (Kb) __stcs(&Kb[0], cur.op);
   }
+  auto put = [&](int j, const RowOut &r, double u, double op) {
+    gam[j * ss] = r.g;
+    uu[j * ss] = u;
+    o1s[j * ss] = r.o1;
+    if (FORM == 1) qs[(j - 1) * ss] = r.q;
+    if (Kb) __stcs(&Kb[j * kz], op);
+  };
   for (int j = 1; j < nz - 1; j++) {
     cur = nxt;
     nxt = opac(j + 1);
     Elim n;
     RowOut r;
-    if (!(center_fast<FORM>(e, cur, nxt.op, dz2, n, r) & nxt.ok)) {
+    if (!(center_fast<FORM>(e, cur, nxt, dz2, n, r) & nxt.wok)) {
       settle_opac<FORM == 1>(nxt);
-      center_slow<FORM>(e, cur, nxt.op, dz2, n, r, bad);
+      center_slow<FORM>(e, cur, nxt, dz2, n, r, bad);
     }
-    gam[j * ss] = r.g;
-    uu[j * ss] = n.u;
-    o1s[j * ss] = r.o1;
-    if (FORM == 1) qs[(j - 1) * ss] = r.q;
-    if (Kb) __stcs(&Kb[j * kz], cur.op);
+    put(j, r, n.u, cur.op);
     e = n;
   }
   { /* fill_boundary_coeffs :193-197 */
-    const int j = nz - 1;
-    const double op = nxt.op, o1 = 1.0 / op, o2 = op * op;
+    const double op = nxt.op, o2 = op * op;
     const double zt = ((op * dz2) * nxt.w) * 0.25;
     const double dd = -((nxt.S * zt) * o2);
-    double g, bet;
+    RowOut r;
+    double bet;
+    r.o1 = 1.0 / op;
     if (FORM == 0) {
-      g = e.c / e.d;
-      bet = -(((o1 + dz) + zt) * o2) - op * g;
+      r.g = e.c / e.d;
+      r.q = 0.0;
+      bet = -(((r.o1 + dz) + zt) * o2) - op * r.g;
     } else {
-      g = -(e.c / e.d);
-      qs[(j - 1) * ss] = e.h / e.d; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
+      r.g = -(e.c / e.d);
+      r.q = e.h / e.d; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
       bet = -(0.0 + ((dz + zt) * o2 + (op * e.h) / e.d));
     }
     if (bet == 0.0) bad = true;
     e.u = (dd - op * e.u) / bet;
-    gam[j * ss] = g;
-    uu[j * ss] = e.u;
-    o1s[j * ss] = o1;
-    if (Kb) __stcs(&Kb[j * kz], op);
+    put(nz - 1, r, e.u, op);
   }
   if (!active) return;
   if (bad) {

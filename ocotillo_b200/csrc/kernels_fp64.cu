@@ -113,7 +113,7 @@ struct DirectPillars {
   __device__ __forceinline__ GlobalRec at(int z) { return GlobalRec{base + (int64_t)z * NF}; }
 };
 
-constexpr int ZC = 12;            /* z records per staged chunk (static shared memory up to 48 KB) */
+constexpr int ZC = 11;            /* z records per staged chunk (static shared memory up to 48 KB) */
 constexpr int WARPS_PER_BLOCK = 4; /* k_solve runs 128-thread blocks */
 constexpr long long kSpinLimit = 1ll << 26;
 
@@ -141,7 +141,8 @@ struct StagedPillars {
   double *buf;    /* shared: [2][ZC*NF] */
   uint32_t bar0;  /* shared address of two mbarriers (8 B each) */
   const double *src;
-  int nz, nchunks, cur;
+  const double *rec; /* next record, left of them in the buffer */
+  int nz, nchunks, cur, left;
   uint32_t waits;    /* bit b: parity of the next wait on buffer b */
   uint32_t inflight; /* bit b: a copy into buffer b has been issued and not yet waited for */
   bool failed;
@@ -173,23 +174,29 @@ struct StagedPillars {
   __device__ __forceinline__ void begin(const double *column, int lane) {
     src = column;
     cur = -1;
+    left = 0;
     nchunks = (nz + ZC - 1) / ZC;
     __syncwarp();
     if (lane == 0) issue(0);
     note_issue(0);
   }
-  __device__ __forceinline__ SharedRec at(int z) {
-    const int c = z / ZC;
-    if (c != cur) { /* c == cur + 1 */
+  /* The next record; z counts up from 0. */
+  __device__ __forceinline__ SharedRec at(int) {
+    if (left == 0) {
+      const int c = ++cur;
       __syncwarp();
       if (!failed && c + 1 < nchunks) {
         if ((threadIdx.x & 31) == 0) issue(c + 1);
         note_issue(c + 1);
       }
       if (!failed && !wait(c & 1)) failed = true;
-      cur = c;
+      rec = buf + (c & 1) * (ZC * NF);
+      left = ZC;
     }
-    return SharedRec{buf + (c & 1) * (ZC * NF) + (z - c * ZC) * NF};
+    left--;
+    const SharedRec r{rec};
+    rec += NF;
+    return r;
   }
 };
 
@@ -261,7 +268,7 @@ template <int FORM, bool GREY>
 __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
   __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
   __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
-  __shared__ double s_tc[WARPS_PER_BLOCK][NTC * 32]; /* the lanes' temperature factors */
+  __shared__ double2 s_tc[WARPS_PER_BLOCK][NTC / 2 * 32]; /* the lanes' temperature factors */
   __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -296,10 +303,10 @@ __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
     const bool active = iw_raw < a.nw;
     const int iw = active ? iw_raw : a.nw - 1;
     pa.begin(a.pil + cl * (int64_t)a.nz * NF, lane);
-    if (!GREY) store_lam_shared(&s_lam[wib][lane], a.lam, iw, a.nw);
+    if (!GREY) store_lam_shared(s_lam[wib], lane, a.lam, iw, a.nw);
     __syncwarp();
     solve_item<FORM, GREY, BlockItem, StagedPillars, LamS>(BlockItem{a, cl, iw}, active, pa, gam, uu, o1, qs,
-                                                          &s_lam[wib][lane], TCacheS{&s_tc[wib][lane]});
+                                                          s_lam[wib], TCacheS{s_tc[wib] + lane});
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
       /* let copies still in flight land (bounded) before the block's shared memory is released */
@@ -348,7 +355,7 @@ template <int FORM>
 __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArgs b) {
   __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
   __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
-  __shared__ double s_tc[WARPS_PER_BLOCK][NTC * 32]; /* the lanes' temperature factors */
+  __shared__ double2 s_tc[WARPS_PER_BLOCK][NTC / 2 * 32]; /* the lanes' temperature factors */
   __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -382,10 +389,10 @@ __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArg
     const int iw = active ? iw_raw : nw - 1;
     pa.nz = __ldg(&c->nz);
     pa.begin(b.pil + __ldg(&c->rec_off) * NF, lane);
-    store_lam_shared(&s_lam[wib][lane], b.lam + __ldg(&c->lam_off), iw, nw);
+    store_lam_shared(s_lam[wib], lane, b.lam + __ldg(&c->lam_off), iw, nw);
     __syncwarp();
     solve_item<FORM, false, BatchItem, StagedPillars, LamS>(BatchItem{b, c, (int64_t)t.x, iw}, active, pa, gam, uu, o1,
-                                                           qs, &s_lam[wib][lane], TCacheS{&s_tc[wib][lane]});
+                                                           qs, s_lam[wib], TCacheS{s_tc[wib] + lane});
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
       pa.wait(0);

@@ -23,19 +23,21 @@ inline bool block_elements_fit(int nx, int ny, int nz, int nw) {
  * (gas_state.f90:30-110 plus every factor of continuous_opacity.f90 that depends on z
  * only).  Layout [col][z][NF] doubles. */
 enum PillarField {
-  F_RHO = 0,   /* rho */
-  F_RHO1,      /* 1/rho */
-  F_T1,        /* 1/T */
+  /* read at every point, in 16-byte pairs */
+  F_IONF = 0,  /* nHI/(nHI+nHII) */
+  F_HMBF,      /* H- bound-free factor (c_o :161) */
+  F_AFF,       /* ionf*ne*k*T (H- free-free prefactor, c_o :339) */
+  F_ESCAT,     /* Thomson cross-section per H (c_o :149) */
+  F_RHO,       /* rho */
+  F_EF,        /* H free-free energy factor (c_o :265) */
+  F_ESCM,      /* e_scatter*mp1 (albedo numerator, c_o :195) */
+  F_FLAGS,     /* integer bits in the low word: FLAG_NEUTRAL, FLAG_SAME_T, FLAG_ESC_OK */
+  /* read where the temperature changes */
   F_DFT1,      /* damping_factor_const*T1 (source function, c_o :399) */
   F_THETA,     /* 5040/T */
   F_TH1L,      /* theta1*log10e (H free-free Gaunt factor, c_o :264) */
   F_LGT,       /* log10(theta) */
   F_LGT2,      /* log10(theta)**2 */
-  F_IONF,      /* nHI/(nHI+nHII) */
-  F_ESCAT,     /* Thomson cross-section per H (c_o :149) */
-  F_ESCM,      /* e_scatter*mp1 (albedo numerator, c_o :195) */
-  F_HMBF,      /* H- bound-free factor (c_o :161) */
-  F_FLAGS,     /* integer bits in the low word: FLAG_NEUTRAL, FLAG_SAME_T */
   F_E1,        /* exp(-chi_n(n)*k1*T1), n = 1..6 (c_o :238) */
   F_E2,
   F_E3,
@@ -43,16 +45,19 @@ enum PillarField {
   F_E5,
   F_E6,
   F_UNSOLD,    /* Unsold integral (c_o :242) */
-  F_AFF,       /* ionf*ne*k*T (H- free-free prefactor, c_o :339) */
-  F_EF,        /* H free-free energy factor (c_o :265) */
+  /* read at ionized points */
+  F_RHO1,      /* 1/rho */
+  F_T1,        /* 1/T */
   F_TPOW,      /* (T*1e-4)**(-1.5) (bremsstrahlung Gaunt factor, c_o :290) */
   F_LZ,        /* log(ne*(nHI+nHII)) + 2*log(1) - 0.5*log(T) (c_o :292-294) */
-  F_LNRHO,     /* log(rho) (mixed form) */
-  F_PAD,
+  F_PAD0,
+  F_PAD1,
   NF
 };
+static_assert(NF % 2 == 0, "records are read in 16-byte pairs");
 constexpr int FLAG_NEUTRAL = 1; /* (1 - NHII/N) > switch_ionfraction (c_o :262) */
 constexpr int FLAG_SAME_T = 2;  /* T equals the level below's bit for bit (never set at z = 0) */
+constexpr int FLAG_ESC_OK = 4;  /* e_scatter*mp1 passes div_a_ok (recip_div.h) */
 /* Grey RT re-uses the slots (continuous_opacity.f90:377-390). */
 enum GreyField { G_RHO = F_RHO, G_S = F_RHO1, G_ALPHA = F_T1 };
 
