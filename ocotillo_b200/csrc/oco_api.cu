@@ -773,11 +773,6 @@ static int epilogue_args(oco_ctx *c, const oco_params *p, EpilogueArgs &a) {
   return OCO_OK;
 }
 
-static int epilogue_blocks(oco_ctx *c, int64_t items) {
-  const int64_t want = (items + 255) / 256, cap = (int64_t)c->num_sms * 8;
-  return (int)std::max<int64_t>(1, std::min(want, cap));
-}
-
 extern "C" int oco_intensities_device(oco_ctx *c, const oco_params *p, const double *U, const double *V, double *Ip,
                                       double *Im, void *stream) {
   EpilogueArgs a;
@@ -789,7 +784,7 @@ extern "C" int oco_intensities_device(oco_ctx *c, const oco_params *p, const dou
   a.Ip = Ip;
   a.Im = Im;
   CU(cudaSetDevice(c->device));
-  CU(launch_intensities(a, epilogue_blocks(c, a.ncol * a.nw), (cudaStream_t)stream));
+  CU(launch_intensities(a, c->num_sms, (cudaStream_t)stream));
   c->launches++;
   return OCO_OK;
 }
@@ -807,7 +802,7 @@ extern "C" int oco_optical_depth_device(oco_ctx *c, const oco_params *p, const d
   a.photo = photo_index;
   a.target = target_tau;
   CU(cudaSetDevice(c->device));
-  CU(launch_optical_depth(a, epilogue_blocks(c, a.ncol * a.nw), (cudaStream_t)stream));
+  CU(launch_optical_depth(a, (cudaStream_t)stream));
   c->launches++;
   return OCO_OK;
 }
@@ -820,7 +815,7 @@ extern "C" int oco_integrated_flux_device(oco_ctx *c, const oco_params *p, const
   if (!V || !F) return oco_set_err(c, OCO_EINVAL, "V and F are required");
   const int64_t ncol = (int64_t)p->nx * p->ny;
   CU(cudaSetDevice(c->device));
-  CU(launch_integrated_flux(V, c->trapw.as<double>(), ncol, p->nw, ncol, F, epilogue_blocks(c, ncol),
+  CU(launch_integrated_flux(V, c->trapw.as<double>(), ncol, p->nw, ncol, F, c->num_sms,
                             (cudaStream_t)stream));
   c->launches++;
   return OCO_OK;
