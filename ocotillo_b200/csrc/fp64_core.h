@@ -340,32 +340,127 @@ __device__ __forceinline__ Opac opacity_grey(const R P, double sg) {
 }
 
 /* ---- the solve ----------------------------------------------------------------------- */
-/* Solves one (column, wavelength) item.  `active` false: the lane only keeps the warp's
- * shared pipeline in step (staged path, wavelength index beyond nw) and stores nothing. */
-/* The reverse sweep of one item (back-substitution, tridag :43-45; ghost zones :49-62; flux
- * :96-109) from the forward sweep's last u and its scratch (gam, uu, o1s and, stable form, qs at
- * stride it.ss()), storing U, V and the emergent fluxes through the item accessor. */
 /* Issues an L2 prefetch of the line holding p. */
 __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }
 
-constexpr int RING = 6; /* levels of scratch that the stable form's reverse sweep keeps in registers */
+/* Where the reverse sweep's outputs go.  LaneStores: each lane writes its item's levels itself
+ * (coalesced where lambda is the fastest index).  active false: nothing is written. */
+template <class IT>
+struct LaneStores {
+  /* kappa leaves in the forward sweep and the scratch holds 1/kappa (false), or the scratch holds
+   * kappa, which leaves with U and V, and the reverse sweep takes 1/kappa */
+  static constexpr bool KAPPA_REVERSE = false;
+  double *Ub, *Kb, *Vb;
+  int64_t uz, kz, vz;
+  __device__ __forceinline__ LaneStores(const IT &it, bool active)
+      : Ub(active ? it.U() : nullptr), Kb(active ? it.K() : nullptr), Vb(active ? it.V() : nullptr), uz(it.uz()),
+        kz(it.kz()), vz(it.vz()) {}
+  __device__ __forceinline__ void u(int m, double x) const {
+    if (Ub) __stcs(&Ub[m * uz], x);
+  }
+  __device__ __forceinline__ void k(int j, double op) const {
+    if (Kb) __stcs(&Kb[j * kz], op);
+  }
+  __device__ __forceinline__ void v(int j, double x, double) const {
+    if (Vb) __stcs(&Vb[j * vz], x);
+  }
+  /* U_k and V of level k + 3, slot q of a group of 8 levels in decreasing order; a: that level's
+   * scratch value */
+  __device__ __forceinline__ void put(int, int k, double U, double x, double a) const {
+    u(3 + k, U);
+    v(k + 3, x, a);
+  }
+  __device__ __forceinline__ void flush(int, int) const {}
+};
 
-/* PF: the scratch was written long before (by another kernel) and few warps run, so its loads
- * are DRAM latency: 1/kappa is loaded with the other scratch arrays 8 levels ahead of the
- * serial chain and the next blocks of 8 levels are prefetched into L2 (the block solves keep
- * PF off: their scratch is recent and many warps hide its latency). */
-template <int FORM, class IT, bool PF = false>
-__device__ __forceinline__ void solve_reverse(const IT &it, double u, const double *__restrict__ gam,
-                                              const double *__restrict__ uu, const double *__restrict__ o1s,
-                                              const double *__restrict__ qs) {
+/* Layouts with z fastest (the reference's): neighbouring lanes' levels lie a row apart, so a
+ * group of 8 levels of the warp's 32 items is gathered in shared memory (tile [3][8][TILE_ROW])
+ * and written as 64-byte runs, four rows per store instruction; the few edge levels are stored
+ * lane by lane.  ROWS: the warp's rows are equally spaced (one column's wavelengths), otherwise
+ * each row's address comes from its lane.  The stores are plain ones: a run's first and last
+ * sectors are completed by the neighbouring groups in L2.  Measured: see k_solve_staged. */
+constexpr int TILE_Z = 8, TILE_ROW = 36; /* 36: conflict-free both ways */
+constexpr int TILE_DOUBLES = 3 * TILE_Z * TILE_ROW;
+template <class IT, bool ROWS>
+struct TileStores : LaneStores<IT> {
+  static constexpr bool KAPPA_REVERSE = true;
+  double *tile;
+  double *U0, *K0, *V0; /* row of lane 0 (ROWS) or of the lane */
+  int64_t us, ks;       /* elements between rows */
+  int nrows;
+  __device__ __forceinline__ TileStores(const IT &it, bool active, double *t)
+      : LaneStores<IT>(it, active), tile(t), U0(it.U()), K0(it.K()), V0(it.V()), us(it.urow()), ks(it.krow()) {
+    nrows = __popc(__ballot_sync(0xffffffffu, active)); /* active lanes come first */
+    if (ROWS) {
+      U0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)U0, 0);
+      K0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)K0, 0);
+      V0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)V0, 0);
+    }
+  }
+  __device__ __forceinline__ void v(int j, double x, double op) const {
+    LaneStores<IT>::v(j, x, op);
+    LaneStores<IT>::k(j, op);
+  }
+  __device__ __forceinline__ void put(int q, int, double U, double v, double op) const {
+    double *t = tile + q * TILE_ROW + (threadIdx.x & 31);
+    t[0] = U;
+    t[TILE_Z * TILE_ROW] = v;
+    t[2 * TILE_Z * TILE_ROW] = op;
+  }
+  __device__ __forceinline__ void rows(double *base, int64_t stride, const double *t, int z, int n) const {
+    if (!base) return;
+    const int lane = threadIdx.x & 31, s = lane & (TILE_Z - 1), r = lane / TILE_Z;
+    const double *p = t + (n - 1 - s) * TILE_ROW + r;
+    double *g = base + r * stride + z + s;
+    if (ROWS && n == TILE_Z && nrows == 32) { /* nearly always */
+#pragma unroll
+      for (int i = 0; i < 32 / 4; i++) g[(int64_t)(4 * i) * stride] = p[4 * i];
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < 32 / 4; i++) {
+      double *d = ROWS ? g + (int64_t)(4 * i) * stride
+                       : (double *)__shfl_sync(0xffffffffu, (unsigned long long)base, 4 * i + r) + z + s;
+      if (s < n && 4 * i + r < nrows) *d = p[4 * i];
+    }
+  }
+  /* writes the n levels put last, k the lowest */
+  __device__ __forceinline__ void flush(int k, int n) const {
+    __syncwarp();
+    rows(U0, us, tile, 3 + k, n);
+    rows(V0, ks, tile + TILE_Z * TILE_ROW, 3 + k, n);
+    rows(K0, ks, tile + 2 * TILE_Z * TILE_ROW, 3 + k, n);
+    __syncwarp();
+  }
+};
+
+/* 1/kappa of a scratch value (see KAPPA_REVERSE), rounded as the division. */
+template <class ST>
+__device__ __forceinline__ double scratch_o1(double a) {
+  if (!ST::KAPPA_REVERSE) return a;
+  double y = div_recip(a);
+  if (!op_ok(a)) y = 1.0 / a;
+  return y;
+}
+
+constexpr int RING = 4; /* levels of scratch that the stable form's reverse sweep keeps in registers */
+
+/* The reverse sweep of one item (back-substitution, tridag :43-45; ghost zones :49-62; flux
+ * :96-109) from the forward sweep's last u and its scratch (gamma, u, kap: 1/kappa or kappa, and, stable form, q at
+ * stride it.ss()), storing U, V (and kappa) through st and the emergent fluxes through the item
+ * accessor.  PF: the scratch was written long before (by another kernel) and few warps run, so its
+ * loads are DRAM latency: blocks of 8 levels are loaded ahead of the serial chain and the next
+ * blocks prefetched into L2 (the block solves keep PF off: their scratch is recent and many warps
+ * hide its latency). */
+template <int FORM, bool PF = false, class IT, class ST>
+__device__ __forceinline__ void solve_reverse(const IT &it, bool active, double u, const double *__restrict__ gam,
+                                              const double *__restrict__ uu, const double *__restrict__ kap,
+                                              const double *__restrict__ qs, const ST &st) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
-  double *Ub = it.U();
-  double *Vb = it.V();
   const double dz1 = it.dz1();
-  const int64_t uz = it.uz();
   double vtop = 0.0, vbot = 0.0;
   if (FORM == 1 && nz >= 4) {
     /* Stable form: the differences D_k = U_k - U_{k+1} = u_k - q_k U_{k+1} come out of the
@@ -374,7 +469,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
      * stencil on U, accurate where U's differences are below its resolution. */
     const int n = nz;
     double Un = u; /* U_{n-1} */
-    if (Ub) __stcs(&Ub[(3 + n - 1) * uz], Un);
+    st.u(3 + n - 1, Un);
     double Uk[3], Dt[3];
     for (int t = 0; t < 3; t++) {
       const int k = n - 2 - t;
@@ -382,34 +477,34 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
       Dt[t] = uf - qs[k * ss] * Un;
       Un = uf - gam[(k + 1) * ss] * Un;
       Uk[t] = Un;
-      if (Ub) __stcs(&Ub[(3 + k) * uz], Un);
+      st.u(3 + k, Un);
     }
     const double fn = u;
-    if (Ub) __stcs(&Ub[(n + 3) * uz], 2.0 * fn - Uk[0]);
-    if (Ub) __stcs(&Ub[(n + 4) * uz], 2.0 * fn - Uk[1]);
-    if (Ub) __stcs(&Ub[(n + 5) * uz], 2.0 * fn - Uk[2]);
+    st.u(n + 3, 2.0 * fn - Uk[0]);
+    st.u(n + 4, 2.0 * fn - Uk[1]);
+    st.u(n + 5, 2.0 * fn - Uk[2]);
     double d0 = Dt[2], d1 = Dt[1], d2 = Dt[0], d3 = Dt[0], d4 = Dt[1], d5 = Dt[2];
-    auto emitDo = [&](int j, double o1j) -> double {
+    auto flux = [&](double op) -> double {
       const double s1 = d2 + d3;
       const double s2 = (s1 + d1) + d4;
       const double s3 = (s2 + d0) + d5;
       const double df = -((1.0 / 60.0) * (((45.0 * s1) - 9.0 * s2) + s3));
-      const double v = ((-1.0 * o1j) * df) * dz1;
-      if (Vb) __stcs(&Vb[j * it.vz()], v);
+      return ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
+    };
+    auto edge = [&](int j) -> double {
+      const double op = kap[j * ss], v = flux(op);
+      st.v(j, v, op);
       return v;
     };
-    auto emitD = [&](int j) -> double { return emitDo(j, o1s[j * ss]); };
-    vtop = emitD(n - 1);
+    vtop = edge(n - 1);
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = u; /* the four lowest U seen so far */
-    auto stepDo = [&](int k, double uf, double qk, double gk1, double o1k3) {
+    auto step = [&](int slot, int k, double uf, double qk, double gk1, double op) {
       const double Dk = uf - qk * Un;
       Un = uf - gk1 * Un;
-      if (Ub) __stcs(&Ub[(3 + k) * uz], Un);
       U3 = U2; U2 = U1; U1 = U0; U0 = Un;
       d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = Dk;
-      emitDo(k + 3, o1k3);
+      st.put(slot, k, Un, flux(op), op);
     };
-    auto stepD = [&](int k, double uf, double qk, double gk1) { stepDo(k, uf, qk, gk1, o1s[(k + 3) * ss]); };
     int k = n - 5;
     if (PF) {
       for (; k >= 7; k -= 8) { /* scratch loads of 8 steps hoisted off the serial chain */
@@ -418,123 +513,124 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
           prefetch_l2(&uu[(k - q) * ss]);
           prefetch_l2(&qs[(k - q) * ss]);
           prefetch_l2(&gam[(k - q + 1) * ss]);
-          prefetch_l2(&o1s[(k - q + 3) * ss]);
+          prefetch_l2(&kap[(k - q + 3) * ss]);
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) {
           ub[q] = uu[(k - q) * ss];
           qb[q] = qs[(k - q) * ss];
           gb[q] = gam[(k - q + 1) * ss];
-          ob[q] = o1s[(k - q + 3) * ss];
+          ob[q] = kap[(k - q + 3) * ss];
         }
 #pragma unroll
-        for (int q = 0; q < 8; q++) stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
+        for (int q = 0; q < 8; q++) step(q, k - q, ub[q], qb[q], gb[q], ob[q]);
+        st.flush(k - 7, 8);
       }
-    } else if (k >= RING - 1) { /* the scratch of RING levels in registers, as the plain form below */
-      constexpr int R = RING;
-      double ub[R], qb[R], gb[R], ob[R];
+    } else if (k >= 7) {
+      /* the scratch of RING levels in registers: a level's slot is reloaded for RING levels
+       * further down as soon as it is used, so that loads stay in flight throughout */
+      double ub[RING], qb[RING], gb[RING], ob[RING];
 #pragma unroll
-      for (int q = 0; q < R; q++) {
+      for (int q = 0; q < RING; q++) {
         ub[q] = uu[(k - q) * ss];
         qb[q] = qs[(k - q) * ss];
         gb[q] = gam[(k - q + 1) * ss];
-        ob[q] = o1s[(k - q + 3) * ss];
+        ob[q] = kap[(k - q + 3) * ss];
       }
-      for (; k >= 2 * R - 1; k -= R) {
+      for (; k >= 7; k -= 8) {
 #pragma unroll
-        for (int q = 0; q < R; q++) {
-          const int kn = k - R - q;
-          stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
-          ub[q] = uu[kn * ss];
-          qb[q] = qs[kn * ss];
-          gb[q] = gam[(kn + 1) * ss];
-          ob[q] = o1s[(kn + 3) * ss];
+        for (int q = 0; q < 8; q++) {
+          const int r = q % RING, kn = max(k - RING - q, 0);
+          step(q, k - q, ub[r], qb[r], gb[r], ob[r]);
+          ub[r] = uu[kn * ss];
+          qb[r] = qs[kn * ss];
+          gb[r] = gam[(kn + 1) * ss];
+          ob[r] = kap[(kn + 3) * ss];
         }
+        st.flush(k - 7, 8);
       }
-#pragma unroll
-      for (int q = 0; q < R; q++) stepDo(k - q, ub[q], qb[q], gb[q], ob[q]);
-      k -= R;
     }
-    for (; k >= 0; k--) stepD(k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss]);
-    if (Ub) __stcs(&Ub[2 * uz], 2.0 * U0 - U1);
-    if (Ub) __stcs(&Ub[1 * uz], 2.0 * U0 - U2);
-    if (Ub) __stcs(&Ub[0], 2.0 * U0 - U3);
+    if (k >= 0) {
+      const int m = k + 1;
+      for (int q = 0; k >= 0; k--, q++) step(q, k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss], kap[(k + 3) * ss]);
+      st.flush(0, m);
+    }
+    st.u(2, 2.0 * U0 - U1);
+    st.u(1, 2.0 * U0 - U2);
+    st.u(0, 2.0 * U0 - U3);
     const double D0 = d0, D1 = d1, D2 = d2;
     d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D0;
-    emitD(2);
+    edge(2);
     d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D1;
-    emitD(1);
+    edge(1);
     d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D2;
-    vbot = emitD(0);
+    vbot = edge(0);
   } else if (nz >= 4) {
-    auto emitV = [&](int j, double o1j, double w0, double w1, double w2, double w4, double w5, double w6) -> double {
-      double df = (1.0 / 60.0) * (((45.0 * (w4 - w2)) - 9.0 * (w5 - w1)) + (w6 - w0));
-      double v = ((-1.0 * o1j) * df) * dz1;
-      if (Vb) __stcs(&Vb[j * it.vz()], v);
-      return v;
-    };
     const int n = nz;
     double u1 = u; /* U_{n-1} */
     double u2 = uu[(n - 2) * ss] - gam[(n - 1) * ss] * u1;
     double u3 = uu[(n - 3) * ss] - gam[(n - 2) * ss] * u2;
     double u4 = uu[(n - 4) * ss] - gam[(n - 3) * ss] * u3;
-    if (Ub) __stcs(&Ub[(3 + n - 1) * uz], u1);
-    if (Ub) __stcs(&Ub[(3 + n - 2) * uz], u2);
-    if (Ub) __stcs(&Ub[(3 + n - 3) * uz], u3);
-    if (Ub) __stcs(&Ub[(3 + n - 4) * uz], u4);
+    st.u(3 + n - 1, u1);
+    st.u(3 + n - 2, u2);
+    st.u(3 + n - 3, u3);
+    st.u(3 + n - 4, u4);
     double g1 = 2.0 * u1 - u2, g2 = 2.0 * u1 - u3, g3 = 2.0 * u1 - u4;
-    if (Ub) __stcs(&Ub[(n + 3) * uz], g1);
-    if (Ub) __stcs(&Ub[(n + 4) * uz], g2);
-    if (Ub) __stcs(&Ub[(n + 5) * uz], g3);
+    st.u(n + 3, g1);
+    st.u(n + 4, g2);
+    st.u(n + 5, g3);
     double w0 = u4, w1 = u3, w2 = u2, w3 = u1, w4 = g1, w5 = g2, w6 = g3;
-    vtop = emitV(n - 1, o1s[(n - 1) * ss], w0, w1, w2, w4, w5, w6);
+    auto flux = [&](double op) -> double {
+      double df = (1.0 / 60.0) * (((45.0 * (w4 - w2)) - 9.0 * (w5 - w1)) + (w6 - w0));
+      return ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
+    };
+    auto edge = [&](int j) -> double {
+      const double op = kap[j * ss], v = flux(op);
+      st.v(j, v, op);
+      return v;
+    };
+    vtop = edge(n - 1);
+    auto step = [&](int slot, int k, double uk, double gk1, double op) {
+      double Uk = uk - gk1 * w0;
+      w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = Uk;
+      st.put(slot, k, Uk, flux(op), op);
+    };
     int kk = n - 5;
-    /* the scratch of 8 levels in registers: a level's slot is reloaded for 8 levels further down
-     * as soon as it is used, so that loads stay in flight throughout */
-    if (kk >= 7) {
+    if (kk >= 7) { /* the scratch of 8 levels in registers, as above */
       double ub[8], gb[8], ob[8];
 #pragma unroll
       for (int q = 0; q < 8; q++) {
         ub[q] = uu[(kk - q) * ss];
         gb[q] = gam[(kk - q + 1) * ss];
-        ob[q] = o1s[(kk - q + 3) * ss];
+        ob[q] = kap[(kk - q + 3) * ss];
       }
-      auto step = [&](int k, double uk, double gk1, double o1k3) {
-        double Uk = uk - gk1 * w0;
-        if (Ub) __stcs(&Ub[(3 + k) * uz], Uk);
-        w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = Uk;
-        emitV(k + 3, o1k3, w0, w1, w2, w4, w5, w6);
-      };
-      for (; kk >= 15; kk -= 8) {
+      for (; kk >= 7; kk -= 8) {
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-          const int kn = kk - 8 - q;
-          step(kk - q, ub[q], gb[q], ob[q]);
+          const int kn = max(kk - 8 - q, 0);
+          step(q, kk - q, ub[q], gb[q], ob[q]);
           ub[q] = uu[kn * ss];
           gb[q] = gam[(kn + 1) * ss];
-          ob[q] = o1s[(kn + 3) * ss];
+          ob[q] = kap[(kn + 3) * ss];
         }
+        st.flush(kk - 7, 8);
       }
-#pragma unroll
-      for (int q = 0; q < 8; q++) step(kk - q, ub[q], gb[q], ob[q]);
-      kk -= 8;
     }
-    for (; kk >= 0; kk--) {
-      double Uk = uu[kk * ss] - gam[(kk + 1) * ss] * w0;
-      if (Ub) __stcs(&Ub[(3 + kk) * uz], Uk);
-      w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = Uk;
-      emitV(kk + 3, o1s[(kk + 3) * ss], w0, w1, w2, w4, w5, w6);
+    if (kk >= 0) {
+      const int m = kk + 1;
+      for (int q = 0; kk >= 0; kk--, q++) step(q, kk, uu[kk * ss], gam[(kk + 1) * ss], kap[(kk + 3) * ss]);
+      st.flush(0, m);
     }
     double b1 = 2.0 * w0 - w1, b2 = 2.0 * w0 - w2, b3 = 2.0 * w0 - w3;
-    if (Ub) __stcs(&Ub[2 * uz], b1);
-    if (Ub) __stcs(&Ub[1 * uz], b2);
-    if (Ub) __stcs(&Ub[0], b3);
+    st.u(2, b1);
+    st.u(1, b2);
+    st.u(0, b3);
     w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b1;
-    emitV(2, o1s[2 * ss], w0, w1, w2, w4, w5, w6);
+    edge(2);
     w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b2;
-    emitV(1, o1s[1 * ss], w0, w1, w2, w4, w5, w6);
+    edge(1);
     w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b3;
-    vbot = emitV(0, o1s[0], w0, w1, w2, w4, w5, w6);
+    vbot = edge(0);
   } else { /* nz = 2 or 3: the reference's ghost update order matters (ghosts feed ghosts) */
     double f[9];
     const int n1 = 3, n2 = nz + 2;
@@ -544,18 +640,19 @@ __device__ __forceinline__ void solve_reverse(const IT &it, double u, const doub
       f[n1 - i] = 2.0 * f[n1] - f[n1 + i];
       f[n2 + i] = 2.0 * f[n2] - f[n2 - i];
     }
-    if (Ub)
-      for (int m = 0; m < nz + 6; m++) __stcs(&Ub[m * uz], f[m]);
+    for (int m = 0; m < nz + 6; m++) st.u(m, f[m]);
     for (int j = 0; j < nz; j++) {
       int c = n1 + j;
       double df = (1.0 / 60.0) * (((45.0 * (f[c + 1] - f[c - 1])) - 9.0 * (f[c + 2] - f[c - 2])) +
                                   (f[c + 3] - f[c - 3]));
-      double v = ((-1.0 * o1s[j * ss]) * df) * dz1;
-      if (Vb) __stcs(&Vb[j * it.vz()], v);
+      const double op = kap[j * ss];
+      double v = ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
+      st.v(j, v, op);
       if (j == 0) vbot = v;
       if (j == nz - 1) vtop = v;
     }
   }
+  if (!active) return;
   if (double *p = it.vtop()) __stcs(p, vtop);
   if (double *p = it.vbot()) __stcs(p, vbot);
 }
@@ -571,7 +668,7 @@ struct Elim {
   double yd, yk; /* 1/d, 1/kh */
   int ok;        /* d, c, (h) and kh pass the checks */
 };
-/* What a row leaves in the scratch: gamma, u, 1/kappa and (stable) q of the row below. */
+/* What a row leaves in the scratch beside u: gamma, (stable) q of the row below, 1/kappa. */
 struct RowOut {
   double g, q, o1;
 };
@@ -587,8 +684,8 @@ __device__ __forceinline__ void elim_checks(Elim &e, int ook) {
 
 /* Centre row (fill_center_coeffs :159-165; tridag :34-40 or its difference form
  * bet = -(c + h), h = e + a h_prev/(c_prev + h_prev)) from the row below's state, with every
- * quotient from a shared reciprocal: 1/kappa, c and a share the mean opacities' reciprocals with
- * the neighbouring rows; gamma and u the pivot's (plain); gamma, q, a h and u the same divisor's
+ * quotient from a shared reciprocal: c and a share the mean opacities' reciprocals with the
+ * neighbouring rows; gamma and u the pivot's (plain); gamma, q, a h and u the same divisor's
  * (stable; -bet of a row is the next row's c + h).  Returns whether every operand passed its
  * check (kh lies between two opacities that did; c, an opacity squared over a mean, is then in
  * range). */
@@ -596,7 +693,7 @@ template <int FORM>
 __device__ __forceinline__ int center_fast(const Elim &e, const Opac &cur, const Opac &nxt, double dz2, Elim &n,
                                            RowOut &r) {
   const double op = cur.op, o2 = op * op;
-  r.o1 = div_recip(op);
+  r.o1 = div_recip(op); /* dead where the scratch holds kappa */
   n.kh = 0.5 * (nxt.op + op);
   n.yk = div_recip(n.kh);
   const double aa = div_quot(o2, e.kh, e.yk), cc = div_quot(o2, n.kh, n.yk);
@@ -671,16 +768,14 @@ __device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, cons
  * columns 3.67 -> 3.53 ms.  Not faster: row j's elimination beside the opacity of level j + 2
  * (7.53 ms; 0.39 ms), the exponentials and logarithms behind calls (7.45; 14.5 for 13.6 ms on the
  * warm disk), five blocks per SM at 96 registers (7.8 ms). */
-template <int FORM, bool GREY, class IT, class PA, class LMT, class TC>
+template <int FORM, bool GREY, class IT, class PA, class LMT, class TC, class ST>
 __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, double *__restrict__ gam,
-                                           double *__restrict__ uu, double *__restrict__ o1s,
-                                           double *__restrict__ qs, const double *lam_table, TC tc) {
+                                           double *__restrict__ uu, double *__restrict__ kap,
+                                           double *__restrict__ qs, const double *lam_table, TC tc, const ST &st) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
   const LMT L(it, lam_table, !GREY);
-  double *Kb = active ? it.K() : nullptr;
   const double dz = it.dz(), dz2 = it.dz2();
-  const int64_t kz = it.kz();
   bool bad = false;
   auto opac = [&](int z) -> Opac {
     if (GREY) return opacity_grey<FORM == 1>(pa.at(z), it.sigma_grey());
@@ -710,15 +805,15 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
     e.kh = 0.5 * (nxt.op + cur.op); /* kappa_p(1) = kappa_m(2), :147-154 */
     elim_checks<FORM>(e, cur.ook & nxt.ook);
     uu[0] = e.u;
-    o1s[0] = o1;
-    if (Kb) __stcs(&Kb[0], cur.op);
+    kap[0] = ST::KAPPA_REVERSE ? cur.op : o1;
+    if (!ST::KAPPA_REVERSE) st.k(0, cur.op);
   }
   auto put = [&](int j, const RowOut &r, double u, double op) {
     gam[j * ss] = r.g;
     uu[j * ss] = u;
-    o1s[j * ss] = r.o1;
+    kap[j * ss] = ST::KAPPA_REVERSE ? op : r.o1;
+    if (!ST::KAPPA_REVERSE) st.k(j, op);
     if (FORM == 1) qs[(j - 1) * ss] = r.q;
-    if (Kb) __stcs(&Kb[j * kz], op);
   };
   for (int j = 1; j < nz - 1; j++) {
     cur = nxt;
@@ -752,13 +847,12 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
     e.u = (dd - op * e.u) / bet;
     put(nz - 1, r, e.u, op);
   }
-  if (!active) return;
-  if (bad) {
+  if (active && bad) {
     atomicAdd(&it.status()[0], 1ull);
     atomicMin(&it.status()[1], it.id());
   }
-
-  solve_reverse<FORM>(it, e.u, gam, uu, o1s, qs);
+  __syncwarp();
+  solve_reverse<FORM>(it, active, e.u, gam, uu, kap, qs, st);
 }
 
 }  // namespace oco

@@ -10,10 +10,11 @@
  *               of 32 consecutive items (lambda fastest) from a device counter.  Per item:
  *               opacity, albedo and source function (continuous_opacity.f90:175-201,
  *               :377-409), tridiagonal coefficients (auxiliary.f90:111-201), the Thomas
- *               forward sweep (auxiliary.f90:14-41) streaming gamma, u and 1/kappa to a
+ *               forward sweep (auxiliary.f90:14-41) streaming gamma, u and kappa to a
  *               per-warp-slot scratch, then the back-substitution (:43-45), ghost zones
  *               (:49-62) and 6th-order flux (:64-109) in one reverse sweep with a 7-point
- *               register window.
+ *               register window.  All outputs leave in the reverse sweep (fp64_core.h: LaneStores,
+ *               TileStores).
  *
  * Output stores (U, kappa, V and the emergent flux) use the streaming cache hint (st.global.cs,
  * evict first): they are never read back, and L2 then keeps more of the forward sweep's scratch
@@ -176,6 +177,7 @@ struct StagedPillars {
     cur = -1;
     left = 0;
     nchunks = (nz + ZC - 1) / ZC;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); /* this lane's tile accesses before the copies */
     __syncwarp();
     if (lane == 0) issue(0);
     note_issue(0);
@@ -227,6 +229,9 @@ struct BlockItem {
   __device__ __forceinline__ int64_t vz() const { return a.V_zs; }
   __device__ __forceinline__ double *vtop() const { return a.Vtop ? a.Vtop + pidx() : nullptr; }
   __device__ __forceinline__ double *vbot() const { return a.Vbot ? a.Vbot + pidx() : nullptr; }
+  /* z fastest: elements between the rows of neighbouring wavelengths */
+  __device__ __forceinline__ int64_t urow() const { return a.ld_col * a.U_is; }
+  __device__ __forceinline__ int64_t krow() const { return a.ld_col * (int64_t)a.nz; }
   __device__ __forceinline__ int64_t ss() const { return 32; }
   __device__ __forceinline__ unsigned long long *status() const { return a.status; }
   __device__ __forceinline__ unsigned long long id() const {
@@ -234,9 +239,20 @@ struct BlockItem {
   }
 };
 
-/* Generic path: warp tasks are 32 consecutive items of the flattened (column, lambda) index. */
-template <int FORM, bool GREY>
+/* The stores of a warp's outputs: lane by lane, or (REF, z fastest) through the tile. */
+template <bool REF, bool ROWS, class IT>
+__device__ __forceinline__ auto make_stores(const IT &it, bool active, double *tile) {
+  if constexpr (REF)
+    return TileStores<IT, ROWS>(it, active, tile);
+  else
+    return LaneStores<IT>(it, active);
+}
+
+/* Generic path: warp tasks are 32 consecutive items of the flattened (column, lambda) index (lanes
+ * past the last item repeat it and store nothing). */
+template <int FORM, bool GREY, bool REF>
 __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
+  __shared__ double s_tile[WARPS_PER_BLOCK][REF ? TILE_DOUBLES : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nitems = a.ncol * a.nw;
@@ -244,54 +260,73 @@ __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
   const int64_t wbase = slot * 32 * (int64_t)a.nz + lane; /* each warp's scratch [z][lane], contiguous */
   double *gam = a.gam + wbase;
   double *uu = a.uu + wbase;
-  double *o1 = a.o1 + wbase;
+  double *kap = a.kap + wbase;
   double *qs = a.q + wbase;
   for (;;) {
     unsigned long long task = 0;
     if (lane == 0) task = atomicAdd(a.work, 1ull);
     task = __shfl_sync(0xffffffffu, task, 0);
     if (task >= ntasks) break;
-    const int64_t item = (int64_t)task * 32 + lane;
-    if (item < nitems) {
-      const int64_t cl = item / a.nw;
-      const int iw = (int)(item - cl * a.nw);
-      DirectPillars pa{a.pil + cl * (int64_t)a.nz * NF};
-      solve_item<FORM, GREY, BlockItem, DirectPillars, LamR>(BlockItem{a, cl, iw}, true, pa, gam, uu, o1, qs, nullptr,
-                                                             TCacheR{});
-    }
+    const bool active = (int64_t)task * 32 + lane < nitems;
+    const int64_t item = active ? (int64_t)task * 32 + lane : nitems - 1;
+    const int64_t cl = item / a.nw;
+    const int iw = (int)(item - cl * a.nw);
+    DirectPillars pa{a.pil + cl * (int64_t)a.nz * NF};
+    const BlockItem it{a, cl, iw};
+    solve_item<FORM, GREY, BlockItem, DirectPillars, LamR>(it, active, pa, gam, uu, kap, qs, nullptr, TCacheR{},
+                                                           make_stores<REF, false>(it, active, s_tile[threadIdx.x >> 5]));
   }
 }
 
+/* A staged warp's shared memory.  The reverse sweep needs none of it: its output tile takes the
+ * record buffers and the constants over (both are rewritten by the next task, the buffers by bulk
+ * copies ordered after the tile's last use by the fence in StagedPillars::begin). */
+struct StagedSmem {
+  double pil[2 * ZC * NF];
+  double lam[NLF * 32];        /* the task's 32 wavelengths' constants */
+  double2 tc[NTC / 2 * 32];    /* the lanes' temperature factors */
+  unsigned long long bar[2];
+  __device__ __forceinline__ double *tile() { return pil; }
+};
+static_assert(sizeof(StagedSmem::pil) + sizeof(StagedSmem::lam) >= TILE_DOUBLES * sizeof(double), "output tile");
+static_assert(sizeof(StagedSmem) % 16 == 0 && sizeof(StagedSmem::pil) % 16 == 0, "bulk copies and 16-byte pairs");
+
+__device__ __forceinline__ void init_staged(StagedPillars &pa, StagedSmem &sm) {
+  pa.buf = sm.pil;
+  pa.bar0 = smem_addr(&sm.bar[0]);
+  pa.waits = 0;
+  pa.inflight = 0;
+  pa.failed = false;
+  if ((threadIdx.x & 31) == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0 + 8u) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+}
+
 /* Staged path: warp tasks are (column, tile of 32 wavelengths); the column's pillar records
- * are streamed into shared memory by bulk copies (see StagedPillars). */
-template <int FORM, bool GREY>
+ * are streamed into shared memory by bulk copies (see StagedPillars).  REF: outputs with z fastest
+ * through the tile (a warm disk of 1800 columns x 500 x 250, plain: 13.6 ms with lambda-fastest
+ * temporaries and three transposes, 12.7 ms so; ragged batch of 400 columns with each lane storing
+ * its own rows 3.55 ms, 2.57 ms so).  With lambda fastest the same disk takes 11.4 ms: the tile's
+ * 45 instructions per level and the larger code (instruction-cache misses) are the rest. */
+template <int FORM, bool REF>
 __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
-  __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
-  __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
-  __shared__ double2 s_tc[WARPS_PER_BLOCK][NTC / 2 * 32]; /* the lanes' temperature factors */
-  __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  __shared__ __align__(128) StagedSmem s_warp[WARPS_PER_BLOCK];
+  StagedSmem &sm = s_warp[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int ntiles = (a.nw + 31) / 32;
   const unsigned long long ntasks = (unsigned long long)a.ncol * ntiles;
   const int64_t wbase = slot * 32 * (int64_t)a.nz + lane; /* each warp's scratch [z][lane], contiguous */
   double *gam = a.gam + wbase;
   double *uu = a.uu + wbase;
-  double *o1 = a.o1 + wbase;
+  double *kap = a.kap + wbase;
   double *qs = a.q + wbase;
   StagedPillars pa;
-  pa.buf = s_pil[wib];
-  pa.bar0 = smem_addr(&s_bar[wib][0]);
   pa.nz = a.nz;
-  pa.waits = 0;
-  pa.inflight = 0;
-  pa.failed = false;
-  if (lane == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0 + 8u) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
+  init_staged(pa, sm);
   for (;;) {
     unsigned long long task = 0;
     if (lane == 0) task = atomicAdd(a.work, 1ull);
@@ -303,10 +338,12 @@ __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
     const bool active = iw_raw < a.nw;
     const int iw = active ? iw_raw : a.nw - 1;
     pa.begin(a.pil + cl * (int64_t)a.nz * NF, lane);
-    if (!GREY) store_lam_shared(s_lam[wib], lane, a.lam, iw, a.nw);
+    store_lam_shared(sm.lam, lane, a.lam, iw, a.nw);
     __syncwarp();
-    solve_item<FORM, GREY, BlockItem, StagedPillars, LamS>(BlockItem{a, cl, iw}, active, pa, gam, uu, o1, qs,
-                                                          s_lam[wib], TCacheS{s_tc[wib] + lane});
+    const BlockItem it{a, cl, iw};
+    solve_item<FORM, false, BlockItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
+                                                          TCacheS{sm.tc + lane},
+                                                          make_stores<REF, true>(it, active, sm.tile()));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
       /* let copies still in flight land (bounded) before the block's shared memory is released */
@@ -343,6 +380,8 @@ struct BatchItem {
   __device__ __forceinline__ int64_t vz() const { return uz(); }
   __device__ __forceinline__ double *vtop() const { return b.Vtop ? b.Vtop + __ldg(&c->flux_off) + w : nullptr; }
   __device__ __forceinline__ double *vbot() const { return b.Vbot ? b.Vbot + __ldg(&c->flux_off) + w : nullptr; }
+  __device__ __forceinline__ int64_t urow() const { return nz() + 6; }
+  __device__ __forceinline__ int64_t krow() const { return nz(); }
   __device__ __forceinline__ int64_t ss() const { return 32; }
   __device__ __forceinline__ unsigned long long *status() const { return b.status; }
   __device__ __forceinline__ unsigned long long id() const { return ((unsigned long long)col << 32) | (unsigned)w; }
@@ -351,31 +390,19 @@ struct BatchItem {
 /* Warp-column tiling: tasks (column, 32-wavelength tile) from the device queue, longest
  * columns first; the column's records stream through the warp's shared-memory buffers and
  * the tile's wavelength constants sit in the warp's shared-memory table (as k_solve_staged). */
-template <int FORM>
+template <int FORM, bool REF>
 __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArgs b) {
-  __shared__ __align__(128) double s_pil[WARPS_PER_BLOCK][2 * ZC * NF];
-  __shared__ __align__(16) double s_lam[WARPS_PER_BLOCK][NLF * 32]; /* the task's 32 wavelengths' constants */
-  __shared__ double2 s_tc[WARPS_PER_BLOCK][NTC / 2 * 32]; /* the lanes' temperature factors */
-  __shared__ __align__(8) unsigned long long s_bar[WARPS_PER_BLOCK][2];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  __shared__ __align__(128) StagedSmem s_warp[WARPS_PER_BLOCK];
+  StagedSmem &sm = s_warp[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t wbase = slot * 32 * (int64_t)b.max_nz + lane; /* each warp's scratch [z][lane], contiguous */
   double *gam = b.gam + wbase;
   double *uu = b.uu + wbase;
-  double *o1 = b.o1 + wbase;
+  double *kap = b.kap + wbase;
   double *qs = b.q + wbase;
   StagedPillars pa;
-  pa.buf = s_pil[wib];
-  pa.bar0 = smem_addr(&s_bar[wib][0]);
-  pa.waits = 0;
-  pa.inflight = 0;
-  pa.failed = false;
-  if (lane == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0 + 8u) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
+  init_staged(pa, sm);
   for (;;) {
     unsigned long long task = 0;
     if (lane == 0) task = atomicAdd(b.work, 1ull);
@@ -389,10 +416,12 @@ __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArg
     const int iw = active ? iw_raw : nw - 1;
     pa.nz = __ldg(&c->nz);
     pa.begin(b.pil + __ldg(&c->rec_off) * NF, lane);
-    store_lam_shared(s_lam[wib], lane, b.lam + __ldg(&c->lam_off), iw, nw);
+    store_lam_shared(sm.lam, lane, b.lam + __ldg(&c->lam_off), iw, nw);
     __syncwarp();
-    solve_item<FORM, false, BatchItem, StagedPillars, LamS>(BatchItem{b, c, (int64_t)t.x, iw}, active, pa, gam, uu, o1,
-                                                           qs, s_lam[wib], TCacheS{s_tc[wib] + lane});
+    const BatchItem it{b, c, (int64_t)t.x, iw};
+    solve_item<FORM, false, BatchItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
+                                                           TCacheS{sm.tc + lane},
+                                                           make_stores<REF, true>(it, active, sm.tile()));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
       pa.wait(0);
@@ -410,18 +439,19 @@ cudaError_t launch_pillars_batch(const double *rho, const double *T, const MBatc
   return cudaGetLastError();
 }
 
+static const void *batch_fn(int form, bool ref) {
+  if (form == 0) return ref ? (const void *)k_batch_fp64_staged<0, true> : (const void *)k_batch_fp64_staged<0, false>;
+  return ref ? (const void *)k_batch_fp64_staged<1, true> : (const void *)k_batch_fp64_staged<1, false>;
+}
+
 cudaError_t launch_batch_fp64(const FP64BatchArgs &a, int form, int blocks, int threads, cudaStream_t s) {
-  if (form == 0)
-    k_batch_fp64_staged<0><<<blocks, threads, 0, s>>>(a);
-  else
-    k_batch_fp64_staged<1><<<blocks, threads, 0, s>>>(a);
-  return cudaGetLastError();
+  void *args[] = {(void *)&a};
+  return cudaLaunchKernel(batch_fn(form, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 int batch_fp64_max_blocks_per_sm(int form, int threads) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &n, form == 0 ? (const void *)k_batch_fp64_staged<0> : (const void *)k_batch_fp64_staged<1>, threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_fn(form, false), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
@@ -436,20 +466,22 @@ cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int
 
 bool solve_uses_staging(int nw) { return nw >= 64 || (nw % 32) == 0; }
 
-static const void *solve_fn(int form, int grey, bool staged) {
-  if (staged) {
-    if (form == 0) return grey ? (const void *)k_solve_staged<0, true> : (const void *)k_solve_staged<0, false>;
-    return grey ? (const void *)k_solve_staged<1, true> : (const void *)k_solve_staged<1, false>;
-  }
-  if (form == 0) return grey ? (const void *)k_solve<0, true> : (const void *)k_solve<0, false>;
-  return grey ? (const void *)k_solve<1, true> : (const void *)k_solve<1, false>;
+template <bool REF>
+static const void *solve_fn_of(int form, int grey, bool staged) {
+  if (staged)
+    return form == 0 ? (const void *)k_solve_staged<0, REF> : (const void *)k_solve_staged<1, REF>;
+  if (form == 0) return grey ? (const void *)k_solve<0, true, REF> : (const void *)k_solve<0, false, REF>;
+  return grey ? (const void *)k_solve<1, true, REF> : (const void *)k_solve<1, false, REF>;
+}
+static const void *solve_fn(int form, int grey, bool staged, bool ref) {
+  return ref ? solve_fn_of<true>(form, grey, staged) : solve_fn_of<false>(form, grey, staged);
 }
 
 int solve_fp64_max_blocks_per_sm(int form, int grey, int threads) {
   int nb = 0, nb2 = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, solve_fn(form, grey, false), threads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, solve_fn(form, grey, false, false), threads, 0) != cudaSuccess)
     nb = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, solve_fn(form, grey, true), threads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, solve_fn(form, grey, true, false), threads, 0) != cudaSuccess)
     nb2 = 1;
   nb = nb > nb2 ? nb : nb2;
   return nb > 0 ? nb : 1;
@@ -484,7 +516,7 @@ cudaError_t launch_bounded_wait_check(long long limit, unsigned long long *statu
 cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int blocks, int threads, cudaStream_t s) {
   const bool staged = !grey && solve_uses_staging(a.nw);
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_fn(form, grey, staged), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(solve_fn(form, grey, staged, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

@@ -143,9 +143,9 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
       Opac o = opacity_at<true>(SharedRec{rec}, L, tc);
       settle_opac<true>(o);
       g.op[k] = o.op;
+      if (Kb && k >= 1 && k <= n) Kb[z * kz] = o.op;
       g.oma[k] = o.w;
       g.S[k] = o.S;
-      if (Kb && k >= 1 && k <= n) Kb[z * kz] = o.op;
     }
     __syncwarp();
     /* 2. the rows' coefficients (solve_item's forward sweep, stable form, without the
@@ -212,7 +212,8 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
     atomicMin(&it.status()[1], it.id());
   }
   /* 4. the reverse sweep: back-substitution, ghosts, flux (scratch at stride 1) */
-  solve_reverse<1>(UnitStride<IT>{it}, u, gam, uu, o1, qs);
+  const UnitStride<IT> iu{it};
+  solve_reverse<1>(iu, true, u, gam, uu, o1, qs, LaneStores<UnitStride<IT>>(iu, true));
 }
 
 /* ---- coefficient slots ------------------------------------------------------------------ */
@@ -374,7 +375,7 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
     atomicAdd(&it.status()[0], 1ull);
     atomicMin(&it.status()[1], it.id());
   }
-  solve_reverse<1, IT, true>(it, u, aa, dd, S.o1 + q0, ee);
+  solve_reverse<1, true>(it, true, u, aa, dd, S.o1 + q0, ee, LaneStores<IT>(it, true));
 }
 
 __global__ void __launch_bounds__(REPAIR_THREADS, 6) k_repair_solve(const RepairArgs a) {

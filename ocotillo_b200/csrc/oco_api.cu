@@ -318,7 +318,7 @@ static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz,
 /* Reference-layout outputs of a device solve go through lambda-fastest temporaries and a
  * tiled transpose (coalesced stores) unless disabled or pointless (grey / few wavelengths). */
 static bool uses_transpose(const oco_ctx *c, const oco_params *p, bool u, bool k, bool v) {
-  return c->ref_transpose && p->layout == OCO_LAYOUT_REFERENCE && !p->lgrey && p->nw >= 8 && (u || k || v);
+  return p->form == OCO_FORM_MIXED && c->ref_transpose && p->layout == OCO_LAYOUT_REFERENCE && !p->lgrey && p->nw >= 8 && (u || k || v);
 }
 
 /* Bytes of the per-(column, z) record of a form: the FP64 pillar or the mixed record. */
@@ -476,8 +476,8 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
   a.ncol = nb;
   a.gam = c->scratch.as<double>();
   a.uu = a.gam + slots * p->nz;
-  a.o1 = a.uu + slots * p->nz;
-  a.q = a.o1 + slots * p->nz;
+  a.kap = a.uu + slots * p->nz;
+  a.q = a.kap + slots * p->nz;
   a.slot_stride = (int64_t)slots;
   a.work = c->work.as<unsigned long long>();
   a.status = c->status.as<unsigned long long>();

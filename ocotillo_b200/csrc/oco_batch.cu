@@ -146,7 +146,7 @@ static FP64BatchArgs fp64_args(const oco_batch *b) {
   double *sc = b->scratch.as<double>();
   a.gam = sc;
   a.uu = sc + plane;
-  a.o1 = sc + 2 * plane;
+  a.kap = sc + 2 * plane;
   a.q = sc + 3 * plane;
   a.slot_stride = b->slots;
   a.max_nz = b->max_nz;

@@ -102,8 +102,8 @@ struct SolveArgs {
   int64_t ld_col, c_off;
   int layout;
   /* Scratch [warp slot][nz][32] each (slot_stride*nz values): forward-sweep gamma, u,
-   * 1/kappa and (stable form) q, one contiguous block per warp. */
-  double *gam, *uu, *o1, *q;
+   * kappa and (stable form) q, one contiguous block per warp. */
+  double *gam, *uu, *kap, *q;
   int64_t slot_stride; /* resident threads the scratch is sized for (each warp's block is 32*nz) */
   unsigned long long *work;   /* persistent-kernel work counter (warp tasks) */
   unsigned long long *status; /* [0] zero-pivot count, [1] first bad item (min), [2] timeout flag */
@@ -232,7 +232,7 @@ struct FP64BatchArgs {
   int64_t ntasks;
   double *U, *K, *V, *Vtop, *Vbot;
   int layout;
-  double *gam, *uu, *o1, *q; /* scratch [warp slot][max_nz][32] each */
+  double *gam, *uu, *kap, *q; /* scratch [warp slot][max_nz][32] each */
   int64_t slot_stride; /* resident threads the scratch is sized for */
   int max_nz;
   unsigned long long *work;

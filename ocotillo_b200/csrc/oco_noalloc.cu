@@ -75,7 +75,7 @@ int fail(int code, const char *fmt, ...) {
 
 constexpr size_t round256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-/* Bytes of one 128-thread block of Thomas scratch (gamma, u, 1/kappa, q: 4 doubles per z per
+/* Bytes of one 128-thread block of Thomas scratch (gamma, u, kappa, q: 4 doubles per z per
  * thread) and of one column of pillar records. */
 constexpr size_t scratch_block_bytes(size_t nz) { return nz * 4 * sizeof(double) * kThreads; }
 constexpr size_t pillar_column_bytes(size_t nz) { return nz * NF * sizeof(double); }
@@ -191,7 +191,7 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
     const size_t slots = (size_t)blocks * kThreads;
     a.gam = scr;
     a.uu = scr + slots * nz;
-    a.o1 = scr + 2 * slots * nz;
+    a.kap = scr + 2 * slots * nz;
     a.q = scr + 3 * slots * nz;
     a.slot_stride = (int64_t)slots;
     a.work = ctr;
