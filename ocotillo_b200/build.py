@@ -38,7 +38,7 @@ UNITS = [
 ]
 HOST_UNITS = [("oco_deck.cpp", [])]
 
-HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "fp64_core.h", "recip_div.h", "disk_core.h",
+HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "fp64_core.h", "recip_div.h", "stores.h", "disk_core.h",
            "batch_layout.h", "fortran_records.h"]
 
 

@@ -24,6 +24,7 @@
 #include "oco_consts.h"
 #include "oco_internal.h"
 #include "recip_div.h"
+#include "stores.h"
 
 namespace oco {
 using namespace k;
@@ -345,97 +346,6 @@ __device__ __forceinline__ void prefetch_l2(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }
 
-/* Where the reverse sweep's outputs go.  LaneStores: each lane writes its item's levels itself
- * (coalesced where lambda is the fastest index).  active false: nothing is written. */
-template <class IT>
-struct LaneStores {
-  /* kappa leaves in the forward sweep and the scratch holds 1/kappa (false), or the scratch holds
-   * kappa, which leaves with U and V, and the reverse sweep takes 1/kappa */
-  static constexpr bool KAPPA_REVERSE = false;
-  double *Ub, *Kb, *Vb;
-  int64_t uz, kz, vz;
-  __device__ __forceinline__ LaneStores(const IT &it, bool active)
-      : Ub(active ? it.U() : nullptr), Kb(active ? it.K() : nullptr), Vb(active ? it.V() : nullptr), uz(it.uz()),
-        kz(it.kz()), vz(it.vz()) {}
-  __device__ __forceinline__ void u(int m, double x) const {
-    if (Ub) __stcs(&Ub[m * uz], x);
-  }
-  __device__ __forceinline__ void k(int j, double op) const {
-    if (Kb) __stcs(&Kb[j * kz], op);
-  }
-  __device__ __forceinline__ void v(int j, double x, double) const {
-    if (Vb) __stcs(&Vb[j * vz], x);
-  }
-  /* U_k and V of level k + 3, slot q of a group of 8 levels in decreasing order; a: that level's
-   * scratch value */
-  __device__ __forceinline__ void put(int, int k, double U, double x, double a) const {
-    u(3 + k, U);
-    v(k + 3, x, a);
-  }
-  __device__ __forceinline__ void flush(int, int) const {}
-};
-
-/* Layouts with z fastest (the reference's): neighbouring lanes' levels lie a row apart, so a
- * group of 8 levels of the warp's 32 items is gathered in shared memory (tile [3][8][TILE_ROW])
- * and written as 64-byte runs, four rows per store instruction; the few edge levels are stored
- * lane by lane.  ROWS: the warp's rows are equally spaced (one column's wavelengths), otherwise
- * each row's address comes from its lane.  The stores are plain ones: a run's first and last
- * sectors are completed by the neighbouring groups in L2.  Measured: see k_solve_staged. */
-constexpr int TILE_Z = 8, TILE_ROW = 36; /* 36: conflict-free both ways */
-constexpr int TILE_DOUBLES = 3 * TILE_Z * TILE_ROW;
-template <class IT, bool ROWS>
-struct TileStores : LaneStores<IT> {
-  static constexpr bool KAPPA_REVERSE = true;
-  double *tile;
-  double *U0, *K0, *V0; /* row of lane 0 (ROWS) or of the lane */
-  int64_t us, ks;       /* elements between rows */
-  int nrows;
-  __device__ __forceinline__ TileStores(const IT &it, bool active, double *t)
-      : LaneStores<IT>(it, active), tile(t), U0(it.U()), K0(it.K()), V0(it.V()), us(it.urow()), ks(it.krow()) {
-    nrows = __popc(__ballot_sync(0xffffffffu, active)); /* active lanes come first */
-    if (ROWS) {
-      U0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)U0, 0);
-      K0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)K0, 0);
-      V0 = (double *)__shfl_sync(0xffffffffu, (unsigned long long)V0, 0);
-    }
-  }
-  __device__ __forceinline__ void v(int j, double x, double op) const {
-    LaneStores<IT>::v(j, x, op);
-    LaneStores<IT>::k(j, op);
-  }
-  __device__ __forceinline__ void put(int q, int, double U, double v, double op) const {
-    double *t = tile + q * TILE_ROW + (threadIdx.x & 31);
-    t[0] = U;
-    t[TILE_Z * TILE_ROW] = v;
-    t[2 * TILE_Z * TILE_ROW] = op;
-  }
-  __device__ __forceinline__ void rows(double *base, int64_t stride, const double *t, int z, int n) const {
-    if (!base) return;
-    const int lane = threadIdx.x & 31, s = lane & (TILE_Z - 1), r = lane / TILE_Z;
-    const double *p = t + (n - 1 - s) * TILE_ROW + r;
-    double *g = base + r * stride + z + s;
-    if (ROWS && n == TILE_Z && nrows == 32) { /* nearly always */
-#pragma unroll
-      for (int i = 0; i < 32 / 4; i++) g[(int64_t)(4 * i) * stride] = p[4 * i];
-      return;
-    }
-#pragma unroll
-    for (int i = 0; i < 32 / 4; i++) {
-      double *d = ROWS ? g + (int64_t)(4 * i) * stride
-                       : (double *)__shfl_sync(0xffffffffu, (unsigned long long)base, 4 * i + r) + z + s;
-      if (s < n && 4 * i + r < nrows) *d = p[4 * i];
-    }
-  }
-  /* writes the n levels put last, k the lowest */
-  __device__ __forceinline__ void flush(int k, int n) const {
-    __syncwarp();
-    rows(U0, us, tile, 3 + k, n);
-    rows(V0, ks, tile + TILE_Z * TILE_ROW, 3 + k, n);
-    rows(K0, ks, tile + 2 * TILE_Z * TILE_ROW, 3 + k, n);
-    __syncwarp();
-  }
-};
-
 /* 1/kappa of a scratch value (see KAPPA_REVERSE), rounded as the division. */
 template <class ST>
 __device__ __forceinline__ double scratch_o1(double a) {
@@ -457,7 +367,7 @@ constexpr int RING = 4; /* levels of scratch that the stable form's reverse swee
 template <int FORM, bool PF = false, class IT, class ST>
 __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double u, const double *__restrict__ gam,
                                               const double *__restrict__ uu, const double *__restrict__ kap,
-                                              const double *__restrict__ qs, const ST &st) {
+                                              const double *__restrict__ qs, ST &st) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
   const double dz1 = it.dz1();
@@ -468,21 +378,23 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
      * (ghost differences mirror the interior ones); exact in the same arithmetic as the
      * stencil on U, accurate where U's differences are below its resolution. */
     const int n = nz;
+    st.open(n);
     double Un = u; /* U_{n-1} */
-    st.u(3 + n - 1, Un);
+    st.push_u(3, n + 2, Un);
     double Uk[3], Dt[3];
+#pragma unroll
     for (int t = 0; t < 3; t++) {
       const int k = n - 2 - t;
       const double uf = uu[k * ss];
       Dt[t] = uf - qs[k * ss] * Un;
       Un = uf - gam[(k + 1) * ss] * Un;
       Uk[t] = Un;
-      st.u(3 + k, Un);
+      if (t < 2) st.push_u(4 + t, 3 + k, Un);
     }
     const double fn = u;
-    st.u(n + 3, 2.0 * fn - Uk[0]);
-    st.u(n + 4, 2.0 * fn - Uk[1]);
-    st.u(n + 5, 2.0 * fn - Uk[2]);
+    st.push_u(2, n + 3, 2.0 * fn - Uk[0]);
+    st.push_u(1, n + 4, 2.0 * fn - Uk[1]);
+    st.push_u(0, n + 5, 2.0 * fn - Uk[2]);
     double d0 = Dt[2], d1 = Dt[1], d2 = Dt[0], d3 = Dt[0], d4 = Dt[1], d5 = Dt[2];
     auto flux = [&](double op) -> double {
       const double s1 = d2 + d3;
@@ -491,19 +403,19 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       const double df = -((1.0 / 60.0) * (((45.0 * s1) - 9.0 * s2) + s3));
       return ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
     };
-    auto edge = [&](int j) -> double {
-      const double op = kap[j * ss], v = flux(op);
-      st.v(j, v, op);
-      return v;
-    };
-    vtop = edge(n - 1);
+    {
+      const double op = kap[(n - 1) * ss];
+      vtop = flux(op);
+      st.push(6, n - 1, Un, vtop, op); /* U_{n-4}, V_{n-1} */
+      st.group(n - 1, 7);
+    }
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = u; /* the four lowest U seen so far */
     auto step = [&](int slot, int k, double uf, double qk, double gk1, double op) {
       const double Dk = uf - qk * Un;
       Un = uf - gk1 * Un;
       U3 = U2; U2 = U1; U1 = U0; U0 = Un;
       d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = Dk;
-      st.put(slot, k, Un, flux(op), op);
+      st.push(slot, 3 + k, Un, flux(op), op);
     };
     int k = n - 5;
     if (PF) {
@@ -524,7 +436,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
         }
 #pragma unroll
         for (int q = 0; q < 8; q++) step(q, k - q, ub[q], qb[q], gb[q], ob[q]);
-        st.flush(k - 7, 8);
+        st.group(3 + k - 7, 8);
       }
     } else if (k >= 7) {
       /* the scratch of RING levels in registers: a level's slot is reloaded for RING levels
@@ -547,53 +459,60 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
           gb[r] = gam[(kn + 1) * ss];
           ob[r] = kap[(kn + 3) * ss];
         }
-        st.flush(k - 7, 8);
+        st.group(3 + k - 7, 8);
       }
     }
-    if (k >= 0) {
-      const int m = k + 1;
-      for (int q = 0; k >= 0; k--, q++) step(q, k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss], kap[(k + 3) * ss]);
-      st.flush(0, m);
+    int q = 0;
+    for (; k >= 0; k--) {
+      step(q, k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss], kap[(k + 3) * ss]);
+      if (++q == 8) {
+        st.group(3 + k, 8);
+        q = 0;
+      }
     }
-    st.u(2, 2.0 * U0 - U1);
-    st.u(1, 2.0 * U0 - U2);
-    st.u(0, 2.0 * U0 - U3);
-    const double D0 = d0, D1 = d1, D2 = d2;
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D0;
-    edge(2);
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D1;
-    edge(1);
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D2;
-    vbot = edge(0);
+    const double g[3] = {2.0 * U0 - U3, 2.0 * U0 - U2, 2.0 * U0 - U1}; /* ghosts 0, 1, 2 */
+    const double D[3] = {d2, d1, d0};
+#pragma unroll
+    for (int j = 2; j >= 0; j--) { /* ghost differences D_{-1}, D_{-2}, D_{-3} mirror D_0, D_1, D_2 */
+      d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D[j];
+      const double op = kap[j * ss];
+      vbot = flux(op);
+      st.push(q, j, g[j], vbot, op);
+      if (++q == 8) {
+        st.group(j, 8);
+        q = 0;
+      }
+    }
+    st.finish(q);
   } else if (nz >= 4) {
     const int n = nz;
     double u1 = u; /* U_{n-1} */
     double u2 = uu[(n - 2) * ss] - gam[(n - 1) * ss] * u1;
     double u3 = uu[(n - 3) * ss] - gam[(n - 2) * ss] * u2;
     double u4 = uu[(n - 4) * ss] - gam[(n - 3) * ss] * u3;
-    st.u(3 + n - 1, u1);
-    st.u(3 + n - 2, u2);
-    st.u(3 + n - 3, u3);
-    st.u(3 + n - 4, u4);
     double g1 = 2.0 * u1 - u2, g2 = 2.0 * u1 - u3, g3 = 2.0 * u1 - u4;
-    st.u(n + 3, g1);
-    st.u(n + 4, g2);
-    st.u(n + 5, g3);
+    st.open(n);
+    st.push_u(0, n + 5, g3);
+    st.push_u(1, n + 4, g2);
+    st.push_u(2, n + 3, g1);
+    st.push_u(3, n + 2, u1);
+    st.push_u(4, n + 1, u2);
+    st.push_u(5, n, u3);
     double w0 = u4, w1 = u3, w2 = u2, w3 = u1, w4 = g1, w5 = g2, w6 = g3;
     auto flux = [&](double op) -> double {
       double df = (1.0 / 60.0) * (((45.0 * (w4 - w2)) - 9.0 * (w5 - w1)) + (w6 - w0));
       return ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
     };
-    auto edge = [&](int j) -> double {
-      const double op = kap[j * ss], v = flux(op);
-      st.v(j, v, op);
-      return v;
-    };
-    vtop = edge(n - 1);
+    {
+      const double op = kap[(n - 1) * ss];
+      vtop = flux(op);
+      st.push(6, n - 1, u4, vtop, op);
+      st.group(n - 1, 7);
+    }
     auto step = [&](int slot, int k, double uk, double gk1, double op) {
       double Uk = uk - gk1 * w0;
       w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = Uk;
-      st.put(slot, k, Uk, flux(op), op);
+      st.push(slot, 3 + k, Uk, flux(op), op);
     };
     int kk = n - 5;
     if (kk >= 7) { /* the scratch of 8 levels in registers, as above */
@@ -613,24 +532,30 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
           gb[q] = gam[(kn + 1) * ss];
           ob[q] = kap[(kn + 3) * ss];
         }
-        st.flush(kk - 7, 8);
+        st.group(3 + kk - 7, 8);
       }
     }
-    if (kk >= 0) {
-      const int m = kk + 1;
-      for (int q = 0; kk >= 0; kk--, q++) step(q, kk, uu[kk * ss], gam[(kk + 1) * ss], kap[(kk + 3) * ss]);
-      st.flush(0, m);
+    int q = 0;
+    for (; kk >= 0; kk--) {
+      step(q, kk, uu[kk * ss], gam[(kk + 1) * ss], kap[(kk + 3) * ss]);
+      if (++q == 8) {
+        st.group(3 + kk, 8);
+        q = 0;
+      }
     }
-    double b1 = 2.0 * w0 - w1, b2 = 2.0 * w0 - w2, b3 = 2.0 * w0 - w3;
-    st.u(2, b1);
-    st.u(1, b2);
-    st.u(0, b3);
-    w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b1;
-    edge(2);
-    w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b2;
-    edge(1);
-    w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b3;
-    vbot = edge(0);
+    const double b[3] = {2.0 * w0 - w3, 2.0 * w0 - w2, 2.0 * w0 - w1}; /* ghosts 0, 1, 2 */
+#pragma unroll
+    for (int j = 2; j >= 0; j--) {
+      w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b[j];
+      const double op = kap[j * ss];
+      vbot = flux(op);
+      st.push(q, j, b[j], vbot, op);
+      if (++q == 8) {
+        st.group(j, 8);
+        q = 0;
+      }
+    }
+    st.finish(q);
   } else { /* nz = 2 or 3: the reference's ghost update order matters (ghosts feed ghosts) */
     double f[9];
     const int n1 = 3, n2 = nz + 2;
@@ -647,7 +572,8 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
                                   (f[c + 3] - f[c - 3]));
       const double op = kap[j * ss];
       double v = ((-1.0 * scratch_o1<ST>(op)) * df) * dz1;
-      st.v(j, v, op);
+      st.v(j, v);
+      if (ST::KAPPA_REVERSE) st.k(j, op);
       if (j == 0) vbot = v;
       if (j == nz - 1) vtop = v;
     }
@@ -771,7 +697,7 @@ __device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, cons
 template <int FORM, bool GREY, class IT, class PA, class LMT, class TC, class ST>
 __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, double *__restrict__ gam,
                                            double *__restrict__ uu, double *__restrict__ kap,
-                                           double *__restrict__ qs, const double *lam_table, TC tc, const ST &st) {
+                                           double *__restrict__ qs, const double *lam_table, TC tc, ST st) {
   const int nz = it.nz();
   const int64_t ss = it.ss();
   const LMT L(it, lam_table, !GREY);

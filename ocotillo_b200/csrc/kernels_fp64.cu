@@ -13,8 +13,7 @@
  *               forward sweep (auxiliary.f90:14-41) streaming gamma, u and kappa to a
  *               per-warp-slot scratch, then the back-substitution (:43-45), ghost zones
  *               (:49-62) and 6th-order flux (:64-109) in one reverse sweep with a 7-point
- *               register window.  All outputs leave in the reverse sweep (fp64_core.h: LaneStores,
- *               TileStores).
+ *               register window.  All outputs leave in the reverse sweep (stores.h).
  *
  * Output stores (U, kappa, V and the emergent flux) use the streaming cache hint (st.global.cs,
  * evict first): they are never read back, and L2 then keeps more of the forward sweep's scratch
@@ -114,7 +113,7 @@ struct DirectPillars {
   __device__ __forceinline__ GlobalRec at(int z) { return GlobalRec{base + (int64_t)z * NF}; }
 };
 
-constexpr int ZC = 11;            /* z records per staged chunk (static shared memory up to 48 KB) */
+constexpr int ZC = 12;            /* z records per staged chunk (static shared memory up to 48 KB) */
 constexpr int WARPS_PER_BLOCK = 4; /* k_solve runs 128-thread blocks */
 constexpr long long kSpinLimit = 1ll << 26;
 
@@ -239,20 +238,16 @@ struct BlockItem {
   }
 };
 
-/* The stores of a warp's outputs: lane by lane, or (REF, z fastest) through the tile. */
-template <bool REF, bool ROWS, class IT>
-__device__ __forceinline__ auto make_stores(const IT &it, bool active, double *tile) {
-  if constexpr (REF)
-    return TileStores<IT, ROWS>(it, active, tile);
-  else
-    return LaneStores<IT>(it, active);
+template <class IT>
+__device__ __forceinline__ OutPtrs out_ptrs(const IT &it) {
+  return OutPtrs{it.U(), it.K(), it.V(), it.uz(), it.kz(), it.vz(), it.urow(), it.krow()};
 }
 
 /* Generic path: warp tasks are 32 consecutive items of the flattened (column, lambda) index (lanes
  * past the last item repeat it and store nothing). */
 template <int FORM, bool GREY, bool REF>
 __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
-  __shared__ double s_tile[WARPS_PER_BLOCK][REF ? TILE_DOUBLES : 1];
+  __shared__ RingSmem<double> s_ring[REF ? WARPS_PER_BLOCK : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nitems = a.ncol * a.nw;
@@ -274,22 +269,26 @@ __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
     DirectPillars pa{a.pil + cl * (int64_t)a.nz * NF};
     const BlockItem it{a, cl, iw};
     solve_item<FORM, GREY, BlockItem, DirectPillars, LamR>(it, active, pa, gam, uu, kap, qs, nullptr, TCacheR{},
-                                                           make_stores<REF, false>(it, active, s_tile[threadIdx.x >> 5]));
+                                                           make_stores<REF, false, false>(out_ptrs(it), active, &s_ring[REF ? threadIdx.x >> 5 : 0]));
   }
 }
 
-/* A staged warp's shared memory.  The reverse sweep needs none of it: its output tile takes the
- * record buffers and the constants over (both are rewritten by the next task, the buffers by bulk
- * copies ordered after the tile's last use by the fence in StagedPillars::begin). */
+/* A staged warp's shared memory.  The reverse sweep needs none of the forward sweep's: its output
+ * ring takes it over (the next task rewrites it, the buffers by bulk copies ordered after the
+ * ring's last use by the fence in StagedPillars::begin). */
 struct StagedSmem {
-  double pil[2 * ZC * NF];
-  double lam[NLF * 32];        /* the task's 32 wavelengths' constants */
-  double2 tc[NTC / 2 * 32];    /* the lanes' temperature factors */
+  union {
+    struct {
+      double pil[2 * ZC * NF];
+      double lam[NLF * 32];     /* the task's 32 wavelengths' constants */
+      double2 tc[NTC / 2 * 32]; /* the lanes' temperature factors */
+    };
+    RingSmem<double> ring;
+  };
   unsigned long long bar[2];
-  __device__ __forceinline__ double *tile() { return pil; }
+  __device__ StagedSmem() = delete;
 };
-static_assert(sizeof(StagedSmem::pil) + sizeof(StagedSmem::lam) >= TILE_DOUBLES * sizeof(double), "output tile");
-static_assert(sizeof(StagedSmem) % 16 == 0 && sizeof(StagedSmem::pil) % 16 == 0, "bulk copies and 16-byte pairs");
+static_assert(sizeof(StagedSmem) % 16 == 0 && (2 * ZC * NF * sizeof(double)) % 16 == 0, "bulk copies and 16-byte pairs");
 
 __device__ __forceinline__ void init_staged(StagedPillars &pa, StagedSmem &sm) {
   pa.buf = sm.pil;
@@ -307,14 +306,15 @@ __device__ __forceinline__ void init_staged(StagedPillars &pa, StagedSmem &sm) {
 
 /* Staged path: warp tasks are (column, tile of 32 wavelengths); the column's pillar records
  * are streamed into shared memory by bulk copies (see StagedPillars).  REF: outputs with z fastest
- * through the tile (a warm disk of 1800 columns x 500 x 250, plain: 13.6 ms with lambda-fastest
- * temporaries and three transposes, 12.7 ms so; ragged batch of 400 columns with each lane storing
- * its own rows 3.55 ms, 2.57 ms so).  With lambda fastest the same disk takes 11.4 ms: the tile's
- * 45 instructions per level and the larger code (instruction-cache misses) are the rest. */
+ * through the ring (a warm disk of 1800 columns x 500 x 250, plain: 13.65 ms with lambda-fastest
+ * temporaries and three transposes, 12.8 ms so; the AGN profile 4.8 ms, runs off the 64-byte
+ * boundaries 6.4 ms; ragged batch of 400 columns with each lane storing its own rows 3.55 ms, 2.65
+ * ms so).  With lambda fastest the warm disk takes 11.4 ms: the ring's instructions and the larger
+ * code (instruction-cache misses) are the rest. */
 template <int FORM, bool REF>
 __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
-  __shared__ __align__(128) StagedSmem s_warp[WARPS_PER_BLOCK];
-  StagedSmem &sm = s_warp[threadIdx.x >> 5];
+  __shared__ __align__(128) unsigned char s_warp[WARPS_PER_BLOCK * sizeof(StagedSmem)];
+  StagedSmem &sm = reinterpret_cast<StagedSmem *>(s_warp)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int ntiles = (a.nw + 31) / 32;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
     const BlockItem it{a, cl, iw};
     solve_item<FORM, false, BlockItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
                                                           TCacheS{sm.tc + lane},
-                                                          make_stores<REF, true>(it, active, sm.tile()));
+                                                          make_stores<REF, true, false>(out_ptrs(it), active, &sm.ring));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
       /* let copies still in flight land (bounded) before the block's shared memory is released */
@@ -392,8 +392,8 @@ struct BatchItem {
  * the tile's wavelength constants sit in the warp's shared-memory table (as k_solve_staged). */
 template <int FORM, bool REF>
 __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArgs b) {
-  __shared__ __align__(128) StagedSmem s_warp[WARPS_PER_BLOCK];
-  StagedSmem &sm = s_warp[threadIdx.x >> 5];
+  __shared__ __align__(128) unsigned char s_warp[WARPS_PER_BLOCK * sizeof(StagedSmem)];
+  StagedSmem &sm = reinterpret_cast<StagedSmem *>(s_warp)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t wbase = slot * 32 * (int64_t)b.max_nz + lane; /* each warp's scratch [z][lane], contiguous */
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArg
     const BatchItem it{b, c, (int64_t)t.x, iw};
     solve_item<FORM, false, BatchItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
                                                            TCacheS{sm.tc + lane},
-                                                           make_stores<REF, true>(it, active, sm.tile()));
+                                                           make_stores<REF, true, false>(out_ptrs(it), active, &sm.ring));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
       pa.wait(0);

@@ -7,24 +7,26 @@
  *                     items with direct loads when nw is small.  Forward sweep: log2-space
  *                     opacity, scaled rows and the difference-form Thomas elimination in FP32
  *                     (the source function's exponent as integer + FP32 fraction),
- *                     writing kappa and a scratch record per z (|gamma| or q, 1/kappa, u
- *                     mantissa and exponent); reverse sweep: extended-range FP32
- *                     back-substitution, the differences D_j, and the flux from a 6-value
- *                     window of differences, with FP64 outputs.
- * Output stores carry the streaming cache hint (st.global.cs): they are never read back here,
- * and L2 keeps more of the scratch for the reverse sweep (ragged batch -0.3%).
+ *                     writing a scratch record per z (|gamma| or q, kappa, u mantissa and
+ *                     exponent); reverse sweep: extended-range FP32 back-substitution, the
+ *                     differences D_j, and the flux from a 6-value window of differences, with
+ *                     FP64 outputs (stores.h).
  * See mixed_core.h for the arithmetic and its relation to the reference.
  */
 #include <cuda_runtime.h>
 
 #include "mixed_core.h"
 #include "oco_internal.h"
+#include "stores.h"
 
 namespace oco {
 using namespace oco::mx;
 
-constexpr int MZC = 20;            /* z records per staged chunk (20 x 256 B) */
+constexpr int MZC = 14;            /* z records per staged chunk (14 x 256 B) */
 constexpr int MWARPS = 4;          /* warps per 128-thread block */
+#ifndef MBLOCKS
+#define MBLOCKS 5 /* resident blocks per SM */
+#endif
 constexpr long long kMSpinLimit = 1ll << 26;
 #ifndef OCO_MIXED_PREFETCH
 #define OCO_MIXED_PREFETCH 4 /* reverse-sweep steps whose scratch loads are issued together */
@@ -61,8 +63,8 @@ __device__ __forceinline__ bool mtry_wait(uint32_t bar, uint32_t parity) {
 struct MStaged {
   float *buf;
   uint32_t bar0;
-  const float *src;
-  int nz, nchunks, cur;
+  const float *src, *rec; /* the column; the next record in the buffer */
+  int nz, nchunks, cur, left;
   uint32_t waits, inflight;
   bool failed;
   __device__ __forceinline__ void issue(int c) {
@@ -90,23 +92,30 @@ struct MStaged {
   __device__ __forceinline__ void begin(const float *column) {
     src = column;
     cur = -1;
+    left = 0;
     nchunks = (nz + MZC - 1) / MZC;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); /* this lane's tile accesses before the copies */
     __syncwarp();
     if ((threadIdx.x & 31) == 0) issue(0);
     inflight |= 1u;
   }
-  __device__ __forceinline__ MRec at(int z) {
-    const int c = z / MZC;
-    if (c != cur) {
+  /* The next record; z counts up from 0. */
+  __device__ __forceinline__ MRec at(int) {
+    if (left == 0) {
+      const int c = ++cur;
       __syncwarp();
       if (!failed && c + 1 < nchunks) {
         if ((threadIdx.x & 31) == 0) issue(c + 1);
         inflight |= 1u << ((c + 1) & 1);
       }
       if (!failed && !wait(c & 1)) failed = true;
-      cur = c;
+      rec = buf + (c & 1) * (MZC * MZN);
+      left = MZC;
     }
-    return MRec{buf + (c & 1) * (MZC * MZN) + (z - c * MZC) * MZN};
+    left--;
+    const MRec r{rec};
+    rec += MZN;
+    return r;
   }
 };
 
@@ -115,8 +124,21 @@ struct MDirect {
   __device__ __forceinline__ MGRec at(int z) { return MGRec{base + (int64_t)z * MZN}; }
 };
 
-__device__ __forceinline__ void load_lam32(Lam32 &L, const float *__restrict__ t, int iw, int nw) {
+/* Wavelength constants: most are read only where T changes or at ionized points, so a staged warp
+ * keeps them in its shared table [MLN][32] and leaves their registers to the sweep; the lanes of the
+ * other kernels hold theirs in registers. */
+struct MLamS {
+  const float *p; /* &table[0][lane] */
+  __device__ __forceinline__ float operator()(int k) const { return p[k * 32]; }
+};
+__device__ __forceinline__ Lam32 load_lam32(const float *__restrict__ t, int iw, int nw) {
+  Lam32 L;
   lam32_from(L, [&](int f) { return __ldg(t + (int64_t)f * nw + iw); });
+  return L;
+}
+__device__ __forceinline__ void store_lam32_shared(float *table, int lane, const float *__restrict__ t, int iw, int nw) {
+#pragma unroll
+  for (int k = 0; k < MLN; k++) table[k * 32 + lane] = __ldg(t + (int64_t)k * nw + iw);
 }
 
 /* Everything one (column, wavelength) item needs besides its records. */
@@ -127,9 +149,7 @@ struct MItem {
   float ldz2i, ldz2f; /* log2(dz^2) = integer + fraction */
   float dz2f;       /* dz^2 */
   double dz1;       /* 1/dz */
-  double *U;        /* U of z = 0 (ghost zone 0), stride uz, or NULL; written only when active */
-  double *K, *V;    /* kappa and V of z = 0 or NULL, strides kz, vz */
-  int64_t uz, kz, vz;
+  OutPtrs o;        /* U, kappa, V; written only when active */
   double *vtop, *vbot; /* emergent-flux destinations or NULL */
 };
 
@@ -146,12 +166,14 @@ __device__ __forceinline__ MItem block_item(const MixedArgs &a, int64_t cl, int 
   it.dz2f = (float)(a.dz * a.dz);
   it.dz1 = 1.0 / a.dz;
   const int64_t idx = (a.layout == 0) ? (int64_t)iw * a.ld_col + a.c_off + cl : (a.c_off + cl) * a.nw + iw;
-  it.U = a.U ? a.U + idx * a.U_is : nullptr;
-  it.K = a.K ? a.K + idx * a.K_is : nullptr;
-  it.V = a.V ? a.V + idx * a.V_is : nullptr;
-  it.uz = a.U_zs;
-  it.kz = a.K_zs;
-  it.vz = a.V_zs;
+  it.o.U = a.U ? a.U + idx * a.U_is : nullptr;
+  it.o.K = a.K ? a.K + idx * a.K_is : nullptr;
+  it.o.V = a.V ? a.V + idx * a.V_is : nullptr;
+  it.o.uz = a.U_zs;
+  it.o.kz = a.K_zs;
+  it.o.vz = a.V_zs;
+  it.o.urow = a.ld_col * a.U_is;
+  it.o.krow = a.ld_col * (int64_t)a.nz;
   const int64_t pidx = (int64_t)iw * a.ld_col + a.c_off + cl;
   it.vtop = a.Vtop ? a.Vtop + pidx : nullptr;
   it.vbot = a.Vbot ? a.Vbot + pidx : nullptr;
@@ -159,10 +181,10 @@ __device__ __forceinline__ MItem block_item(const MixedArgs &a, int64_t cl, int 
 }
 
 /* The warp's Thomas scratch, one sequential stream per warp.  A record per level is
- * {v, 1/kappa, u mantissa, u exponent} (see the forward sweep); two formats:
+ * {v, kappa, u mantissa, u exponent} (see the forward sweep); two formats:
  *   MScratch16  one float4 per lane, 512 bytes per level;
- *   MScratch12  12 bytes per lane, 384 per level: the 32 lanes' {v, 1/kappa} pairs (float2),
- *               then their u mantissas, with u's exponent packed into the spare bits of 1/kappa
+ *   MScratch12  12 bytes per lane, 384 per level: the 32 lanes' {v, kappa} pairs (float2),
+ *               then their u mantissas, with u's exponent packed into the spare bits of kappa
  *               and of the mantissa (pack_o1_u, mixed_core.h: u's mantissa lies in [1, 2)).  A
  *               record whose u does not fit (exponent outside [-512, 511], or a mantissa that
  *               is not normal) makes put() return false and the item is flagged for the FP64
@@ -183,7 +205,7 @@ struct MScratch16 {
     return true;
   }
   __device__ __forceinline__ float4 get(int j) const { return *p(j); }
-  __device__ __forceinline__ float o1(int j) const { return p(j)->y; }
+  __device__ __forceinline__ float kappa(int j) const { return p(j)->y; }
 };
 struct MScratch12 {
   static constexpr int LEVEL = 32 * 12;
@@ -201,12 +223,12 @@ struct MScratch12 {
   }
   __device__ __forceinline__ float4 get(int j) const {
     const float2 a = *p2(j);
-    float o1, m;
+    float kc, m;
     int e;
-    unpack_o1_u(__float_as_int(a.y), __float_as_int(*p1(j)), o1, m, e);
-    return make_float4(a.x, o1, m, __int_as_float(e));
+    unpack_o1_u(__float_as_int(a.y), __float_as_int(*p1(j)), kc, m, e);
+    return make_float4(a.x, kc, m, __int_as_float(e));
   }
-  __device__ __forceinline__ float o1(int j) const { return __int_as_float(__float_as_int(p2(j)->y) & 0x7fffffff); }
+  __device__ __forceinline__ float kappa(int j) const { return __int_as_float(__float_as_int(p2(j)->y) & 0x7fffffff); }
 };
 /* One (column, wavelength) item, its scratch records in sc.  An inactive lane runs the forward
  * sweep (to keep a staged warp in step) and writes nothing. */
@@ -219,36 +241,40 @@ struct MScratch12 {
  * FP32 leaves relative errors of a few 1e-6 in u, q and U, so above `cond` the item is
  * flagged for the FP64 re-solve (kernels_repair.cu).  Columns with nz < 4 are not tested (their flux is the
  * reference's stencil on U).  An item whose scratch records do not fit MScratch is flagged too. */
-template <class PA, class SC>
-__device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa, const SC &sc, float cond) {
+template <class PA, class LA, class SC, class ST>
+__device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa, const LA &L, const SC &sc,
+                                            ST st, float cond) {
   const int nz = it.nz;
-  Lam32 L;
-  load_lam32(L, it.lam, it.iw, it.nw);
-  double *Ub = active ? it.U : nullptr;
-  double *Kb = active ? it.K : nullptr;
-  double *Vb = active ? it.V : nullptr;
   const float dzf = it.dzf, dz2f = it.dz2f, ldz2i = it.ldz2i, ldz2f = it.ldz2f;
 
-  Opac32 cur = opacity(pa.at(0), L);
-  Opac32 nxt = opacity(pa.at(1), L);
+  /* The (T, lambda) part is taken again while the record says that T has not changed: most levels
+   * of a disk sit at its temperature floor.  356 -> 300 instructions per point on the AGN grid
+   * (4096 columns x 512 x 256, all of the kernel: 6.77 -> 6.1 ms). */
+  const LamPt c = lam_point(L);
+  TF32 t;
+  auto opac = [&](int z) -> Opac32 {
+    const auto Z = pa.at(z);
+    if (!(f2bits(Z[MZ_FLAGS]) & MZF_SAME_T)) t = tfac(Z, L);
+    return opacity(Z, L, c, t);
+  };
+  Opac32 cur = opac(0);
+  Opac32 nxt = opac(1);
   float kc = kappa_lin(cur), kn = kappa_lin(nxt);
   Row32 r = row_boundary(kc, cur, dzf, dz2f, ldz2i, ldz2f, false);
   float h = r.e, cprev = r.c;
   float an = 2.0f * rcp(kn + kc); /* a' of row 1; then c' of the row below */
   XF u = xexp2(r.ldi, r.ldf);
   u = xnorm(u.m * (r.w * rcp(r.c + h)), u.e);
-  float o1 = rcp(kc);
-  if (Kb) __stcs(&Kb[0], (double)kc);
-  /* scratch record of z = j: {v_j, 1/kappa_j, u_j mantissa, u_j exponent (int bits)} where v_j holds the
+  /* scratch record of z = j: {v_j, kappa_j, u_j mantissa, u_j exponent (int bits)} where v_j holds the
    * smaller of q_j = h_j/(c_j+h_j) and |gamma_{j+1}| = c_j/(c_j+h_j) (they sum to 1; a negative
    * v_j stores -|gamma_{j+1}|), written once row j+1 is known */
-  float4 pend = make_float4(0.0f, o1, u.m, __int_as_float(u.e));
+  float4 pend = make_float4(0.0f, kc, u.m, __int_as_float(u.e));
   bool fits = true;
   for (int j = 1; j < nz; j++) {
     cur = nxt;
     kc = kn;
     if (j < nz - 1) {
-      nxt = opacity(pa.at(j + 1), L);
+      nxt = opac(j + 1);
       kn = kappa_lin(nxt);
       r = row_center(an, kc, kn, cur, dz2f, ldz2i, ldz2f);
       an = r.c;
@@ -262,36 +288,32 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
     h = r.e + (r.a * rr) * h; /* a'/(c'+h) is O(1); a' h alone can overflow */
     const float rb = rcp(r.c + h);
     u = xaxpy(xexp2(r.ldi, r.ldf), r.w * rb, u, r.a * rb);
-    o1 = rcp(kc);
-    if (Kb) __stcs(&Kb[(int64_t)j * it.kz], (double)kc);
-    pend = make_float4(0.0f, o1, u.m, __int_as_float(u.e));
+    pend = make_float4(0.0f, kc, u.m, __int_as_float(u.e));
     cprev = r.c;
   }
   fits &= sc.put(nz - 1, pend);
-  if (!active) return false;
   bool flag = !fits;
 
   /* reverse sweep */
   const int n = nz;
   const double dz1 = it.dz1;
-  const int64_t uz = it.uz;
   XF Un = u; /* U_{n-1} */
-  if (Ub) __stcs(&Ub[(int64_t)(3 + n - 1) * uz], xtod(Un));
   double vtop = 0.0, vbot = 0.0;
   if (nz >= 4) {
+    st.open(n);
+    st.push_u(3, n + 2, xtod(Un));
     /* window of differences d0..d5 = D_k..D_{k+5}; V_{k+3} from it */
     double d0, d1, d2, d3, d4, d5;
     double Uk[3];
     /* D_{n-2}, D_{n-3}, D_{n-4} first (top ghosts mirror them) */
     double Dt[3];
-    const float nx4_top_o1 = sc.o1(n - 1); /* 1/kappa_{n-1} */
-    float o1t[3];
+    float kt[3];
     double Ct[3]; /* C_k = u_k + q_k U_{k+1} of the top differences */
 #pragma unroll
     for (int t = 0; t < 3; t++) {
       const int k = n - 2 - t;
       const float4 w = sc.get(k);
-      o1t[t] = w.y;
+      kt[t] = w.y;
       const float g1 = (w.x >= 0.0f) ? 1.0f - w.x : -w.x;
       const float qk = (w.x >= 0.0f) ? w.x : 1.0f + w.x;
       XF uj;
@@ -302,34 +324,34 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       XF Dj;
       xaxpy2(uj, Un, g1, -qk, Un, Dj);
       Uk[t] = xtod(Un);
-      if (Ub) __stcs(&Ub[(int64_t)(3 + k) * uz], Uk[t]);
+      if (t < 2) st.push_u(4 + t, 3 + k, Uk[t]);
       Dt[t] = xtod(Dj);
     }
-    flag = !(37.0 * Ct[0] + 8.0 * Ct[1] + Ct[2] <= (double)cond * fabs(37.0 * Dt[0] - 8.0 * Dt[1] + Dt[2]));
-    const float o1_nm2 = o1t[0], o1_nm3 = o1t[1], o1_nm4 = o1t[2];
+    flag = flag || !(37.0 * Ct[0] + 8.0 * Ct[1] + Ct[2] <= (double)cond * fabs(37.0 * Dt[0] - 8.0 * Dt[1] + Dt[2]));
     /* top ghosts f(n2+i) = 2 f(n2) - f(n2-i) */
     const double fn = xtod(u);
-    if (Ub) {
-      __stcs(&Ub[(int64_t)(n + 3) * uz], 2.0 * fn - Uk[0]);
-      __stcs(&Ub[(int64_t)(n + 4) * uz], 2.0 * fn - Uk[1]);
-      __stcs(&Ub[(int64_t)(n + 5) * uz], 2.0 * fn - Uk[2]);
-    }
+    st.push_u(2, n + 3, 2.0 * fn - Uk[0]);
+    st.push_u(1, n + 4, 2.0 * fn - Uk[1]);
+    st.push_u(0, n + 5, 2.0 * fn - Uk[2]);
     /* window for V_{n-1}: D_{n-4} .. D_{n+1} = Dt[2], Dt[1], Dt[0], D_{n-1}=Dt[0], D_n=Dt[1], D_{n+1}=Dt[2] */
     d0 = Dt[2]; d1 = Dt[1]; d2 = Dt[0]; d3 = Dt[0]; d4 = Dt[1]; d5 = Dt[2];
-    auto emit = [&](int j, float o1j) -> double {
+    auto flux = [&](float kj) -> double {
       const double s1 = d2 + d3;
       const double s2 = (s1 + d1) + d4;
       const double s3 = (s2 + d0) + d5;
       const double df = -((1.0 / 60.0) * (((45.0 * s1) - 9.0 * s2) + s3));
-      const double v = ((-(double)o1j) * df) * dz1;
-      if (Vb) __stcs(&Vb[(int64_t)j * it.vz], v);
-      return v;
+      return ((-(double)rcp(kj)) * df) * dz1;
     };
-    vtop = emit(n - 1, nx4_top_o1);
+    {
+      const float kj = sc.kappa(n - 1);
+      vtop = flux(kj);
+      st.push(6, n - 1, Uk[2], vtop, (double)kj); /* U_{n-4}, V_{n-1} */
+      st.group(n - 1, 7);
+    }
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = fn; /* the four lowest U seen so far */
-    /* o1 ring: r1, r2, r3 = 1/kappa of k+1, k+2, k+3 before step k */
-    float r1 = o1_nm4, r2 = o1_nm3, r3 = o1_nm2;
-    auto step = [&](int k, const float4 &w) {
+    /* kappa ring: r1, r2, r3 = kappa of k+1, k+2, k+3 before step k */
+    float r1 = kt[2], r2 = kt[1], r3 = kt[0];
+    auto step = [&](int slot, int k, const float4 &w) {
       const float g1 = (w.x >= 0.0f) ? 1.0f - w.x : -w.x; /* |gamma_{k+1}| */
       const float qk = (w.x >= 0.0f) ? w.x : 1.0f + w.x;  /* q_k */
       XF uj;
@@ -338,30 +360,42 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       XF Dj;
       xaxpy2(uj, Un, g1, -qk, Un, Dj);
       const double Uv = xtod(Un);
-      if (Ub) __stcs(&Ub[(int64_t)(3 + k) * uz], Uv);
       U3 = U2; U2 = U1; U1 = U0; U0 = Uv;
       d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = xtod(Dj);
-      emit(k + 3, r3);
+      st.push(slot, 3 + k, Uv, flux(r3), (double)r3);
       r3 = r2; r2 = r1; r1 = w.y;
     };
     int k = n - 5;
     constexpr int PF = OCO_MIXED_PREFETCH;
-    for (; k >= PF - 1; k -= PF) { /* scratch loads of PF steps hoisted off the serial chain */
-      float4 w[PF];
-      /* the PF scratch levels OCO_MIXED_L2_AHEAD steps ahead into L2, one bulk request from lane
-       * 0 (the warp's levels are contiguous; they were written a whole forward sweep ago and
-       * have usually left L2) */
-      if (k - PF + 1 - OCO_MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0) /* PF levels, one bulk request */
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(
-                         sc.level(k - PF + 1 - OCO_MIXED_L2_AHEAD))),
-                     "r"((uint32_t)(PF * SC::LEVEL))
-                     : "memory");
+    static_assert(8 % PF == 0, "groups of 8 levels");
+    for (; k >= 7; k -= 8) {
 #pragma unroll
-      for (int q = 0; q < PF; q++) w[q] = sc.get(k - q);
+      for (int g = 0; g < 8; g += PF) { /* scratch loads of PF steps hoisted off the serial chain */
+        const int kg = k - g;
+        float4 w[PF];
+        /* the PF scratch levels OCO_MIXED_L2_AHEAD steps ahead into L2, one bulk request from lane
+         * 0 (the warp's levels are contiguous; they were written a whole forward sweep ago and
+         * have usually left L2) */
+        if (kg - PF + 1 - OCO_MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0) /* PF levels, one bulk request */
+          asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(
+                           sc.level(kg - PF + 1 - OCO_MIXED_L2_AHEAD))),
+                       "r"((uint32_t)(PF * SC::LEVEL))
+                       : "memory");
 #pragma unroll
-      for (int q = 0; q < PF; q++) step(k - q, w[q]);
+        for (int q = 0; q < PF; q++) w[q] = sc.get(kg - q);
+#pragma unroll
+        for (int q = 0; q < PF; q++) step(g + q, kg - q, w[q]);
+      }
+      st.group(3 + k - 7, 8);
     }
-    for (; k >= 0; k--) step(k, sc.get(k));
+    int q = 0;
+    for (; k >= 0; k--) {
+      step(q, k, sc.get(k));
+      if (++q == 8) {
+        st.group(3 + k, 8);
+        q = 0;
+      }
+    }
     { /* condition number of the bottom flux from D_0, D_1, D_2 (d0, d1, d2) and U_1..U_3 */
       double Cb = 0.0;
 #pragma unroll
@@ -377,18 +411,20 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       flag = flag || !(Cb <= (double)cond * fabs(37.0 * d0 - 8.0 * d1 + d2));
     }
     /* bottom ghosts f(n1-i) = 2 f(n1) - f(n1+i); ghost differences mirror D_0, D_1, D_2 */
-    if (Ub) {
-      __stcs(&Ub[(int64_t)2 * uz], 2.0 * U0 - U1);
-      __stcs(&Ub[(int64_t)1 * uz], 2.0 * U0 - U2);
-      __stcs(&Ub[0], 2.0 * U0 - U3);
+    const double g[3] = {2.0 * U0 - U3, 2.0 * U0 - U2, 2.0 * U0 - U1}; /* ghosts 0, 1, 2 */
+    const double D[3] = {d2, d1, d0};
+    const float kb[3] = {r1, r2, r3};
+#pragma unroll
+    for (int j = 2; j >= 0; j--) { /* D_{-1} = D_0, D_{-2} = D_1, D_{-3} = D_2 */
+      d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D[j];
+      vbot = flux(kb[j]);
+      st.push(q, j, g[j], vbot, (double)kb[j]);
+      if (++q == 8) {
+        st.group(j, 8);
+        q = 0;
+      }
     }
-    const double D0 = d0, D1 = d1, D2 = d2;
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D0; /* D_{-1} = D_0 */
-    emit(2, r3);
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D1; /* D_{-2} = D_1 */
-    emit(1, r2);
-    d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D2; /* D_{-3} = D_2 */
-    vbot = emit(0, r1);
+    st.finish(q);
   } else { /* nz = 2 or 3: U stencil on the ghosted array (the reference's update order) */
     double f[9];
     const int n1 = 3, n2 = nz + 2;
@@ -407,17 +443,19 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       f[n1 - i] = 2.0 * f[n1] - f[n1 + i];
       f[n2 + i] = 2.0 * f[n2] - f[n2 - i];
     }
-    if (Ub)
-      for (int m = 0; m < nz + 6; m++) __stcs(&Ub[(int64_t)m * uz], f[m]);
+    for (int m = 0; m < nz + 6; m++) st.u(m, f[m]);
     for (int j = 0; j < nz; j++) {
       const int c = n1 + j;
       const double df = (1.0 / 60.0) * (((45.0 * (f[c + 1] - f[c - 1])) - 9.0 * (f[c + 2] - f[c - 2])) + (f[c + 3] - f[c - 3]));
-      const double v = ((-(double)sc.o1(j)) * df) * dz1;
-      if (Vb) __stcs(&Vb[(int64_t)j * it.vz], v);
+      const float kj = sc.kappa(j);
+      const double v = ((-(double)rcp(kj)) * df) * dz1;
+      st.v(j, v);
+      st.k(j, (double)kj);
       if (j == 0) vbot = v;
       if (j == nz - 1) vtop = v;
     }
   }
+  if (!active) return false;
   if (it.vtop) __stcs(it.vtop, vtop);
   if (it.vbot) __stcs(it.vbot, vbot);
   return flag;
@@ -463,28 +501,49 @@ __device__ __forceinline__ void mark_items(bool flag, int64_t word, int iw, unsi
   list_items(flag, m, id, word, iw, ilist, icount, slot);
 }
 
-template <class SC>
-__global__ void __launch_bounds__(128, 5) k_solve_mixed_staged(const MixedArgs a) {
-  __shared__ __align__(128) float s_rec[MWARPS][2 * MZC * MZN];
-  __shared__ __align__(8) unsigned long long s_bar[MWARPS][2];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int ntiles = (a.nw + 31) / 32;
-  const unsigned long long ntasks = (unsigned long long)a.ncol * ntiles;
-  const SC sc{(char *)(a.s4 + slot * 32 * (int64_t)a.nz), lane}; /* the warp's scratch, contiguous */
-  MStaged pa;
-  pa.buf = s_rec[wib];
-  pa.bar0 = msmem(&s_bar[wib][0]);
-  pa.nz = a.nz;
+/* A staged warp's shared memory; the output ring of the reverse sweep takes over what the forward
+ * sweep used (the next task rewrites it; see MStaged::begin). */
+struct MStagedSmem {
+  union {
+    struct {
+      float rec[2 * MZC * MZN];
+      float lam[MLN * 32]; /* the task's 32 wavelengths' constants */
+    };
+    RingSmem<float> ring;
+  };
+  unsigned long long bar[2];
+  __device__ MStagedSmem() = delete;
+};
+static_assert(sizeof(MStagedSmem) % 16 == 0, "bulk copies");
+
+__device__ __forceinline__ void init_staged(MStaged &pa, MStagedSmem &sm) {
+  pa.buf = sm.rec;
+  pa.bar0 = msmem(&sm.bar[0]);
   pa.waits = 0;
   pa.inflight = 0;
   pa.failed = false;
-  if (lane == 0) {
+  if ((threadIdx.x & 31) == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0 + 8u) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
+}
+
+/* REF: outputs with z fastest through the ring (AGN grid of 1600 columns x 512 x 256: 5.04 ms with
+ * lambda-fastest temporaries and three transposes, 3.43 ms so; with lambda fastest 2.95 ms). */
+template <class SC, bool REF>
+__global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const MixedArgs a) {
+  __shared__ __align__(128) unsigned char s_warp[MWARPS * sizeof(MStagedSmem)];
+  MStagedSmem &sm = reinterpret_cast<MStagedSmem *>(s_warp)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int ntiles = (a.nw + 31) / 32;
+  const unsigned long long ntasks = (unsigned long long)a.ncol * ntiles;
+  const SC sc{(char *)(a.s4 + slot * 32 * (int64_t)a.nz), lane}; /* the warp's scratch, contiguous */
+  MStaged pa;
+  pa.nz = a.nz;
+  init_staged(pa, sm);
   for (;;) {
     unsigned long long task = 0;
     if (lane == 0) task = atomicAdd(a.work, 1ull);
@@ -496,7 +555,11 @@ __global__ void __launch_bounds__(128, 5) k_solve_mixed_staged(const MixedArgs a
     const bool active = iw_raw < a.nw;
     const int iw = active ? iw_raw : a.nw - 1;
     pa.begin(a.rec + cl * (int64_t)a.nz * MZN);
-    const bool flag = msolve_item(block_item(a, cl, iw), active, pa, sc, a.repair_cond) ||
+    store_lam32_shared(sm.lam, lane, a.lam, iw, a.nw);
+    __syncwarp();
+    const MItem it = block_item(a, cl, iw);
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<REF, true, true>(it.o, active, &sm.ring),
+                                  a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
@@ -509,8 +572,11 @@ __global__ void __launch_bounds__(128, 5) k_solve_mixed_staged(const MixedArgs a
   }
 }
 
-template <class SC>
-__global__ void __launch_bounds__(128, 5) k_solve_mixed(const MixedArgs a) {
+/* Few wavelengths: 32 consecutive items per warp (lanes past the last item repeat it and store
+ * nothing). */
+template <class SC, bool REF>
+__global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
+  __shared__ RingSmem<float> s_ring[REF ? MWARPS : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nitems = a.ncol * a.nw;
@@ -521,36 +587,37 @@ __global__ void __launch_bounds__(128, 5) k_solve_mixed(const MixedArgs a) {
     if (lane == 0) task = atomicAdd(a.work, 1ull);
     task = __shfl_sync(0xffffffffu, task, 0);
     if (task >= ntasks) break;
-    const int64_t item = (int64_t)task * 32 + lane;
-    bool flag = false;
-    int64_t word = 0;
-    int iw = 0;
-    if (item < nitems) {
-      const int64_t cl = item / a.nw;
-      iw = (int)(item - cl * a.nw);
-      MDirect pa{a.rec + cl * (int64_t)a.nz * MZN};
-      flag = msolve_item(block_item(a, cl, iw), true, pa, sc, a.repair_cond) || __ldg(a.colflag + cl) != 0u;
-      word = cl * ((a.nw + 31) / 32) + iw / 32;
-    }
-    mark_items(flag, word, iw, (unsigned long long)item, a.rbits, a.rslot, a.rlist, a.rcount, a.ilist, a.icount);
+    const bool active = (int64_t)task * 32 + lane < nitems;
+    const int64_t item = active ? (int64_t)task * 32 + lane : nitems - 1;
+    const int64_t cl = item / a.nw;
+    const int iw = (int)(item - cl * a.nw);
+    MDirect pa{a.rec + cl * (int64_t)a.nz * MZN};
+    const MItem it = block_item(a, cl, iw);
+    const bool flag = msolve_item(it, active, pa, load_lam32(it.lam, iw, it.nw), sc,
+                                  make_stores<REF, false, true>(it.o, active, &s_ring[REF ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
+                      (active && __ldg(a.colflag + cl) != 0u);
+    mark_items(flag, cl * ((a.nw + 31) / 32) + iw / 32, iw, (unsigned long long)item, a.rbits, a.rslot, a.rlist, a.rcount,
+               a.ilist, a.icount);
   }
 }
 
 static bool mixed_uses_staging(int nw) { return (nw >= 64) || (nw % 32) == 0; }
 
-static const void *solve_mixed_fn(int nw) {
-  return mixed_uses_staging(nw) ? (const void *)k_solve_mixed_staged<MScratch16> : (const void *)k_solve_mixed<MScratch16>;
+static const void *solve_mixed_fn(int nw, bool ref) {
+  if (mixed_uses_staging(nw))
+    return ref ? (const void *)k_solve_mixed_staged<MScratch16, true> : (const void *)k_solve_mixed_staged<MScratch16, false>;
+  return ref ? (const void *)k_solve_mixed<MScratch16, true> : (const void *)k_solve_mixed<MScratch16, false>;
 }
 
 int solve_mixed_max_blocks_per_sm(int threads, int nw) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw), threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw, false), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
 cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_mixed_fn(a.nw), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(solve_mixed_fn(a.nw, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 /* ---- ragged batches ---------------------------------------------------------------------- */
@@ -568,16 +635,18 @@ __device__ __forceinline__ MItem batch_item(const MixedBatchArgs &b, const MBatc
   it.dz2f = (float)c.dz2; /* as block_item's (float)(dz * dz) */
   it.dz1 = c.dz1;
   if (b.layout == 0) { /* per column [lambda][z] (z fastest) */
-    it.U = b.U ? b.U + c.u_off + (int64_t)iw * (c.nz + 6) : nullptr;
-    it.K = b.K ? b.K + c.kv_off + (int64_t)iw * c.nz : nullptr;
-    it.V = b.V ? b.V + c.kv_off + (int64_t)iw * c.nz : nullptr;
-    it.uz = it.kz = it.vz = 1;
+    it.o.U = b.U ? b.U + c.u_off + (int64_t)iw * (c.nz + 6) : nullptr;
+    it.o.K = b.K ? b.K + c.kv_off + (int64_t)iw * c.nz : nullptr;
+    it.o.V = b.V ? b.V + c.kv_off + (int64_t)iw * c.nz : nullptr;
+    it.o.uz = it.o.kz = it.o.vz = 1;
   } else { /* per column [z][lambda] */
-    it.U = b.U ? b.U + c.u_off + iw : nullptr;
-    it.K = b.K ? b.K + c.kv_off + iw : nullptr;
-    it.V = b.V ? b.V + c.kv_off + iw : nullptr;
-    it.uz = it.kz = it.vz = c.nw;
+    it.o.U = b.U ? b.U + c.u_off + iw : nullptr;
+    it.o.K = b.K ? b.K + c.kv_off + iw : nullptr;
+    it.o.V = b.V ? b.V + c.kv_off + iw : nullptr;
+    it.o.uz = it.o.kz = it.o.vz = c.nw;
   }
+  it.o.urow = c.nz + 6;
+  it.o.krow = c.nz;
   it.vtop = b.Vtop ? b.Vtop + c.flux_off + iw : nullptr;
   it.vbot = b.Vbot ? b.Vbot + c.flux_off + iw : nullptr;
   return it;
@@ -585,25 +654,15 @@ __device__ __forceinline__ MItem batch_item(const MixedBatchArgs &b, const MBatc
 
 /* Warp-column tiling: tasks (column, 32-wavelength tile) from the device queue, longest
  * columns first; the column's records stream through the warp's shared-memory buffers. */
-template <class SC>
-__global__ void __launch_bounds__(128, 5) k_batch_mixed_staged(const MixedBatchArgs b) {
-  __shared__ __align__(128) float s_rec[MWARPS][2 * MZC * MZN];
-  __shared__ __align__(8) unsigned long long s_bar[MWARPS][2];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+template <class SC, bool REF>
+__global__ void __launch_bounds__(128, MBLOCKS) k_batch_mixed_staged(const MixedBatchArgs b) {
+  __shared__ __align__(128) unsigned char s_warp[MWARPS * sizeof(MStagedSmem)];
+  MStagedSmem &sm = reinterpret_cast<MStagedSmem *>(s_warp)[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const SC sc{(char *)(b.s4 + slot * 32 * (int64_t)b.max_nz), lane}; /* the warp's scratch, contiguous */
   MStaged pa;
-  pa.buf = s_rec[wib];
-  pa.bar0 = msmem(&s_bar[wib][0]);
-  pa.waits = 0;
-  pa.inflight = 0;
-  pa.failed = false;
-  if (lane == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0) : "memory");
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(pa.bar0 + 8u) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncwarp();
+  init_staged(pa, sm);
   for (;;) {
     unsigned long long task = 0;
     if (lane == 0) task = atomicAdd(b.work, 1ull);
@@ -616,7 +675,11 @@ __global__ void __launch_bounds__(128, 5) k_batch_mixed_staged(const MixedBatchA
     const int iw = active ? iw_raw : c.nw - 1;
     pa.nz = c.nz;
     pa.begin(b.rec + c.rec_off * MZN);
-    const bool flag = msolve_item(batch_item(b, c, iw), active, pa, sc, b.repair_cond) ||
+    store_lam32_shared(sm.lam, lane, b.lam + c.lam_off, iw, c.nw);
+    __syncwarp();
+    const MItem it = batch_item(b, c, iw);
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<REF, true, true>(it.o, active, &sm.ring),
+                                  b.repair_cond) ||
                       (active && __ldg(b.colflag + t.x) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
@@ -633,7 +696,7 @@ __global__ void __launch_bounds__(128, 5) k_batch_mixed_staged(const MixedBatchA
  * form one list; a warp takes 32 consecutive items, so partial wavelength tiles of one column
  * are filled with the next column's items (similar nz, as the list is sorted). */
 template <class SC>
-__global__ void __launch_bounds__(128, 5) k_batch_mixed_packed(const MixedBatchArgs b) {
+__global__ void __launch_bounds__(128, 4) k_batch_mixed_packed(const MixedBatchArgs b) {
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const SC sc{(char *)(b.s4 + slot * 32 * (int64_t)b.max_nz), lane}; /* the warp's scratch, contiguous */
@@ -659,28 +722,31 @@ __global__ void __launch_bounds__(128, 5) k_batch_mixed_packed(const MixedBatchA
       iw = (int)(item - __ldg(b.item_pre + lo));
       const MBatchCol c = b.cols[col];
       MDirect pa{b.rec + c.rec_off * MZN};
-      flag = msolve_item(batch_item(b, c, iw), true, pa, sc, b.repair_cond) || __ldg(b.colflag + col) != 0u;
+      /* the lanes' columns differ in depth: each stores its own levels */
+      const MItem it = batch_item(b, c, iw);
+      flag = msolve_item(it, true, pa, load_lam32(it.lam, iw, it.nw), sc, LaneStores<true>(it.o, true), b.repair_cond) ||
+             __ldg(b.colflag + col) != 0u;
     }
     mark_items(flag, (int64_t)col * b.rwstride + iw / 32, iw, ((unsigned long long)(unsigned)col << 32) | (unsigned)iw,
                b.rbits, b.rslot, b.rlist, b.rcount, b.ilist, b.icount);
   }
 }
 
-static const void *batch_mixed_fn(int tiling) {
-  return tiling == BATCH_TILING_PACKED ? (const void *)k_batch_mixed_packed<MScratch12>
-                                       : (const void *)k_batch_mixed_staged<MScratch12>;
+static const void *batch_mixed_fn(int tiling, bool ref) {
+  if (tiling == BATCH_TILING_PACKED) return (const void *)k_batch_mixed_packed<MScratch12>;
+  return ref ? (const void *)k_batch_mixed_staged<MScratch12, true> : (const void *)k_batch_mixed_staged<MScratch12, false>;
 }
 
 int batch_mixed_max_blocks_per_sm(int tiling, int threads) {
   int n = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_fn(tiling), threads, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_fn(tiling, false), threads, 0);
   if (e != cudaSuccess || n < 1) n = 1;
   return n;
 }
 
 cudaError_t launch_batch_mixed(const MixedBatchArgs &a, int tiling, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(batch_mixed_fn(tiling), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(batch_mixed_fn(tiling, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

@@ -43,6 +43,10 @@ __device__ __forceinline__ void store_records(const float *r, float *__restrict_
   }
 }
 
+__device__ __forceinline__ bool same_bits(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+
 /* colflag[col] is set to 1 when a cell of the column has a negative neutral fraction (see
  * mx::pillar); the caller clears it first. */
 __global__ void __launch_bounds__(PM_THREADS) k_pillars_mixed(const double *__restrict__ rho,
@@ -55,7 +59,8 @@ __global__ void __launch_bounds__(PM_THREADS) k_pillars_mixed(const double *__re
   if (i0 >= n) return; /* whole warp past the end */
   float r[MZN];
   if (i < n) {
-    if (pillar(rho[i], T[i], fully_ionized_T, r)) colflag[i / nz] = 1u;
+    const bool same = i % nz != 0 && same_bits(T[i], T[i - 1]);
+    if (pillar(rho[i], T[i], fully_ionized_T, r, same)) colflag[i / nz] = 1u;
   } else {
 #pragma unroll
     for (int k = 0; k < MZN; k++) r[k] = 0.0f; /* not stored */
@@ -97,7 +102,8 @@ __global__ void __launch_bounds__(PM_THREADS) k_pillars_mixed_batch(const double
         hi = mid;
     }
     const int64_t src = cols[lo].in_off + (i - rec_pre[lo]);
-    if (pillar(rho[src], T[src], fully_ionized_T, r)) colflag[lo] = 1u;
+    const bool same = i != rec_pre[lo] && same_bits(T[src], T[src - 1]);
+    if (pillar(rho[src], T[src], fully_ionized_T, r, same)) colflag[lo] = 1u;
   } else {
 #pragma unroll
     for (int k = 0; k < MZN; k++) r[k] = 0.0f; /* not stored */

@@ -101,6 +101,11 @@ struct RBatchItem {
   __device__ __forceinline__ const double *T() const { return a.T + c.in_off; }
 };
 
+template <class IT>
+__device__ __forceinline__ LaneStores<false> lane_stores(const IT &it) {
+  return LaneStores<false>(OutPtrs{it.U(), it.K(), it.V(), it.uz(), it.kz(), it.vz(), 0, 0}, true);
+}
+
 /* An item whose scratch is one lane's contiguous arrays (the by-item path). */
 template <class IT>
 struct UnitStride : IT {
@@ -213,7 +218,8 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
   }
   /* 4. the reverse sweep: back-substitution, ghosts, flux (scratch at stride 1) */
   const UnitStride<IT> iu{it};
-  solve_reverse<1>(iu, true, u, gam, uu, o1, qs, LaneStores<UnitStride<IT>>(iu, true));
+  LaneStores<false> st = lane_stores(iu);
+  solve_reverse<1>(iu, true, u, gam, uu, o1, qs, st);
 }
 
 /* ---- coefficient slots ------------------------------------------------------------------ */
@@ -375,7 +381,8 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
     atomicAdd(&it.status()[0], 1ull);
     atomicMin(&it.status()[1], it.id());
   }
-  solve_reverse<1, true>(it, true, u, aa, dd, S.o1 + q0, ee, LaneStores<IT>(it, true));
+  LaneStores<false> st = lane_stores(it);
+  solve_reverse<1, true>(it, true, u, aa, dd, S.o1 + q0, ee, st);
 }
 
 __global__ void __launch_bounds__(REPAIR_THREADS, 6) k_repair_solve(const RepairArgs a) {

@@ -16,7 +16,8 @@
  *     FP32, the fractions keep ~3e-8 absolute precision, and every 2^x is taken as
  *     2^int * ex2(fraction): kappa and the source function come out to a few 1e-7.  The
  *     Planck exponent x*log2(e) is a double-float product (FMA two-product of split FP32
- *     factors) for the same reason.  The H bound-free level sum
+ *     factors) for the same reason.  What depends on (T, lambda) only (TF32) is kept from one
+ *     level to the next while T does not change by a bit.  The H bound-free level sum
  *     sum_n g(lambda,n) n^-3 exp(-chi_n/kT) (:237-239) is factored by its first non-zero
  *     level n0(lambda): E_n0 * (g_n0 + sum_{n>n0} g_n * E_n/E_n0), with the ratios E_n/E_n0
  *     precomputed per z.  The absorption fraction 1 - omega = kappa_abs/kappa_rad is a linear
@@ -45,8 +46,10 @@
 
 #ifdef __CUDACC__
 #define MX_HD static __host__ __device__ __forceinline__
+#define MX_HD_MEMBER __host__ __device__ __forceinline__
 #else
 #define MX_HD static inline
+#define MX_HD_MEMBER inline
 #endif
 
 namespace oco {
@@ -57,21 +60,25 @@ namespace mx {
  * small logarithms or linear values.  damping_factor_const/T is split into hi + lo (the Planck
  * exponent needs it to ~1e-12). */
 enum MixedZ {
-  MZ_TH = 0,        /* theta = 5040/T */
-  MZ_PU,            /* log2(ionf * Unsold integral) [2] */
-  MZ_PE = MZ_PU + 2, /* log2(ionf * exp(-chi_n/kT)), n = 1..6 [2 each] */
-  MZ_LHM = MZ_PE + 12, /* log2(hm_bf_factor * ionf) [2] */
+  /* read at every point, in 16-byte groups */
+  MZ_LHM = 0,       /* log2(hm_bf_factor * ionf) [2] */
   MZ_LAFF = MZ_LHM + 2, /* log2(ionf ne k T) [2] */
   MZ_LESC = MZ_LAFF + 2, /* log2(e_scatter) [2] */
   MZ_LIONFEF = MZ_LESC + 2, /* log2(ionf * energyfactor) [2] */
   MZ_LRHO = MZ_LIONFEF + 2, /* log2(rho) [2] */
-  MZ_LZ2 = MZ_LRHO + 2, /* log2(ne (nHI+nHII) T^-1/2) [2] */
-  MZ_LGT = MZ_LZ2 + 2, /* log10(theta) */
-  MZ_LGT2,          /* log10(theta)^2 */
-  MZ_NEUTRAL,       /* 1 if (1 - NHII/N) > switch_ionfraction */
-  MZ_TH1L,          /* theta1 * log10e */
-  MZ_LNTPOW,        /* ln((T*1e-4)^-1.5) */
+  MZ_PU = MZ_LRHO + 2, /* log2(ionf * Unsold integral) [2] */
+  MZ_FLAGS = MZ_PU + 2, /* integer bits MZF_NEUTRAL, MZF_SAME_T */
+  MZ_PAD,
+  MZ_PE,            /* log2(ionf * exp(-chi_n/kT)), n = 1..6 [2 each] */
+  /* read at ionized points */
+  MZ_LZ2 = MZ_PE + 12, /* log2(ne (nHI+nHII) T^-1/2) [2] */
+  MZ_LNTPOW = MZ_LZ2 + 2, /* ln((T*1e-4)^-1.5) */
   MZ_T1,            /* 1/T */
+  /* read where the temperature changes */
+  MZ_TH,            /* theta = 5040/T */
+  MZ_LGT,           /* log10(theta) */
+  MZ_LGT2,          /* log10(theta)^2 */
+  MZ_TH1L,          /* theta1 * log10e */
   MZ_DFT1,          /* damping_factor_const / T, high part */
   MZ_DFT1L,         /* low part */
   MZ_R,             /* level ratios E_n/E_n0 by first level n0 = 1..6: row n0 at MZ_R + rrow(n0)
@@ -80,6 +87,8 @@ enum MixedZ {
   MZ_END = MZ_R + 26,
   MZN = 64          /* 256 B */
 };
+constexpr int MZF_NEUTRAL = 1; /* (1 - NHII/N) > switch_ionfraction */
+constexpr int MZF_SAME_T = 2;  /* T equals the level below's bit for bit (never set at z = 0) */
 /* start of row n0 (1..6) of the level-ratio table: sum over m < n0 of (7 - m) */
 MX_HD int rrow(int n0) { return (n0 - 1) * 7 - ((n0 - 1) * n0) / 2; }
 static_assert(MZ_END <= MZN && MZN % 4 == 0, "mixed record layout");
@@ -145,6 +154,24 @@ MX_HD float rcp(float x) {
 #endif
 }
 
+MX_HD int f2bits(float f) {
+#ifdef __CUDA_ARCH__
+  return __float_as_int(f);
+#else
+  int i;
+  memcpy(&i, &f, 4);
+  return i;
+#endif
+}
+MX_HD float bits2f(int i) {
+#ifdef __CUDA_ARCH__
+  return __int_as_float(i);
+#else
+  float f;
+  memcpy(&f, &i, 4);
+  return f;
+#endif
+}
 MX_HD float fmaxf_(float a, float b) { return a > b ? a : b; }
 /* log2(1 - 2^-t) for t > 0 (accurate to a few 1e-7 relative of the result's argument
  * for t >= 2^-6; a two-term series below that). */
@@ -182,7 +209,7 @@ MX_HD double dexp(double v) { return exp(v); }
  * proportional to ionf (continuous_opacity.f90:237-244, :318-322, :337-339, :265) turn negative.
  * Logarithms cannot carry that (the record holds such terms as vanishing): a column with such a
  * cell is solved in FP64 instead. */
-MX_HD bool pillar(double r, double t, double fully_ionized_T, float *o) {
+MX_HD bool pillar(double r, double t, double fully_ionized_T, float *o, bool same_T = false) {
   using namespace oco::k;
   const double rho1 = 1.0 / r, T1 = 1.0 / t;
   double c_ion = (mp * rho1) * (saha_const * oco_pow(t, 1.5) * oco_exp(-((T1 * hydrogen_ionization_eV) * k1_eV)));
@@ -234,12 +261,13 @@ MX_HD bool pillar(double r, double t, double fully_ionized_T, float *o) {
   put_l2(nprod > 0.0 ? (dlog(nprod) - 0.5 * dlog(t)) * kLog2e : (double)kNeg, o + MZ_LZ2);
   o[MZ_LGT] = (float)(lgt);
   o[MZ_LGT2] = (float)((lgt * lgt));
-  o[MZ_NEUTRAL] = (float)(((1.0 - x) > switch_ionfraction) ? 1.0 : 0.0);
+  o[MZ_FLAGS] = bits2f((((1.0 - x) > switch_ionfraction) ? MZF_NEUTRAL : 0) | (same_T ? MZF_SAME_T : 0));
+  o[MZ_PAD] = 0.0f;
+  for (int k2 = MZ_END; k2 < MZN; k2++) o[k2] = 0.0f;
   o[MZ_TH1L] = (float)((theta1 * log10e));
   o[MZ_LNTPOW] = (float)((-1.5 * dlog(t * 1e-4)));
   o[MZ_T1] = (float)(T1);
   split2(damping_factor_const * T1, o[MZ_DFT1], o[MZ_DFT1L]);
-  for (int k2 = MZ_END; k2 < MZN; k2++) o[k2] = 0.0f;
   return nHI < 0.0;
 }
 
@@ -274,41 +302,16 @@ MX_HD void lambda_record(const LamIn &L, float *o) {
   o[ML_LSF] = (float)(lsw5 - fl);
 }
 
-/* Wavelength constants held in registers by the solve; *i members are the integer parts of
- * the large logarithms (value = member + member_i). */
+/* Wavelength constants by MixedL field. */
 struct Lam32 {
-  float cl2, law, lawi, gs[6], ls, lsi_, fc, fci, f2, f3, lal0w, lal0wi, gff, chi1, lnnu9, hnuk, l3nu, l3nui;
-  float ch, cl;   /* log2(e)/lambda_cm = ch + cl */
-  float lsi, lsf; /* log2(2 h c^2 lambda_cm^-5) = lsi + lsf, lsi an integer */
-  int roff, peoff; /* MixedZ offsets of the level-ratio row and of log2(ionf E_n0) */
+  float f[MLN];
+  MX_HD_MEMBER float operator()(int k) const { return f[k]; }
 };
 /* Lam32 from a record laid out as MixedL (field f at t[f * stride]). */
 template <class Get>
 MX_HD void lam32_from(Lam32 &L, Get t) {
-  L.cl2 = t(ML_CL2);
-  L.law = t(ML_LAW);
-  L.lawi = t(ML_LAW + 1);
-  for (int q = 0; q < 6; q++) L.gs[q] = t(ML_GS + q);
-  L.roff = (int)t(ML_ROFF);
-  L.peoff = (int)t(ML_PEOFF);
-  L.ls = t(ML_LS);
-  L.lsi_ = t(ML_LS + 1);
-  L.fc = t(ML_FC);
-  L.fci = t(ML_FC + 1);
-  L.f2 = t(ML_F2);
-  L.f3 = t(ML_F3);
-  L.lal0w = t(ML_LAL0W);
-  L.lal0wi = t(ML_LAL0W + 1);
-  L.gff = t(ML_GFF);
-  L.chi1 = t(ML_CHI1);
-  L.lnnu9 = t(ML_LNNU9);
-  L.hnuk = t(ML_HNUK);
-  L.l3nu = t(ML_L3NU);
-  L.l3nui = t(ML_L3NU + 1);
-  L.ch = t(ML_CH);
-  L.cl = t(ML_CL);
-  L.lsi = t(ML_LSI);
-  L.lsf = t(ML_LSF);
+#pragma unroll
+  for (int k = 0; k < MLN; k++) L.f[k] = t(k);
 }
 
 /* Opacity, absorption fraction and source function of one (z, lambda):
@@ -357,48 +360,104 @@ MX_HD float pow2_expo(float w) {
 constexpr float kLog2mp1I = 79.0f, kLog2mp1F = -0.0158371009f;
 constexpr float kBremsI = 28.0f, kBremsF = 0.459963723f;
 
-template <class Rec>
-MX_HD Opac32 opacity(const Rec &Z, const Lam32 &L) {
+/* The (T, lambda) part of a point. */
+struct TF32 {
+  float ls;     /* log2(1 - 10^(-chi theta)), c_o :171 */
+  float sm;     /* sum over levels from n0 of g_n E_n/E_n0 */
+  float ff;     /* f2 lgt + f3 lgt^2, log2 */
+  float lgff;   /* log2 of the free-free Gaunt factor */
+  float Si, Sf; /* log2 S before the binary exponent of 1 - omega, integer + fraction */
+};
+
+template <class Rec, class LA>
+MX_HD TF32 tfac(const Rec &Z, const LA &L) {
+  TF32 t;
   /* stim = 1 - 10^(-chi theta) (c_o :171) */
-  const float t10 = L.cl2 * Z[MZ_TH];
-  const float ls = (t10 > 40.0f) ? 0.0f : log2_one_minus_exp2neg(t10);
-  /* H bound-free (c_o :233-244): AHbf wa^3 stim ionf (Unsold + E_n0 sm), sm = sum over
-   * t = 0..5 of g_{n0+t} E_{n0+t}/E_n0: six FMAs down row n0 of the ratio table (levels below
-   * n0 have g = 0 and drop out; past level 6 the weights are 0) */
-  float ai = Z[MZ_PU + 1], af = Z[MZ_PU];
-  float sm = 0.0f;
+  const float t10 = L(ML_CL2) * Z[MZ_TH];
+  t.ls = (t10 > 40.0f) ? 0.0f : log2_one_minus_exp2neg(t10);
+  /* H bound-free (c_o :233-244): sm = sum over t = 0..5 of g_{n0+t} E_{n0+t}/E_n0: six FMAs down
+   * row n0 of the ratio table (levels below n0 have g = 0 and drop out; past level 6 the weights
+   * are 0) */
+  const int roff = (int)L(ML_ROFF);
+  t.sm = 0.0f;
 #pragma unroll
-  for (int t = 0; t < 6; t++) sm = fmaf(L.gs[t], Z[L.roff + t], sm);
+  for (int q = 0; q < 6; q++) t.sm = fmaf(L(ML_GS + q), Z[roff + q], t.sm);
+  t.ff = L(ML_F2) * Z[MZ_LGT] + L(ML_F3) * Z[MZ_LGT2];
+  const float gff = 1.0f + L(ML_GFF) * (Z[MZ_TH1L] * L(ML_CHI1) + 0.5f);
+  t.lgff = lg2(gff);
+  /* Planck function (c_o :399-407): S = sw5 / (e^x - 1), x = dft1/lambda_cm clamped at 308.
+   * t2 = x log2(e) = (dft1_hi + dft1_lo)(ch + cl) as hi + lo (FMA two-product). */
+  const float dh = Z[MZ_DFT1], dl = Z[MZ_DFT1L], ch = L(ML_CH);
+  float p = dh * ch;
+  float lo = fmaf(dh, ch, -p) + (dh * L(ML_CL) + dl * ch);
+  if (p > kT2Clamp) {
+    p = kT2Clamp;
+    lo = kT2ClampLo;
+  }
+  const float ti = floorf(p);
+  const float tf = (p - ti) + lo; /* t2 = ti + tf */
+  const float lm = (p > 40.0f) ? 0.0f : log2_one_minus_exp2neg(p);
+  t.Si = L(ML_LSI) - ti;
+  t.Sf = (L(ML_LSF) - tf) - lm;
+  return t;
+}
+
+/* Wavelength constants that every point needs (the others stay in memory behind LA). */
+struct LamPt {
+  float law, lawi, ls, lsi, fc, fci, lal0w, lal0wi;
+  int peoff;
+};
+template <class LA>
+MX_HD LamPt lam_point(const LA &L) {
+  LamPt c;
+  c.law = L(ML_LAW);
+  c.lawi = L(ML_LAW + 1);
+  c.ls = L(ML_LS);
+  c.lsi = L(ML_LS + 1);
+  c.fc = L(ML_FC);
+  c.fci = L(ML_FC + 1);
+  c.lal0w = L(ML_LAL0W);
+  c.lal0wi = L(ML_LAL0W + 1);
+  c.peoff = (int)L(ML_PEOFF);
+  return c;
+}
+
+/* The point from its (T, lambda) part and the record's density-dependent logarithms. */
+template <class Rec, class LA>
+MX_HD Opac32 opacity(const Rec &Z, const LA &L, const LamPt &c, const TF32 &t) {
+  /* H bound-free (c_o :233-244): AHbf wa^3 stim ionf (Unsold + E_n0 sm) */
+  float ai = Z[MZ_PU + 1], af = Z[MZ_PU];
   {
-    const float ef = Z[L.peoff], ei = Z[L.peoff + 1]; /* log2(ionf E_n0); = MZ_PU (d = 0) if no level */
+    const float ef = Z[c.peoff], ei = Z[c.peoff + 1]; /* log2(ionf E_n0); = MZ_PU (d = 0) if no level */
     /* log2(Unsold) - log2(E_n0), both times ionf; the larger one sets the scale */
     const float d = (ai - ei) + (af - ef);
     const bool ug = d >= 0.0f;
     const float x = ex2(-fabsf(d)); /* branch-free: one ex2 and one lg2 whichever side is larger */
-    const float arg = ug ? fmaf(x, sm, 1.0f) : x + sm;
+    const float arg = ug ? fmaf(x, t.sm, 1.0f) : x + t.sm;
     af = (ug ? af : ef) + lg2(arg);
     ai = ug ? ai : ei;
   }
-  const float Ai = ai + L.lawi, Af = (L.law + ls) + af;
+  const float Ai = ai + c.lawi, Af = (c.law + t.ls) + af;
   /* H- bound-free (c_o :318-322) */
-  const float Bi = Z[MZ_LHM + 1] + L.lsi_, Bf = (ls + Z[MZ_LHM]) + L.ls;
+  const float Bi = Z[MZ_LHM + 1] + c.lsi, Bf = (t.ls + Z[MZ_LHM]) + c.ls;
   /* H- free-free (c_o :337-339): log2(ionf ne k T) + (f1 + f2 lgt + f3 lgt^2 - 26) log2(10) */
-  const float Ci = Z[MZ_LAFF + 1] + L.fci, Cf = (Z[MZ_LAFF] + L.fc) + (L.f2 * Z[MZ_LGT] + L.f3 * Z[MZ_LGT2]);
+  const float Ci = Z[MZ_LAFF + 1] + c.fci, Cf = (Z[MZ_LAFF] + c.fc) + t.ff;
   const float Di = Z[MZ_LESC + 1], Df = Z[MZ_LESC];
   /* scale 2^mi, mi the largest integer part: each 2^(term - mi) = ex2((int diff, exact) + frac) */
   const float mi = fmaxf_(fmaxf_(Ai, Bi), fmaxf_(Ci, Di));
   const float eA = ex2((Ai - mi) + Af), eB = ex2((Bi - mi) + Bf), eC = ex2((Ci - mi) + Cf), eD = ex2((Di - mi) + Df);
-  const float S4 = (eA + eB) + (eC + eD); /* sum per H / 2^mi */
-  const float S3 = (eA + eB) + eC;        /* absorption part (no Thomson) */
+  const float eAB = eA + eB;
+  const float S4 = eAB + (eC + eD); /* sum per H / 2^mi */
+  const float S3 = eAB + eC;        /* absorption part (no Thomson) */
   /* per-mass scale of S4 and S3: 2^(Xi + Xf) */
   const float Xi = mi + kLog2mp1I, Xf = kLog2mp1F;
+  const float lrhoi = Z[MZ_LRHO + 1], lrhof = Z[MZ_LRHO];
   /* kappa and kappa_rad are one lg2 each of a linear combination scaled to M = max(X, extra
    * term); of the two scale factors one is exactly 1.  1 - omega = kappa_abs / kappa_rad. */
   Opac32 o;
   float Mi, Mf, es, ex, num, den, lin;
-  if (Z[MZ_NEUTRAL] != 0.0f) { /* c_o :262-268: kappa = rho (2 kr0 + kHff/mp), kappa_rad = kr0 + kHff/mp */
-    const float gff = 1.0f + L.gff * (Z[MZ_TH1L] * L.chi1 + 0.5f);
-    const float Hi = Z[MZ_LIONFEF + 1] + L.lal0wi, Hf = ((ls + Z[MZ_LIONFEF]) + L.lal0w) + lg2(gff); /* kHff mp1 */
+  if (f2bits(Z[MZ_FLAGS]) & MZF_NEUTRAL) { /* c_o :262-268: kappa = rho (2 kr0 + kHff/mp), kappa_rad = kr0 + kHff/mp */
+    const float Hi = Z[MZ_LIONFEF + 1] + c.lal0wi, Hf = ((t.ls + Z[MZ_LIONFEF]) + c.lal0w) + t.lgff; /* kHff mp1 */
     const float dx = (Xi - Hi) + (Xf - Hf);
     const bool xs = dx >= 0.0f;
     const float e = ex2(-fabsf(dx));
@@ -410,13 +469,13 @@ MX_HD Opac32 opacity(const Rec &Z, const Lam32 &L) {
     num = S3 * es + ex;
     den = S4 * es + ex;
   } else { /* c_o :270-275, bremsstrahlung :281-300: kappa = rho kr0 + kb, kappa_rad = 2 kr0 + kb/rho */
-    const float y = 5.960f - 0.551328895f * (L.lnnu9 + Z[MZ_LNTPOW]); /* sqrt(3)/pi */
+    const float y = 5.960f - 0.551328895f * (L(ML_LNNU9) + Z[MZ_LNTPOW]); /* sqrt(3)/pi */
     const float gaunt = kLn2_f * lg2(ex2(y * kLog2e_f) + 2.71828183f);
-    const float xh = L.hnuk * Z[MZ_T1];
+    const float xh = L(ML_HNUK) * Z[MZ_T1];
     const float lq = (xh > 30.0f) ? 0.0f : log2_one_minus_exp2neg(xh * kLog2e_f); /* log2(1 - e^-xh) */
     /* log2(kb / rho) = log2(369234910.67735046 ne n T^-1/2 nu^-3 (1 - e^-xh) gaunt / rho) */
-    const float Ki = ((Z[MZ_LZ2 + 1] - L.l3nui) - Z[MZ_LRHO + 1]) + kBremsI;
-    const float Kf = ((Z[MZ_LZ2] - L.l3nu) - Z[MZ_LRHO]) + ((lq + lg2(gaunt)) + kBremsF);
+    const float Ki = ((Z[MZ_LZ2 + 1] - L(ML_L3NU + 1)) - lrhoi) + kBremsI;
+    const float Kf = ((Z[MZ_LZ2] - L(ML_L3NU)) - lrhof) + ((lq + lg2(gaunt)) + kBremsF);
     const float dx = (Xi - Ki) + (Xf - Kf);
     const bool xs = dx >= 0.0f;
     const float e = ex2(-fabsf(dx));
@@ -428,25 +487,17 @@ MX_HD Opac32 opacity(const Rec &Z, const Lam32 &L) {
     num = (2.0f * S3 + eD) * es + ex;
     den = 2.0f * S4 * es + ex;
   }
-  o.lki = Z[MZ_LRHO + 1] + Mi;
-  o.lkf = (Z[MZ_LRHO] + Mf) + lg2(lin);
+  o.lki = lrhoi + Mi;
+  o.lkf = (lrhof + Mf) + lg2(lin);
   const float w = num * rcp(den);
   o.omw = w > 1.0f ? 1.0f : (w < 1.17549435e-38f ? 1.17549435e-38f : w); /* [2^-126, 1] */
-  /* Planck function (c_o :399-407): S = sw5 / (e^x - 1), x = dft1/lambda_cm clamped at 308.
-   * t2 = x log2(e) = (dft1_hi + dft1_lo)(ch + cl) as hi + lo (FMA two-product). */
-  const float dh = Z[MZ_DFT1], dl = Z[MZ_DFT1L];
-  float p = dh * L.ch;
-  float lo = fmaf(dh, L.ch, -p) + (dh * L.cl + dl * L.ch);
-  if (p > kT2Clamp) {
-    p = kT2Clamp;
-    lo = kT2ClampLo;
-  }
-  const float ti = floorf(p);
-  const float tf = (p - ti) + lo; /* t2 = ti + tf */
-  const float lm = (p > 40.0f) ? 0.0f : log2_one_minus_exp2neg(p);
-  o.lSi = (L.lsi - ti) + pow2_expo(o.omw);
-  o.lSf = (L.lsf - tf) - lm;
+  o.lSi = t.Si + pow2_expo(o.omw);
+  o.lSf = t.Sf;
   return o;
+}
+template <class Rec, class LA>
+MX_HD Opac32 opacity(const Rec &Z, const LA &L) {
+  return opacity(Z, L, lam_point(L), tfac(Z, L));
 }
 
 /* ---- extended-exponent numbers: value = m * 2^e, m FP32, e int ------------------------ */
@@ -454,24 +505,6 @@ struct XF {
   float m;
   int e;
 };
-MX_HD int f2bits(float f) {
-#ifdef __CUDA_ARCH__
-  return __float_as_int(f);
-#else
-  int i;
-  memcpy(&i, &f, 4);
-  return i;
-#endif
-}
-MX_HD float bits2f(int i) {
-#ifdef __CUDA_ARCH__
-  return __int_as_float(i);
-#else
-  float f;
-  memcpy(&f, &i, 4);
-  return f;
-#endif
-}
 /* 2^k as a float for -126 <= k <= 127; +0 below (k = -127 is the zero bit pattern). */
 MX_HD float pow2f(int k) { return bits2f(((k < -127 ? -127 : k) + 127) << 23); }
 /* renormalise so that |m| is in [1, 2) with bit operations: the exponent field moves into e.
@@ -516,7 +549,7 @@ MX_HD double xtod(XF x) {
   return (double)x.m * oco_u2d((uint64_t)(int64_t)(x.e + 1023) << 52);
 }
 
-/* 1/kappa (> 0) and an XF u = m 2^e with m in [1, 2) in two 32-bit words: w1 = 1/kappa with
+/* kappa (> 0) and an XF u = m 2^e with m in [1, 2) in two 32-bit words: w1 = kappa with
  * bit 9 of e + 512 in its sign bit, w2 = m's 23 fraction bits with bits 0-8 of e + 512 in its
  * sign and exponent field.  Returns whether the pair fits (e in [-512, 511], m normal in
  * [1, 2)); unpacking a fitting pair gives the same bits back. */

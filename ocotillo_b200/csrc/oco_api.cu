@@ -75,7 +75,6 @@ extern "C" int oco_create(oco_ctx **out, int device) {
     oco_destroy(c);
     return code;
   }
-  if (const char *r = getenv("OCO_REFERENCE_STORES")) c->ref_transpose = strcmp(r, "direct") != 0;
   if (const char *g = getenv("OCO_WORKSPACE_GB")) {
     double gb = atof(g);
     if (gb > 0.0) c->budget_bytes = std::max<size_t>((size_t)(gb * (1ull << 30)), 1);
@@ -96,9 +95,6 @@ extern "C" void oco_destroy(oco_ctx *c) {
   c->trapw.release();
   c->pil.release();
   c->scratch.release();
-  c->tmpU.release();
-  c->tmpK.release();
-  c->tmpV.release();
   c->work.release();
   c->status.release();
   c->rbits.release();
@@ -315,12 +311,6 @@ static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz,
   return OCO_OK;
 }
 
-/* Reference-layout outputs of a device solve go through lambda-fastest temporaries and a
- * tiled transpose (coalesced stores) unless disabled or pointless (grey / few wavelengths). */
-static bool uses_transpose(const oco_ctx *c, const oco_params *p, bool u, bool k, bool v) {
-  return p->form == OCO_FORM_MIXED && c->ref_transpose && p->layout == OCO_LAYOUT_REFERENCE && !p->lgrey && p->nw >= 8 && (u || k || v);
-}
-
 /* Bytes of the per-(column, z) record of a form: the FP64 pillar or the mixed record. */
 static size_t record_bytes(int form) {
   return form == OCO_FORM_MIXED ? MIXED_ZN * sizeof(float) : NF * sizeof(double);
@@ -336,9 +326,6 @@ static int64_t chunk_columns(oco_ctx *c, const oco_params *p, bool host_path, bo
                          (planes ? 2 : 0);
     per_col += 2 * ((size_t)p->nz * 2 + (size_t)p->nw * per_w) * sizeof(double);
   }
-  if (!host_path && uses_transpose(c, p, u, k, v)) /* lambda-fastest temporaries of the chunk */
-    per_col += (size_t)p->nw * ((u ? (size_t)(p->nz + 6) : 0) + (k ? (size_t)p->nz : 0) + (v ? (size_t)p->nz : 0)) *
-               sizeof(double);
   int64_t ch = (int64_t)std::max<size_t>(1, c->budget_bytes / per_col);
   if (p->form == OCO_FORM_MIXED) /* the FP64 re-solve indexes a chunk's flagged items with 32-bit slots */
     ch = std::min<int64_t>(ch, std::max<int64_t>(1, INT32_MAX / p->nw));
@@ -548,10 +535,9 @@ static void fill_strides(SolveArgs &a, const oco_params *p, int layout, int64_t 
 }
 
 /* One chunk [c0, c0 + nb) of a device solve into the caller's arrays (whole-block strides, layout
- * p->layout); reference-layout U, kappa, V go through lambda-fastest temporaries and a transpose. */
+ * p->layout). */
 static int device_chunk(oco_ctx *c, const oco_params *p, const double *rho, const double *T, int64_t c0, int64_t nb,
                         double *U, double *kappa, double *V, double *Vtop, double *Vbot, cudaStream_t s) {
-  const int64_t ncol = (int64_t)p->nx * p->ny;
   SolveArgs a{};
   a.nz = p->nz;
   a.nw = p->nw;
@@ -559,38 +545,14 @@ static int device_chunk(oco_ctx *c, const oco_params *p, const double *rho, cons
   a.dz1 = 1.0 / p->dz;
   a.dz2 = p->dz * p->dz;
   a.sigma_grey = p->sigma_grey;
-  if (!uses_transpose(c, p, U != nullptr, kappa != nullptr, V != nullptr)) {
-    fill_strides(a, p, p->layout, ncol);
-    a.U = U;
-    a.K = kappa;
-    a.V = V;
-    a.Vtop = Vtop;
-    a.Vbot = Vbot;
-    a.c_off = c0;
-    return run_chunk(c, p, rho + c0 * p->nz, T + c0 * p->nz, nb, a, s);
-  }
-  const int nz = p->nz, nw = p->nw, mz = nz + 6;
-  const int64_t items = nb * nw;
-  if (U) CU(c->tmpU.ensure((size_t)items * mz * sizeof(double)));
-  if (kappa) CU(c->tmpK.ensure((size_t)items * nz * sizeof(double)));
-  if (V) CU(c->tmpV.ensure((size_t)items * nz * sizeof(double)));
-  a.layout = OCO_LAYOUT_LAMBDA_FASTEST;
-  a.ld_col = ncol; /* emergent planes: caller's plane, offset below */
-  a.c_off = 0;
-  a.U_zs = a.K_zs = a.V_zs = items;
-  a.U_is = a.K_is = a.V_is = 1;
-  a.U = U ? c->tmpU.as<double>() : nullptr;
-  a.K = kappa ? c->tmpK.as<double>() : nullptr;
-  a.V = V ? c->tmpV.as<double>() : nullptr;
-  a.Vtop = Vtop ? Vtop + c0 : nullptr;
-  a.Vbot = Vbot ? Vbot + c0 : nullptr;
-  int rc = run_chunk(c, p, rho + c0 * p->nz, T + c0 * p->nz, nb, a, s);
-  if (rc) return rc;
-  if (U) CU(launch_lambda_to_reference(c->tmpU.as<double>(), items, U, ncol, c0, nb, mz, nw, c->num_sms, s));
-  if (kappa) CU(launch_lambda_to_reference(c->tmpK.as<double>(), items, kappa, ncol, c0, nb, nz, nw, c->num_sms, s));
-  if (V) CU(launch_lambda_to_reference(c->tmpV.as<double>(), items, V, ncol, c0, nb, nz, nw, c->num_sms, s));
-  c->launches += (U ? 1 : 0) + (kappa ? 1 : 0) + (V ? 1 : 0);
-  return OCO_OK;
+  fill_strides(a, p, p->layout, (int64_t)p->nx * p->ny);
+  a.U = U;
+  a.K = kappa;
+  a.V = V;
+  a.Vtop = Vtop;
+  a.Vbot = Vbot;
+  a.c_off = c0;
+  return run_chunk(c, p, rho + c0 * p->nz, T + c0 * p->nz, nb, a, s);
 }
 
 extern "C" int oco_solve_block_device(oco_ctx *c, const oco_params *p, const double *rho, const double *T,
