@@ -209,7 +209,7 @@ struct Opac {
 template <bool STABLE>
 __device__ __forceinline__ void settle_opac(Opac &o) {
   if (!o.wok) {
-    const double q = o.num / o.kr;
+    const double q = div_call(o.num, o.kr);
     o.w = STABLE ? q : 1.0 - q;
     o.wok = 1;
   }
@@ -271,12 +271,12 @@ __device__ __forceinline__ void pow10_pow10_exp(double y1, double y2, double x3,
 }
 
 template <bool STABLE, class R, class LM, class TC>
-__device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc) {
+__device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc, bool fresh = false) {
   const double2 em = P.pair(F_ESCM);
   const int flags = __double2loint(em.y);
   const bool neutral = flags & FLAG_NEUTRAL;
   TFac t;
-  if (flags & FLAG_SAME_T) {
+  if ((flags & FLAG_SAME_T) && !fresh) { /* fresh: tc does not hold the level below */
     t = tc.get();
   } else {
     double damping = P[F_DFT1] * L.wcm1();
@@ -351,20 +351,26 @@ template <class ST>
 __device__ __forceinline__ double scratch_o1(double a) {
   if (!ST::KAPPA_REVERSE) return a;
   double y = div_recip(a);
-  if (!op_ok(a)) y = 1.0 / a;
+  if (!op_ok(a)) y = div_call(1.0, a);
   return y;
 }
 
-constexpr int RING = 4; /* levels of scratch that the stable form's reverse sweep keeps in registers */
+/* The sweeps over stored levels load them in two groups of G (4 or 8) that take turns: one is used
+ * while the other is in flight.  (A ring whose slots are reloaded one by one waits a full latency
+ * per level: a warp has six scoreboards and waits for all loads that share one.)  4 where registers
+ * are short and many warps run, 8 where a warp is alone with the latency (k_chain, 16 columns x 500
+ * x 250: 455 us with a ring of 8, 281 us with groups of 4, 277 us with 8). */
+constexpr int RG = 4, RG_ALONE = 8;
+/* Shorter columns take the sweeps' rolled loops level by level: fetching straight-line code that runs
+ * once or twice costs more than the loads' latency. */
+constexpr int LONG_NZ = 48;
 
 /* The reverse sweep of one item (back-substitution, tridag :43-45; ghost zones :49-62; flux
  * :96-109) from the forward sweep's last u and its scratch (gamma, u, kap: 1/kappa or kappa, and, stable form, q at
  * stride it.ss()), storing U, V (and kappa) through st and the emergent fluxes through the item
- * accessor.  PF: the scratch was written long before (by another kernel) and few warps run, so its
- * loads are DRAM latency: blocks of 8 levels are loaded ahead of the serial chain and the next
- * blocks prefetched into L2 (the block solves keep PF off: their scratch is recent and many warps
- * hide its latency). */
-template <int FORM, bool PF = false, class IT, class ST>
+ * accessor.  PF: the scratch was written long before (by another kernel) and few warps run, so the
+ * next groups are prefetched into L2 as well. */
+template <int FORM, int G = RG, bool PF = false, class IT, class ST>
 __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double u, const double *__restrict__ gam,
                                               const double *__restrict__ uu, const double *__restrict__ kap,
                                               const double *__restrict__ qs, ST &st) {
@@ -407,7 +413,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       const double op = kap[(n - 1) * ss];
       vtop = flux(op);
       st.push(6, n - 1, Un, vtop, op); /* U_{n-4}, V_{n-1} */
-      st.group(n - 1, 7);
+      st.template group<false>(n - 1, 7);
     }
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = u; /* the four lowest U seen so far */
     auto step = [&](int slot, int k, double uf, double qk, double gk1, double op) {
@@ -418,68 +424,64 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       st.push(slot, 3 + k, Un, flux(op), op);
     };
     int k = n - 5;
-    if (PF) {
-      for (; k >= 7; k -= 8) { /* scratch loads of 8 steps hoisted off the serial chain */
-        double ub[8], qb[8], gb[8], ob[8];
-        for (int q = 16; q < 24 && k - q >= 0; q++) { /* the block after next */
-          prefetch_l2(&uu[(k - q) * ss]);
-          prefetch_l2(&qs[(k - q) * ss]);
-          prefetch_l2(&gam[(k - q + 1) * ss]);
-          prefetch_l2(&kap[(k - q + 3) * ss]);
-        }
+    struct Lev {
+      double u, q, g, o;
+    } A[G], B[G];
+    auto load = [&](Lev *l, int k0) {
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          ub[q] = uu[(k - q) * ss];
-          qb[q] = qs[(k - q) * ss];
-          gb[q] = gam[(k - q + 1) * ss];
-          ob[q] = kap[(k - q + 3) * ss];
-        }
-#pragma unroll
-        for (int q = 0; q < 8; q++) step(q, k - q, ub[q], qb[q], gb[q], ob[q]);
-        st.group(3 + k - 7, 8);
+      for (int i = 0; i < G; i++) {
+        const int kl = max(k0 - i, 0);
+        l[i] = Lev{uu[kl * ss], qs[kl * ss], gam[(kl + 1) * ss], kap[(kl + 3) * ss]};
       }
-    } else if (k >= 7) {
-      /* the scratch of RING levels in registers: a level's slot is reloaded for RING levels
-       * further down as soon as it is used, so that loads stay in flight throughout */
-      double ub[RING], qb[RING], gb[RING], ob[RING];
+    };
+    auto steps = [&](const Lev *l, int slot, int k0) { /* G levels */
 #pragma unroll
-      for (int q = 0; q < RING; q++) {
-        ub[q] = uu[(k - q) * ss];
-        qb[q] = qs[(k - q) * ss];
-        gb[q] = gam[(k - q + 1) * ss];
-        ob[q] = kap[(k - q + 3) * ss];
-      }
-      for (; k >= 7; k -= 8) {
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const int r = q % RING, kn = max(k - RING - q, 0);
-          step(q, k - q, ub[r], qb[r], gb[r], ob[r]);
-          ub[r] = uu[kn * ss];
-          qb[r] = qs[kn * ss];
-          gb[r] = gam[(kn + 1) * ss];
-          ob[r] = kap[(kn + 3) * ss];
+      for (int i = 0; i < G; i++) step(slot + i, k0 - i, l[i].u, l[i].q, l[i].g, l[i].o);
+      if (slot + G == 8) st.template group<true>(3 + k0 - G + 1, 8);
+    };
+    load(A, k);
+#pragma unroll 1
+    for (; k >= 2 * G - 1 && nz >= LONG_NZ; k -= 2 * G) {
+      if (PF)
+        for (int p = 4 * G; p < 6 * G && k - p >= 0; p++) { /* two pairs of groups ahead into L2 */
+          prefetch_l2(&uu[(k - p) * ss]);
+          prefetch_l2(&qs[(k - p) * ss]);
+          prefetch_l2(&gam[(k - p + 1) * ss]);
+          prefetch_l2(&kap[(k - p + 3) * ss]);
         }
-        st.group(3 + k - 7, 8);
-      }
+      load(B, k - G);
+      steps(A, 0, k);
+      load(A, k - 2 * G);
+      steps(B, G % 8, k - G);
     }
+    /* the remaining levels, then the ghosts: 0, 1, 2 levels above the bottom, whose differences
+     * D_{-1}, D_{-2}, D_{-3} mirror D_0, D_1, D_2; one level loaded ahead */
+    double g0 = 0.0, g1 = 0.0, g2 = 0.0, D1 = 0.0, D2 = 0.0, Dn = 0.0;
+    Lev x = A[0];
     int q = 0;
-    for (; k >= 0; k--) {
-      step(q, k, uu[k * ss], qs[k * ss], gam[(k + 1) * ss], kap[(k + 3) * ss]);
-      if (++q == 8) {
-        st.group(3 + k, 8);
-        q = 0;
+#pragma unroll 1
+    for (; k >= -3; k--) {
+      if (k >= 0) {
+        const int kn = max(k - 1, 0);
+        const Lev nx{uu[kn * ss], qs[kn * ss], gam[(kn + 1) * ss], kap[(kn + 3) * ss]};
+        step(q, k, x.u, x.q, x.g, x.o);
+        x = nx;
+      } else {
+        if (k == -1) {
+          g2 = 2.0 * U0 - U1;
+          g1 = 2.0 * U0 - U2;
+          g0 = 2.0 * U0 - U3;
+          Dn = d0;
+          D1 = d1;
+          D2 = d2;
+        }
+        d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = k == -1 ? Dn : (k == -2 ? D1 : D2);
+        const double op = kap[(3 + k) * ss];
+        vbot = flux(op);
+        st.push(q, 3 + k, k == -1 ? g2 : (k == -2 ? g1 : g0), vbot, op);
       }
-    }
-    const double g[3] = {2.0 * U0 - U3, 2.0 * U0 - U2, 2.0 * U0 - U1}; /* ghosts 0, 1, 2 */
-    const double D[3] = {d2, d1, d0};
-#pragma unroll
-    for (int j = 2; j >= 0; j--) { /* ghost differences D_{-1}, D_{-2}, D_{-3} mirror D_0, D_1, D_2 */
-      d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D[j];
-      const double op = kap[j * ss];
-      vbot = flux(op);
-      st.push(q, j, g[j], vbot, op);
       if (++q == 8) {
-        st.group(j, 8);
+        st.template group<false>(3 + k, 8);
         q = 0;
       }
     }
@@ -507,7 +509,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       const double op = kap[(n - 1) * ss];
       vtop = flux(op);
       st.push(6, n - 1, u4, vtop, op);
-      st.group(n - 1, 7);
+      st.template group<false>(n - 1, 7);
     }
     auto step = [&](int slot, int k, double uk, double gk1, double op) {
       double Uk = uk - gk1 * w0;
@@ -515,43 +517,54 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       st.push(slot, 3 + k, Uk, flux(op), op);
     };
     int kk = n - 5;
-    if (kk >= 7) { /* the scratch of 8 levels in registers, as above */
-      double ub[8], gb[8], ob[8];
+    struct Lev {
+      double u, g, o;
+    } A[G], B[G];
+    auto load = [&](Lev *l, int k0) {
 #pragma unroll
-      for (int q = 0; q < 8; q++) {
-        ub[q] = uu[(kk - q) * ss];
-        gb[q] = gam[(kk - q + 1) * ss];
-        ob[q] = kap[(kk - q + 3) * ss];
+      for (int i = 0; i < G; i++) {
+        const int kl = max(k0 - i, 0);
+        l[i] = Lev{uu[kl * ss], gam[(kl + 1) * ss], kap[(kl + 3) * ss]};
       }
-      for (; kk >= 7; kk -= 8) {
+    };
+    auto steps = [&](const Lev *l, int slot, int k0) { /* G levels */
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          const int kn = max(kk - 8 - q, 0);
-          step(q, kk - q, ub[q], gb[q], ob[q]);
-          ub[q] = uu[kn * ss];
-          gb[q] = gam[(kn + 1) * ss];
-          ob[q] = kap[(kn + 3) * ss];
-        }
-        st.group(3 + kk - 7, 8);
-      }
+      for (int i = 0; i < G; i++) step(slot + i, k0 - i, l[i].u, l[i].g, l[i].o);
+      if (slot + G == 8) st.template group<true>(3 + k0 - G + 1, 8);
+    };
+    load(A, kk);
+#pragma unroll 1
+    for (; kk >= 2 * G - 1 && nz >= LONG_NZ; kk -= 2 * G) {
+      load(B, kk - G);
+      steps(A, 0, kk);
+      load(A, kk - 2 * G);
+      steps(B, G % 8, kk - G);
     }
+    /* the remaining levels, then the ghosts, one level loaded ahead */
+    double b0 = 0.0, b1 = 0.0, b2 = 0.0;
+    Lev x = A[0];
     int q = 0;
-    for (; kk >= 0; kk--) {
-      step(q, kk, uu[kk * ss], gam[(kk + 1) * ss], kap[(kk + 3) * ss]);
-      if (++q == 8) {
-        st.group(3 + kk, 8);
-        q = 0;
+#pragma unroll 1
+    for (; kk >= -3; kk--) {
+      if (kk >= 0) {
+        const int kn = max(kk - 1, 0);
+        const Lev nx{uu[kn * ss], gam[(kn + 1) * ss], kap[(kn + 3) * ss]};
+        step(q, kk, x.u, x.g, x.o);
+        x = nx;
+      } else {
+        if (kk == -1) {
+          b2 = 2.0 * w0 - w1;
+          b1 = 2.0 * w0 - w2;
+          b0 = 2.0 * w0 - w3;
+        }
+        const double b = kk == -1 ? b2 : (kk == -2 ? b1 : b0);
+        w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b;
+        const double op = kap[(3 + kk) * ss];
+        vbot = flux(op);
+        st.push(q, 3 + kk, b, vbot, op);
       }
-    }
-    const double b[3] = {2.0 * w0 - w3, 2.0 * w0 - w2, 2.0 * w0 - w1}; /* ghosts 0, 1, 2 */
-#pragma unroll
-    for (int j = 2; j >= 0; j--) {
-      w6 = w5; w5 = w4; w4 = w3; w3 = w2; w2 = w1; w1 = w0; w0 = b[j];
-      const double op = kap[j * ss];
-      vbot = flux(op);
-      st.push(q, j, b[j], vbot, op);
       if (++q == 8) {
-        st.group(j, 8);
+        st.template group<false>(3 + kk, 8);
         q = 0;
       }
     }
@@ -657,29 +670,102 @@ template <int FORM>
 __device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, const Opac &nxt, double dz2, Elim &n,
                                             RowOut &r, bool &bad) {
   const double op = cur.op, o2 = op * op;
-  r.o1 = 1.0 / op;
+  r.o1 = div_call(1.0, op);
   n.kh = 0.5 * (nxt.op + op);
-  const double aa = o2 / e.kh, cc = o2 / n.kh;
+  const double aa = div_call(o2, e.kh), cc = div_call(o2, n.kh);
   const double z3 = (dz2 * (op * (op * op))) * cur.w;
   const double dd = -(cur.S * z3);
   n.c = cc;
   double bet;
   if (FORM == 0) {
     const double bb = -((aa + cc) + z3);
-    r.g = e.c / e.d;
+    r.g = div_call(e.c, e.d);
     r.q = 0.0;
     n.h = 0.0;
     n.d = bet = bb - aa * r.g;
   } else {
-    r.g = -(e.c / e.d);
-    r.q = e.h / e.d;
-    n.h = z3 + (aa * e.h) / e.d;
+    r.g = -div_call(e.c, e.d);
+    r.q = div_call(e.h, e.d);
+    n.h = z3 + div_call(aa * e.h, e.d);
     n.d = cc + n.h;
     bet = -n.d;
   }
   if (bet == 0.0) bad = true;
-  n.u = (dd - aa * e.u) / bet;
+  n.u = div_call(dd - aa * e.u, bet);
   elim_checks<FORM>(n, cur.ook & nxt.ook);
+}
+
+/* The elimination over rows whose coefficients are given (the split block solve and the mixed form's
+ * re-solve): state between two rows, d as in Elim. */
+struct Chain {
+  double c, h, d, yd, u;
+  int ok; /* c, (h) and d pass the checks */
+};
+template <int FORM>
+__device__ __forceinline__ void chain_checks(Chain &e) {
+  e.yd = div_recip(e.d);
+  e.ok = div_b_ok(e.d) & div_a_ok(e.c);
+  if (FORM == 1) e.ok &= div_a_ok(e.h);
+}
+/* Row 0: x is its diagonal (plain) or h (stable). */
+template <int FORM>
+__device__ __forceinline__ Chain chain_first(double x, double cc, double dd, bool &bad) {
+  Chain e;
+  e.c = cc;
+  e.h = FORM == 0 ? 0.0 : x;
+  e.d = FORM == 0 ? x : cc + x;
+  const double bet = FORM == 0 ? x : -e.d;
+  if (bet == 0.0) bad = true;
+  e.u = dd / bet;
+  chain_checks<FORM>(e);
+  return e;
+}
+/* A row above: x is its diagonal (plain) or its diagonal excess (stable).  The serial chain is one
+ * reciprocal, one quotient and two operations per row (plain; stable: one more quotient's), where
+ * the operator's divisions put 2 x 124 cycles and their branches on it. */
+template <int FORM>
+__device__ __forceinline__ void chain_step(Chain &e, double aa, double x, double cc, double dd, double &g, double &q,
+                                           bool &bad) {
+  Chain n;
+  const double num = dd - aa * e.u;
+  int ok = e.ok & div_a_ok(num);
+  n.c = cc;
+  if (FORM == 0) {
+    g = div_quot(e.c, e.d, e.yd);
+    q = n.h = 0.0;
+    n.d = x - aa * g;
+    n.yd = div_recip(n.d);
+    n.u = div_quot(num, n.d, n.yd);
+  } else {
+    const double ah = aa * e.h;
+    g = -div_quot(e.c, e.d, e.yd);
+    q = div_quot(e.h, e.d, e.yd);
+    n.h = x + div_quot(ah, e.d, e.yd);
+    n.d = cc + n.h;
+    n.yd = div_recip(n.d);
+    n.u = -div_quot(num, n.d, n.yd);
+    ok &= div_a_ok(ah);
+  }
+  const int dok = div_b_ok(n.d);
+  n.ok = dok & div_a_ok(cc);
+  if (FORM == 1) n.ok &= div_a_ok(n.h);
+  if (!(ok & dok)) { /* as above with the operator */
+    double bet;
+    if (FORM == 0) {
+      g = div_call(e.c, e.d);
+      n.d = bet = x - aa * g;
+    } else {
+      g = -div_call(e.c, e.d);
+      q = div_call(e.h, e.d);
+      n.h = x + div_call(aa * e.h, e.d);
+      n.d = cc + n.h;
+      bet = -n.d;
+    }
+    if (bet == 0.0) bad = true;
+    n.u = div_call(num, bet);
+    chain_checks<FORM>(n);
+  }
+  e = n;
 }
 
 /* Levels are bound by dependent FP64 latency, not by a pipe: a warp alone on its SM needed as long
@@ -689,9 +775,8 @@ __device__ __forceinline__ void center_slow(const Elim &e, const Opac &cur, cons
  * (without the kept factors: AGN grid plain 11.84 -> 11.05 ms, 16 columns x 500 x 250 stable
  * 1.03 -> 0.80 ms; with them 7.2 and 0.49 ms).  The GPU then runs this kernel at its 1000 W limit
  * (1.82 GHz), so what counts is instructions per point: records, kept factors and constants are
- * read in 16-byte pairs, the record pointer is advanced instead of computed, and the reverse
- * sweep's loads never pause (ring of levels): 7.48 -> 7.37 ms, 0.49 -> 0.41 ms, batch of 400
- * columns 3.67 -> 3.53 ms.  Not faster: row j's elimination beside the opacity of level j + 2
+ * read in 16-byte pairs and the record pointer is advanced instead of computed: 7.48 -> 7.37 ms,
+ * 0.49 -> 0.41 ms, batch of 400 columns 3.67 -> 3.53 ms.  Not faster: row j's elimination beside the opacity of level j + 2
  * (7.53 ms; 0.39 ms), the exponentials and logarithms behind calls (7.45; 14.5 for 13.6 ms on the
  * warm disk), five blocks per SM at 96 registers (7.8 ms). */
 template <int FORM, bool GREY, class IT, class PA, class LMT, class TC, class ST>

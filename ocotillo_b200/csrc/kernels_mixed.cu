@@ -28,12 +28,8 @@ constexpr int MWARPS = 4;          /* warps per 128-thread block */
 #define MBLOCKS 5 /* resident blocks per SM */
 #endif
 constexpr long long kMSpinLimit = 1ll << 26;
-#ifndef OCO_MIXED_PREFETCH
-#define OCO_MIXED_PREFETCH 4 /* reverse-sweep steps whose scratch loads are issued together */
-#endif
-#ifndef OCO_MIXED_L2_AHEAD
-#define OCO_MIXED_L2_AHEAD 8 /* reverse-sweep steps between the L2 prefetch and the load of a scratch level */
-#endif
+constexpr int MG = 4;              /* reverse sweep: levels per group of scratch loads */
+constexpr int MIXED_L2_AHEAD = 8;  /* reverse sweep: steps between the L2 prefetch and the load of a level */
 
 /* Shared-memory record accessor. */
 struct MRec {
@@ -346,7 +342,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       const float kj = sc.kappa(n - 1);
       vtop = flux(kj);
       st.push(6, n - 1, Uk[2], vtop, (double)kj); /* U_{n-4}, V_{n-1} */
-      st.group(n - 1, 7);
+      st.template group<false>(n - 1, 7);
     }
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = fn; /* the four lowest U seen so far */
     /* kappa ring: r1, r2, r3 = kappa of k+1, k+2, k+3 before step k */
@@ -366,33 +362,39 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       r3 = r2; r2 = r1; r1 = w.y;
     };
     int k = n - 5;
-    constexpr int PF = OCO_MIXED_PREFETCH;
-    static_assert(8 % PF == 0, "groups of 8 levels");
-    for (; k >= 7; k -= 8) {
-#pragma unroll
-      for (int g = 0; g < 8; g += PF) { /* scratch loads of PF steps hoisted off the serial chain */
-        const int kg = k - g;
-        float4 w[PF];
-        /* the PF scratch levels OCO_MIXED_L2_AHEAD steps ahead into L2, one bulk request from lane
-         * 0 (the warp's levels are contiguous; they were written a whole forward sweep ago and
-         * have usually left L2) */
-        if (kg - PF + 1 - OCO_MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0) /* PF levels, one bulk request */
+    /* Scratch levels in two groups of MG that take turns (one in use, one in flight); one bulk request
+     * from lane 0 brings the MG levels MIXED_L2_AHEAD steps further down into L2 (the warp's levels
+     * are contiguous; they were written a whole forward sweep ago and have usually left L2). */
+    if (k >= 7) {
+      float4 A[MG], B[MG];
+      auto load = [&](float4 *w, int k0) {
+        if (k0 - MG + 1 - MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0)
           asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(
-                           sc.level(kg - PF + 1 - OCO_MIXED_L2_AHEAD))),
-                       "r"((uint32_t)(PF * SC::LEVEL))
+                           sc.level(k0 - MG + 1 - MIXED_L2_AHEAD))),
+                       "r"((uint32_t)(MG * SC::LEVEL))
                        : "memory");
 #pragma unroll
-        for (int q = 0; q < PF; q++) w[q] = sc.get(kg - q);
+        for (int i = 0; i < MG; i++) w[i] = sc.get(max(k0 - i, 0));
+      };
+      auto steps = [&](const float4 *w, int slot, int k0) {
 #pragma unroll
-        for (int q = 0; q < PF; q++) step(g + q, kg - q, w[q]);
+        for (int i = 0; i < MG; i++) step(slot + i, k0 - i, w[i]);
+      };
+      load(A, k);
+      for (; k >= 7; k -= 8) {
+        load(B, k - MG);
+        steps(A, 0, k);
+        load(A, k - 8);
+        steps(B, MG, k - MG);
+        st.template group<true>(3 + k - 7, 8);
       }
-      st.group(3 + k - 7, 8);
     }
     int q = 0;
+#pragma unroll 1
     for (; k >= 0; k--) {
       step(q, k, sc.get(k));
       if (++q == 8) {
-        st.group(3 + k, 8);
+        st.template group<false>(3 + k, 8);
         q = 0;
       }
     }
@@ -411,16 +413,15 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       flag = flag || !(Cb <= (double)cond * fabs(37.0 * d0 - 8.0 * d1 + d2));
     }
     /* bottom ghosts f(n1-i) = 2 f(n1) - f(n1+i); ghost differences mirror D_0, D_1, D_2 */
-    const double g[3] = {2.0 * U0 - U3, 2.0 * U0 - U2, 2.0 * U0 - U1}; /* ghosts 0, 1, 2 */
-    const double D[3] = {d2, d1, d0};
-    const float kb[3] = {r1, r2, r3};
-#pragma unroll
+    const double g0 = 2.0 * U0 - U3, g1 = 2.0 * U0 - U2, g2 = 2.0 * U0 - U1, D0 = d0, D1 = d1, D2 = d2;
+#pragma unroll 1
     for (int j = 2; j >= 0; j--) { /* D_{-1} = D_0, D_{-2} = D_1, D_{-3} = D_2 */
-      d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = D[j];
-      vbot = flux(kb[j]);
-      st.push(q, j, g[j], vbot, (double)kb[j]);
+      d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = j == 2 ? D0 : (j == 1 ? D1 : D2);
+      const float kj = j == 2 ? r3 : (j == 1 ? r2 : r1);
+      vbot = flux(kj);
+      st.push(q, j, j == 2 ? g2 : (j == 1 ? g1 : g0), vbot, (double)kj);
       if (++q == 8) {
-        st.group(j, 8);
+        st.template group<false>(j, 8);
         q = 0;
       }
     }

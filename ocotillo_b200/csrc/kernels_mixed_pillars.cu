@@ -52,9 +52,10 @@ __device__ __forceinline__ bool same_bits(double a, double b) {
 __global__ void __launch_bounds__(PM_THREADS) k_pillars_mixed(const double *__restrict__ rho,
                                                               const double *__restrict__ T, int64_t n, int nz,
                                                               double fully_ionized_T, float *__restrict__ rec,
-                                                              unsigned *__restrict__ colflag) {
+                                                              unsigned *__restrict__ colflag, const ChunkInit init) {
   __shared__ __align__(16) float s_buf[PM_THREADS / 32][32 * PM_STRIDE];
   const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  chunk_init(init, i, (int64_t)gridDim.x * blockDim.x);
   const int64_t i0 = i - (threadIdx.x & 31);
   if (i0 >= n) return; /* whole warp past the end */
   float r[MZN];
@@ -71,11 +72,11 @@ __global__ void __launch_bounds__(PM_THREADS) k_pillars_mixed(const double *__re
 static_assert(MZN == MIXED_ZN, "mixed record size");
 
 cudaError_t launch_pillars_mixed(const double *rho, const double *T, int64_t ncol, int nz, double fully_ionized_T,
-                                 float *rec, unsigned *colflag, cudaStream_t s) {
+                                 float *rec, unsigned *colflag, const ChunkInit &init, cudaStream_t s) {
   const int64_t n = ncol * nz;
   if (n == 0) return cudaSuccess;
   k_pillars_mixed<<<(unsigned)((n + PM_THREADS - 1) / PM_THREADS), PM_THREADS, 0, s>>>(rho, T, n, nz, fully_ionized_T,
-                                                                                      rec, colflag);
+                                                                                      rec, colflag, init);
   return cudaGetLastError();
 }
 

@@ -339,23 +339,15 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
   const int64_t q0 = S.at(pos, 0);
   double *aa = S.aa + q0, *dd = S.dd + q0, *ee = S.ee + q0;
   const double *cc = S.cc + q0;
-  double h = ee[0];
-  double bet = -(cc[0] + h);
-  bool bad = bet == 0.0;
-  double u = dd[0] / bet;
-  dd[0] = u;
-  double c_prev = cc[0];
+  bool bad = false;
+  Chain e = chain_first<1>(ee[0], cc[0], dd[0], bad);
+  dd[0] = e.u;
   auto step = [&](int j, double a_, double c_, double d_, double e_) {
-    const double den = c_prev + h;
-    const double g = -(c_prev / den);
-    ee[(j - 1) * 32] = h / den; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
-    h = e_ + (a_ * h) / den;
-    bet = -(c_ + h);
-    if (bet == 0.0) bad = true;
-    u = (d_ - a_ * u) / bet;
+    double g, q;
+    chain_step<1>(e, a_, e_, c_, d_, g, q, bad);
+    ee[(j - 1) * 32] = q; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
     aa[j * 32] = g;
-    dd[j * 32] = u;
-    c_prev = c_;
+    dd[j * 32] = e.u;
   };
   int j = 1;
   for (; j + 8 <= nz; j += 8) { /* the coefficients of 8 levels loaded ahead of the serial chain */
@@ -382,7 +374,7 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
     atomicMin(&it.status()[1], it.id());
   }
   LaneStores<false> st = lane_stores(it);
-  solve_reverse<1, true>(it, true, u, aa, dd, S.o1 + q0, ee, st);
+  solve_reverse<1, RG, true>(it, true, e.u, aa, dd, S.o1 + q0, ee, st);
 }
 
 __global__ void __launch_bounds__(REPAIR_THREADS, 6) k_repair_solve(const RepairArgs a) {

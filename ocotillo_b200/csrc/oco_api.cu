@@ -311,16 +311,21 @@ static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz,
   return OCO_OK;
 }
 
-/* Bytes of the per-(column, z) record of a form: the FP64 pillar or the mixed record. */
-static size_t record_bytes(int form) {
-  return form == OCO_FORM_MIXED ? MIXED_ZN * sizeof(float) : NF * sizeof(double);
+/* Bytes per (column, z) that a chunk keeps beside its outputs: the FP64 pillar or the mixed record;
+ * grey transfer has the split solve's rows instead (per column, in tiles of 32). */
+static size_t record_bytes(const oco_params *p) {
+  if (p->lgrey) return 5 * sizeof(double);
+  return p->form == OCO_FORM_MIXED ? MIXED_ZN * sizeof(float) : NF * sizeof(double);
+}
+static cudaError_t ensure_records(oco_ctx *c, const oco_params *p, int64_t ncol) {
+  return p->lgrey ? cudaSuccess : c->pil.ensure((size_t)ncol * p->nz * record_bytes(p));
 }
 
 /* Columns per chunk so that pillars (+ staged outputs on the host path) fit the budget. */
 static int64_t chunk_columns(oco_ctx *c, const oco_params *p, bool host_path, bool u = true, bool k = true,
                              bool v = true, bool planes = true) {
   const int64_t ncol = (int64_t)p->nx * p->ny;
-  size_t per_col = (size_t)p->nz * record_bytes(p->form);
+  size_t per_col = (size_t)p->nz * record_bytes(p);
   if (host_path) { /* two staging sets of the requested outputs */
     const size_t per_w = (u ? (size_t)(p->nz + 6) : 0) + (k ? (size_t)p->nz : 0) + (v ? (size_t)p->nz : 0) +
                          (planes ? 2 : 0);
@@ -337,6 +342,15 @@ int64_t oco_ctx_repair_slots(const oco_ctx *c, int64_t cap) {
   return cap;
 }
 
+/* The counters that the chunk's first kernel sets up (the status once per call). */
+static ChunkInit take_init(oco_ctx *c) {
+  ChunkInit i{};
+  i.work = c->work.as<unsigned long long>();
+  if (c->status_reset) i.status = c->status.as<unsigned long long>();
+  c->status_reset = false;
+  return i;
+}
+
 /* One chunk: pillars + persistent solve. Outputs described by the strides in a. */
 static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, const double *T, int64_t nb,
                            const SolveArgs &a64, cudaStream_t s) {
@@ -351,7 +365,13 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
   float *rec = c->pil.as<float>();
   CU(c->colflag.ensure((size_t)nb * sizeof(unsigned)));
   CU(cudaMemsetAsync(c->colflag.p, 0, (size_t)nb * sizeof(unsigned), s));
-  CU(launch_pillars_mixed(rho, T, nb, p->nz, p->fully_ionized_T, rec, c->colflag.as<unsigned>(), s));
+  const int64_t nwords = (p->nw + 31) / 32;
+  CU(c->rbits.ensure((size_t)nb * nwords * sizeof(unsigned)));
+  ChunkInit init = take_init(c);
+  init.lists = c->stats.as<unsigned long long>() + 1; /* rcount, icount, the re-solve's queue */
+  init.rbits = c->rbits.as<unsigned>();
+  init.nrbits = nb * nwords;
+  CU(launch_pillars_mixed(rho, T, nb, p->nz, p->fully_ionized_T, rec, c->colflag.as<unsigned>(), init, s));
   if (c->prof) {
     CU(cudaEventRecord(e1, s));
     c->ev_pil.emplace_back(e0, e1);
@@ -382,8 +402,6 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
   a.status = c->status.as<unsigned long long>();
   a.repair_cond = c->repair_cond;
   a.colflag = c->colflag.as<unsigned>();
-  const int64_t nwords = (p->nw + 31) / 32;
-  CU(c->rbits.ensure((size_t)nb * nwords * sizeof(unsigned)));
   CU(c->rlist.ensure((size_t)nb * nwords * sizeof(unsigned long long)));
   CU(c->ilist.ensure((size_t)nb * p->nw * sizeof(unsigned long long)));
   CU(c->rslot.ensure((size_t)nb * nwords * 32 * sizeof(int)));
@@ -393,9 +411,6 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
   a.rcount = c->stats.as<unsigned long long>() + 1;
   a.ilist = c->ilist.as<unsigned long long>();
   a.icount = c->stats.as<unsigned long long>() + 2;
-  CU(cudaMemsetAsync(a.rcount, 0, 3 * sizeof(unsigned long long), s)); /* rcount, icount, the re-solve's queue */
-  CU(cudaMemsetAsync(a.rbits, 0, (size_t)nb * nwords * sizeof(unsigned), s));
-  CU(cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s));
   /* the FP64 re-solve of the flagged items (stable form), after the mixed solve */
   RepairArgs r{};
   r.list = a.rlist;
@@ -449,17 +464,25 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
     e3 = c->take_event();
     CU(cudaEventRecord(e0, s));
   }
-  CU(launch_pillars(rho, T, nb, p->nz, p->fully_ionized_T, grey, c->pil.as<double>(), s));
+  const bool split = solve_is_split(grey, nb, p->nw, c->num_sms);
+  const ChunkInit init = take_init(c);
+  if (!grey) CU(launch_pillars(rho, T, nb, p->nz, p->fully_ionized_T, 0, c->pil.as<double>(), init, s));
   if (c->prof) {
     CU(cudaEventRecord(e1, s));
     c->ev_pil.emplace_back(e0, e1);
   }
   int blocks = 0;
-  int rc = prepare_solve(c, p->form, grey, nb * p->nw, p->nz, &blocks);
-  if (rc) return rc;
-  size_t slots = (size_t)blocks * kSolveThreads;
+  if (split) {
+    CU(c->scratch.ensure(split_scratch_doubles(split_tiles(nb, p->nw), p->nz) * sizeof(double)));
+  } else {
+    int rc = prepare_solve(c, p->form, grey, nb * p->nw, p->nz, &blocks);
+    if (rc) return rc;
+  }
+  const size_t slots = (size_t)blocks * kSolveThreads;
   a.pil = c->pil.as<double>();
   a.lam = grey ? nullptr : c->lam.as<double>();
+  a.rho = rho;
+  a.T = T;
   a.ncol = nb;
   a.gam = c->scratch.as<double>();
   a.uu = a.gam + slots * p->nz;
@@ -468,19 +491,23 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
   a.slot_stride = (int64_t)slots;
   a.work = c->work.as<unsigned long long>();
   a.status = c->status.as<unsigned long long>();
-  CU(cudaMemsetAsync(a.work, 0, sizeof(unsigned long long), s));
+  const int form = p->form == OCO_FORM_STABLE ? 1 : 0;
   if (c->prof) CU(cudaEventRecord(e2, s));
-  CU(launch_solve_fp64(a, p->form == OCO_FORM_STABLE ? 1 : 0, grey, blocks, kSolveThreads, s));
+  if (split)
+    CU(launch_solve_split(a, form, grey, grey ? init : ChunkInit{}, s));
+  else
+    CU(launch_solve_fp64(a, form, grey, blocks, kSolveThreads, s));
   if (c->prof) {
     CU(cudaEventRecord(e3, s));
     c->ev_solve.emplace_back(e2, e3);
   }
-  c->launches += 2;
+  c->launches += (grey ? 0 : 1) + (split ? 2 : 1);
   return OCO_OK;
 }
 
 /* status[0] = number of items with a zero pivot, status[1] = smallest such item index. */
 static int reset_status(oco_ctx *c, cudaStream_t s) {
+  c->status_reset = false;
   if (c->status_pending) return OCO_OK; /* accumulate until the pending status is read */
   CU(cudaMemsetAsync(c->status.p, 0, sizeof(unsigned long long), s));
   CU(cudaMemsetAsync(c->status.as<unsigned long long>() + 1, 0xff, sizeof(unsigned long long), s));
@@ -573,8 +600,8 @@ extern "C" int oco_solve_block_device(oco_ctx *c, const oco_params *p, const dou
   }
   const int64_t ncol = (int64_t)p->nx * p->ny;
   const int64_t ch = chunk_columns(c, p, false, U != nullptr, kappa != nullptr, V != nullptr, Vtop || Vbot);
-  CU(c->pil.ensure((size_t)ch * p->nz * record_bytes(p->form)));
-  if ((rc = reset_status(c, s))) return rc;
+  CU(ensure_records(c, p, ch));
+  c->status_reset = !c->status_pending; /* pending: accumulate until it is read */
   for (int64_t c0 = 0; c0 < ncol; c0 += ch) {
     const int64_t nb = std::min(ch, ncol - c0);
     if ((rc = device_chunk(c, p, rho, T, c0, nb, U, kappa, V, Vtop, Vbot, s))) return rc;
@@ -593,7 +620,7 @@ extern "C" int oco_solve_block_device(oco_ctx *c, const oco_params *p, const dou
 int oco_ctx_run_columns(oco_ctx *c, const oco_params *p, const double *rho, const double *T, int64_t c0, int64_t nb,
                         double *U, double *kappa, double *V, double *Vtop, double *Vbot, int max_blocks,
                         cudaStream_t s) {
-  CU(c->pil.ensure((size_t)nb * p->nz * record_bytes(p->form)));
+  CU(ensure_records(c, p, nb));
   c->max_blocks = max_blocks;
   const int rc = device_chunk(c, p, rho, T, c0, nb, U, kappa, V, Vtop, Vbot, s);
   c->max_blocks = 0;
@@ -631,7 +658,7 @@ extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rh
   const int64_t ncol = (int64_t)p->nx * p->ny;
   const int nz = p->nz, nw = p->nw, mz = nz + 6;
   const int64_t ch = chunk_columns(c, p, true, U != nullptr, kappa != nullptr, V != nullptr, Vtop || Vbot);
-  CU(c->pil.ensure((size_t)ch * nz * record_bytes(p->form)));
+  CU(ensure_records(c, p, ch));
   for (auto &st : c->stage) {
     CU(st.rho.ensure((size_t)ch * nz * sizeof(double)));
     CU(st.T.ensure((size_t)ch * nz * sizeof(double)));
@@ -642,7 +669,7 @@ extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rh
     if (Vbot) CU(st.bot.ensure((size_t)ch * nw * sizeof(double)));
   }
   if (c->status_pending && (rc = oco_synchronize(c))) return rc;
-  if ((rc = reset_status(c, c->stream))) return rc;
+  c->status_reset = true;
   SolveArgs a{};
   a.nz = nz;
   a.nw = nw;

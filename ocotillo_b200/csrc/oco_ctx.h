@@ -71,6 +71,7 @@ struct oco_ctx {
   bool prof = false;
   /* device-array calls defer the zero-pivot check to oco_synchronize */
   bool status_pending = false;
+  bool status_reset = false; /* the next chunk's first kernel clears the status (ChunkInit) */
   cudaStream_t status_stream = nullptr;
   oco_params status_params{};  /* the first pending call's, which locate the first bad item */
   bool status_dims_mixed = false; /* pending calls of different nx, ny or nw: no location */

@@ -81,6 +81,32 @@ enum LambdaField {
   NL
 };
 
+/* Counters that the first kernel of a chunk sets up for the ones after it, instead of a memset each
+ * (they cost a small block's launches as much as its kernels do): pointers may be NULL. */
+struct ChunkInit {
+  unsigned long long *work;   /* = 0 */
+  unsigned long long *status; /* = {0, ~0, 0} (once per call) */
+  unsigned long long *lists;  /* [3] = 0: the re-solve's counters */
+  unsigned *rbits;            /* [nrbits] = 0 */
+  int64_t nrbits;
+};
+#ifdef __CUDACC__
+/* Called by every thread of the grid (i its index, n the threads). */
+__device__ __forceinline__ void chunk_init(const ChunkInit &c, int64_t i, int64_t n) {
+  if (i == 0) {
+    if (c.work) c.work[0] = 0ull;
+    if (c.status) {
+      c.status[0] = 0ull;
+      c.status[1] = ~0ull;
+      c.status[2] = 0ull;
+    }
+    if (c.lists) c.lists[0] = c.lists[1] = c.lists[2] = 0ull;
+  }
+  if (c.rbits)
+    for (int64_t k = i; k < c.nrbits; k += n) c.rbits[k] = 0u;
+}
+#endif
+
 /* Arguments of the FP64 solve kernels (plain and stable forms, grey or not). */
 struct SolveArgs {
   const double *pil; /* [ncol][nz][NF] pillars of this chunk */
@@ -107,7 +133,14 @@ struct SolveArgs {
   int64_t slot_stride; /* resident threads the scratch is sized for (each warp's block is 32*nz) */
   unsigned long long *work;   /* persistent-kernel work counter (warp tasks) */
   unsigned long long *status; /* [0] zero-pivot count, [1] first bad item (min), [2] timeout flag */
+  const double *rho, *T;      /* split solve of a grey chunk: its inputs [ncol][nz] */
 };
+/* The split block solve (kernels_fp64.cu: k_rows, k_chain): warp tiles of a chunk, the doubles of its
+ * scratch (SolveArgs::gam) and whether a chunk takes it. */
+int64_t split_tiles(int64_t ncol, int nw);
+inline size_t split_scratch_doubles(int64_t tiles, int nz) { return (size_t)tiles * 32 * (size_t)nz * 5; }
+bool solve_is_split(int grey, int64_t ncol, int nw, int num_sms);
+cudaError_t launch_solve_split(const SolveArgs &a, int form, int grey, const ChunkInit &init, cudaStream_t s);
 
 /* Arguments of the mixed-precision solve kernels. */
 struct MixedArgs {
@@ -289,7 +322,7 @@ void fill_lambda_table(const double *waves, int nw, double *tab);
 
 /* Kernel launchers (defined in kernels_fp64.cu). Return cudaGetLastError(). */
 cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int nz,
-                           double fully_ionized_T, int grey, double *pil, cudaStream_t s);
+                           double fully_ionized_T, int grey, double *pil, const ChunkInit &init, cudaStream_t s);
 cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int nslot_blocks,
                               int threads, cudaStream_t s);
 int solve_fp64_max_blocks_per_sm(int form, int grey, int threads);
@@ -305,7 +338,7 @@ constexpr float MIXED_REPAIR_COND = 100.0f;
 constexpr int MIXED_LN = 29; /* fields of the mixed wavelength table */
 /* colflag[ncol] (cleared by the caller) marks columns to re-solve in FP64 (mx::pillar). */
 cudaError_t launch_pillars_mixed(const double *rho, const double *T, int64_t ncol, int nz, double fully_ionized_T,
-                                 float *rec, unsigned *colflag, cudaStream_t s);
+                                 float *rec, unsigned *colflag, const ChunkInit &init, cudaStream_t s);
 cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s);
 int solve_mixed_max_blocks_per_sm(int threads, int nw); /* occupancy of the kernel used for nw */
 /* Fills tab32[MIXED_LN*nw] from the FP64 table tab[NL*nw]. */

@@ -165,10 +165,6 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
     CUN(cudaMemcpyAsync(lam, g_host_table, (size_t)NL * nw * sizeof(double), cudaMemcpyHostToDevice, s));
   }
   const int rc = drained([&]() -> int {
-    CUN(cudaMemsetAsync(ctr + 1, 0, sizeof(unsigned long long), s));
-    CUN(cudaMemsetAsync(ctr + 2, 0xff, sizeof(unsigned long long), s));
-    CUN(cudaMemsetAsync(ctr + 3, 0, sizeof(unsigned long long), s));
-
     SolveArgs a{};
     a.nz = nz;
     a.nw = nw;
@@ -200,8 +196,10 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
       const int64_t nb = std::min(chunk, ncol - c0);
       a.ncol = nb;
       a.c_off = c0;
-      CUN(launch_pillars(rho + c0 * nz, T + c0 * nz, nb, nz, p->fully_ionized_T, grey, pil, s));
-      CUN(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), s));
+      ChunkInit init{};
+      init.work = ctr;
+      if (c0 == 0) init.status = ctr + 1;
+      CUN(launch_pillars(rho + c0 * nz, T + c0 * nz, nb, nz, p->fully_ionized_T, grey, pil, init, s));
       const int64_t nblk = std::min<int64_t>(blocks, (nb * nw + kThreads - 1) / kThreads);
       CUN(launch_solve_fp64(a, p->form == OCO_FORM_STABLE ? 1 : 0, grey, (int)nblk, kThreads, s));
     }

@@ -80,4 +80,10 @@ OCO_HD int div_b_frac_ok(double b) { return ((div_hi(b) + 1u) & 0xfffffu) != 0u;
 OCO_HD int div_b_ok(double b) { return div_in_range(b, 200, 200) & div_b_frac_ok(b); }
 OCO_HD int div_a_ok(double a) { return div_in_range(a, 760, 480); }
 
+#ifdef __CUDACC__
+/* The operator where a check fails, out of line: the fast paths around it stay small enough for the
+ * instruction caches. */
+static __device__ __noinline__ double div_call(double a, double b) { return a / b; }
+#endif
+
 #endif /* OCO_RECIP_DIV_H */

@@ -60,6 +60,7 @@ struct LaneStores {
     v(m, V);
     if (KREV) k(m, K);
   }
+  template <bool FULL>
   __device__ __forceinline__ void group(int, int) {}
   __device__ __forceinline__ void finish(int) {}
 };
@@ -106,10 +107,10 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
   }
   /* One array's runs after every level above lo (ring slot slo) has been pushed: row r, whose
    * element 0 lies ph elements past a 64-byte boundary, writes levels w .. w + 7 with w the lowest
-   * level >= lo on a boundary.  top: levels above are not stored; masked: some may not be, or
-   * lie below 0, or rows are missing. */
+   * level >= lo on a boundary.  top: levels above are not stored; full: all 8 levels of every
+   * row are. */
   template <class T>
-  __device__ __forceinline__ void runs(const T *a, double *p, int64_t stride, int lo, int slo, int top, bool masked) const {
+  __device__ __forceinline__ void runs(const T *a, double *p, int64_t stride, int lo, int slo, int top, bool full) const {
     if (!p) return;
     const int lane = threadIdx.x & 31, s = lane & 7, r = lane / 8;
     if (ROWS) {
@@ -119,7 +120,7 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
       const T *ae = a + (slo - oe + (slo < oe ? RING_Z : 0)) * RING_ROW + r;
       const T *ao = a + (slo - oo + (slo < oo ? RING_Z : 0)) * RING_ROW + r;
       double *ge = p + lo + oe, *go = p + lo + oo;
-      if (!masked) {
+      if (full) {
 #pragma unroll
         for (int i = 0; i < 8; i++) ((i & 1) ? go : ge)[(int64_t)(4 * i) * stride] = (double)((i & 1) ? ao : ae)[4 * i];
       } else {
@@ -139,23 +140,23 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
       }
     }
   }
-  __device__ __forceinline__ void flush(int lo, int slo) const {
-    const bool masked = lo > nz - 17 || lo < 0 || nrows < 32;
-    __syncwarp();
-    runs(ring->U, U0, us, lo, slo, nz + 5, masked);
-    runs(ring->V, V0, ks, lo, slo, nz - 1, masked);
-    runs(ring->K, K0, ks, lo, slo, nz - 1, masked);
-    __syncwarp();
-  }
-  /* a group of n levels, the lowest lo, is complete */
+  /* a group of n levels, the lowest lo, is complete; FULL: worth the straight-line code for runs
+   * without masks (the main loop's) */
+  template <bool FULL>
   __device__ __forceinline__ void group(int lo, int n) {
-    flush(lo, wrap(base + n - 1));
+    const int slo = wrap(base + n - 1);
+    const bool full = FULL && lo <= nz - 17 && nrows == 32;
+    __syncwarp();
+    runs(ring->U, U0, us, lo, slo, nz + 5, full);
+    runs(ring->V, V0, ks, lo, slo, nz - 1, full);
+    runs(ring->K, K0, ks, lo, slo, nz - 1, full);
+    __syncwarp();
     base = wrap(base + n);
   }
   /* level 0 was the q-th level (from 1) of its group, or q = 0: no group open */
   __device__ __forceinline__ void finish(int q) {
 #pragma unroll 1
-    for (int t = 0; t < 2; t++) group(q - 8 - 8 * t, 8);
+    for (int t = 0; t < 2; t++) group<false>(q - 8 - 8 * t, 8);
   }
 };
 
