@@ -30,6 +30,7 @@ UNITS = [
     ("kernels_repair.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_mixed_pillars.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("oco_api.cu", []),
+    ("host_copy.cu", []),
     ("oco_noalloc.cu", []),
     ("oco_batch.cu", []),
     ("kernels_epilogue.cu", ["-fmad=false"]),
@@ -38,7 +39,7 @@ UNITS = [
 ]
 HOST_UNITS = [("oco_deck.cpp", [])]
 
-HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "fp64_core.h", "recip_div.h", "stores.h", "disk_core.h",
+HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "fp64_core.h", "recip_div.h", "stores.h", "host_copy.h", "disk_core.h",
            "batch_layout.h", "fortran_records.h"]
 
 

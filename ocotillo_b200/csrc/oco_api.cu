@@ -103,6 +103,7 @@ extern "C" void oco_destroy(oco_ctx *c) {
   c->stats.release();
   c->colflag.release();
   c->rlist.release();
+  c->host_copy.release();
   for (auto &s : c->stage) {
     s.rho.release();
     s.T.release();
@@ -648,8 +649,34 @@ int oco_ctx_full_blocks(oco_ctx *c, int form, int grey) {
   return bps * c->num_sms;
 }
 
-extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rho, const double *T, double *U,
-                               double *kappa, double *V, double *Vtop, double *Vbot) {
+/* Copies a finished chunk's outputs [c0, c0 + nb) from its staging set into the host arrays on the
+ * copy stream: pinned arrays by DMA (asynchronous), pageable ones through the context's pinned
+ * slots (complete on return). */
+static int copy_out(oco_ctx *c, const oco_params *p, Stage &st, int64_t c0, int64_t nb, double *U, double *kappa,
+                    double *V, double *Vtop, double *Vbot, const bool *pageable) {
+  const int64_t ncol = (int64_t)p->nx * p->ny;
+  struct {
+    double *host;
+    const DevBuf *dev;
+    int64_t len;
+  } const arr[5] = {{U, &st.U, p->nz + 6}, {kappa, &st.K, p->nz}, {V, &st.V, p->nz}, {Vtop, &st.top, 1}, {Vbot, &st.bot, 1}};
+  std::vector<HostCopy> slow;
+  for (int i = 0; i < 5; i++) {
+    if (!arr[i].host) continue;
+    const size_t pitch = (size_t)(ncol * arr[i].len) * sizeof(double), row = (size_t)(nb * arr[i].len) * sizeof(double);
+    double *dst = arr[i].host + c0 * arr[i].len;
+    if (pageable[i])
+      slow.push_back({(const char *)arr[i].dev->p, (char *)dst, row, pitch, (size_t)p->nw});
+    else
+      CU(cudaMemcpy2DAsync(dst, pitch, arr[i].dev->p, row, row, p->nw, cudaMemcpyDeviceToHost, c->copy));
+  }
+  if (!slow.empty()) CU(c->host_copy.run(c->device, c->copy, slow));
+  CU(cudaEventRecord(st.done, c->copy));
+  return OCO_OK;
+}
+
+static int solve_block(oco_ctx *c, const oco_params *p, const double *rho, const double *T, double *U, double *kappa,
+                       double *V, double *Vtop, double *Vbot) {
   int rc = check_params(c, p);
   if (rc) return rc;
   if (p->form == OCO_FORM_MIXED && p->lgrey) return oco_set_err(c, OCO_EINVAL, "the mixed form has no grey variant");
@@ -668,6 +695,14 @@ extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rh
     if (Vtop) CU(st.top.ensure((size_t)ch * nw * sizeof(double)));
     if (Vbot) CU(st.bot.ensure((size_t)ch * nw * sizeof(double)));
   }
+  /* Small outputs: the driver's copies (a thread's start costs more than their faults); so too without
+   * memory for the pinned slots. */
+  const double *host[5] = {U, kappa, V, Vtop, Vbot};
+  bool pageable[5], any = false;
+  const size_t out_bytes = (size_t)ncol * nw * ((U ? mz : 0) + (kappa ? nz : 0) + (V ? nz : 0)) * sizeof(double);
+  for (int i = 0; i < 5; i++) any |= pageable[i] = out_bytes >= HOST_COPY_MIN && host[i] && host_pageable(host[i]);
+  if (any && !c->host_copy.ready(out_bytes))
+    for (bool &b : pageable) b = false;
   if (c->status_pending && (rc = oco_synchronize(c))) return rc;
   c->status_reset = true;
   SolveArgs a{};
@@ -678,6 +713,10 @@ extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rh
   a.dz2 = p->dz * p->dz;
   a.sigma_grey = p->sigma_grey;
   int k = 0;
+  int64_t last = -1; /* first column of the chunk whose outputs are still to be copied */
+  auto out = [&](int set) {
+    return copy_out(c, p, c->stage[set], last, std::min(ch, ncol - last), U, kappa, V, Vtop, Vbot, pageable);
+  };
   for (int64_t c0 = 0; c0 < ncol; c0 += ch, k ^= 1) {
     const int64_t nb = std::min(ch, ncol - c0);
     Stage &st = c->stage[k];
@@ -695,24 +734,28 @@ extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rh
     a.Vbot = Vbot ? st.bot.as<double>() : nullptr;
     a.c_off = 0;
     if ((rc = run_chunk(c, p, st.rho.as<double>(), st.T.as<double>(), nb, a, c->stream))) return rc;
-    /* copy-back on the copy stream, after the kernels */
+    /* the previous chunk's outputs go out while this chunk's kernels run; then the copy stream waits
+     * for these */
+    if (last >= 0 && (rc = out(k ^ 1))) return rc;
     cudaEvent_t ready;
     CU(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
     CU(cudaEventRecord(ready, c->stream));
     CU(cudaStreamWaitEvent(c->copy, ready, 0));
     CU(cudaEventDestroy(ready));
-    const size_t dp_u = (size_t)ncol * mz * sizeof(double), sp_u = (size_t)nb * mz * sizeof(double);
-    if (U) CU(cudaMemcpy2DAsync(U + c0 * mz, dp_u, st.U.p, sp_u, sp_u, nw, cudaMemcpyDeviceToHost, c->copy));
-    const size_t dp_k = (size_t)ncol * nz * sizeof(double), sp_k = (size_t)nb * nz * sizeof(double);
-    if (kappa) CU(cudaMemcpy2DAsync(kappa + c0 * nz, dp_k, st.K.p, sp_k, sp_k, nw, cudaMemcpyDeviceToHost, c->copy));
-    if (V) CU(cudaMemcpy2DAsync(V + c0 * nz, dp_k, st.V.p, sp_k, sp_k, nw, cudaMemcpyDeviceToHost, c->copy));
-    const size_t dp_p = (size_t)ncol * sizeof(double), sp_p = (size_t)nb * sizeof(double);
-    if (Vtop) CU(cudaMemcpy2DAsync(Vtop + c0, dp_p, st.top.p, sp_p, sp_p, nw, cudaMemcpyDeviceToHost, c->copy));
-    if (Vbot) CU(cudaMemcpy2DAsync(Vbot + c0, dp_p, st.bot.p, sp_p, sp_p, nw, cudaMemcpyDeviceToHost, c->copy));
-    CU(cudaEventRecord(st.done, c->copy));
+    last = c0;
   }
+  if ((rc = out(k ^ 1))) return rc;
   CU(cudaStreamSynchronize(c->copy));
   return read_status(c, c->stream, p);
+}
+
+extern "C" int oco_solve_block(oco_ctx *c, const oco_params *p, const double *rho, const double *T, double *U,
+                               double *kappa, double *V, double *Vtop, double *Vbot) {
+  try {
+    return solve_block(c, p, rho, T, U, kappa, V, Vtop, Vbot);
+  } catch (const std::bad_alloc &) {
+    return oco_set_err(c, OCO_ENOMEM, "oco_solve_block: out of host memory");
+  }
 }
 
 extern "C" int oco_synchronize(oco_ctx *c) {

@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/oco.h"
+#include "host_copy.h"
 
 struct DevBuf {
   void *p = nullptr;
@@ -64,6 +65,7 @@ struct oco_ctx {
   float repair_cond = 100.0f; /* oco_set_mixed_repair */
   int64_t repair_slots_max = -1; /* OCO_REPAIR_SLOTS: caps the re-solve's slots (the rest go one warp per item) */
   Stage stage[2];
+  oco::HostCopier host_copy; /* outputs of the host-array path into pageable arrays */
   int64_t launches = 0;
   size_t budget_bytes = 8ull << 30; /* chunk budget for pillars + staged outputs */
   int max_blocks = 0;               /* cap on the persistent grid (0: occupancy limit x SMs) */
