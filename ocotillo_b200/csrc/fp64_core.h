@@ -365,6 +365,35 @@ constexpr int RG = 4, RG_ALONE = 8;
  * once or twice costs more than the loads' latency. */
 constexpr int LONG_NZ = 48;
 
+/* U_{k+1} -> U at the level above the returned k, which leaves at least the four bottom levels. */
+template <int G>
+__device__ __forceinline__ double back_substitute(int &k, double U, const double *__restrict__ gam,
+                                                  const double *__restrict__ uu, int64_t ss, int nz) {
+  struct Lev {
+    double u, g;
+  } A[G], B[G];
+  auto load = [&](Lev *l, int k0) {
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      const int kl = max(k0 - i, 0);
+      l[i] = Lev{uu[kl * ss], gam[(kl + 1) * ss]};
+    }
+  };
+  auto steps = [&](const Lev *l) {
+#pragma unroll
+    for (int i = 0; i < G; i++) U = l[i].u - l[i].g * U;
+  };
+  load(A, k);
+#pragma unroll 1
+  for (; k >= 2 * G + 3 && nz >= LONG_NZ; k -= 2 * G) {
+    load(B, k - G);
+    steps(A);
+    load(A, k - 2 * G);
+    steps(B);
+  }
+  return U;
+}
+
 /* The reverse sweep of one item (back-substitution, tridag :43-45; ghost zones :49-62; flux
  * :96-109) from the forward sweep's last u and its scratch (gamma, u, kap: 1/kappa or kappa, and, stable form, q at
  * stride it.ss()), storing U, V (and kappa) through st and the emergent fluxes through the item
@@ -439,9 +468,11 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       for (int i = 0; i < G; i++) step(slot + i, k0 - i, l[i].u, l[i].q, l[i].g, l[i].o);
       if (slot + G == 8) st.template group<true>(3 + k0 - G + 1, 8);
     };
+    if (ST::PLANES) /* U alone down to the bottom's last levels */
+      Un = back_substitute<G>(k, Un, gam, uu, ss, nz);
     load(A, k);
 #pragma unroll 1
-    for (; k >= 2 * G - 1 && nz >= LONG_NZ; k -= 2 * G) {
+    for (; !ST::PLANES && k >= 2 * G - 1 && nz >= LONG_NZ; k -= 2 * G) {
       if (PF)
         for (int p = 4 * G; p < 6 * G && k - p >= 0; p++) { /* two pairs of groups ahead into L2 */
           prefetch_l2(&uu[(k - p) * ss]);
@@ -532,9 +563,10 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       for (int i = 0; i < G; i++) step(slot + i, k0 - i, l[i].u, l[i].g, l[i].o);
       if (slot + G == 8) st.template group<true>(3 + k0 - G + 1, 8);
     };
+    if (ST::PLANES) w0 = back_substitute<G>(kk, w0, gam, uu, ss, nz);
     load(A, kk);
 #pragma unroll 1
-    for (; kk >= 2 * G - 1 && nz >= LONG_NZ; kk -= 2 * G) {
+    for (; !ST::PLANES && kk >= 2 * G - 1 && nz >= LONG_NZ; kk -= 2 * G) {
       load(B, kk - G);
       steps(A, 0, kk);
       load(A, kk - 2 * G);
@@ -822,7 +854,7 @@ __device__ __forceinline__ void solve_item(const IT &it, bool active, PA &pa, do
   auto put = [&](int j, const RowOut &r, double u, double op) {
     gam[j * ss] = r.g;
     uu[j * ss] = u;
-    kap[j * ss] = ST::KAPPA_REVERSE ? op : r.o1;
+    if (!ST::PLANES || j == nz - 1) kap[j * ss] = ST::KAPPA_REVERSE ? op : r.o1;
     if (!ST::KAPPA_REVERSE) st.k(j, op);
     if (FORM == 1) qs[(j - 1) * ss] = r.q;
   };

@@ -246,9 +246,9 @@ __device__ __forceinline__ OutPtrs out_ptrs(const IT &it) {
 
 /* Generic path: warp tasks are 32 consecutive items of the flattened (column, lambda) index (lanes
  * past the last item repeat it and store nothing). */
-template <int FORM, bool GREY, bool REF>
+template <int FORM, bool GREY, int MODE>
 __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
-  __shared__ RingSmem<double> s_ring[REF ? WARPS_PER_BLOCK : 1];
+  __shared__ RingSmem<double> s_ring[MODE == ST_RING ? WARPS_PER_BLOCK : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nitems = a.ncol * a.nw;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
     DirectPillars pa{a.pil + cl * (int64_t)a.nz * NF};
     const BlockItem it{a, cl, iw};
     solve_item<FORM, GREY, BlockItem, DirectPillars, LamR>(it, active, pa, gam, uu, kap, qs, nullptr, TCacheR{},
-                                                           make_stores<REF, false, false>(out_ptrs(it), active, &s_ring[REF ? threadIdx.x >> 5 : 0]));
+                                                           make_stores<MODE, false, false>(out_ptrs(it), active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]));
   }
 }
 
@@ -306,13 +306,13 @@ __device__ __forceinline__ void init_staged(StagedPillars &pa, StagedSmem &sm) {
 }
 
 /* Staged path: warp tasks are (column, tile of 32 wavelengths); the column's pillar records
- * are streamed into shared memory by bulk copies (see StagedPillars).  REF: outputs with z fastest
+ * are streamed into shared memory by bulk copies (see StagedPillars).  ST_RING: outputs with z fastest
  * through the ring (a warm disk of 1800 columns x 500 x 250, plain: 13.65 ms with lambda-fastest
  * temporaries and three transposes, 12.8 ms so; the AGN profile 4.8 ms, runs off the 64-byte
  * boundaries 6.4 ms; ragged batch of 400 columns with each lane storing its own rows 3.55 ms, 2.65
  * ms so).  With lambda fastest the warm disk takes 11.4 ms: the ring's instructions and the larger
  * code (instruction-cache misses) are the rest. */
-template <int FORM, bool REF>
+template <int FORM, int MODE>
 __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
   __shared__ __align__(128) unsigned char s_warp[WARPS_PER_BLOCK * sizeof(StagedSmem)];
   StagedSmem &sm = reinterpret_cast<StagedSmem *>(s_warp)[threadIdx.x >> 5];
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_staged(const SolveArgs a) {
     const BlockItem it{a, cl, iw};
     solve_item<FORM, false, BlockItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
                                                           TCacheS{sm.tc + lane},
-                                                          make_stores<REF, true, false>(out_ptrs(it), active, &sm.ring));
+                                                          make_stores<MODE, true, false>(out_ptrs(it), active, &sm.ring));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&a.status[2], 1ull);
       /* let copies still in flight land (bounded) before the block's shared memory is released */
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles) 
     atomicMin(&it.status()[1], it.id());
   }
   __syncwarp();
-  auto st = make_stores<REF, TILE, false>(out_ptrs(it), active, s_ring);
+  auto st = make_stores<REF ? ST_RING : ST_LANE, TILE, false>(out_ptrs(it), active, s_ring);
   solve_reverse<FORM, RG_ALONE>(it, active, e.u, S.aa, S.dd, S.kap, S.xx, st);
 }
 
@@ -636,7 +636,7 @@ struct BatchItem {
 /* Warp-column tiling: tasks (column, 32-wavelength tile) from the device queue, longest
  * columns first; the column's records stream through the warp's shared-memory buffers and
  * the tile's wavelength constants sit in the warp's shared-memory table (as k_solve_staged). */
-template <int FORM, bool REF>
+template <int FORM, int MODE>
 __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArgs b) {
   __shared__ __align__(128) unsigned char s_warp[WARPS_PER_BLOCK * sizeof(StagedSmem)];
   StagedSmem &sm = reinterpret_cast<StagedSmem *>(s_warp)[threadIdx.x >> 5];
@@ -667,7 +667,7 @@ __global__ void __launch_bounds__(128, 4) k_batch_fp64_staged(const FP64BatchArg
     const BatchItem it{b, c, (int64_t)t.x, iw};
     solve_item<FORM, false, BatchItem, StagedPillars, LamS>(it, active, pa, gam, uu, kap, qs, sm.lam,
                                                            TCacheS{sm.tc + lane},
-                                                           make_stores<REF, true, false>(out_ptrs(it), active, &sm.ring));
+                                                           make_stores<MODE, true, false>(out_ptrs(it), active, &sm.ring));
     if (__any_sync(0xffffffffu, pa.failed)) {
       if (lane == 0) atomicOr(&b.status[2], 1ull);
       pa.wait(0);
@@ -685,19 +685,24 @@ cudaError_t launch_pillars_batch(const double *rho, const double *T, const MBatc
   return cudaGetLastError();
 }
 
-static const void *batch_fn(int form, bool ref) {
-  if (form == 0) return ref ? (const void *)k_batch_fp64_staged<0, true> : (const void *)k_batch_fp64_staged<0, false>;
-  return ref ? (const void *)k_batch_fp64_staged<1, true> : (const void *)k_batch_fp64_staged<1, false>;
+template <int FORM>
+static const void *batch_fn_of(StoreMode m) {
+  switch (m) {
+    case ST_RING: return (const void *)k_batch_fp64_staged<FORM, ST_RING>;
+    case ST_PLANES: return (const void *)k_batch_fp64_staged<FORM, ST_PLANES>;
+    default: return (const void *)k_batch_fp64_staged<FORM, ST_LANE>;
+  }
 }
+static const void *batch_fn(int form, StoreMode m) { return form == 0 ? batch_fn_of<0>(m) : batch_fn_of<1>(m); }
 
 cudaError_t launch_batch_fp64(const FP64BatchArgs &a, int form, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(batch_fn(form, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(batch_fn(form, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 int batch_fp64_max_blocks_per_sm(int form, int threads) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_fn(form, false), threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_fn(form, ST_LANE), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
@@ -712,22 +717,29 @@ cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int
 
 bool solve_uses_staging(int nw) { return nw >= 64 || (nw % 32) == 0; }
 
-template <bool REF>
-static const void *solve_fn_of(int form, int grey, bool staged) {
-  if (staged)
-    return form == 0 ? (const void *)k_solve_staged<0, REF> : (const void *)k_solve_staged<1, REF>;
-  if (form == 0) return grey ? (const void *)k_solve<0, true, REF> : (const void *)k_solve<0, false, REF>;
-  return grey ? (const void *)k_solve<1, true, REF> : (const void *)k_solve<1, false, REF>;
+template <int FORM>
+static const void *staged_fn_of(StoreMode m) {
+  switch (m) {
+    case ST_RING: return (const void *)k_solve_staged<FORM, ST_RING>;
+    case ST_PLANES: return (const void *)k_solve_staged<FORM, ST_PLANES>;
+    default: return (const void *)k_solve_staged<FORM, ST_LANE>;
+  }
 }
-static const void *solve_fn(int form, int grey, bool staged, bool ref) {
-  return ref ? solve_fn_of<true>(form, grey, staged) : solve_fn_of<false>(form, grey, staged);
+template <int FORM, bool GREY>
+static const void *direct_fn_of(StoreMode m) { /* planes: the lane-by-lane kernel stores no level either */
+  return m == ST_RING ? (const void *)k_solve<FORM, GREY, ST_RING> : (const void *)k_solve<FORM, GREY, ST_LANE>;
+}
+static const void *solve_fn(int form, int grey, bool staged, StoreMode m) {
+  if (staged) return form == 0 ? staged_fn_of<0>(m) : staged_fn_of<1>(m);
+  if (grey) return form == 0 ? direct_fn_of<0, true>(m) : direct_fn_of<1, true>(m);
+  return form == 0 ? direct_fn_of<0, false>(m) : direct_fn_of<1, false>(m);
 }
 
 int solve_fp64_max_blocks_per_sm(int form, int grey, int threads) {
   int nb = 0, nb2 = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, solve_fn(form, grey, false, false), threads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, solve_fn(form, grey, false, ST_LANE), threads, 0) != cudaSuccess)
     nb = 1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, solve_fn(form, grey, true, false), threads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb2, solve_fn(form, grey, true, ST_LANE), threads, 0) != cudaSuccess)
     nb2 = 1;
   nb = nb > nb2 ? nb : nb2;
   return nb > 0 ? nb : 1;
@@ -762,7 +774,7 @@ cudaError_t launch_bounded_wait_check(long long limit, unsigned long long *statu
 cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int blocks, int threads, cudaStream_t s) {
   const bool staged = !grey && solve_uses_staging(a.nw);
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_fn(form, grey, staged, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(solve_fn(form, grey, staged, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

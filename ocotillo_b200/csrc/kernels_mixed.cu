@@ -226,6 +226,26 @@ struct MScratch12 {
   }
   __device__ __forceinline__ float kappa(int j) const { return __int_as_float(__float_as_int(p2(j)->y) & 0x7fffffff); }
 };
+/* MScratch12P: 12 bytes without kappa, for solves that store no level (the kappa of the two ends stays
+ * with the item): {v, u mantissa} (float2), then u's exponents; no packing, any exponent. */
+struct MScratch12P {
+  static constexpr int LEVEL = 32 * 12;
+  char *w; /* the warp's level 0 */
+  int lane;
+  __device__ __forceinline__ float2 *p2(int j) const { return (float2 *)(w + (int64_t)j * LEVEL) + lane; }
+  __device__ __forceinline__ float *p1(int j) const { return (float *)(w + (int64_t)j * LEVEL + 256) + lane; }
+  __device__ __forceinline__ const char *level(int j) const { return w + (int64_t)j * LEVEL; }
+  __device__ __forceinline__ bool put(int j, const float4 &r) const {
+    *p2(j) = make_float2(r.x, r.z);
+    *p1(j) = r.w;
+    return true;
+  }
+  __device__ __forceinline__ float4 get(int j) const {
+    const float2 a = *p2(j);
+    return make_float4(a.x, 0.0f, a.y, *p1(j));
+  }
+  __device__ __forceinline__ float kappa(int) const { return 0.0f; } /* not kept */
+};
 /* One (column, wavelength) item, its scratch records in sc.  An inactive lane runs the forward
  * sweep (to keep a staged warp in step) and writes nothing. */
 /* Returns whether the item's emergent flux is ill-conditioned for this arithmetic: with
@@ -256,6 +276,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
   Opac32 cur = opac(0);
   Opac32 nxt = opac(1);
   float kc = kappa_lin(cur), kn = kappa_lin(nxt);
+  const float k0 = kc; /* kappa of the bottom level */
   Row32 r = row_boundary(kc, cur, dzf, dz2f, ldz2i, ldz2f, false);
   float h = r.e, cprev = r.c;
   float an = 2.0f * rcp(kn + kc); /* a' of row 1; then c' of the row below */
@@ -339,7 +360,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       return ((-(double)rcp(kj)) * df) * dz1;
     };
     {
-      const float kj = sc.kappa(n - 1);
+      const float kj = kc; /* the top level's */
       vtop = flux(kj);
       st.push(6, n - 1, Uk[2], vtop, (double)kj); /* U_{n-4}, V_{n-1} */
       st.template group<false>(n - 1, 7);
@@ -365,7 +386,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
     /* Scratch levels in two groups of MG that take turns (one in use, one in flight); one bulk request
      * from lane 0 brings the MG levels MIXED_L2_AHEAD steps further down into L2 (the warp's levels
      * are contiguous; they were written a whole forward sweep ago and have usually left L2). */
-    if (k >= 7) {
+    if (k >= 7 + (ST::PLANES ? 4 : 0)) {
       float4 A[MG], B[MG];
       auto load = [&](float4 *w, int k0) {
         if (k0 - MG + 1 - MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0)
@@ -378,10 +399,17 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       };
       auto steps = [&](const float4 *w, int slot, int k0) {
 #pragma unroll
-        for (int i = 0; i < MG; i++) step(slot + i, k0 - i, w[i]);
+        for (int i = 0; i < MG; i++) {
+          if constexpr (ST::PLANES) { /* U alone down to the bottom's last levels */
+            const XF uj{w[i].z, __float_as_int(w[i].w)};
+            Un = xaxpy1(uj, Un, (w[i].x >= 0.0f) ? 1.0f - w[i].x : -w[i].x);
+          } else {
+            step(slot + i, k0 - i, w[i]);
+          }
+        }
       };
       load(A, k);
-      for (; k >= 7; k -= 8) {
+      for (; k >= 7 + (ST::PLANES ? 4 : 0); k -= 8) {
         load(B, k - MG);
         steps(A, 0, k);
         load(A, k - 8);
@@ -417,7 +445,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
 #pragma unroll 1
     for (int j = 2; j >= 0; j--) { /* D_{-1} = D_0, D_{-2} = D_1, D_{-3} = D_2 */
       d5 = d4; d4 = d3; d3 = d2; d2 = d1; d1 = d0; d0 = j == 2 ? D0 : (j == 1 ? D1 : D2);
-      const float kj = j == 2 ? r3 : (j == 1 ? r2 : r1);
+      const float kj = ST::PLANES ? k0 : j == 2 ? r3 : (j == 1 ? r2 : r1);
       vbot = flux(kj);
       st.push(q, j, j == 2 ? g2 : (j == 1 ? g1 : g0), vbot, (double)kj);
       if (++q == 8) {
@@ -448,7 +476,7 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
     for (int j = 0; j < nz; j++) {
       const int c = n1 + j;
       const double df = (1.0 / 60.0) * (((45.0 * (f[c + 1] - f[c - 1])) - 9.0 * (f[c + 2] - f[c - 2])) + (f[c + 3] - f[c - 3]));
-      const float kj = sc.kappa(j);
+      const float kj = ST::PLANES ? (j == 0 ? k0 : kc) : sc.kappa(j);
       const double v = ((-(double)rcp(kj)) * df) * dz1;
       st.v(j, v);
       st.k(j, (double)kj);
@@ -531,9 +559,9 @@ __device__ __forceinline__ void init_staged(MStaged &pa, MStagedSmem &sm) {
   __syncwarp();
 }
 
-/* REF: outputs with z fastest through the ring (AGN grid of 1600 columns x 512 x 256: 5.04 ms with
+/* ST_RING: outputs with z fastest through the ring (AGN grid of 1600 columns x 512 x 256: 5.04 ms with
  * lambda-fastest temporaries and three transposes, 3.43 ms so; with lambda fastest 2.95 ms). */
-template <class SC, bool REF>
+template <class SC, int MODE>
 __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const MixedArgs a) {
   __shared__ __align__(128) unsigned char s_warp[MWARPS * sizeof(MStagedSmem)];
   MStagedSmem &sm = reinterpret_cast<MStagedSmem *>(s_warp)[threadIdx.x >> 5];
@@ -559,7 +587,7 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const Mixed
     store_lam32_shared(sm.lam, lane, a.lam, iw, a.nw);
     __syncwarp();
     const MItem it = block_item(a, cl, iw);
-    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<REF, true, true>(it.o, active, &sm.ring),
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, true>(it.o, active, &sm.ring),
                                   a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
@@ -575,9 +603,9 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const Mixed
 
 /* Few wavelengths: 32 consecutive items per warp (lanes past the last item repeat it and store
  * nothing). */
-template <class SC, bool REF>
+template <class SC, int MODE>
 __global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
-  __shared__ RingSmem<float> s_ring[REF ? MWARPS : 1];
+  __shared__ RingSmem<float> s_ring[MODE == ST_RING ? MWARPS : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nitems = a.ncol * a.nw;
@@ -595,7 +623,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
     MDirect pa{a.rec + cl * (int64_t)a.nz * MZN};
     const MItem it = block_item(a, cl, iw);
     const bool flag = msolve_item(it, active, pa, load_lam32(it.lam, iw, it.nw), sc,
-                                  make_stores<REF, false, true>(it.o, active, &s_ring[REF ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
+                                  make_stores<MODE, false, true>(it.o, active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     mark_items(flag, cl * ((a.nw + 31) / 32) + iw / 32, iw, (unsigned long long)item, a.rbits, a.rslot, a.rlist, a.rcount,
                a.ilist, a.icount);
@@ -604,21 +632,24 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
 
 static bool mixed_uses_staging(int nw) { return (nw >= 64) || (nw % 32) == 0; }
 
-static const void *solve_mixed_fn(int nw, bool ref) {
-  if (mixed_uses_staging(nw))
-    return ref ? (const void *)k_solve_mixed_staged<MScratch16, true> : (const void *)k_solve_mixed_staged<MScratch16, false>;
-  return ref ? (const void *)k_solve_mixed<MScratch16, true> : (const void *)k_solve_mixed<MScratch16, false>;
+static const void *solve_mixed_fn(int nw, StoreMode m) {
+  if (mixed_uses_staging(nw)) switch (m) {
+      case ST_RING: return (const void *)k_solve_mixed_staged<MScratch16, ST_RING>;
+      case ST_PLANES: return (const void *)k_solve_mixed_staged<MScratch12P, ST_PLANES>;
+      default: return (const void *)k_solve_mixed_staged<MScratch16, ST_LANE>;
+    }
+  return m == ST_RING ? (const void *)k_solve_mixed<MScratch16, ST_RING> : (const void *)k_solve_mixed<MScratch16, ST_LANE>;
 }
 
 int solve_mixed_max_blocks_per_sm(int threads, int nw) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw, false), threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw, ST_LANE), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
 cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_mixed_fn(a.nw, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(solve_mixed_fn(a.nw, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 /* ---- ragged batches ---------------------------------------------------------------------- */
@@ -655,7 +686,7 @@ __device__ __forceinline__ MItem batch_item(const MixedBatchArgs &b, const MBatc
 
 /* Warp-column tiling: tasks (column, 32-wavelength tile) from the device queue, longest
  * columns first; the column's records stream through the warp's shared-memory buffers. */
-template <class SC, bool REF>
+template <class SC, int MODE>
 __global__ void __launch_bounds__(128, MBLOCKS) k_batch_mixed_staged(const MixedBatchArgs b) {
   __shared__ __align__(128) unsigned char s_warp[MWARPS * sizeof(MStagedSmem)];
   MStagedSmem &sm = reinterpret_cast<MStagedSmem *>(s_warp)[threadIdx.x >> 5];
@@ -679,7 +710,7 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_batch_mixed_staged(const Mixed
     store_lam32_shared(sm.lam, lane, b.lam + c.lam_off, iw, c.nw);
     __syncwarp();
     const MItem it = batch_item(b, c, iw);
-    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<REF, true, true>(it.o, active, &sm.ring),
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, true>(it.o, active, &sm.ring),
                                   b.repair_cond) ||
                       (active && __ldg(b.colflag + t.x) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
@@ -733,21 +764,25 @@ __global__ void __launch_bounds__(128, 4) k_batch_mixed_packed(const MixedBatchA
   }
 }
 
-static const void *batch_mixed_fn(int tiling, bool ref) {
+static const void *batch_mixed_fn(int tiling, StoreMode m) {
   if (tiling == BATCH_TILING_PACKED) return (const void *)k_batch_mixed_packed<MScratch12>;
-  return ref ? (const void *)k_batch_mixed_staged<MScratch12, true> : (const void *)k_batch_mixed_staged<MScratch12, false>;
+  switch (m) {
+    case ST_RING: return (const void *)k_batch_mixed_staged<MScratch12, ST_RING>;
+    case ST_PLANES: return (const void *)k_batch_mixed_staged<MScratch12P, ST_PLANES>;
+    default: return (const void *)k_batch_mixed_staged<MScratch12, ST_LANE>;
+  }
 }
 
 int batch_mixed_max_blocks_per_sm(int tiling, int threads) {
   int n = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_fn(tiling, false), threads, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_mixed_fn(tiling, ST_LANE), threads, 0);
   if (e != cudaSuccess || n < 1) n = 1;
   return n;
 }
 
 cudaError_t launch_batch_mixed(const MixedBatchArgs &a, int tiling, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(batch_mixed_fn(tiling, a.layout == 0), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(batch_mixed_fn(tiling, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

@@ -544,6 +544,14 @@ MX_HD void xaxpy2(XF x, XF y, float t1, float t2, XF &r1, XF &r2) {
   r1 = xnorm(ge ? fmaf(b1, p, x.m) : fmaf(x.m, p, b1), e);
   r2 = xnorm(ge ? fmaf(b2, p, x.m) : fmaf(x.m, p, b2), e);
 }
+/* The first of them alone. */
+MX_HD XF xaxpy1(XF x, XF y, float t1) {
+  const int d = x.e - y.e;
+  const bool ge = d >= 0;
+  const float p = pow2f(ge ? -d : d);
+  const float b1 = y.m * t1;
+  return xnorm(ge ? fmaf(b1, p, x.m) : fmaf(x.m, p, b1), ge ? x.e : y.e);
+}
 MX_HD double xtod(XF x) {
   if (x.m == 0.0f || x.e < -1000) return 0.0;
   return (double)x.m * oco_u2d((uint64_t)(int64_t)(x.e + 1023) << 52);

@@ -38,7 +38,7 @@ struct OutPtrs {
  * forward sweep has stored it (k) and the argument is ignored. */
 template <bool KREV>
 struct LaneStores {
-  static constexpr bool KAPPA_REVERSE = KREV;
+  static constexpr bool KAPPA_REVERSE = KREV, PLANES = false;
   double *Ub, *Kb, *Vb;
   int64_t uz, kz, vz;
   __device__ __forceinline__ LaneStores(const OutPtrs &o, bool active)
@@ -60,6 +60,22 @@ struct LaneStores {
     v(m, V);
     if (KREV) k(m, K);
   }
+  template <bool FULL>
+  __device__ __forceinline__ void group(int, int) {}
+  __device__ __forceinline__ void finish(int) {}
+};
+
+/* Only the emergent planes are wanted (a serving job without fields): nothing is stored per level.
+ * The sweeps then form the fluxes and differences of the bottom levels alone, and the scratch keeps
+ * kappa of the two ends only. */
+struct PlaneStores {
+  static constexpr bool KAPPA_REVERSE = false, PLANES = true;
+  __device__ __forceinline__ void u(int, double) const {}
+  __device__ __forceinline__ void k(int, double) const {}
+  __device__ __forceinline__ void v(int, double) const {}
+  __device__ __forceinline__ void open(int) {}
+  __device__ __forceinline__ void push_u(int, int, double) {}
+  __device__ __forceinline__ void push(int, int, double, double, double) {}
   template <bool FULL>
   __device__ __forceinline__ void group(int, int) {}
   __device__ __forceinline__ void finish(int) {}
@@ -160,11 +176,18 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
   }
 };
 
-/* The stores of a warp's outputs: lane by lane, or (REF, z fastest) through the ring. */
-template <bool REF, bool ROWS, bool KREV, class KT>
+/* How a kernel's warps store their outputs: lane by lane, through the ring (z fastest), or only the
+ * emergent planes. */
+enum StoreMode { ST_LANE = 0, ST_RING = 1, ST_PLANES = 2 };
+inline StoreMode store_mode(const void *U, const void *K, const void *V, int layout) {
+  return !U && !K && !V ? ST_PLANES : layout == 0 ? ST_RING : ST_LANE;
+}
+template <int MODE, bool ROWS, bool KREV, class KT>
 __device__ __forceinline__ auto make_stores(const OutPtrs &o, bool active, RingSmem<KT> *ring) {
-  if constexpr (REF)
+  if constexpr (MODE == ST_RING)
     return RingStores<ROWS, KT>(o, active, ring);
+  else if constexpr (MODE == ST_PLANES)
+    return PlaneStores{};
   else
     return LaneStores<KREV>(o, active);
 }
