@@ -248,6 +248,10 @@ struct TCacheS { /* the lane's pairs in the warp's shared table [NTC/2][32] */
   }
 };
 
+/* The rare full evaluations, out of line. */
+static __device__ __noinline__ double exp_dd_call(double xh, double xl) { return oco_exp_dd(xh, xl); }
+static __device__ __noinline__ double log_call(double x) { return oco_log(x); }
+
 /* calc_opacity_and_albedo for one (z, lambda), continuous_opacity.f90:175-201 with
  * :171, :233-244, :318-322, :337-339, :261-277, :290-298, :399-407. */
 /* 10^y1, 10^y2 and e^x3 as oco_pow10, oco_pow10 and oco_exp compute them, with the three
@@ -262,12 +266,29 @@ __device__ __forceinline__ void pow10_pow10_exp(double y1, double y2, double x3,
   const int ok1 = oco_exp_fast_nb(p1, l1, &f1);
   const int ok2 = oco_exp_fast_nb(p2, l2, &f2);
   const int ok3 = oco_exp_fast_nb(x3, 0.0, &f3);
-  if (!ok1) f1 = oco_exp_dd(p1, l1);
-  if (!ok2) f2 = oco_exp_dd(p2, l2);
-  if (!ok3) f3 = oco_exp_dd(x3, 0.0);
+  if (!ok1) f1 = exp_dd_call(p1, l1);
+  if (!ok2) f2 = exp_dd_call(p2, l2);
+  if (!ok3) f3 = exp_dd_call(x3, 0.0);
   r1 = OCO_M(1.0, f1);
   r2 = OCO_M(1.0, f2);
   r3 = f3;
+}
+
+/* bremsstrahlung_absorptionCoeff (c_o :281-300): the Gaunt factor's log, exp and log and the other
+ * factor's exp, log and exp side by side without branches (each would be a chain of its own behind
+ * its special cases), and the full functions where an argument is not an ordinary one or a fast
+ * exponential cannot decide its rounding (a warm disk of 1800 columns x 500 x 250, 62% of the points
+ * ionized: 12.6 -> 11.07 ms). */
+__device__ __forceinline__ double bremsstrahlung(double a, double b, double c) {
+  double a1, b1, a2, b2, a3, b3;
+  int ok = oco_log_nb(a, &a1) & oco_exp_fast_nb(b, 0.0, &b1);
+  ok &= oco_exp_fast_nb(5.960 - (sqrt3 * pi1) * a1, 0.0, &a2) & oco_log_nb(1.0 - b1, &b2);
+  ok &= oco_log_nb(a2 + exp1, &a3) & oco_exp_fast_nb(c + b2, 0.0, &b3);
+  if (!ok) {
+    a3 = log_call(exp_dd_call(5.960 - (sqrt3 * pi1) * log_call(a), 0.0) + exp1);
+    b3 = exp_dd_call(c + log_call(1.0 - exp_dd_call(b, 0.0)), 0.0);
+  }
+  return (bremsstrahlung_constant * b3) * a3;
 }
 
 template <bool STABLE, class R, class LM, class TC>
@@ -307,10 +328,7 @@ __device__ __forceinline__ Opac opacity_at(const R P, const LM &L, TC &tc, bool 
     kr = kr + x;
     op = op + kr * rho;
   } else {
-    double gaunt = oco_log(oco_exp(5.960 - (sqrt3 * pi1) * oco_log(L.nu9() * P[F_TPOW])) + exp1);
-    double lnq = (P[F_LZ] - L.l3nu()) + oco_log(1.0 - oco_exp(-(L.hnuk() * P[F_T1])));
-    double krho = (bremsstrahlung_constant * oco_exp(lnq)) * gaunt;
-    op = op + krho;
+    op = op + bremsstrahlung(L.nu9() * P[F_TPOW], -(L.hnuk() * P[F_T1]), P[F_LZ] - L.l3nu());
     x = op * P[F_RHO1];
     kr = kr + x;
   }

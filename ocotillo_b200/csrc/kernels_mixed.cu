@@ -200,6 +200,9 @@ struct MScratch16 {
     *p(j) = r;
     return true;
   }
+  using Raw = float4; /* a record as loaded; opened where it is used, so that the load stays in flight */
+  __device__ __forceinline__ Raw load(int j) const { return *p(j); }
+  static __device__ __forceinline__ float4 open(const Raw &r) { return r; }
   __device__ __forceinline__ float4 get(int j) const { return *p(j); }
   __device__ __forceinline__ float kappa(int j) const { return p(j)->y; }
 };
@@ -217,13 +220,18 @@ struct MScratch12 {
     *p1(j) = __int_as_float(w2);
     return fits;
   }
-  __device__ __forceinline__ float4 get(int j) const {
-    const float2 a = *p2(j);
+  struct Raw {
+    float2 a;
+    float m;
+  };
+  __device__ __forceinline__ Raw load(int j) const { return Raw{*p2(j), *p1(j)}; }
+  static __device__ __forceinline__ float4 open(const Raw &r) {
     float kc, m;
     int e;
-    unpack_o1_u(__float_as_int(a.y), __float_as_int(*p1(j)), kc, m, e);
-    return make_float4(a.x, kc, m, __int_as_float(e));
+    unpack_o1_u(__float_as_int(r.a.y), __float_as_int(r.m), kc, m, e);
+    return make_float4(r.a.x, kc, m, __int_as_float(e));
   }
+  __device__ __forceinline__ float4 get(int j) const { return open(load(j)); }
   __device__ __forceinline__ float kappa(int j) const { return __int_as_float(__float_as_int(p2(j)->y) & 0x7fffffff); }
 };
 /* MScratch12P: 12 bytes without kappa, for solves that store no level (the kappa of the two ends stays
@@ -240,10 +248,13 @@ struct MScratch12P {
     *p1(j) = r.w;
     return true;
   }
-  __device__ __forceinline__ float4 get(int j) const {
-    const float2 a = *p2(j);
-    return make_float4(a.x, 0.0f, a.y, *p1(j));
-  }
+  struct Raw {
+    float2 a;
+    float e;
+  };
+  __device__ __forceinline__ Raw load(int j) const { return Raw{*p2(j), *p1(j)}; }
+  static __device__ __forceinline__ float4 open(const Raw &r) { return make_float4(r.a.x, 0.0f, r.a.y, r.e); }
+  __device__ __forceinline__ float4 get(int j) const { return open(load(j)); }
   __device__ __forceinline__ float kappa(int) const { return 0.0f; } /* not kept */
 };
 /* One (column, wavelength) item, its scratch records in sc.  An inactive lane runs the forward
@@ -387,24 +398,25 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
      * from lane 0 brings the MG levels MIXED_L2_AHEAD steps further down into L2 (the warp's levels
      * are contiguous; they were written a whole forward sweep ago and have usually left L2). */
     if (k >= 7 + (ST::PLANES ? 4 : 0)) {
-      float4 A[MG], B[MG];
-      auto load = [&](float4 *w, int k0) {
+      typename SC::Raw A[MG], B[MG];
+      auto load = [&](typename SC::Raw *w, int k0) {
         if (k0 - MG + 1 - MIXED_L2_AHEAD >= 0 && (threadIdx.x & 31) == 0)
           asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(
                            sc.level(k0 - MG + 1 - MIXED_L2_AHEAD))),
                        "r"((uint32_t)(MG * SC::LEVEL))
                        : "memory");
 #pragma unroll
-        for (int i = 0; i < MG; i++) w[i] = sc.get(max(k0 - i, 0));
+        for (int i = 0; i < MG; i++) w[i] = sc.load(max(k0 - i, 0));
       };
-      auto steps = [&](const float4 *w, int slot, int k0) {
+      auto steps = [&](const typename SC::Raw *w, int slot, int k0) {
 #pragma unroll
         for (int i = 0; i < MG; i++) {
+          const float4 x = SC::open(w[i]);
           if constexpr (ST::PLANES) { /* U alone down to the bottom's last levels */
-            const XF uj{w[i].z, __float_as_int(w[i].w)};
-            Un = xaxpy1(uj, Un, (w[i].x >= 0.0f) ? 1.0f - w[i].x : -w[i].x);
+            const XF uj{x.z, __float_as_int(x.w)};
+            Un = xaxpy1(uj, Un, (x.x >= 0.0f) ? 1.0f - x.x : -x.x);
           } else {
-            step(slot + i, k0 - i, w[i]);
+            step(slot + i, k0 - i, x);
           }
         }
       };

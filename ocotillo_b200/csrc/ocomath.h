@@ -310,6 +310,61 @@ OCO_HD void oco_log_dd(double x, double *lh, double *ll) {
   *ll = OCO_S(lo, OCO_S(r, s2));
 }
 
+/* oco_log without branches: for a finite normal x > 0 the same operations as oco_log_dd, and 1; 0
+ * otherwise (*res is then meaningless).  Several of these and of oco_exp_fast_nb can be
+ * interleaved by the compiler. */
+OCO_HD int oco_log_nb(double x, double *res) {
+  const uint64_t u = oco_d2u(x);
+  const uint64_t hi = u >> 52;
+  const int ok = (hi - 1 < 0x7fe); /* positive, neither subnormal nor infinite nor NaN */
+  int e = (int)hi - 1023;
+  double m = oco_u2d((u & 0x000fffffffffffffULL) | 0x3ff0000000000000ULL);
+  const int big = m >= 1.5;
+  m = big ? OCO_M(m, 0.5) : m;
+  e += big;
+  const double shift = 0x1.8p52;
+  const double jd = OCO_S(OCO_A(OCO_M(OCO_S(m, 1.0), (double)OCO_LOG_N), shift), shift);
+  const int j = (int)jd;
+  const double F = OCO_A(1.0, OCO_M(jd, 1.0 / OCO_LOG_N));
+  const double f = OCO_S(m, F);
+  const int idx = 2 * (j - OCO_LOG_JMIN);
+  const double ih = OCO_TAB(oco_invF_tab, idx), il = OCO_TAB(oco_invF_tab, idx + 1);
+  double uh = OCO_M(f, ih);
+  const double ue = OCO_FMA(f, ih, -uh);
+  double ul = OCO_A(ue, OCO_M(f, il));
+  const double u0 = OCO_A(uh, ul);
+  ul = OCO_S(ul, OCO_S(u0, uh));
+  uh = u0;
+  const double s = OCO_M(uh, uh);
+  const double se = OCO_FMA(uh, uh, -s);
+  const double half = OCO_M(0.5, s);
+  const double halfe = OCO_A(OCO_M(0.5, se), OCO_M(uh, ul));
+  double P = OCO_FMA(-uh, OCO_LOG_C11, OCO_LOG_C10);
+  P = OCO_FMA(-uh, P, OCO_LOG_C9);
+  P = OCO_FMA(-uh, P, OCO_LOG_C8);
+  P = OCO_FMA(-uh, P, OCO_LOG_C7);
+  P = OCO_FMA(-uh, P, OCO_LOG_C6);
+  P = OCO_FMA(-uh, P, OCO_LOG_C5);
+  P = OCO_FMA(-uh, P, OCO_LOG_C4);
+  P = OCO_FMA(-uh, P, OCO_LOG_C3);
+  P = OCO_M(OCO_M(s, uh), P);
+  const double qh = OCO_S(uh, half);
+  const double ql = OCO_A(OCO_S(OCO_S(uh, qh), half), OCO_A(OCO_S(ul, halfe), P));
+  const double ed = (double)e;
+  const double A = OCO_M(ed, OCO_LN2_HI);
+  const double B = OCO_TAB(oco_logF_tab, idx);
+  const double s1 = OCO_A(A, B);
+  double bb = OCO_S(s1, A);
+  const double t1 = OCO_A(OCO_S(A, OCO_S(s1, bb)), OCO_S(B, bb));
+  const double s2 = OCO_A(s1, qh);
+  bb = OCO_S(s2, s1);
+  const double t2 = OCO_A(OCO_S(s1, OCO_S(s2, bb)), OCO_S(qh, bb));
+  const double lo = OCO_A(OCO_A(t1, t2),
+                          OCO_A(OCO_A(OCO_M(ed, OCO_LN2_LO), OCO_TAB(oco_logF_tab, idx + 1)), ql));
+  *res = OCO_A(s2, lo);
+  return ok;
+}
+
 /* Natural exponential. */
 OCO_HD double oco_exp(double x) { return oco_exp_dd(x, 0.0); }
 
