@@ -2,6 +2,7 @@
 #include "host_copy.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <system_error>
 #include <thread>
@@ -24,15 +25,15 @@ void HostCopier::release() {
   }
   if (pinned_) cudaFreeHost(pinned_);
   pinned_ = nullptr;
-  slot_ = 0;
+  half_ = 0;
 }
 
-cudaError_t HostCopier::ensure(size_t slot) {
+cudaError_t HostCopier::ensure(size_t half) {
   cudaError_t e = cudaSuccess;
-  if (slot_ < slot) {
+  if (half_ < half) {
     release();
-    e = cudaHostAlloc((void **)&pinned_, 2 * HOST_COPY_THREADS * slot, cudaHostAllocDefault);
-    if (e == cudaSuccess) slot_ = slot;
+    e = cudaHostAlloc((void **)&pinned_, 2 * half, cudaHostAllocDefault);
+    if (e == cudaSuccess) half_ = half;
   }
   for (auto &v : ev_)
     if (e == cudaSuccess && !v) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
@@ -40,66 +41,87 @@ cudaError_t HostCopier::ensure(size_t slot) {
 }
 
 namespace {
-/* Bytes [off, off + n) of the copies laid end to end, from the slot to their destinations. */
-void scatter(const std::vector<HostCopy> &copies, size_t i, size_t off, const char *slot, size_t n) {
-  const HostCopy &c = copies[i];
-  while (n) {
-    const size_t row = off / c.row_bytes, at = off - row * c.row_bytes, k = std::min(n, c.row_bytes - at);
-    memcpy(c.dst + row * c.dst_pitch + at, slot, k);
-    slot += k;
-    off += k;
-    n -= k;
+/* Calls f(copy, offset in it, n) for the parts of bytes [lo, hi) of the copies laid end to end. */
+template <class F>
+void parts(const std::vector<HostCopy> &copies, size_t lo, size_t hi, F f) {
+  size_t at = 0;
+  for (const auto &c : copies) {
+    const size_t end = at + c.bytes();
+    const size_t a = std::max(lo, at), b = std::min(hi, end);
+    if (a < b) f(c, a - at, b - a);
+    at = end;
   }
 }
 
-struct Piece {
-  size_t copy, off, n;
-};
+/* Bytes [lo, hi), which lie at slot, to their destinations. */
+void scatter(const std::vector<HostCopy> &copies, size_t lo, size_t hi, const char *slot) {
+  parts(copies, lo, hi, [&](const HostCopy &c, size_t off, size_t n) {
+    while (n) {
+      const size_t row = off / c.row_bytes, in = off - row * c.row_bytes, k = std::min(n, c.row_bytes - in);
+      memcpy(c.dst + row * c.dst_pitch + in, slot, k);
+      slot += k;
+      off += k;
+      n -= k;
+    }
+  });
+}
 }  // namespace
 
 cudaError_t HostCopier::run(int device, cudaStream_t s, const std::vector<HostCopy> &copies) {
-  cudaError_t e = cudaSuccess;
+  (void)device; /* the calling thread's; the others do not talk to the driver */
   size_t total = 0;
   for (const auto &c : copies) total += c.bytes();
-  /* small outputs: one piece per thread, of at least a few pages */
-  const size_t share = (total / HOST_COPY_THREADS + 4095) & ~(size_t)4095;
-  const size_t size = std::min(slot_, std::max<size_t>(share, 64u << 10));
-  std::vector<Piece> pieces;
-  for (size_t i = 0; i < copies.size(); i++)
-    for (size_t o = 0; o < copies[i].bytes(); o += size) pieces.push_back({i, o, std::min(size, copies[i].bytes() - o)});
-  const int nt = (int)std::min<size_t>(HOST_COPY_THREADS, pieces.size());
-  cudaError_t err[HOST_COPY_THREADS];
-  std::fill(err, err + HOST_COPY_THREADS, cudaSuccess);
-  auto work = [&](int t, int step) { /* pieces t, t + step, ... through the thread's two slots */
-    cudaError_t q = cudaSetDevice(device);
-    auto start = [&](size_t p, int b) {
-      const Piece &x = pieces[p];
-      char *slot = pinned_ + (2 * t + b) * slot_;
-      q = cudaMemcpyAsync(slot, copies[x.copy].src + x.off, x.n, cudaMemcpyDeviceToHost, s);
-      if (q == cudaSuccess) q = cudaEventRecord(ev_[2 * t + b], s);
-    };
-    int b = 0;
-    if (q == cudaSuccess && (size_t)t < pieces.size()) start(t, 0);
-    for (size_t p = t; q == cudaSuccess && p < pieces.size(); p += step, b ^= 1) {
-      if (p + step < pieces.size()) start(p + step, b ^ 1);
-      if (q == cudaSuccess) q = cudaEventSynchronize(ev_[2 * t + b]);
-      if (q == cudaSuccess)
-        scatter(copies, pieces[p].copy, pieces[p].off, pinned_ + (2 * t + b) * slot_, pieces[p].n);
-    }
-    err[t] = q;
+  const size_t rounds = (total + half_ - 1) / half_;
+  const unsigned cores = std::thread::hardware_concurrency();
+  const int nt = (int)std::max<size_t>(1, std::min<size_t>({(size_t)HOST_COPY_THREADS, total >> 19, cores / 2}));
+  int made = 1;                     /* threads with a share, this one included */
+  std::atomic<size_t> round{0};     /* rounds published; ~0: no more */
+  std::atomic<int> left{0};         /* shares of the round still to be stored */
+  auto share = [&](size_t r, int t, int n) { /* the t-th of n shares of round r */
+    const size_t lo = r * half_, len = std::min(half_, total - lo);
+    const size_t a = len * t / n, b = len * (t + 1) / n;
+    scatter(copies, lo + a, lo + b, pinned_ + (r & 1) * half_ + a);
   };
+  std::atomic<int> team{0}; /* = made once it is known */
+  auto work = [&](int t) {
+    for (size_t seen = 0;;) {
+      size_t r;
+      while ((r = round.load(std::memory_order_acquire)) == seen) std::this_thread::yield();
+      if (r == ~(size_t)0) return;
+      share(r - 1, t, team.load(std::memory_order_relaxed));
+      seen = r;
+      left.fetch_sub(1, std::memory_order_release);
+    }
+  };
+  auto start = [&](size_t r) { /* the DMA of round r into its half */
+    const size_t lo = r * half_, hi = std::min(total, lo + half_);
+    char *slot = pinned_ + (r & 1) * half_;
+    cudaError_t e = cudaSuccess;
+    parts(copies, lo, hi, [&](const HostCopy &c, size_t off, size_t n) {
+      if (e == cudaSuccess) e = cudaMemcpyAsync(slot, c.src + off, n, cudaMemcpyDeviceToHost, s);
+      slot += n;
+    });
+    return e == cudaSuccess ? cudaEventRecord(ev_[r & 1], s) : e;
+  };
+  cudaError_t e = rounds ? start(0) : cudaSuccess;
   std::thread th[HOST_COPY_THREADS];
-  int made = 1;
   try {
-    for (; made < nt; made++) th[made] = std::thread(work, made, nt);
-  } catch (const std::system_error &) { /* fewer threads: this one takes the others' pieces below */
+    for (; made < nt; made++) th[made] = std::thread(work, made);
+  } catch (const std::system_error &) { /* fewer threads: larger shares */
   }
-  if (nt > 0) work(0, nt);
-  for (int t = made; t < nt; t++) work(t, nt);
+  team.store(made, std::memory_order_relaxed);
+  for (size_t r = 0; r < rounds && e == cudaSuccess; r++) {
+    if (r + 1 < rounds) e = start(r + 1); /* its half was stored in round r - 1 */
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev_[r & 1]);
+    if (e != cudaSuccess) break;
+    left.store(made - 1, std::memory_order_relaxed);
+    round.store(r + 1, std::memory_order_release);
+    share(r, 0, made);
+    while (left.load(std::memory_order_acquire) > 0) std::this_thread::yield();
+  }
+  round.store(~(size_t)0, std::memory_order_release);
   for (int t = 1; t < made; t++) th[t].join();
-  for (int t = 0; t < nt; t++)
-    if (err[t] != cudaSuccess) e = err[t];
-  if (e != cudaSuccess) cudaStreamSynchronize(s); /* nothing may still write the slots */
+  if (e != cudaSuccess) cudaStreamSynchronize(s); /* nothing may still write the halves */
   return e;
 }
 
