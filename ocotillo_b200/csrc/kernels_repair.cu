@@ -349,35 +349,54 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
     aa[j * 32] = g;
     dd[j * 32] = e.u;
   };
+  /* two groups of levels that take turns, and the next pair of groups into L2 */
+  constexpr int G = RG_ALONE;
+  struct Row {
+    double a, c, d, e;
+  } A[G], B[G];
+  auto load = [&](Row *l, int j0) {
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      const int k = min(j0 + i, nz - 1) * 32;
+      l[i] = Row{aa[k], cc[k], dd[k], ee[k]};
+    }
+  };
+  auto steps = [&](const Row *l, int j0) {
+#pragma unroll
+    for (int i = 0; i < G; i++) step(j0 + i, l[i].a, l[i].c, l[i].d, l[i].e);
+  };
   int j = 1;
-  for (; j + 8 <= nz; j += 8) { /* the coefficients of 8 levels loaded ahead of the serial chain */
-    for (int t = 16; t < 24 && j + t < nz; t++) { /* the block after next into L2 */
+  load(A, 1);
+#pragma unroll 1
+  for (; j + 2 * G <= nz; j += 2 * G) {
+    for (int t = 4 * G; t < 6 * G && j + t < nz; t++) {
       prefetch_l2(&aa[(j + t) * 32]);
       prefetch_l2(&cc[(j + t) * 32]);
       prefetch_l2(&dd[(j + t) * 32]);
       prefetch_l2(&ee[(j + t) * 32]);
     }
-    double ab[8], cb[8], db[8], eb[8];
-#pragma unroll
-    for (int t = 0; t < 8; t++) {
-      ab[t] = aa[(j + t) * 32];
-      cb[t] = cc[(j + t) * 32];
-      db[t] = dd[(j + t) * 32];
-      eb[t] = ee[(j + t) * 32];
-    }
-#pragma unroll
-    for (int t = 0; t < 8; t++) step(j + t, ab[t], cb[t], db[t], eb[t]);
+    load(B, j + G);
+    steps(A, j);
+    load(A, j + 2 * G);
+    steps(B, j + G);
   }
-  for (; j < nz; j++) step(j, aa[j * 32], cc[j * 32], dd[j * 32], ee[j * 32]);
+  Row x = A[0];
+#pragma unroll 1
+  for (; j < nz; j++) { /* one level loaded ahead */
+    const int k = min(j + 1, nz - 1) * 32;
+    const Row nx{aa[k], cc[k], dd[k], ee[k]};
+    step(j, x.a, x.c, x.d, x.e);
+    x = nx;
+  }
   if (bad) {
     atomicAdd(&it.status()[0], 1ull);
     atomicMin(&it.status()[1], it.id());
   }
   LaneStores<false> st = lane_stores(it);
-  solve_reverse<1, RG, true>(it, true, e.u, aa, dd, S.o1 + q0, ee, st);
+  solve_reverse<1, RG_ALONE, true>(it, true, e.u, aa, dd, S.o1 + q0, ee, st);
 }
 
-__global__ void __launch_bounds__(REPAIR_THREADS, 6) k_repair_solve(const RepairArgs a) {
+__global__ void __launch_bounds__(REPAIR_THREADS, 4) k_repair_solve(const RepairArgs a) {
   __shared__ __align__(16) double s_seg[RWARPS][sizeof(RSeg) / sizeof(double)];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;

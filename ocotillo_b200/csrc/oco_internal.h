@@ -250,7 +250,7 @@ struct RepairArgs {
 };
 /* Threads per block of k_repair_solve. */
 constexpr int REPAIR_THREADS = 64;
-constexpr int REPAIR_SOLVE_BLOCKS_PER_SM = 6;
+constexpr int REPAIR_SOLVE_BLOCKS_PER_SM = 4;
 constexpr int REPAIR_COEF_BLOCKS_PER_SM = 4;
 /* Slots that a scratch of scratch_bytes holds beside k_repair_solve's per-warp arrays. */
 int64_t repair_capacity(size_t scratch_bytes, int max_nz, int solve_blocks);
