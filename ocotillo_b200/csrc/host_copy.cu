@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <cstring>
 #include <system_error>
 #include <thread>
@@ -86,7 +87,12 @@ cudaError_t HostCopier::run(int device, cudaStream_t s, const std::vector<HostCo
   auto work = [&](int t) {
     for (size_t seen = 0;;) {
       size_t r;
-      while ((r = round.load(std::memory_order_acquire)) == seen) std::this_thread::yield();
+      for (int spins = 0; (r = round.load(std::memory_order_acquire)) == seen;) {
+        if (++spins < 4096) /* a round takes some 20 us; the first waits for the kernels */
+          std::this_thread::yield();
+        else
+          std::this_thread::sleep_for(std::chrono::microseconds(50));
+      }
       if (r == ~(size_t)0) return;
       share(r - 1, t, team.load(std::memory_order_relaxed));
       seen = r;
