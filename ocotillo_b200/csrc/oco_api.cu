@@ -6,8 +6,9 @@
  * wavelength-independent per-(column, z) quantities, then the persistent solve kernel
  * processes the chunk's (column, wavelength) items.  The device-array entry point writes
  * straight into the caller's arrays (either layout); the host-array entry point stages
- * each chunk through device buffers in the reference layout and copies them back with one
- * pitched copy per output, overlapping the next chunk's kernels with the copy-back.
+ * each chunk through device buffers in the reference layout and copies them back (pinned
+ * arrays with one pitched copy per output, large pageable ones through host_copy.h),
+ * overlapping the next chunk's kernels with the copy-back.
  */
 #include <cuda_runtime.h>
 

@@ -128,7 +128,8 @@ struct SolveArgs {
   int64_t ld_col, c_off;
   int layout;
   /* Scratch [warp slot][nz][32] each (slot_stride*nz values): forward-sweep gamma, u,
-   * kappa and (stable form) q, one contiguous block per warp. */
+   * 1/kappa (kappa where the reverse sweep stores it) and (stable form) q, one contiguous block
+   * per warp; the split solve lays its five arrays out from gam instead. */
   double *gam, *uu, *kap, *q;
   int64_t slot_stride; /* resident threads the scratch is sized for (each warp's block is 32*nz) */
   unsigned long long *work;   /* persistent-kernel work counter (warp tasks) */
