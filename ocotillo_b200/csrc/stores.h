@@ -108,9 +108,12 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
       if (V0) V0 += r8 * ks;
     }
   }
+  /* Before an item's first push.  The ring may lie over shared memory that the forward sweep read
+   * (StagedSmem, MStagedSmem): no lane writes it before every lane has left that sweep. */
   __device__ __forceinline__ void open(int n) {
     nz = n;
     base = 0;
+    __syncwarp();
   }
   static __device__ __forceinline__ int wrap(int s) { return s >= RING_Z ? s - RING_Z : s; }
   /* level m, the q-th of its group */
