@@ -185,16 +185,17 @@ __device__ __forceinline__ void store_lam_shared(double *table, int lane, const 
   for (int k = 0; k < NLF - 2; k++) table[64 + k * 32 + lane] = __ldg(lam + (int64_t)src[k] * nw + iw);
 }
 
-/* One pillar record, read through the read-only cache (global) or from shared memory. */
+/* One pillar record, read through the read-only cache (global, 16-byte aligned) or from shared or
+ * local memory. */
 struct GlobalRec {
   const double *p;
   __device__ __forceinline__ double operator[](int f) const { return __ldg(p + f); }
   __device__ __forceinline__ double2 pair(int f) const { return __ldg(reinterpret_cast<const double2 *>(p + f)); }
 };
 struct SharedRec {
-  const double *p;
-  __device__ __forceinline__ double operator[](int f) const { return p[f]; }
-  __device__ __forceinline__ double2 pair(int f) const { return *reinterpret_cast<const double2 *>(p + f); }
+  const PillarRecord *p;
+  __device__ __forceinline__ double operator[](int f) const { return p->f[f]; }
+  __device__ __forceinline__ double2 pair(int f) const { return *reinterpret_cast<const double2 *>(p->f + f); }
 };
 
 /* Opacity and source function of one (z, lambda), and the absorption fraction w = 1 - albedo

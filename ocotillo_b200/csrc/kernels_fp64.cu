@@ -139,10 +139,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
  * z, one at a time: entering chunk c frees the buffer of chunk c-1, which then receives
  * chunk c+1.  Waits are bounded; on timeout the warp records the failure and stops. */
 struct StagedPillars {
-  double *buf;    /* shared: [2][ZC*NF] */
+  PillarRecord *buf; /* shared: [2][ZC] */
   uint32_t bar0;  /* shared address of two mbarriers (8 B each) */
   const double *src;
-  const double *rec; /* next record, left of them in the buffer */
+  const PillarRecord *rec; /* next record, left of them in the buffer */
   int nz, nchunks, cur, left;
   uint32_t waits;    /* bit b: parity of the next wait on buffer b */
   uint32_t inflight; /* bit b: a copy into buffer b has been issued and not yet waited for */
@@ -152,7 +152,7 @@ struct StagedPillars {
     const int rows = min(ZC, nz - c * ZC);
     const uint32_t bytes = (uint32_t)(rows * NF * sizeof(double));
     const uint32_t bar = bar0 + 8u * (c & 1);
-    const uint32_t dst = smem_addr(buf + (c & 1) * (ZC * NF));
+    const uint32_t dst = smem_addr(buf + (c & 1) * ZC);
     const size_t g = __cvta_generic_to_global(src + (int64_t)c * ZC * NF);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -192,12 +192,12 @@ struct StagedPillars {
         note_issue(c + 1);
       }
       if (!failed && !wait(c & 1)) failed = true;
-      rec = buf + (c & 1) * (ZC * NF);
+      rec = buf + (c & 1) * ZC;
       left = ZC;
     }
     left--;
     const SharedRec r{rec};
-    rec += NF;
+    rec++;
     return r;
   }
 };
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
 struct StagedSmem {
   union {
     struct {
-      double pil[2 * ZC * NF];
+      PillarRecord pil[2 * ZC];
       double lam[NLF * 32];     /* the task's 32 wavelengths' constants */
       double2 tc[NTC / 2 * 32]; /* the lanes' temperature factors */
     };
@@ -289,7 +289,7 @@ struct StagedSmem {
   unsigned long long bar[2];
   __device__ StagedSmem() = delete;
 };
-static_assert(sizeof(StagedSmem) % 16 == 0 && (2 * ZC * NF * sizeof(double)) % 16 == 0, "bulk copies and 16-byte pairs");
+static_assert(sizeof(StagedSmem) % 16 == 0, "bulk copies and 16-byte pairs");
 
 __device__ __forceinline__ void init_staged(StagedPillars &pa, StagedSmem &sm) {
   pa.buf = sm.pil;

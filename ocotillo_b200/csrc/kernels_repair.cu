@@ -142,10 +142,10 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
     for (int k = lane; k < n + 2; k += 32) {
       const int z = z0 - 1 + k;
       if (z < 0 || z >= nz) continue;
-      double rec[NF];
-      pillar_record(rho[z], T[z], fit, 0, false, rec);
+      PillarRecord rec;
+      pillar_record(rho[z], T[z], fit, 0, false, rec.f);
       TCacheR tc;
-      Opac o = opacity_at<true>(SharedRec{rec}, L, tc);
+      Opac o = opacity_at<true>(SharedRec{&rec}, L, tc);
       settle_opac<true>(o);
       g.op[k] = o.op;
       if (Kb && k >= 1 && k <= n) Kb[z * kz] = o.op;
@@ -247,14 +247,14 @@ constexpr int CZ = 30;
 /* One flagged item's rows for the task's levels: lane l holds level zl = c*CZ - 1 + l and its
  * record rec (valid: 0 <= zl < nz). */
 template <class IT>
-__device__ __forceinline__ void coef_item(const IT &it, const double *rec, int zl, bool valid, const Slots &S,
+__device__ __forceinline__ void coef_item(const IT &it, const PillarRecord &rec, int zl, bool valid, const Slots &S,
                                           int64_t pos) {
   const int lane = threadIdx.x & 31;
   const LamR L(it, nullptr);
   Opac o{};
   if (valid) {
     TCacheR tc;
-    o = opacity_at<true>(SharedRec{rec}, L, tc);
+    o = opacity_at<true>(SharedRec{&rec}, L, tc);
     settle_opac<true>(o);
   }
   const double op_lo = __shfl_up_sync(0xffffffffu, o.op, 1), op_hi = __shfl_down_sync(0xffffffffu, o.op, 1);
@@ -290,13 +290,13 @@ __device__ __forceinline__ void coef_item(const IT &it, const double *rec, int z
 constexpr int CWARPS = 4; /* warps per block of k_repair_coef */
 
 __global__ void __launch_bounds__(CWARPS * 32, 4) k_repair_coef(const RepairArgs a) {
-  __shared__ __align__(16) double s_rec[CWARPS][32 * NF];
+  __shared__ PillarRecord s_rec[CWARPS][32];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const int64_t n_words = (int64_t)*a.count;
   const int nch = (a.max_nz + CZ - 1) / CZ;
   const unsigned long long ntasks = (unsigned long long)(n_words * nch);
   const Slots S(a);
-  double *rec = &s_rec[wib][lane * NF]; /* each lane reads only its own record */
+  PillarRecord &rec = s_rec[wib][lane]; /* each lane reads only its own record */
   /* tasks from a device counter, chunk-major (task t: chunk t / n_words of word t % n_words):
    * a task's cost grows with its word's flagged items, so a fixed assignment would leave some
    * warps with several times the mean */
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(CWARPS * 32, 4) k_repair_coef(const RepairArgs
     const double *T = a.block ? a.T + col * a.nz : a.T + bc->in_off;
     const int zl = c * CZ - 1 + lane;
     const bool valid = zl >= 0 && zl < nz && lane <= CZ + 1;
-    if (valid) pillar_record(rho[zl], T[zl], a.fully_ionized_T, 0, false, rec);
+    if (valid) pillar_record(rho[zl], T[zl], a.fully_ionized_T, 0, false, rec.f);
     for (unsigned m = a.bits[w]; m; m &= m - 1) {
       const int b = __ffs(m) - 1;
       const int64_t pos = a.slot[w * 32 + b];

@@ -54,7 +54,11 @@ enum PillarField {
   F_PAD1,
   NF
 };
-static_assert(NF % 2 == 0, "records are read in 16-byte pairs");
+/* A record in shared or local memory: the 16-byte pairs need its alignment wherever it is held. */
+struct alignas(16) PillarRecord {
+  double f[NF];
+};
+static_assert(sizeof(PillarRecord) == NF * sizeof(double), "records lie one after another");
 constexpr int FLAG_NEUTRAL = 1; /* (1 - NHII/N) > switch_ionfraction (c_o :262) */
 constexpr int FLAG_SAME_T = 2;  /* T equals the level below's bit for bit (never set at z = 0) */
 constexpr int FLAG_ESC_OK = 4;  /* e_scatter*mp1 passes div_a_ok (recip_div.h) */
