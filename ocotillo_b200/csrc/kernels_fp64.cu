@@ -413,12 +413,13 @@ __device__ __forceinline__ bool split_item(const SolveArgs &a, int64_t t, int64_
   return i < n;
 }
 
-/* Coefficient arrays of the tiles: [tile][z][32], in this order after one another. */
+/* Coefficient arrays of the tiles: [tile][z][32], in this order after one another; at level z0 of
+ * tile t. */
 struct SplitRows {
   double *aa, *xx, *cc, *dd, *kap; /* xx: diagonal (plain), its excess (stable); kap as the sweep's scratch */
-  __device__ __forceinline__ SplitRows(const SolveArgs &a, int64_t tiles, int64_t t) {
+  __device__ __forceinline__ SplitRows(const SolveArgs &a, int64_t tiles, int64_t t, int z0) {
     const int64_t plane = tiles * 32 * a.nz;
-    aa = a.gam + t * 32 * a.nz + (threadIdx.x & 31);
+    aa = a.gam + t * 32 * a.nz + tile_level(z0) + (threadIdx.x & 31);
     xx = aa + plane;
     cc = xx + plane;
     dd = cc + plane;
@@ -441,7 +442,7 @@ __global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tile
   const LamR L(it, nullptr, !GREY);
   TCacheR tc;
   GreyCell gc;
-  const SplitRows S(a, tiles, t);
+  const SplitRows S(a, tiles, t, z0);
   const int zf = max(z0 - 1, 0); /* first level computed */
   auto opac = [&](int z) -> Opac {
     Opac o;
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tile
     cur = up;
   }
   for (int j = z0; j < z1; j++) {
-    const int i = j * 32;
+    const int i = (j - z0) * 32;
     const double op = cur.op, o2 = op * op;
     double o1 = div_recip(op);
     if (!cur.ook) o1 = div_call(1.0, op);
@@ -513,16 +514,16 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles) 
   int iw;
   const bool active = split_item<TILE>(a, t, cl, iw);
   const BlockItem it{a, cl, iw};
-  const SplitRows S(a, tiles, t);
+  const SplitRows S(a, tiles, t, 0);
   bool bad = false;
   Chain e = chain_first<FORM>(S.xx[0], S.cc[0], S.dd[0], bad);
   S.dd[0] = e.u;
   auto step = [&](int j, double aa, double xx, double cc, double dd) {
     double g, q;
     chain_step<FORM>(e, aa, xx, cc, dd, g, q, bad);
-    S.aa[j * 32] = g;
-    S.dd[j * 32] = e.u;
-    if (FORM == 1) S.xx[(j - 1) * 32] = q; /* q_{j-1} over the excess of row j - 1 */
+    S.aa[tile_level(j)] = g;
+    S.dd[tile_level(j)] = e.u;
+    if (FORM == 1) S.xx[tile_level(j - 1)] = q; /* q_{j-1} over the excess of row j - 1 */
   };
   constexpr int G = RG_ALONE;
   struct Row {
@@ -531,7 +532,7 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles) 
   auto load = [&](Row *l, int j0) {
 #pragma unroll
     for (int i = 0; i < G; i++) {
-      const int k = min(j0 + i, nz - 1) * 32;
+      const int64_t k = tile_level(min(j0 + i, nz - 1));
       l[i] = Row{S.aa[k], S.xx[k], S.cc[k], S.dd[k]};
     }
   };
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles) 
   Row x = A[0];
 #pragma unroll 1
   for (; j < nz; j++) { /* one level loaded ahead */
-    const int k = min(j + 1, nz - 1) * 32;
+    const int64_t k = tile_level(min(j + 1, nz - 1));
     const Row nx{S.aa[k], S.xx[k], S.cc[k], S.dd[k]};
     step(j, x.a, x.x, x.c, x.d);
     x = nx;

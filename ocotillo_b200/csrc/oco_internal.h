@@ -143,6 +143,9 @@ struct SolveArgs {
 /* The split block solve (kernels_fp64.cu: k_rows, k_chain): warp tiles of a chunk, the doubles of its
  * scratch (SolveArgs::gam) and whether a chunk takes it. */
 int64_t split_tiles(int64_t ncol, int nw);
+/* Offset of level z in a warp tile's [z][32] arrays: 64 bits, since a lone column that fits the device
+ * can be taller than 2^26 levels. */
+__host__ __device__ constexpr int64_t tile_level(int z) { return (int64_t)z * 32; }
 inline size_t split_scratch_doubles(int64_t tiles, int nz) { return (size_t)tiles * 32 * (size_t)nz * 5; }
 bool solve_is_split(int grey, int64_t ncol, int nw, int num_sms);
 cudaError_t launch_solve_split(const SolveArgs &a, int form, int grey, const ChunkInit &init, cudaStream_t s);
