@@ -5,7 +5,6 @@
 #include <atomic>
 #include <chrono>
 #include <cstring>
-#include <system_error>
 #include <thread>
 
 namespace oco {
@@ -113,7 +112,8 @@ cudaError_t HostCopier::run(int device, cudaStream_t s, const std::vector<HostCo
   std::thread th[HOST_COPY_THREADS];
   try {
     for (; made < nt; made++) th[made] = std::thread(work, made);
-  } catch (const std::system_error &) { /* fewer threads: larger shares */
+  } catch (...) { /* no thread or no memory for one: fewer threads, larger shares.  Nothing may leave here
+                     past the started ones, which wait for a round */
   }
   team.store(made, std::memory_order_relaxed);
   for (size_t r = 0; r < rounds && e == cudaSuccess; r++) {
