@@ -7,8 +7,8 @@
  *                     items with direct loads when nw is small.  Forward sweep: log2-space
  *                     opacity, scaled rows and the difference-form Thomas elimination in FP32
  *                     (the source function's exponent as integer + FP32 fraction),
- *                     writing a scratch record per z (|gamma| or q, kappa, u mantissa and
- *                     exponent); reverse sweep: extended-range FP32 back-substitution, the
+ *                     writing a scratch record per z (|gamma| or q, kappa or 1/kappa, u mantissa
+ *                     and exponent); reverse sweep: extended-range FP32 back-substitution, the
  *                     differences D_j, and the flux from a 6-value window of differences, with
  *                     FP64 outputs (stores.h).
  * See mixed_core.h for the arithmetic and its relation to the reference.
@@ -177,7 +177,7 @@ __device__ __forceinline__ MItem block_item(const MixedArgs &a, int64_t cl, int 
 }
 
 /* The warp's Thomas scratch, one sequential stream per warp.  A record per level is
- * {v, kappa, u mantissa, u exponent} (see the forward sweep); two formats:
+ * {v, kappa or 1/kappa, u mantissa, u exponent} (see the forward sweep); two formats:
  *   MScratch16  one float4 per lane, 512 bytes per level;
  *   MScratch12  12 bytes per lane, 384 per level: the 32 lanes' {v, kappa} pairs (float2),
  *               then their u mantissas, with u's exponent packed into the spare bits of kappa
@@ -288,15 +288,23 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
   Opac32 nxt = opac(1);
   float kc = kappa_lin(cur), kn = kappa_lin(nxt);
   const float k0 = kc; /* kappa of the bottom level */
+  /* What a level's scratch record keeps of kappa: kappa itself where it leaves in the reverse sweep (the
+   * ring), else 1/kappa, which is all that the fluxes need then: kappa is stored by the forward sweep,
+   * and the reverse sweep, the longer chain, has no reciprocal, conversion and third store (ragged batch of
+   * 8192 columns 24.0 -> 22.1 ms, AGN grid of 4096 columns 6.60 -> 6.32 ms). */
+  constexpr bool KREV = ST::KAPPA_REVERSE;
+  auto keep = [](float k) -> float { return KREV || ST::PLANES ? k : rcp(k); };
+  auto kept_o1 = [](float y) -> float { return KREV || ST::PLANES ? rcp(y) : y; };
+  if (!KREV) st.k(0, (double)kc);
   Row32 r = row_boundary(kc, cur, dzf, dz2f, ldz2i, ldz2f, false);
   float h = r.e, cprev = r.c;
   float an = 2.0f * rcp(kn + kc); /* a' of row 1; then c' of the row below */
   XF u = xexp2(r.ldi, r.ldf);
   u = xnorm(u.m * (r.w * rcp(r.c + h)), u.e);
-  /* scratch record of z = j: {v_j, kappa_j, u_j mantissa, u_j exponent (int bits)} where v_j holds the
+  /* scratch record of z = j: {v_j, keep(kappa_j), u_j mantissa, u_j exponent (int bits)} where v_j holds the
    * smaller of q_j = h_j/(c_j+h_j) and |gamma_{j+1}| = c_j/(c_j+h_j) (they sum to 1; a negative
    * v_j stores -|gamma_{j+1}|), written once row j+1 is known */
-  float4 pend = make_float4(0.0f, kc, u.m, __int_as_float(u.e));
+  float4 pend = make_float4(0.0f, keep(kc), u.m, __int_as_float(u.e));
   bool fits = true;
   for (int j = 1; j < nz; j++) {
     cur = nxt;
@@ -316,7 +324,8 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
     h = r.e + (r.a * rr) * h; /* a'/(c'+h) is O(1); a' h alone can overflow */
     const float rb = rcp(r.c + h);
     u = xaxpy(xexp2(r.ldi, r.ldf), r.w * rb, u, r.a * rb);
-    pend = make_float4(0.0f, kc, u.m, __int_as_float(u.e));
+    pend = make_float4(0.0f, keep(kc), u.m, __int_as_float(u.e));
+    if (!KREV) st.k(j, (double)kc);
     cprev = r.c;
   }
   fits &= sc.put(nz - 1, pend);
@@ -368,16 +377,16 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       const double s2 = (s1 + d1) + d4;
       const double s3 = (s2 + d0) + d5;
       const double df = -((1.0 / 60.0) * (((45.0 * s1) - 9.0 * s2) + s3));
-      return ((-(double)rcp(kj)) * df) * dz1;
+      return ((-(double)kept_o1(kj)) * df) * dz1;
     };
     {
-      const float kj = kc; /* the top level's */
+      const float kj = keep(kc); /* the top level's */
       vtop = flux(kj);
       st.push(6, n - 1, Uk[2], vtop, (double)kj); /* U_{n-4}, V_{n-1} */
       st.template group<false>(n - 1, 7);
     }
     double U0 = Uk[2], U1 = Uk[1], U2 = Uk[0], U3 = fn; /* the four lowest U seen so far */
-    /* kappa ring: r1, r2, r3 = kappa of k+1, k+2, k+3 before step k */
+    /* r1, r2, r3 = what the records keep of kappa of k+1, k+2, k+3 before step k */
     float r1 = kt[2], r2 = kt[1], r3 = kt[0];
     auto step = [&](int slot, int k, const float4 &w) {
       const float g1 = (w.x >= 0.0f) ? 1.0f - w.x : -w.x; /* |gamma_{k+1}| */
@@ -489,9 +498,9 @@ __device__ __forceinline__ bool msolve_item(const MItem &it, bool active, PA &pa
       const int c = n1 + j;
       const double df = (1.0 / 60.0) * (((45.0 * (f[c + 1] - f[c - 1])) - 9.0 * (f[c + 2] - f[c - 2])) + (f[c + 3] - f[c - 3]));
       const float kj = ST::PLANES ? (j == 0 ? k0 : kc) : sc.kappa(j);
-      const double v = ((-(double)rcp(kj)) * df) * dz1;
+      const double v = ((-(double)kept_o1(kj)) * df) * dz1;
       st.v(j, v);
-      st.k(j, (double)kj);
+      if (KREV) st.k(j, (double)kj);
       if (j == 0) vbot = v;
       if (j == nz - 1) vtop = v;
     }
@@ -599,7 +608,7 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const Mixed
     store_lam32_shared(sm.lam, lane, a.lam, iw, a.nw);
     __syncwarp();
     const MItem it = block_item(a, cl, iw);
-    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, true>(it.o, active, &sm.ring),
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, false>(it.o, active, &sm.ring),
                                   a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
@@ -635,7 +644,7 @@ __global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
     MDirect pa{a.rec + cl * (int64_t)a.nz * MZN};
     const MItem it = block_item(a, cl, iw);
     const bool flag = msolve_item(it, active, pa, load_lam32(it.lam, iw, it.nw), sc,
-                                  make_stores<MODE, false, true>(it.o, active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
+                                  make_stores<MODE, false, false>(it.o, active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     mark_items(flag, cl * ((a.nw + 31) / 32) + iw / 32, iw, (unsigned long long)item, a.rbits, a.rslot, a.rlist, a.rcount,
                a.ilist, a.icount);
@@ -722,7 +731,7 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_batch_mixed_staged(const Mixed
     store_lam32_shared(sm.lam, lane, b.lam + c.lam_off, iw, c.nw);
     __syncwarp();
     const MItem it = batch_item(b, c, iw);
-    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, true>(it.o, active, &sm.ring),
+    const bool flag = msolve_item(it, active, pa, MLamS{sm.lam + lane}, sc, make_stores<MODE, true, false>(it.o, active, &sm.ring),
                                   b.repair_cond) ||
                       (active && __ldg(b.colflag + t.x) != 0u);
     if (__any_sync(0xffffffffu, pa.failed)) {
@@ -768,7 +777,7 @@ __global__ void __launch_bounds__(128, 4) k_batch_mixed_packed(const MixedBatchA
       MDirect pa{b.rec + c.rec_off * MZN};
       /* the lanes' columns differ in depth: each stores its own levels */
       const MItem it = batch_item(b, c, iw);
-      flag = msolve_item(it, true, pa, load_lam32(it.lam, iw, it.nw), sc, LaneStores<true>(it.o, true), b.repair_cond) ||
+      flag = msolve_item(it, true, pa, load_lam32(it.lam, iw, it.nw), sc, LaneStores<false>(it.o, true), b.repair_cond) ||
              __ldg(b.colflag + col) != 0u;
     }
     mark_items(flag, (int64_t)col * b.rwstride + iw / 32, iw, ((unsigned long long)(unsigned)col << 32) | (unsigned)iw,

@@ -557,7 +557,7 @@ MX_HD double xtod(XF x) {
   return (double)x.m * oco_u2d((uint64_t)(int64_t)(x.e + 1023) << 52);
 }
 
-/* kappa (> 0) and an XF u = m 2^e with m in [1, 2) in two 32-bit words: w1 = kappa with
+/* kappa or 1/kappa (> 0) and an XF u = m 2^e with m in [1, 2) in two 32-bit words: w1 = the former with
  * bit 9 of e + 512 in its sign bit, w2 = m's 23 fraction bits with bits 0-8 of e + 512 in its
  * sign and exponent field.  Returns whether the pair fits (e in [-512, 511], m normal in
  * [1, 2)); unpacking a fitting pair gives the same bits back. */

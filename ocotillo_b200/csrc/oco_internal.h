@@ -167,7 +167,7 @@ struct MixedArgs {
   double *Vtop, *Vbot;
   int64_t ld_col, c_off;
   int layout;
-  float4 *s4; /* scratch [warp slot][nz][32]: |gamma| or q, 1/kappa, u mantissa, u exponent (int bits) */
+  float4 *s4; /* scratch [warp slot][nz][32]: |gamma| or q, kappa or 1/kappa, u mantissa, u exponent (int bits) */
   int64_t slot_stride; /* resident threads the scratch is sized for */
   unsigned long long *work;
   unsigned long long *status;
