@@ -245,9 +245,12 @@ __device__ __forceinline__ OutPtrs out_ptrs(const IT &it) {
 }
 
 /* Generic path: warp tasks are 32 consecutive items of the flattened (column, lambda) index (lanes
- * past the last item repeat it and store nothing). */
+ * past the last item repeat it and store nothing).  Bound by latency, so by the warps in flight: at
+ * 202-208 registers two blocks fit an SM, three at 168 with some 50 bytes spilled (128 x 128 turbulent
+ * columns x 256 levels, 17 wavelengths: plain, z fastest 4.35 -> 3.23 ms; stable 4.06 -> 3.07 ms with
+ * lambda fastest, 4.48 -> 3.34 ms with z fastest). */
 template <int FORM, bool GREY, int MODE>
-__global__ void __launch_bounds__(128) k_solve(const SolveArgs a) {
+__global__ void __launch_bounds__(128, 3) k_solve(const SolveArgs a) {
   __shared__ RingSmem<double> s_ring[MODE == ST_RING ? WARPS_PER_BLOCK : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
