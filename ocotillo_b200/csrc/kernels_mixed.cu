@@ -623,9 +623,12 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const Mixed
 }
 
 /* Few wavelengths: 32 consecutive items per warp (lanes past the last item repeat it and store
- * nothing). */
+ * nothing).  Five blocks per SM at 96 registers with 28 bytes spilled (128 x 128 turbulent columns x 256
+ * levels, lambda fastest, four blocks at 126 registers -> five: 5 wavelengths 1.31 -> 1.06 ms, 17 2.06 ->
+ * 1.89 ms, 33 3.24 -> 2.97 ms, 3 0.98 ms both); the ring variant spills twice as much there and gains at
+ * 5 wavelengths only (1.41 -> 1.23 ms; 3 1.04 -> 1.15 ms, 17 and 33 the same). */
 template <class SC, int MODE>
-__global__ void __launch_bounds__(128, 4) k_solve_mixed(const MixedArgs a) {
+__global__ void __launch_bounds__(128, MODE == ST_RING ? 4 : 5) k_solve_mixed(const MixedArgs a) {
   __shared__ RingSmem<float> s_ring[MODE == ST_RING ? MWARPS : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
