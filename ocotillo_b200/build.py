@@ -26,7 +26,13 @@ COMMON = ARCH + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-con
 # (source, extra flags)
 UNITS = [
     ("kernels_fp64.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("kernels_fp64_items.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("kernels_fp64_staged.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("kernels_fp64_split.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
+    ("kernels_fp64_batch.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_mixed.cu", []),
+    ("kernels_mixed_items.cu", []),
+    ("kernels_mixed_batch.cu", []),
     ("kernels_repair.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_mixed_pillars.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("oco_api.cu", []),
@@ -39,7 +45,7 @@ UNITS = [
 ]
 HOST_UNITS = [("oco_deck.cpp", [])]
 
-HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "fp64_core.h", "recip_div.h", "stores.h", "host_copy.h", "disk_core.h",
+HEADERS = ["ocomath.h", "ocomath_tables.h", "oco_consts.h", "oco_internal.h", "oco_ctx.h", "mixed_core.h", "mixed_block.h", "fp64_core.h", "fp64_block.h", "recip_div.h", "stores.h", "host_copy.h", "disk_core.h",
            "batch_layout.h", "fortran_records.h"]
 
 

@@ -1,6 +1,6 @@
 /*
  * fp64_core.h -- the FP64 per-item arithmetic of the plain and stable forms, shared by the
- * FP64 kernels (kernels_fp64.cu) and the mixed kernels' FP64 re-solve of flagged items
+ * FP64 kernels (kernels_fp64*.cu) and the mixed kernels' FP64 re-solve of flagged items
  * (kernels_mixed.cu).
  *
  *   pillar_record  one (column, z) record: Saha ionization and every factor of the
@@ -12,7 +12,7 @@
  *                  Thomas sweep (:14-47) with its scratch, ghosts (:49-62) and flux (:64-109).
  *
  * Bit-faithfulness to the CPU oracle needs this code compiled without FMA contraction
- * (kernels_fp64.cu is built with -fmad=false); the exponentials and logarithms (ocomath) use
+ * (their units are built with -fmad=false); the exponentials and logarithms (ocomath) use
  * non-contracting intrinsics everywhere.
  */
 #ifndef OCO_FP64_CORE_H

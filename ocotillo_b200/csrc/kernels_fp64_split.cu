@@ -1,0 +1,261 @@
+/* kernels_fp64_split.cu -- the split FP64 block solve: few items, grey transfer (see kernels_fp64.cu). */
+#include "fp64_block.h"
+
+namespace oco {
+
+/* ---- the split block solve ------------------------------------------------------------- */
+/* With few items the persistent kernels leave most of the GPU idle while each warp walks its column
+ * alone (2 us per level and warp, whatever the number of warps: 16 columns x 500 x 250 took 1.03
+ * ms, 0.45 ms after the sweep's own changes).  Here everything that is independent along z runs
+ * first, parallel over (warp tile, RZ levels): k_rows writes the rows' coefficients; k_chain then
+ * runs the recurrences, one warp per tile, with nothing but them on its serial chain: 0.23 ms for
+ * those 16 columns.  That moves ~180 B per point instead of ~75, so it is taken while there are at
+ * most two tiles per SM (solve_is_split; a full wave of the persistent kernel holds 16), and for
+ * grey transfer always: it has one wavelength per column (few items) and no opacity sums, and reads
+ * rho and T directly instead of a 208-byte record per cell (16,384 columns x 512: 1.08 -> 0.43 ms).
+ * Per point the operations are solve_item's, so the same bits. */
+constexpr int RZ = 8; /* levels per warp of k_rows: two more are computed for the neighbours */
+
+/* One cell of a grey column (grey_parameters, continuous_opacity.f90:377-390); the factors of an
+ * unchanged temperature are kept. */
+struct GreyCell {
+  double t, p35, S;
+};
+template <bool STABLE>
+__device__ __forceinline__ Opac opacity_grey_cell(double r, double t, double sg, bool fresh, GreyCell &k) {
+  if (fresh || !same_bits(t, k.t)) {
+    const double t2 = t * t;
+    k.t = t;
+    k.S = sigma_sb * (t2 * t2);
+    k.p35 = 3.68e22 * oco_pow(t, -3.5);
+  }
+  const double alpha = k.p35 * r, tot = alpha + sg;
+  Opac o;
+  o.op = tot * r;
+  o.S = k.S;
+  o.num = STABLE ? alpha : sg;
+  o.kr = tot;
+  const double q = div_quot(o.num, tot, div_recip(tot));
+  o.w = STABLE ? q : 1.0 - q;
+  o.wok = div_b_ok(tot) & div_a_ok(o.num);
+  o.ook = op_ok(o.op);
+  return o;
+}
+
+/* The item of a lane: by_tile, wavelength tile*32 + lane of the tile's column, otherwise item
+ * tile*32 + lane of the flattened list; lanes past the end repeat the last. */
+__device__ __forceinline__ bool split_item(const SolveArgs &a, bool by_tile, int64_t t, int64_t &cl, int &iw) {
+  const int lane = threadIdx.x & 31;
+  if (by_tile) {
+    const int ntiles = (a.nw + 31) / 32;
+    cl = t / ntiles;
+    iw = (int)(t - cl * ntiles) * 32 + lane;
+    const bool on = iw < a.nw;
+    if (!on) iw = a.nw - 1;
+    return on;
+  }
+  const int64_t n = a.ncol * a.nw, i = t * 32 + lane, item = i < n ? i : n - 1;
+  cl = item / a.nw;
+  iw = (int)(item - cl * a.nw);
+  return i < n;
+}
+
+/* Coefficient arrays of the tiles: [tile][z][32], in this order after one another; at level z0 of
+ * tile t. */
+struct SplitRows {
+  double *aa, *xx, *cc, *dd, *kap; /* xx: diagonal (plain), its excess (stable); kap as the sweep's scratch */
+  __device__ __forceinline__ SplitRows(const SolveArgs &a, int64_t tiles, int64_t t, int z0) {
+    const int64_t plane = tiles * 32 * a.nz;
+    aa = a.gam + t * 32 * a.nz + tile_level(z0) + (threadIdx.x & 31);
+    xx = aa + plane;
+    cc = xx + plane;
+    dd = cc + plane;
+    kap = dd + plane;
+  }
+};
+
+/* by_tile: see split_item; ring: k_chain's outputs go through the ring, kappa among them (both uniform,
+ * so not worth code of their own: a process pays for loading each variant at its first solve). */
+template <int FORM, bool GREY>
+__global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tiles, bool by_tile, bool ring,
+                                                 const ChunkInit init) {
+  chunk_init(init, blockIdx.x * (int64_t)blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x);
+  const int nch = (a.nz + RZ - 1) / RZ;
+  const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w >= tiles * nch) return;
+  const int64_t t = w / nch;
+  const int nz = a.nz, z0 = (int)(w - t * nch) * RZ, z1 = min(z0 + RZ, nz);
+  int64_t cl;
+  int iw;
+  const bool active = split_item(a, by_tile, t, cl, iw);
+  const BlockItem it{a, cl, iw};
+  const LamR L(it, nullptr, !GREY);
+  TCacheR tc;
+  GreyCell gc;
+  const SplitRows S(a, tiles, t, z0);
+  const int zf = max(z0 - 1, 0); /* first level computed */
+  auto opac = [&](int z) -> Opac {
+    Opac o;
+    if constexpr (GREY)
+      o = opacity_grey_cell<FORM == 1>(__ldg(a.rho + cl * nz + z), __ldg(a.T + cl * nz + z), a.sigma_grey, z == zf, gc);
+    else
+      o = opacity_at<FORM == 1>(GlobalRec{a.pil + (cl * (int64_t)nz + z) * NF}, L, tc, z == zf);
+    settle_opac<FORM == 1>(o);
+    return o;
+  };
+  const double dz = a.dz, dz2 = a.dz2;
+  double *Kb = ring || !active ? nullptr : it.K();
+  const int64_t kz = it.kz();
+  double kh = 1.0, yk = 1.0; /* mean opacity below the level */
+  int okk = 0;
+  Opac cur = opac(zf);
+  auto mean = [&](const Opac &lo, const Opac &hi) {
+    kh = 0.5 * (hi.op + lo.op);
+    yk = div_recip(kh);
+    okk = lo.ook & hi.ook & div_b_frac_ok(kh);
+  };
+  if (z0 > 0) {
+    const Opac up = opac(z0);
+    mean(cur, up);
+    cur = up;
+  }
+  for (int j = z0; j < z1; j++) {
+    const int i = (j - z0) * 32;
+    const double op = cur.op, o2 = op * op;
+    double o1 = div_recip(op);
+    if (!cur.ook) o1 = div_call(1.0, op);
+    Opac nxt{};
+    if (j == 0 || j == nz - 1) { /* fill_boundary_coeffs :187-197 */
+      const double zt = ((op * dz2) * cur.w) * 0.25;
+      S.dd[i] = -((cur.S * zt) * o2);
+      S.xx[i] = FORM == 0 ? -(((o1 + dz) + zt) * o2) : (dz + zt) * o2;
+      S.aa[i] = op; /* row 0: unused */
+      S.cc[i] = j == 0 ? op : 0.0;
+      if (j == 0) {
+        nxt = opac(1);
+        mean(cur, nxt);
+      }
+    } else { /* fill_center_coeffs :159-165 */
+      nxt = opac(j + 1);
+      double aa = div_quot(o2, kh, yk);
+      if (!okk) aa = div_call(o2, kh);
+      mean(cur, nxt);
+      double cc = div_quot(o2, kh, yk);
+      if (!okk) cc = div_call(o2, kh);
+      const double z3 = (dz2 * (op * (op * op))) * cur.w;
+      S.aa[i] = aa;
+      S.cc[i] = cc;
+      S.xx[i] = FORM == 0 ? -((aa + cc) + z3) : z3;
+      S.dd[i] = -(cur.S * z3);
+    }
+    S.kap[i] = ring ? op : o1;
+    if (Kb) __stcs(&Kb[j * kz], op);
+    cur = nxt;
+  }
+}
+
+/* One warp per block, so that the tiles spread over the SMs.  ROWS: the ring's rows are one column's
+ * (by_tile). */
+template <int FORM, bool RING, bool ROWS>
+__global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, bool by_tile) {
+  __shared__ RingSmem<double> s_ring[1];
+  const int64_t t = blockIdx.x;
+  const int nz = a.nz;
+  int64_t cl;
+  int iw;
+  const bool active = split_item(a, by_tile, t, cl, iw);
+  const BlockItem it{a, cl, iw};
+  const SplitRows S(a, tiles, t, 0);
+  bool bad = false;
+  Chain e = chain_first<FORM>(S.xx[0], S.cc[0], S.dd[0], bad);
+  S.dd[0] = e.u;
+  auto step = [&](int j, double aa, double xx, double cc, double dd) {
+    double g, q;
+    chain_step<FORM>(e, aa, xx, cc, dd, g, q, bad);
+    S.aa[tile_level(j)] = g;
+    S.dd[tile_level(j)] = e.u;
+    if (FORM == 1) S.xx[tile_level(j - 1)] = q; /* q_{j-1} over the excess of row j - 1 */
+  };
+  constexpr int G = RG_ALONE;
+  struct Row {
+    double a, x, c, d;
+  } A[G], B[G];
+  auto load = [&](Row *l, int j0) {
+#pragma unroll
+    for (int i = 0; i < G; i++) {
+      const int64_t k = tile_level(min(j0 + i, nz - 1));
+      l[i] = Row{S.aa[k], S.xx[k], S.cc[k], S.dd[k]};
+    }
+  };
+  auto steps = [&](const Row *l, int j0) {
+#pragma unroll
+    for (int i = 0; i < G; i++) step(j0 + i, l[i].a, l[i].x, l[i].c, l[i].d);
+  };
+  int j = 1;
+  load(A, 1);
+#pragma unroll 1
+  for (; j + 2 * G <= nz && nz >= LONG_NZ; j += 2 * G) {
+    load(B, j + G);
+    steps(A, j);
+    load(A, j + 2 * G);
+    steps(B, j + G);
+  }
+  Row x = A[0];
+#pragma unroll 1
+  for (; j < nz; j++) { /* one level loaded ahead */
+    const int64_t k = tile_level(min(j + 1, nz - 1));
+    const Row nx{S.aa[k], S.xx[k], S.cc[k], S.dd[k]};
+    step(j, x.a, x.x, x.c, x.d);
+    x = nx;
+  }
+  if (active && bad) {
+    atomicAdd(&it.status()[0], 1ull);
+    atomicMin(&it.status()[1], it.id());
+  }
+  __syncwarp();
+  auto st = make_stores<RING ? ST_RING : ST_LANE, ROWS, false>(out_ptrs(it), active, s_ring);
+  solve_reverse<FORM, RG_ALONE>(it, active, e.u, S.aa, S.dd, S.kap, S.xx, st);
+}
+
+static bool split_by_tile(int nw) { return nw >= 64 || nw % 32 == 0; }
+int64_t split_tiles(int64_t ncol, int nw) {
+  return split_by_tile(nw) ? ncol * ((nw + 31) / 32) : (ncol * nw + 31) / 32;
+}
+bool solve_is_split(int grey, int64_t ncol, int nw, int num_sms) {
+  return grey || split_tiles(ncol, nw) <= 2 * (int64_t)num_sms;
+}
+
+/* Outputs with z fastest: through the ring only where they do not fit in L2, which otherwise joins the
+ * lanes' own stores into whole lines for nothing (16 columns x 500 x 250, 48 MB: 0.33 ms with the
+ * ring, 0.23 ms without; 16,384 grey columns, 201 MB: 0.44 and 0.42 ms). */
+constexpr int64_t SPLIT_RING_BYTES = 256ll << 20;
+
+template <int FORM>
+static cudaError_t launch_chain(const SolveArgs &a, int64_t tiles, bool by_tile, bool ring, cudaStream_t s) {
+  if (!ring)
+    k_chain<FORM, false, false><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, by_tile);
+  else if (by_tile)
+    k_chain<FORM, true, true><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, true);
+  else
+    k_chain<FORM, true, false><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, false);
+  return cudaGetLastError();
+}
+/* init: set up by k_rows where no record kernel comes before it (grey). */
+template <int FORM>
+static cudaError_t split_launch(const SolveArgs &a, int grey, const ChunkInit &init, cudaStream_t s) {
+  const bool by_tile = !grey && split_by_tile(a.nw);
+  const int64_t tiles = split_tiles(a.ncol, a.nw), warps = tiles * ((a.nz + RZ - 1) / RZ);
+  const bool ring = a.layout == 0 && tiles * 32 * (int64_t)a.nz * 24 > SPLIT_RING_BYTES;
+  const unsigned blocks = (unsigned)((warps + 3) / 4);
+  if (grey)
+    k_rows<FORM, true><<<blocks, 128, 0, s>>>(a, tiles, by_tile, ring, init);
+  else
+    k_rows<FORM, false><<<blocks, 128, 0, s>>>(a, tiles, by_tile, ring, init);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? launch_chain<FORM>(a, tiles, by_tile, ring, s) : e;
+}
+cudaError_t launch_solve_split(const SolveArgs &a, int form, int grey, const ChunkInit &init, cudaStream_t s) {
+  return form == 0 ? split_launch<0>(a, grey, init, s) : split_launch<1>(a, grey, init, s);
+}
+
+}  // namespace oco

@@ -300,10 +300,10 @@ static const int kSolveThreads = 128;
 
 /* Grid of the persistent solve kernel and its scratch: per resident thread and z, FP64
  * gamma, u, 1/kappa, q (32 B) or, for the mixed form, one record of at most 16 B. */
-static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz, int *blocks) {
+static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz, int nw, StoreMode mode, int *blocks) {
   const bool mixed = form == OCO_FORM_MIXED;
-  int bps = mixed ? solve_mixed_max_blocks_per_sm(kSolveThreads, c->nw)
-                  : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey, kSolveThreads);
+  int bps = mixed ? solve_mixed_max_blocks_per_sm(kSolveThreads, nw, mode)
+                  : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey, kSolveThreads, nw, mode);
   int64_t maxb = (int64_t)bps * c->num_sms;
   if (c->max_blocks > 0) maxb = std::min<int64_t>(maxb, c->max_blocks);
   int64_t need = (nitems + kSolveThreads - 1) / kSolveThreads;
@@ -379,7 +379,7 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
     c->ev_pil.emplace_back(e0, e1);
   }
   int blocks = 0;
-  int rc = prepare_solve(c, OCO_FORM_MIXED, 0, nb * p->nw, p->nz, &blocks);
+  int rc = prepare_solve(c, OCO_FORM_MIXED, 0, nb * p->nw, p->nz, p->nw, store_mode(a64.U, a64.K, a64.V, a64.layout), &blocks);
   if (rc) return rc;
   const size_t slots = (size_t)blocks * kSolveThreads;
   /* the re-solve takes over the mixed solve's scratch: at least its per-warp arrays and 32 slots */
@@ -477,7 +477,7 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
   if (split) {
     CU(c->scratch.ensure(split_scratch_doubles(split_tiles(nb, p->nw), p->nz) * sizeof(double)));
   } else {
-    int rc = prepare_solve(c, p->form, grey, nb * p->nw, p->nz, &blocks);
+    int rc = prepare_solve(c, p->form, grey, nb * p->nw, p->nz, p->nw, store_mode(a.U, a.K, a.V, a.layout), &blocks);
     if (rc) return rc;
   }
   const size_t slots = (size_t)blocks * kSolveThreads;
@@ -644,9 +644,9 @@ int oco_ctx_check_params(oco_ctx *c, const oco_params *p) {
 }
 
 int oco_ctx_full_blocks(oco_ctx *c, int form, int grey) {
-  const int bps = form == OCO_FORM_MIXED ? solve_mixed_max_blocks_per_sm(kSolveThreads, 64)
+  const int bps = form == OCO_FORM_MIXED ? solve_mixed_max_blocks_per_sm(kSolveThreads, 64, ST_LANE)
                                          : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey,
-                                                                        kSolveThreads);
+                                                                        kSolveThreads, 64, ST_LANE);
   return bps * c->num_sms;
 }
 

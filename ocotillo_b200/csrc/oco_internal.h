@@ -18,6 +18,13 @@ inline bool block_elements_fit(int nx, int ny, int nz, int nw) {
   return (double)nx * (double)ny * (double)nw * ((double)nz + 6.0) <= 72057594037927936.0;
 }
 
+/* How a kernel's warps store their outputs: lane by lane, through the ring of stores.h (z fastest), or
+ * only the emergent planes. */
+enum StoreMode { ST_LANE = 0, ST_RING = 1, ST_PLANES = 2 };
+inline StoreMode store_mode(const void *U, const void *K, const void *V, int layout) {
+  return !U && !K && !V ? ST_PLANES : layout == 0 ? ST_RING : ST_LANE;
+}
+
 /* Per-(column, z) quantities written by the pillar kernel and read by the solve kernels:
  * the wavelength-independent part of the reference's per-(z, lambda) work
  * (gas_state.f90:30-110 plus every factor of continuous_opacity.f90 that depends on z
@@ -140,7 +147,7 @@ struct SolveArgs {
   unsigned long long *status; /* [0] zero-pivot count, [1] first bad item (min), [2] timeout flag */
   const double *rho, *T;      /* split solve of a grey chunk: its inputs [ncol][nz] */
 };
-/* The split block solve (kernels_fp64.cu: k_rows, k_chain): warp tiles of a chunk, the doubles of its
+/* The split block solve (kernels_fp64_split.cu: k_rows, k_chain): warp tiles of a chunk, the doubles of its
  * scratch (SolveArgs::gam) and whether a chunk takes it. */
 int64_t split_tiles(int64_t ncol, int nw);
 /* Offset of level z in a warp tile's [z][32] arrays: 64 bits, since a lone column that fits the device
@@ -333,7 +340,10 @@ cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int
                            double fully_ionized_T, int grey, double *pil, const ChunkInit &init, cudaStream_t s);
 cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int nslot_blocks,
                               int threads, cudaStream_t s);
-int solve_fp64_max_blocks_per_sm(int form, int grey, int threads);
+/* Occupancy of the kernel used for nw and m (another's would be loaded for the question alone). */
+int solve_fp64_max_blocks_per_sm(int form, int grey, int threads, int nw, StoreMode m);
+const void *solve_items_fn(int form, int grey, StoreMode m);
+const void *solve_staged_fn(int form, StoreMode m);
 /* Runs the bounded-wait diagnostic kernel (one warp) on s; sets status[2] when the wait ran out. */
 cudaError_t launch_bounded_wait_check(long long limit, unsigned long long *status, cudaStream_t s);
 
@@ -348,7 +358,8 @@ constexpr int MIXED_LN = 29; /* fields of the mixed wavelength table */
 cudaError_t launch_pillars_mixed(const double *rho, const double *T, int64_t ncol, int nz, double fully_ionized_T,
                                  float *rec, unsigned *colflag, const ChunkInit &init, cudaStream_t s);
 cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s);
-int solve_mixed_max_blocks_per_sm(int threads, int nw); /* occupancy of the kernel used for nw */
+int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m);
+const void *solve_mixed_items_fn(StoreMode m);
 /* Fills tab32[MIXED_LN*nw] from the FP64 table tab[NL*nw]. */
 void fill_mixed_lambda_table(const double *tab, int nw, float *tab32);
 

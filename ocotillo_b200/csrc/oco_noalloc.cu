@@ -137,7 +137,8 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
    * column of pillars fits up to OCO_NOALLOC_MAX_NZ (static_assert above). */
   const size_t tab_bytes = grey ? 0 : round256((size_t)NL * nw * sizeof(double));
   const size_t avail = OCO_NOALLOC_WORKSPACE_BYTES - 256 - tab_bytes;
-  int nsm = 0, bps = solve_fp64_max_blocks_per_sm(p->form == OCO_FORM_STABLE ? 1 : 0, grey, kThreads);
+  int nsm = 0, bps = solve_fp64_max_blocks_per_sm(p->form == OCO_FORM_STABLE ? 1 : 0, grey, kThreads, nw,
+                                                  store_mode(U, kappa, V, p->layout));
   CUN(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const size_t per_block = scratch_block_bytes((size_t)nz), per_col = pillar_column_bytes((size_t)nz);
   const int64_t ncol = (int64_t)p->nx * p->ny;

@@ -26,6 +26,8 @@
 
 #include <cuda_runtime.h>
 
+#include "oco_internal.h"
+
 namespace oco {
 
 struct OutPtrs {
@@ -179,12 +181,7 @@ struct RingStores : LaneStores<true> { /* the base's stores serve columns of few
   }
 };
 
-/* How a kernel's warps store their outputs: lane by lane, through the ring (z fastest), or only the
- * emergent planes. */
-enum StoreMode { ST_LANE = 0, ST_RING = 1, ST_PLANES = 2 };
-inline StoreMode store_mode(const void *U, const void *K, const void *V, int layout) {
-  return !U && !K && !V ? ST_PLANES : layout == 0 ? ST_RING : ST_LANE;
-}
+/* The stores of a StoreMode. */
 template <int MODE, bool ROWS, bool KREV, class KT>
 __device__ __forceinline__ auto make_stores(const OutPtrs &o, bool active, RingSmem<KT> *ring) {
   if constexpr (MODE == ST_RING)
