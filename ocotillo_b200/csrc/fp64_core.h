@@ -380,9 +380,6 @@ __device__ __forceinline__ double scratch_o1(double a) {
  * are short and many warps run, 8 where a warp is alone with the latency (k_chain, 16 columns x 500
  * x 250: 455 us with a ring of 8, 281 us with groups of 4, 277 us with 8). */
 constexpr int RG = 4, RG_ALONE = 8;
-/* Shorter columns take the sweeps' rolled loops level by level: fetching straight-line code that runs
- * once or twice costs more than the loads' latency. */
-constexpr int LONG_NZ = 48;
 
 /* U_{k+1} -> U at the level above the returned k, which leaves at least the four bottom levels. */
 template <int G>
@@ -404,7 +401,7 @@ __device__ __forceinline__ double back_substitute(int &k, double U, const double
   };
   load(A, k);
 #pragma unroll 1
-  for (; k >= 2 * G + 3 && nz >= LONG_NZ; k -= 2 * G) {
+  for (; k >= 2 * G + 3; k -= 2 * G) {
     load(B, k - G);
     steps(A);
     load(A, k - 2 * G);
@@ -491,7 +488,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
       Un = back_substitute<G>(k, Un, gam, uu, ss, nz);
     load(A, k);
 #pragma unroll 1
-    for (; !ST::PLANES && k >= 2 * G - 1 && nz >= LONG_NZ; k -= 2 * G) {
+    for (; !ST::PLANES && k >= 2 * G - 1; k -= 2 * G) {
       if (PF)
         for (int p = 4 * G; p < 6 * G && k - p >= 0; p++) { /* two pairs of groups ahead into L2 */
           prefetch_l2(&uu[(k - p) * ss]);
@@ -585,7 +582,7 @@ __device__ __forceinline__ void solve_reverse(const IT &it, bool active, double 
     if (ST::PLANES) w0 = back_substitute<G>(kk, w0, gam, uu, ss, nz);
     load(A, kk);
 #pragma unroll 1
-    for (; !ST::PLANES && kk >= 2 * G - 1 && nz >= LONG_NZ; kk -= 2 * G) {
+    for (; !ST::PLANES && kk >= 2 * G - 1; kk -= 2 * G) {
       load(B, kk - G);
       steps(A, 0, kk);
       load(A, kk - 2 * G);

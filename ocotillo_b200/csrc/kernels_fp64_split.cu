@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, 
   int j = 1;
   load(A, 1);
 #pragma unroll 1
-  for (; j + 2 * G <= nz && nz >= LONG_NZ; j += 2 * G) {
+  for (; j + 2 * G <= nz; j += 2 * G) {
     load(B, j + G);
     steps(A, j);
     load(A, j + 2 * G);
