@@ -80,7 +80,8 @@ int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m) {
 
 cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_mixed_fn(a.nw, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
+  const StoreMode m = mixed_store_mode(a.U, a.K, a.V, a.layout, a.ncol * a.nw, a.nz);
+  return cudaLaunchKernel(solve_mixed_fn(a.nw, m), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

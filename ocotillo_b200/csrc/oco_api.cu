@@ -379,7 +379,8 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
     c->ev_pil.emplace_back(e0, e1);
   }
   int blocks = 0;
-  int rc = prepare_solve(c, OCO_FORM_MIXED, 0, nb * p->nw, p->nz, p->nw, store_mode(a64.U, a64.K, a64.V, a64.layout), &blocks);
+  int rc = prepare_solve(c, OCO_FORM_MIXED, 0, nb * p->nw, p->nz, p->nw,
+                         mixed_store_mode(a64.U, a64.K, a64.V, a64.layout, nb * p->nw, p->nz), &blocks);
   if (rc) return rc;
   const size_t slots = (size_t)blocks * kSolveThreads;
   /* the re-solve takes over the mixed solve's scratch: at least its per-warp arrays and 32 slots */

@@ -25,6 +25,18 @@ inline StoreMode store_mode(const void *U, const void *K, const void *V, int lay
   return !U && !K && !V ? ST_PLANES : layout == 0 ? ST_RING : ST_LANE;
 }
 
+/* The same for a mixed chunk of `items` items: z fastest takes the ring only where the outputs leave L2,
+ * which otherwise joins the lanes' own stores into whole lines, and the warps are few, so that each waits
+ * for its own ring (lanes / ring: 16 columns x 500 levels x 250 wavelengths, 48 MB, 0.37 / 0.51 ms; 16 x
+ * 33 x 5 60 / 71 us; 148 x 512 x 32, 58 MB, the same; 256 x 256 x 64, 101 MB, 0.38 / 0.36 ms; 1024 x 128
+ * x 64, 201 MB, 0.56 / 0.32 ms). */
+constexpr int64_t MIXED_RING_BYTES = 56ll << 20;
+inline StoreMode mixed_store_mode(const void *U, const void *K, const void *V, int layout, int64_t items, int nz) {
+  const int64_t bytes = items * nz * (int64_t)sizeof(double) * ((U != nullptr) + (K != nullptr) + (V != nullptr));
+  const StoreMode m = store_mode(U, K, V, layout);
+  return m == ST_RING && bytes <= MIXED_RING_BYTES ? ST_LANE : m;
+}
+
 /* Per-(column, z) quantities written by the pillar kernel and read by the solve kernels:
  * the wavelength-independent part of the reference's per-(z, lambda) work
  * (gas_state.f90:30-110 plus every factor of continuous_opacity.f90 that depends on z
