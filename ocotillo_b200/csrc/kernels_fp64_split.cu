@@ -14,8 +14,6 @@ namespace oco {
  * grey transfer always: it has one wavelength per column (few items) and no opacity sums, and reads
  * rho and T directly instead of a 208-byte record per cell (16,384 columns x 512: 1.08 -> 0.43 ms).
  * Per point the operations are solve_item's, so the same bits. */
-constexpr int RZ = 8; /* levels per warp of k_rows: two more are computed for the neighbours */
-
 /* One cell of a grey column (grey_parameters, continuous_opacity.f90:377-390); the factors of an
  * unchanged temperature are kept. */
 struct GreyCell {
@@ -217,14 +215,6 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, 
   solve_reverse<FORM, RG_ALONE>(it, active, e.u, S.aa, S.dd, S.kap, S.xx, st);
 }
 
-static bool split_by_tile(int nw) { return nw >= 64 || nw % 32 == 0; }
-int64_t split_tiles(int64_t ncol, int nw) {
-  return split_by_tile(nw) ? ncol * ((nw + 31) / 32) : (ncol * nw + 31) / 32;
-}
-bool solve_is_split(int grey, int64_t ncol, int nw, int num_sms) {
-  return grey || split_tiles(ncol, nw) <= 2 * (int64_t)num_sms;
-}
-
 /* Outputs with z fastest: through the ring only where they do not fit in L2, which otherwise joins the
  * lanes' own stores into whole lines for nothing (16 columns x 500 x 250, 48 MB: 0.33 ms with the
  * ring, 0.23 ms without; 16,384 grey columns, 201 MB: 0.44 and 0.42 ms). */
@@ -244,9 +234,9 @@ static cudaError_t launch_chain(const SolveArgs &a, int64_t tiles, bool by_tile,
 template <int FORM>
 static cudaError_t split_launch(const SolveArgs &a, int grey, const ChunkInit &init, cudaStream_t s) {
   const bool by_tile = !grey && split_by_tile(a.nw);
-  const int64_t tiles = split_tiles(a.ncol, a.nw), warps = tiles * ((a.nz + RZ - 1) / RZ);
+  const int64_t tiles = split_tiles(a.ncol, a.nw);
   const bool ring = a.layout == 0 && tiles * 32 * (int64_t)a.nz * 24 > SPLIT_RING_BYTES;
-  const unsigned blocks = (unsigned)((warps + 3) / 4);
+  const unsigned blocks = (unsigned)split_row_blocks(tiles, a.nz);
   if (grey)
     k_rows<FORM, true><<<blocks, 128, 0, s>>>(a, tiles, by_tile, ring, init);
   else

@@ -467,7 +467,7 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
     e3 = c->take_event();
     CU(cudaEventRecord(e0, s));
   }
-  const bool split = solve_is_split(grey, nb, p->nw, c->num_sms);
+  const bool split = solve_is_split(grey, nb, p->nw, p->nz, c->num_sms, c->max_blocks);
   const ChunkInit init = take_init(c);
   if (!grey) CU(launch_pillars(rho, T, nb, p->nz, p->fully_ionized_T, 0, c->pil.as<double>(), init, s));
   if (c->prof) {

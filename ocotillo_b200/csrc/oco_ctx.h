@@ -68,7 +68,7 @@ struct oco_ctx {
   oco::HostCopier host_copy; /* outputs of the host-array path into pageable arrays */
   int64_t launches = 0;
   size_t budget_bytes = 8ull << 30; /* chunk budget for pillars + staged outputs */
-  int max_blocks = 0;               /* cap on the persistent grid (0: occupancy limit x SMs) */
+  int max_blocks = 0;               /* cap on the solve's grids (0: none; persistent: occupancy limit x SMs) */
   /* kernel timing (oco_set_profiling) */
   bool prof = false;
   /* device-array calls defer the zero-pivot check to oco_synchronize */
@@ -92,8 +92,8 @@ struct oco_ctx {
   }
 };
 
-/* Enqueues columns [c0, c0 + nb) of a block on stream s: the record kernel and the persistent
- * solve, with the solve grid capped at max_blocks (0: no cap).  Outputs (device arrays of the
+/* Enqueues columns [c0, c0 + nb) of a block on stream s: the record kernel and the solve, with the solve's
+ * grids capped at max_blocks (0: no cap; not for grey transfer, which the server does not take).  Outputs (device arrays of the
  * whole block, layout p->layout; any may be NULL) are written for those columns only.  Zero
  * pivots and timeouts accumulate in the context's status until oco_ctx_read_status. */
 int oco_ctx_run_columns(oco_ctx *c, const oco_params *p, const double *rho, const double *T, int64_t c0, int64_t nb,

@@ -161,12 +161,24 @@ struct SolveArgs {
 };
 /* The split block solve (kernels_fp64_split.cu: k_rows, k_chain): warp tiles of a chunk, the doubles of its
  * scratch (SolveArgs::gam) and whether a chunk takes it. */
-int64_t split_tiles(int64_t ncol, int nw);
+constexpr int RZ = 8; /* levels per warp of k_rows: two more are computed for the neighbours */
+inline bool split_by_tile(int nw) { return nw >= 64 || nw % 32 == 0; }
+inline int64_t split_tiles(int64_t ncol, int nw) {
+  return split_by_tile(nw) ? ncol * ((nw + 31) / 32) : (ncol * nw + 31) / 32;
+}
+/* Blocks of k_rows (four warps each); k_chain has a one-warp block per tile. */
+inline int64_t split_row_blocks(int64_t tiles, int nz) { return (tiles * ((nz + RZ - 1) / RZ) + 3) / 4; }
+/* max_blocks: the caller's cap on the grid (0: none), which the split solve's grids must fit. */
+inline bool solve_is_split(int grey, int64_t ncol, int nw, int nz, int num_sms, int max_blocks) {
+  const int64_t tiles = split_tiles(ncol, nw);
+  if (grey) return true;
+  if (max_blocks > 0 && (tiles > max_blocks || split_row_blocks(tiles, nz) > max_blocks)) return false;
+  return tiles <= 2 * (int64_t)num_sms;
+}
 /* Offset of level z in a warp tile's [z][32] arrays: 64 bits, since a lone column that fits the device
  * can be taller than 2^26 levels. */
 __host__ __device__ constexpr int64_t tile_level(int z) { return (int64_t)z * 32; }
 inline size_t split_scratch_doubles(int64_t tiles, int nz) { return (size_t)tiles * 32 * (size_t)nz * 5; }
-bool solve_is_split(int grey, int64_t ncol, int nw, int num_sms);
 cudaError_t launch_solve_split(const SolveArgs &a, int form, int grey, const ChunkInit &init, cudaStream_t s);
 
 /* Arguments of the mixed-precision solve kernels. */

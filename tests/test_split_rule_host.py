@@ -1,0 +1,39 @@
+"""Which chunks take the split block solve (oco_internal.h), compiled for the host: few tiles and grey
+transfer, and never with grids beyond the caller's cap, by which a server shares the GPU between jobs."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+BUILD = os.path.join(ROOT, "tests", "_build")
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def h():
+    os.makedirs(BUILD, exist_ok=True)
+    out = os.path.join(BUILD, "libsplit_rule_host.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-I", "/usr/local/cuda/include", "-I",
+                    os.path.join(ROOT, "ocotillo_b200", "csrc"), "-o", out,
+                    os.path.join(ROOT, "tests", "split_rule_host.cpp")], check=True, capture_output=True)
+    lib = ctypes.CDLL(out)
+    lib.split_rule.argtypes = [ctypes.c_int, ctypes.c_int64] + [ctypes.c_int] * 4
+    lib.split_grid.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int]
+    lib.split_grid.restype = ctypes.c_int64
+    return lib
+
+
+@pytest.mark.parametrize("cap", [1, 7, 74, 148, 592])
+@pytest.mark.parametrize("ncol,nw,nz", [(1, 64, 2), (1, 64, 512), (16, 250, 500), (148, 64, 33), (992, 5, 33), (40, 33, 9)])
+def test_the_split_grids_fit_the_cap(h, cap, ncol, nw, nz):
+    grid = h.split_grid(ncol, nw, nz)
+    assert h.split_rule(0, ncol, nw, nz, SMS, cap) == (grid <= cap)
+    assert h.split_rule(0, ncol, nw, nz, SMS, 0) == 1
+
+
+@pytest.mark.parametrize("ncol,nw,split", [(296, 32, 1), (297, 32, 0), (1894, 5, 1), (1895, 5, 0), (37, 250, 1), (38, 250, 0)])
+def test_two_tiles_per_sm(h, ncol, nw, split):
+    assert h.split_rule(0, ncol, nw, 100, SMS, 0) == split
+    assert h.split_rule(1, ncol, 1, 100, SMS, 0) == 1
