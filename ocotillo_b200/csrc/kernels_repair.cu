@@ -345,9 +345,9 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
   auto step = [&](int j, double a_, double c_, double d_, double e_) {
     double g, q;
     chain_step<1>(e, a_, e_, c_, d_, g, q, bad);
-    ee[(j - 1) * 32] = q; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
-    aa[j * 32] = g;
-    dd[j * 32] = e.u;
+    ee[tile_level(j - 1)] = q; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
+    aa[tile_level(j)] = g;
+    dd[tile_level(j)] = e.u;
   };
   /* two groups of levels that take turns, and the next pair of groups into L2 */
   constexpr int G = RG_ALONE;
@@ -357,7 +357,7 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
   auto load = [&](Row *l, int j0) {
 #pragma unroll
     for (int i = 0; i < G; i++) {
-      const int k = min(j0 + i, nz - 1) * 32;
+      const int64_t k = tile_level(min(j0 + i, nz - 1));
       l[i] = Row{aa[k], cc[k], dd[k], ee[k]};
     }
   };
@@ -370,10 +370,10 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
 #pragma unroll 1
   for (; j + 2 * G <= nz; j += 2 * G) {
     for (int t = 4 * G; t < 6 * G && j + t < nz; t++) {
-      prefetch_l2(&aa[(j + t) * 32]);
-      prefetch_l2(&cc[(j + t) * 32]);
-      prefetch_l2(&dd[(j + t) * 32]);
-      prefetch_l2(&ee[(j + t) * 32]);
+      prefetch_l2(&aa[tile_level(j + t)]);
+      prefetch_l2(&cc[tile_level(j + t)]);
+      prefetch_l2(&dd[tile_level(j + t)]);
+      prefetch_l2(&ee[tile_level(j + t)]);
     }
     load(B, j + G);
     steps(A, j);
@@ -383,7 +383,7 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
   Row x = A[0];
 #pragma unroll 1
   for (; j < nz; j++) { /* one level loaded ahead */
-    const int k = min(j + 1, nz - 1) * 32;
+    const int64_t k = tile_level(min(j + 1, nz - 1));
     const Row nx{aa[k], cc[k], dd[k], ee[k]};
     step(j, x.a, x.c, x.d, x.e);
     x = nx;
