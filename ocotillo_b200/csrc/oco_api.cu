@@ -467,7 +467,7 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
     e3 = c->take_event();
     CU(cudaEventRecord(e0, s));
   }
-  const bool split = solve_is_split(grey, nb, p->nw, p->nz, c->num_sms, c->max_blocks);
+  bool split = solve_is_split(grey, nb, p->nw, p->nz, c->num_sms, c->max_blocks);
   const ChunkInit init = take_init(c);
   if (!grey) CU(launch_pillars(rho, T, nb, p->nz, p->fully_ionized_T, 0, c->pil.as<double>(), init, s));
   if (c->prof) {
@@ -476,8 +476,15 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
   }
   int blocks = 0;
   if (split) {
-    CU(c->scratch.ensure(split_scratch_doubles(split_tiles(nb, p->nw), p->nz) * sizeof(double)));
-  } else {
+    const cudaError_t e = c->scratch.ensure(split_scratch_doubles(split_tiles(nb, p->nw), p->nz) * sizeof(double));
+    if (e == cudaErrorMemoryAllocation && !grey) { /* the persistent solve keeps four fifths of that */
+      cudaGetLastError();
+      split = false;
+    } else {
+      CU(e);
+    }
+  }
+  if (!split) {
     int rc = prepare_solve(c, p->form, grey, nb * p->nw, p->nz, p->nw, store_mode(a.U, a.K, a.V, a.layout), &blocks);
     if (rc) return rc;
   }

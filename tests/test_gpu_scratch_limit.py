@@ -1,0 +1,52 @@
+"""A block whose split-solve scratch does not fit the free device memory, but whose persistent solve's
+does (four fifths of it), is solved all the same, with the same bits."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+NZ, NW = 100_000, 256  # 8 tiles: 1024 MB of split scratch, 819 MB of the persistent solve's
+
+
+@pytest.mark.parametrize("form", ["plain", "stable"])
+def test_split_scratch_does_not_fit(form):
+    import torch
+
+    from ocotillo_b200 import Engine, workloads
+    rho, T, dz = workloads.agn_block(1, 1, NZ, seed=1)
+    r, t = torch.from_numpy(rho).cuda(), torch.from_numpy(T).cuda()
+    new = lambda: {k: torch.full((NW, 1, 1), -1.0, dtype=torch.float64, device="cuda") for k in ("Vtop", "Vbot")}
+
+    def solve(e, out):
+        e.set_wavelengths(workloads.log_wavelengths(NW))
+        e.solve_block_device(r, t, dz, out, form=form)
+        try:
+            e.synchronize()
+        except Exception as x:  # a zero pivot of the plain form
+            assert form == "plain" and "EZEROPIVOT" in str(x)
+        return {k: v.cpu().numpy() for k, v in out.items()}
+
+    e, tight, free = Engine(0), new(), new()
+    # the kernels of both solves loaded, so that the free memory is what the scratch gets
+    for ncol in (1, 40):
+        e.set_wavelengths(workloads.log_wavelengths(NW))
+        a, b, d = workloads.agn_block(1, ncol, 8, seed=2)
+        small = {k: torch.empty((NW, 1, ncol), dtype=torch.float64, device="cuda") for k in ("Vtop", "Vbot")}
+        e.solve_block_device(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), d, small, form=form)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    left = torch.cuda.mem_get_info()[0]
+    fill = torch.empty(left - 940_000_000, dtype=torch.uint8, device="cuda")  # records 21 MB, the rest for the scratch
+    n0 = e.kernel_launches()
+    got = solve(e, tight)
+    assert e.kernel_launches() - n0 == 2  # records and the persistent solve
+    del fill
+    torch.cuda.empty_cache()
+    e.close()
+    e = Engine(0)
+    n0 = e.kernel_launches()
+    ref = solve(e, free)
+    assert e.kernel_launches() - n0 == 3  # records and the split solve's two
+    e.close()
+    for k in ref:
+        assert np.array_equal(got[k].view(np.uint64), ref[k].view(np.uint64)), k
