@@ -20,7 +20,15 @@
 namespace oco {
 
 constexpr int HOST_COPY_THREADS = 8;
-constexpr size_t HOST_COPY_MIN = 512u << 10; /* smaller outputs take the driver's copies */
+/* Smaller outputs take the driver's copies: starting the threads costs a call some 0.1 ms, which arrays that
+ * the caller keeps (no faults) never give back (kept / fresh arrays, driver's copies and these: 2 MB 0.35
+ * and 0.61 ms / 1.21 and 0.84 ms; 3 MB 0.43 and 0.45 / 1.71 and 0.80; 3.5 MB 0.47 and 0.38 / 1.98 and
+ * 0.86). */
+constexpr size_t HOST_COPY_MIN = 3u << 20;
+/* Output bytes that a context has seen when it pins its halves, which takes 1.5-2 ms of that call (4 MB: 4.6
+ * -> 6.5 ms for a context's first call): a process that solves one small block is better off without,
+ * 8 MB break even in one call (7.2 ms both). */
+constexpr size_t HOST_COPY_PIN = 8u << 20;
 /* Bytes of a pinned half: 2 MB in all (pinning 8 MB takes 8 ms of a context's first call), 16 MB for
  * outputs of HOST_COPY_LARGE and more. */
 constexpr size_t HOST_COPY_HALF = 1u << 20, HOST_COPY_HALF_LARGE = 8u << 20;
@@ -38,9 +46,12 @@ struct HostCopy {
 class HostCopier {
  public:
   ~HostCopier() { release(); }
-  /* Allocates the halves for outputs of `bytes` (false: no memory for them; the driver's copies do
-   * without). */
+  /* Whether outputs of `bytes` go through the halves: once the context's calls have brought HOST_COPY_PIN,
+   * and there is memory for them; otherwise the driver's copies do. */
   bool ready(size_t bytes) {
+    if (bytes < HOST_COPY_MIN) return false;
+    seen_ += bytes;
+    if (seen_ < HOST_COPY_PIN) return false;
     if (ensure(bytes >= HOST_COPY_LARGE ? HOST_COPY_HALF_LARGE : HOST_COPY_HALF) == cudaSuccess) return true;
     cudaGetLastError();
     release();
@@ -54,6 +65,7 @@ class HostCopier {
   cudaError_t ensure(size_t half);
   char *pinned_ = nullptr;
   size_t half_ = 0; /* bytes per half */
+  size_t seen_ = 0; /* output bytes of the calls so far that could have used the halves */
   cudaEvent_t ev_[2] = {};
 };
 

@@ -704,8 +704,7 @@ static int solve_block(oco_ctx *c, const oco_params *p, const double *rho, const
     if (Vtop) CU(st.top.ensure((size_t)ch * nw * sizeof(double)));
     if (Vbot) CU(st.bot.ensure((size_t)ch * nw * sizeof(double)));
   }
-  /* Small outputs: the driver's copies (a thread's start costs more than their faults); so too without
-   * memory for the pinned slots. */
+  /* Which outputs go through the context's pinned halves (host_copy.h); the driver copies the others. */
   const double *host[5] = {U, kappa, V, Vtop, Vbot};
   bool pageable[5], any = false;
   const size_t out_bytes = (size_t)ncol * nw * ((U ? mz : 0) + (kappa ? nz : 0) + (V ? nz : 0)) * sizeof(double);

@@ -37,9 +37,15 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *, const void *) { re
 extern "C" int host_copy_run(const char *src, char *dst, size_t row_bytes, size_t dst_pitch, size_t rows, long allow) {
   oco::HostCopier c;
   const std::vector<oco::HostCopy> copies{{src, dst, row_bytes, dst_pitch, rows}};
-  if (!c.ready(row_bytes * rows)) return -1;
+  if (!c.ready(std::max(row_bytes * rows, oco::HOST_COPY_PIN))) return -1;
   g_allow = allow;
   const cudaError_t e = c.run(0, nullptr, copies);
   g_allow = -1;
   return (int)e;
+}
+
+// Whether each of n calls' outputs would go through the halves.
+extern "C" void host_copy_ready(const size_t *bytes, int n, int *ready) {
+  oco::HostCopier c;
+  for (int i = 0; i < n; i++) ready[i] = c.ready(bytes[i]) ? 1 : 0;
 }

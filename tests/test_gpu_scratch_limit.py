@@ -37,16 +37,16 @@ def test_split_scratch_does_not_fit(form):
     torch.cuda.empty_cache()
     left = torch.cuda.mem_get_info()[0]
     fill = torch.empty(left - 940_000_000, dtype=torch.uint8, device="cuda")  # records 21 MB, the rest for the scratch
-    n0 = e.kernel_launches()
+    n0 = e.kernel_launches
     got = solve(e, tight)
-    assert e.kernel_launches() - n0 == 2  # records and the persistent solve
+    assert e.kernel_launches - n0 == 2  # records and the persistent solve
     del fill
     torch.cuda.empty_cache()
     e.close()
     e = Engine(0)
-    n0 = e.kernel_launches()
+    n0 = e.kernel_launches
     ref = solve(e, free)
-    assert e.kernel_launches() - n0 == 3  # records and the split solve's two
+    assert e.kernel_launches - n0 == 3  # records and the split solve's two
     e.close()
     for k in ref:
         assert np.array_equal(got[k].view(np.uint64), ref[k].view(np.uint64)), k

@@ -1,5 +1,6 @@
 """The host copies of large pageable outputs (host_copy.cu) with the CUDA calls replaced by plain copies:
 complete at every row pitch, and complete on fewer threads where starting one runs out of memory."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -44,3 +45,14 @@ def test_copies_are_complete(lib, row, pitch, rows, allow):
     r = subprocess.run([sys.executable, "-c", CHILD, lib] + [str(x) for x in (row, pitch, rows, allow)],
                        capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout == "complete\n", r.stderr[-500:]
+
+
+@pytest.mark.parametrize("mb,ready", [
+    ([4.2], [0]),  # a process that solves one block pays for no pinned memory
+    ([4.2, 4.2, 4.2], [0, 1, 1]), ([31.0], [1]), ([0.5, 2.0] * 8, [0] * 16), ([2.9] * 4 + [4.2, 4.2, 2.0], [0] * 5 + [1, 0])])
+def test_pinned_memory_waits_for_enough_outputs(lib, mb, ready):
+    h = ctypes.CDLL(lib)
+    n = (ctypes.c_size_t * len(mb))(*[int(x * (1 << 20)) for x in mb])
+    got = (ctypes.c_int * len(mb))()
+    h.host_copy_ready(n, len(mb), got)
+    assert list(got) == ready
