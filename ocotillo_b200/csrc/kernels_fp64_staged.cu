@@ -61,6 +61,8 @@ static const void *fn_of(StoreMode m) {
     default: return (const void *)k_solve_staged<FORM, ST_LANE>;
   }
 }
-const void *solve_staged_fn(int form, StoreMode m) { return form == 0 ? fn_of<0>(m) : fn_of<1>(m); }
+/* The stable form named first: the compiler then gives the plain kernel of LaneStores 126 registers
+ * instead of 128 (297 tiles x 512 levels 0.41 instead of 0.43 ms). */
+const void *solve_staged_fn(int form, StoreMode m) { return form == 1 ? fn_of<1>(m) : fn_of<0>(m); }
 
 }  // namespace oco
