@@ -134,7 +134,7 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
   const LamR L(it, nullptr);
   double *Kb = it.K();
   const int64_t kz = it.kz();
-  double h = 0.0, u = 0.0, c_prev = 0.0; /* recurrence state (lane 0) */
+  Chain e{}; /* recurrence state (lane 0) */
   bool bad = false;
   for (int z0 = 0; z0 < nz; z0 += RSEG) {
     const int n = min(RSEG, nz - z0);
@@ -186,27 +186,17 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
     if (lane == 0) {
       int k = 0;
       if (z0 == 0) {
-        h = g.ee[0];
-        const double bet = -(g.cc[0] + h);
-        bad = bet == 0.0;
-        u = g.dd[0] / bet;
-        uu[0] = u;
-        c_prev = g.cc[0];
+        e = chain_first<1>(g.ee[0], g.cc[0], g.dd[0], bad);
+        uu[0] = e.u;
         k = 1;
       }
       for (; k < n; k++) {
         const int j = z0 + k;
-        const double aa = g.aa[k], cc = g.cc[k];
-        const double den = c_prev + h;
-        const double gj = -(c_prev / den);
-        qs[j - 1] = h / den;
-        h = g.ee[k] + (aa * h) / den;
-        const double bet = -(cc + h);
-        if (bet == 0.0) bad = true;
-        u = (g.dd[k] - aa * u) / bet;
+        double gj, qj;
+        chain_step<1>(e, g.aa[k], g.ee[k], g.cc[k], g.dd[k], gj, qj, bad);
+        qs[j - 1] = qj; /* q_{j-1} = h_{j-1}/(c_{j-1} + h_{j-1}) */
         gam[j] = gj;
-        uu[j] = u;
-        c_prev = cc;
+        uu[j] = e.u;
       }
     }
     __syncwarp();
@@ -219,7 +209,7 @@ __device__ __forceinline__ void repair_one(const IT &it, double fit, RSeg &g, do
   /* 4. the reverse sweep: back-substitution, ghosts, flux (scratch at stride 1) */
   const UnitStride<IT> iu{it};
   LaneStores<false> st = lane_stores(iu);
-  solve_reverse<1>(iu, true, u, gam, uu, o1, qs, st);
+  solve_reverse<1>(iu, true, e.u, gam, uu, o1, qs, st);
 }
 
 /* ---- coefficient slots ------------------------------------------------------------------ */
@@ -396,6 +386,10 @@ __device__ __forceinline__ void chain_item(const IT &it, const Slots &S, int64_t
   solve_reverse<1, RG_ALONE, true>(it, true, e.u, aa, dd, S.o1 + q0, ee, st);
 }
 
+/* Four blocks of two warps per SM at 216 registers: the items that the default condition flags need few
+ * warps and short chains.  With every item flagged (1024 AGN columns x 512 x 256, most beyond the slots)
+ * four and six blocks take 62.0 and 58.8 ms, with the default condition 1.92 and 1.94 ms; the ragged batch
+ * of 1024 columns 3.87 and 3.95 ms. */
 __global__ void __launch_bounds__(REPAIR_THREADS, 4) k_repair_solve(const RepairArgs a) {
   __shared__ __align__(16) double s_seg[RWARPS][sizeof(RSeg) / sizeof(double)];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
