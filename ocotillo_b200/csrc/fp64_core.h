@@ -126,8 +126,8 @@ __device__ __forceinline__ void load_lam(Lam &L, const double *__restrict__ lam,
 
 /* The constants as opacity_at reads them: LamR holds them in registers (loaded from the global
  * table); LamS reads them from the warp's shared-memory table [field][32], one column per lane,
- * which frees ~40 registers of the staged kernel (no spills at 128 registers; +3% plain, +5%
- * stable on the AGN grid).  Same values, so the same bits. */
+ * which frees ~40 registers of the staged kernel (at 128 no spills but in the ring variants; +3% plain,
+ * +5% stable on the AGN grid).  Same values, so the same bits. */
 enum { NLF = 20 }; /* fields of the shared table, in the order of store_lam_shared */
 struct LamR {
   Lam L;

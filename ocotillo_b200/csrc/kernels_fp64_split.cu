@@ -10,9 +10,12 @@ namespace oco {
  * first, parallel over (warp tile, RZ levels): k_rows writes the rows' coefficients; k_chain then
  * runs the recurrences, one warp per tile, with nothing but them on its serial chain: 0.23 ms for
  * those 16 columns.  That moves ~180 B per point instead of ~75, so it is taken while there are at
- * most two tiles per SM (solve_is_split; a full wave of the persistent kernel holds 16), and for
- * grey transfer always: it has one wavelength per column (few items) and no opacity sums, and reads
- * rho and T directly instead of a 208-byte record per cell (16,384 columns x 512: 1.08 -> 0.43 ms).
+ * most two tiles per SM (solve_is_split; a full wave of the persistent kernel holds 16).  Split and
+ * persistent solve, plain, tiles of 32 wavelengths x levels: 64 x 512 0.17 and 0.36 ms, 296 x 512 0.35 and
+ * 0.41 ms, 592 x 512 0.55 and 0.45 ms; 64 x 128 83 and 110 us, 296 x 128 112 and 110 us.  With 48
+ * levels and fewer nothing is gained (64 x 48 62 and 58 us, 64 x 16 52 and 44 us); the rule leaves that out.
+ * Grey transfer takes it always: it has one wavelength per column (few items) and no opacity sums, and
+ * reads rho and T directly instead of a 208-byte record per cell (16,384 columns x 512: 1.08 -> 0.41 ms).
  * Per point the operations are solve_item's, so the same bits. */
 /* One cell of a grey column (grey_parameters, continuous_opacity.f90:377-390); the factors of an
  * unchanged temperature are kept. */
@@ -215,9 +218,13 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, 
   solve_reverse<FORM, RG_ALONE>(it, active, e.u, S.aa, S.dd, S.kap, S.xx, st);
 }
 
-/* Outputs with z fastest: through the ring only where they do not fit in L2, which otherwise joins the
- * lanes' own stores into whole lines for nothing (16 columns x 500 x 250, 48 MB: 0.33 ms with the
- * ring, 0.23 ms without; 16,384 grey columns, 201 MB: 0.44 and 0.42 ms). */
+/* Outputs with z fastest from this size on go through the ring, which the single warps of k_chain wait for
+ * but which writes whole runs; below it L2 joins the lanes' own stores into lines.  Which is better turns on
+ * the number of tiles and the shape as much as on the size (ring / lanes, us): 16 columns x 500 x 250, 48 MB,
+ * 330 / 230; grey columns x levels: 4096 x 512, 50 MB, 323 / 194; 16,384 x 512, 201 MB, 441 / 415; 25,600 x
+ * 512, 315 MB, 546 / 640; 16,384 x 1024, 403 MB, 839 / 788; 65,536 x 1024, 1.6 GB, 2384 / 3104; 296 columns
+ * x 32 wavelengths x 1024 levels, 233 MB, 714 / 794, x 2048 1373 / 1891; but 37 x 250 x 2048, 455 MB, 1445 /
+ * 1189, and 1880 x 5 x 2048, 462 MB, 2227 / 1852. */
 constexpr int64_t SPLIT_RING_BYTES = 256ll << 20;
 
 template <int FORM>

@@ -17,11 +17,11 @@
  *                   fill_boundary_coeffs, auxiliary.f90:125-201), stored in the item's slot
  *                   with 1/kappa, and kappa in the output;
  *   k_repair_solve  the recurrences: one lane per slot runs the difference-form elimination over
- *                   the stored coefficients (loads of 8 levels hoisted off the serial chain),
+ *                   the stored coefficients (two groups of 8 levels in flight),
  *                   then the stable form's reverse sweep (solve_reverse: back-substitution,
  *                   ghosts, flux), storing over the mixed results.
  *
- * An item's critical path is thus its elimination alone (two dependent divisions per level)
+ * An item's critical path is thus its elimination alone (a reciprocal and two quotients per level)
  * instead of its whole per-level work, and the per-level work of all items runs at the GPU's
  * throughput.  Items beyond the slots' capacity (the mixed solve's scratch, free once that
  * kernel has finished) are re-solved one warp per item by k_repair_solve (repair_one: the same
