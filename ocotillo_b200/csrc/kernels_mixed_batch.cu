@@ -133,7 +133,8 @@ int batch_mixed_max_blocks_per_sm(int tiling, int threads) {
 
 cudaError_t launch_batch_mixed(const MixedBatchArgs &a, int tiling, int blocks, int threads, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(batch_mixed_fn(tiling, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads), args, 0, s);
+  const StoreMode m = mixed_store_mode(a.U, a.K, a.V, a.layout, a.npoints, 1);
+  return cudaLaunchKernel(batch_mixed_fn(tiling, m), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

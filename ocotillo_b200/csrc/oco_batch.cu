@@ -79,6 +79,7 @@ static MixedBatchArgs batch_args(const oco_batch *b) {
   a.ncol = b->ncol;
   a.ntasks = b->tiling == OCO_TILING_PACKED ? b->ntasks_packed : b->ntasks_tile;
   a.nitems = b->nitems;
+  a.npoints = b->npoints;
   a.U = b->U;
   a.K = b->K;
   a.V = b->V;

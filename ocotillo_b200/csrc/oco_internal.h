@@ -25,11 +25,12 @@ inline StoreMode store_mode(const void *U, const void *K, const void *V, int lay
   return !U && !K && !V ? ST_PLANES : layout == 0 ? ST_RING : ST_LANE;
 }
 
-/* The same for a mixed chunk of `items` items: z fastest takes the ring only where the outputs leave L2,
+/* The same for a mixed chunk of `items` items of nz levels (a batch: its points and 1): z fastest takes the ring only where the outputs leave L2,
  * which otherwise joins the lanes' own stores into whole lines, and the warps are few, so that each waits
  * for its own ring (lanes / ring: 16 columns x 500 levels x 250 wavelengths, 48 MB, 0.37 / 0.51 ms; 16 x
  * 33 x 5 60 / 71 us; 148 x 512 x 32, 58 MB, the same; 256 x 256 x 64, 101 MB, 0.38 / 0.36 ms; 1024 x 128
- * x 64, 201 MB, 0.56 / 0.32 ms). */
+ * x 64, 201 MB, 0.56 / 0.32 ms; ragged batches, 1 to 16 columns of up to 128 levels 102-121 / 129-156 us, 2
+ * of up to 2048, 38 MB, 1.37 / 1.45 ms, 32, 174 MB, 2.05 / 1.83 ms, between those either). */
 constexpr int64_t MIXED_RING_BYTES = 56ll << 20;
 inline StoreMode mixed_store_mode(const void *U, const void *K, const void *V, int layout, int64_t items, int nz) {
   const int64_t bytes = items * nz * (int64_t)sizeof(double) * ((U != nullptr) + (K != nullptr) + (V != nullptr));
@@ -236,7 +237,7 @@ struct MixedBatchArgs {
   const uint2 *tasks;      /* warp-column tiling: (column, 32-wavelength tile), longest first */
   const int32_t *order;    /* packed tiling: columns, longest first */
   const int64_t *item_pre; /* packed tiling: prefix sums of nw over order, ncol + 1 entries */
-  int64_t ncol, ntasks, nitems;
+  int64_t ncol, ntasks, nitems, npoints;
   double *U, *K, *V, *Vtop, *Vbot;
   int layout;
   float4 *s4;        /* scratch: per warp slot max_nz levels of 32 12-byte records (MScratch12) */
