@@ -63,25 +63,25 @@ __global__ void __launch_bounds__(128, MBLOCKS) k_solve_mixed_staged(const Mixed
 
 static bool mixed_uses_staging(int nw) { return (nw >= 64) || (nw % 32) == 0; }
 
-static const void *solve_mixed_fn(int nw, StoreMode m) {
+static const void *solve_mixed_fn(int nw, StoreMode m, bool few) {
   if (mixed_uses_staging(nw)) switch (m) {
       case ST_RING: return (const void *)k_solve_mixed_staged<MScratch16, ST_RING>;
       case ST_PLANES: return (const void *)k_solve_mixed_staged<MScratch12P, ST_PLANES>;
       default: return (const void *)k_solve_mixed_staged<MScratch16, ST_LANE>;
     }
-  return solve_mixed_items_fn(m);
+  return solve_mixed_items_fn(m, few);
 }
 
-int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m) {
+int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m, bool few) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw, m), threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_mixed_fn(nw, m, few), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
-cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s) {
+cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, bool few, cudaStream_t s) {
   void *args[] = {(void *)&a};
   const StoreMode m = mixed_store_mode(a.U, a.K, a.V, a.layout, a.ncol * a.nw, a.nz);
-  return cudaLaunchKernel(solve_mixed_fn(a.nw, m), dim3(blocks), dim3(threads), args, 0, s);
+  return cudaLaunchKernel(solve_mixed_fn(a.nw, m, few), dim3(blocks), dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

@@ -4,12 +4,14 @@
 namespace oco {
 
 /* Few wavelengths: 32 consecutive items per warp (lanes past the last item repeat it and store
- * nothing).  Five blocks per SM at 96 registers with 28 bytes spilled (128 x 128 turbulent columns x 256
- * levels, lambda fastest, four blocks at 126 registers -> five: 5 wavelengths 1.31 -> 1.06 ms, 17 2.06 ->
- * 1.89 ms, 33 3.24 -> 2.97 ms, 3 0.98 ms both); the ring variant spills twice as much there and gains at
- * 5 wavelengths only (1.41 -> 1.23 ms; 3 1.04 -> 1.15 ms, 17 and 33 the same). */
-template <class SC, int MODE>
-__global__ void __launch_bounds__(128, MODE == ST_RING ? 4 : 5) k_solve_mixed(const MixedArgs a) {
+ * nothing).  FEW: every warp has its task at four blocks per SM (mixed_items_few), at 126 registers and with
+ * kappa leaving in the reverse sweep; otherwise five blocks at 96 registers with 28 bytes spilled and kappa
+ * leaving in the forward sweep.  Few / other, lambda fastest, us: 16 columns x 500 levels x 17 wavelengths
+ * 380 / 430 (AGN), 567 / 617 (turbulent); 128 x 128 x 256 turbulent, 5 wavelengths 1336 / 1056, 17 2070 /
+ * 1890, 33 3234 / 2970.  The ring variant spills twice as much at five blocks and gains at 5 wavelengths
+ * only (1.41 -> 1.23 ms; 3 1.04 -> 1.15 ms, 17 and 33 the same): four. */
+template <class SC, int MODE, bool FEW>
+__global__ void __launch_bounds__(128, MODE == ST_RING || FEW ? 4 : 5) k_solve_mixed(const MixedArgs a) {
   __shared__ RingSmem<float> s_ring[MODE == ST_RING ? MWARPS : 1];
   const int lane = threadIdx.x & 31;
   const int64_t slot = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -28,15 +30,16 @@ __global__ void __launch_bounds__(128, MODE == ST_RING ? 4 : 5) k_solve_mixed(co
     MDirect pa{a.rec + cl * (int64_t)a.nz * MZN};
     const MItem it = block_item(a, cl, iw);
     const bool flag = msolve_item(it, active, pa, load_lam32(it.lam, iw, it.nw), sc,
-                                  make_stores<MODE, false, false>(it.o, active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
+                                  make_stores<MODE, false, FEW>(it.o, active, &s_ring[MODE == ST_RING ? threadIdx.x >> 5 : 0]), a.repair_cond) ||
                       (active && __ldg(a.colflag + cl) != 0u);
     mark_items(flag, cl * ((a.nw + 31) / 32) + iw / 32, iw, (unsigned long long)item, a.rbits, a.rslot, a.rlist, a.rcount,
                a.ilist, a.icount);
   }
 }
 
-const void *solve_mixed_items_fn(StoreMode m) {
-  return m == ST_RING ? (const void *)k_solve_mixed<MScratch16, ST_RING> : (const void *)k_solve_mixed<MScratch16, ST_LANE>;
+const void *solve_mixed_items_fn(StoreMode m, bool few) {
+  if (m == ST_RING) return (const void *)k_solve_mixed<MScratch16, ST_RING, false>;
+  return few ? (const void *)k_solve_mixed<MScratch16, ST_LANE, true> : (const void *)k_solve_mixed<MScratch16, ST_LANE, false>;
 }
 
 }  // namespace oco

@@ -302,7 +302,7 @@ static const int kSolveThreads = 128;
  * gamma, u, 1/kappa, q (32 B) or, for the mixed form, one record of at most 16 B. */
 static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz, int nw, StoreMode mode, int *blocks) {
   const bool mixed = form == OCO_FORM_MIXED;
-  int bps = mixed ? solve_mixed_max_blocks_per_sm(kSolveThreads, nw, mode)
+  int bps = mixed ? solve_mixed_max_blocks_per_sm(kSolveThreads, nw, mode, mixed_items_few(nitems, c->num_sms))
                   : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey, kSolveThreads, nw, mode);
   int64_t maxb = (int64_t)bps * c->num_sms;
   if (c->max_blocks > 0) maxb = std::min<int64_t>(maxb, c->max_blocks);
@@ -445,7 +445,7 @@ static int run_chunk_mixed(oco_ctx *c, const oco_params *p, const double *rho, c
   r.repairs = c->stats.as<unsigned long long>();
   r.status = c->status.as<unsigned long long>();
   if (c->prof) CU(cudaEventRecord(e2, s));
-  CU(launch_solve_mixed(a, blocks, kSolveThreads, s));
+  CU(launch_solve_mixed(a, blocks, kSolveThreads, mixed_items_few(nb * p->nw, c->num_sms), s));
   CU(launch_repair(r, rcoef_blocks, rsolve_blocks, s));
   if (c->prof) {
     CU(cudaEventRecord(e3, s));
@@ -652,7 +652,7 @@ int oco_ctx_check_params(oco_ctx *c, const oco_params *p) {
 }
 
 int oco_ctx_full_blocks(oco_ctx *c, int form, int grey) {
-  const int bps = form == OCO_FORM_MIXED ? solve_mixed_max_blocks_per_sm(kSolveThreads, 64, ST_LANE)
+  const int bps = form == OCO_FORM_MIXED ? solve_mixed_max_blocks_per_sm(kSolveThreads, 64, ST_LANE, false)
                                          : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey,
                                                                         kSolveThreads, 64, ST_LANE);
   return bps * c->num_sms;

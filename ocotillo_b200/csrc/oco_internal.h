@@ -382,9 +382,11 @@ constexpr int MIXED_LN = 29; /* fields of the mixed wavelength table */
 /* colflag[ncol] (cleared by the caller) marks columns to re-solve in FP64 (mx::pillar). */
 cudaError_t launch_pillars_mixed(const double *rho, const double *T, int64_t ncol, int nz, double fully_ionized_T,
                                  float *rec, unsigned *colflag, const ChunkInit &init, cudaStream_t s);
-cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, cudaStream_t s);
-int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m);
-const void *solve_mixed_items_fn(StoreMode m);
+/* Whether a by-item mixed chunk's warps all fit four blocks of 128 threads per SM. */
+inline bool mixed_items_few(int64_t items, int num_sms) { return items <= (int64_t)num_sms * 4 * 128; }
+cudaError_t launch_solve_mixed(const MixedArgs &a, int blocks, int threads, bool few, cudaStream_t s);
+int solve_mixed_max_blocks_per_sm(int threads, int nw, StoreMode m, bool few);
+const void *solve_mixed_items_fn(StoreMode m, bool few);
 /* Fills tab32[MIXED_LN*nw] from the FP64 table tab[NL*nw]. */
 void fill_mixed_lambda_table(const double *tab, int nw, float *tab32);
 
