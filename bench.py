@@ -353,15 +353,15 @@ PUBLISHED_POINTS_PER_S = 1e6 / 0.14415
 # FP64 flops = DADD + DMUL + 2 DFMA, FP32 flops = FADD + FMUL + 2 FFMA, and the pipes' activity.
 FP_COUNTERS = {"plain": {"fp64_flops_per_point": 167.2, "fp32_flops_per_point": 0.3, "fp64_pipe_active": 0.404,
                          "fma_pipe_active": 0.106, "xu_active": 0.060},
-               "mixed": {"fp64_flops_per_point": 14.1, "fp32_flops_per_point": 95.1, "fp64_pipe_active": 0.060,
-                         "fma_pipe_active": 0.312, "xu_active": 0.463}}
+               "mixed": {"fp64_flops_per_point": 14.1, "fp32_flops_per_point": 95.1, "fp64_pipe_active": 0.062,
+                         "fma_pipe_active": 0.319, "xu_active": 0.484}}
 FP64_PEAK_TFLOPS, FP32_PEAK_TFLOPS = 37.0, 75.0  # nominal B200 (no measured FP figure in MEASURED_PEAKS.json)
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per mesh*lambda point of the solve
 # kernel, from one ncu --set full capture of a 1024-column launch of this grid (outputs 3.2 GB,
 # larger than L2), scaled to a launch by its points: profiles/k_solve_staged_plain_agn_32x32x512x256.txt
 # and profiles/k_solve_mixed_staged_agn_32x32x512x256.txt.
-TRAFFIC_BYTES_PER_POINT = {"plain": 70.9, "mixed": 56.4}
+TRAFFIC_BYTES_PER_POINT = {"plain": 70.9, "mixed": 56.2}
 
 
 def flux_error(g, form_a, form_b, eps=1e-7, seed=7):
