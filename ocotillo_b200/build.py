@@ -29,7 +29,6 @@ UNITS = [
     ("kernels_fp64_items.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_fp64_staged.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_fp64_split.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
-    ("kernels_fp64_batch.cu", ["-fmad=false", "-prec-div=true", "-prec-sqrt=true"]),
     ("kernels_mixed.cu", []),
     ("kernels_mixed_items.cu", []),
     ("kernels_mixed_batch.cu", []),

@@ -1,8 +1,8 @@
 /*
  * kernels_fp64.cu -- the FP64 hot path on sm_100a.  Its kernels stand in one unit per path (records and
- * dispatch here; kernels_fp64_staged.cu, _items.cu, _split.cu, _batch.cu), because a process loads a
+ * dispatch here; kernels_fp64_staged.cu, _items.cu, _split.cu), because a process loads a
  * unit's module, line tables included, when it first launches one of its kernels: as one unit of 14 MB,
- * which the compiler driver also compresses, that took 13.5 ms of a process's first solve, 2.6 ms so.
+ * which the compiler driver also compresses, that took 13.5 ms of a process's first solve, 2.2-3.7 ms so.
  *
  *   k_pillars   one thread per (column, z): Saha ionization and every factor of the
  *               reference's per-(z, lambda) opacity that depends on z only
@@ -60,13 +60,13 @@ cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int
 
 bool solve_uses_staging(int nw) { return nw >= 64 || (nw % 32) == 0; }
 
-static const void *solve_fn(int form, int grey, int nw, StoreMode m) {
-  return !grey && solve_uses_staging(nw) ? solve_staged_fn(form, m) : solve_items_fn(form, grey, m);
+static const void *solve_fn(int form, int grey, int nw, StoreMode m, bool few) {
+  return !grey && solve_uses_staging(nw) ? solve_staged_fn(form, m) : solve_items_fn(form, grey, m, few);
 }
 
-int solve_fp64_max_blocks_per_sm(int form, int grey, int threads, int nw, StoreMode m) {
+int solve_fp64_max_blocks_per_sm(int form, int grey, int threads, int nw, StoreMode m, bool few) {
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_fn(form, grey, nw, m), threads, 0);
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, solve_fn(form, grey, nw, m, few), threads, 0);
   return (e == cudaSuccess && n > 0) ? n : 1;
 }
 
@@ -96,10 +96,10 @@ cudaError_t launch_bounded_wait_check(long long limit, unsigned long long *statu
   return cudaGetLastError();
 }
 
-cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int blocks, int threads, cudaStream_t s) {
+cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int blocks, int threads, bool few, cudaStream_t s) {
   void *args[] = {(void *)&a};
-  return cudaLaunchKernel(solve_fn(form, grey, a.nw, store_mode(a.U, a.K, a.V, a.layout)), dim3(blocks), dim3(threads),
-                          args, 0, s);
+  return cudaLaunchKernel(solve_fn(form, grey, a.nw, store_mode(a.U, a.K, a.V, a.layout), few), dim3(blocks),
+                          dim3(threads), args, 0, s);
 }
 
 }  // namespace oco

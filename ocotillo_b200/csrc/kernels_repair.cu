@@ -69,7 +69,7 @@ struct RBlockItem {
   __device__ __forceinline__ const double *T() const { return a.T + cl * a.nz; }
 };
 
-/* A flagged item of a ragged batch (cf. BatchItem in kernels_fp64_batch.cu). */
+/* A flagged item of a ragged batch (cf. BatchItem in kernels_fp64_staged.cu). */
 struct RBatchItem {
   const RepairArgs &a;
   const MBatchCol &c;

@@ -303,7 +303,8 @@ static const int kSolveThreads = 128;
 static int prepare_solve(oco_ctx *c, int form, int grey, int64_t nitems, int nz, int nw, StoreMode mode, int *blocks) {
   const bool mixed = form == OCO_FORM_MIXED;
   int bps = mixed ? solve_mixed_max_blocks_per_sm(kSolveThreads, nw, mode, mixed_items_few(nitems, c->num_sms))
-                  : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey, kSolveThreads, nw, mode);
+                  : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey, kSolveThreads, nw, mode,
+                                                 solve_items_few(nitems, c->num_sms));
   int64_t maxb = (int64_t)bps * c->num_sms;
   if (c->max_blocks > 0) maxb = std::min<int64_t>(maxb, c->max_blocks);
   int64_t need = (nitems + kSolveThreads - 1) / kSolveThreads;
@@ -506,7 +507,7 @@ static int run_chunk(oco_ctx *c, const oco_params *p, const double *rho, const d
   if (split)
     CU(launch_solve_split(a, form, grey, grey ? init : ChunkInit{}, s));
   else
-    CU(launch_solve_fp64(a, form, grey, blocks, kSolveThreads, s));
+    CU(launch_solve_fp64(a, form, grey, blocks, kSolveThreads, solve_items_few(nb * p->nw, c->num_sms), s));
   if (c->prof) {
     CU(cudaEventRecord(e3, s));
     c->ev_solve.emplace_back(e2, e3);
@@ -654,7 +655,7 @@ int oco_ctx_check_params(oco_ctx *c, const oco_params *p) {
 int oco_ctx_full_blocks(oco_ctx *c, int form, int grey) {
   const int bps = form == OCO_FORM_MIXED ? solve_mixed_max_blocks_per_sm(kSolveThreads, 64, ST_LANE, false)
                                          : solve_fp64_max_blocks_per_sm(form == OCO_FORM_STABLE ? 1 : 0, grey,
-                                                                        kSolveThreads, 64, ST_LANE);
+                                                                        kSolveThreads, 64, ST_LANE, false);
   return bps * c->num_sms;
 }
 

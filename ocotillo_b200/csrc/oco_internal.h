@@ -363,11 +363,13 @@ void fill_lambda_table(const double *waves, int nw, double *tab);
 /* Kernel launchers (defined in kernels_fp64.cu). Return cudaGetLastError(). */
 cudaError_t launch_pillars(const double *rho, const double *T, int64_t ncol, int nz,
                            double fully_ionized_T, int grey, double *pil, const ChunkInit &init, cudaStream_t s);
+/* Whether a by-item chunk's warps all fit two blocks of 128 threads per SM. */
+inline bool solve_items_few(int64_t items, int num_sms) { return items <= (int64_t)num_sms * 2 * 128; }
 cudaError_t launch_solve_fp64(const SolveArgs &a, int form, int grey, int nslot_blocks,
-                              int threads, cudaStream_t s);
-/* Occupancy of the kernel used for nw and m (another's would be loaded for the question alone). */
-int solve_fp64_max_blocks_per_sm(int form, int grey, int threads, int nw, StoreMode m);
-const void *solve_items_fn(int form, int grey, StoreMode m);
+                              int threads, bool few, cudaStream_t s);
+/* Occupancy of the kernel used for nw, m and few (another's would be loaded for the question alone). */
+int solve_fp64_max_blocks_per_sm(int form, int grey, int threads, int nw, StoreMode m, bool few);
+const void *solve_items_fn(int form, int grey, StoreMode m, bool few);
 const void *solve_staged_fn(int form, StoreMode m);
 /* Runs the bounded-wait diagnostic kernel (one warp) on s; sets status[2] when the wait ran out. */
 cudaError_t launch_bounded_wait_check(long long limit, unsigned long long *status, cudaStream_t s);

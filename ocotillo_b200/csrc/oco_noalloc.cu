@@ -137,9 +137,11 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
    * column of pillars fits up to OCO_NOALLOC_MAX_NZ (static_assert above). */
   const size_t tab_bytes = grey ? 0 : round256((size_t)NL * nw * sizeof(double));
   const size_t avail = OCO_NOALLOC_WORKSPACE_BYTES - 256 - tab_bytes;
-  int nsm = 0, bps = solve_fp64_max_blocks_per_sm(p->form == OCO_FORM_STABLE ? 1 : 0, grey, kThreads, nw,
-                                                  store_mode(U, kappa, V, p->layout));
+  int nsm = 0;
   CUN(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const bool few = solve_items_few((int64_t)p->nx * p->ny * nw, nsm);
+  const int bps = solve_fp64_max_blocks_per_sm(p->form == OCO_FORM_STABLE ? 1 : 0, grey, kThreads, nw,
+                                               store_mode(U, kappa, V, p->layout), few);
   const size_t per_block = scratch_block_bytes((size_t)nz), per_col = pillar_column_bytes((size_t)nz);
   const int64_t ncol = (int64_t)p->nx * p->ny;
   const int64_t need_blocks = (ncol * nw + kThreads - 1) / kThreads;
@@ -202,7 +204,7 @@ extern "C" int oco_solve_block_noalloc(const oco_params *p, const double *wa_ang
       if (c0 == 0) init.status = ctr + 1;
       CUN(launch_pillars(rho + c0 * nz, T + c0 * nz, nb, nz, p->fully_ionized_T, grey, pil, init, s));
       const int64_t nblk = std::min<int64_t>(blocks, (nb * nw + kThreads - 1) / kThreads);
-      CUN(launch_solve_fp64(a, p->form == OCO_FORM_STABLE ? 1 : 0, grey, (int)nblk, kThreads, s));
+      CUN(launch_solve_fp64(a, p->form == OCO_FORM_STABLE ? 1 : 0, grey, (int)nblk, kThreads, few, s));
     }
     return OCO_OK;
   }());

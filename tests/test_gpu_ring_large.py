@@ -1,6 +1,6 @@
-"""The output ring (z fastest) in the block kernels that take it only from a size on: the persistent FP64
-kernels beyond two wavelength tiles per SM, the mixed kernels beyond 56 MiB of outputs, and the split
-solve's chain beyond 256 MiB.  The outputs equal the lambda-fastest ones (stored lane by lane) bit for bit
+"""The output ring (z fastest) in the kernels that take it only from a size on: the persistent FP64 block
+kernels beyond two wavelength tiles per SM, the mixed block and batch kernels beyond 56 MiB of outputs, and
+the split solve's chain beyond 256 MiB.  The outputs equal the lambda-fastest ones (stored lane by lane) bit for bit
 at every remainder of the groups of 8 levels, and nothing outside the arrays is written."""
 import pytest
 
@@ -73,3 +73,43 @@ def test_split_chain(engine, form, ncol, nw, nz0, grey):
     for nz in range(nz0, nz0 + 8):
         _check(engine, ncol, nz, nw, form, grey)
     _pivots(engine, form)
+
+
+def test_mixed_batch(engine):
+    import numpy as np
+    import torch
+
+    from ocotillo_b200 import workloads
+    rng = np.random.default_rng(6)
+    kinds = [(n, int(w)) for n in list(range(2, 40)) + [64, 129] for w in rng.integers(1, 100, 2)]
+    reps = (60 << 20) // (24 * sum(n * w for n, w in kinds)) + 1
+    cols = {n: workloads.athena_column(n, rng, sigma_dex=0.3) for n in {n for n, _ in kinds}}
+    nz, nw = (np.array([k[i] for k in kinds] * reps) for i in (0, 1))
+    assert 24 * int((nz * nw).sum()) > 56 << 20
+    grids = {w: workloads.log_wavelengths(w, 900.0, 40000.0) for w in set(nw.tolist())}
+    at, pos = {}, 0
+    for w, g in grids.items():
+        at[w] = pos
+        pos += len(g)
+    rho, T = (torch.from_numpy(np.concatenate([cols[n][i] for n in nz.tolist()])).cuda() for i in (0, 1))
+    dz = np.array([cols[n][2] for n in nz.tolist()])
+    got = []
+    for layout in (0, 1):
+        b = engine.batch(nz, nw, dz, np.concatenate(list(grids.values())), np.array([at[w] for w in nw.tolist()]),
+                         layout=layout, form="mixed")
+        bufs = {}
+        for k, v in b.alloc().items():
+            buf = torch.full((v.numel() + 64,), -77.0, dtype=torch.float64, device="cuda")
+            bufs[k] = (buf, buf[19:19 + v.numel()])
+        b.bind(rho, T, {k: v[1] for k, v in bufs.items()})
+        b.run()
+        torch.cuda.synchronize()
+        host = {}
+        for k, (buf, view) in bufs.items():
+            assert (buf[:19] == -77.0).all() and (buf[19 + view.numel():] == -77.0).all(), k
+            host[k] = view.cpu()
+        got.append([{k: b.column(host, i, k).contiguous().view(torch.int64) for k in KEYS} for i in range(len(nz))])
+        b.close()
+    for i, (x, y) in enumerate(zip(*got)):
+        for k in KEYS:
+            assert torch.equal(x[k], y[k]), (k, i, kinds[i % len(kinds)])
