@@ -75,8 +75,9 @@ struct SplitRows {
   }
 };
 
-/* by_tile: see split_item; ring: k_chain's outputs go through the ring, kappa among them (both uniform,
- * so not worth code of their own: a process pays for loading each variant at its first solve). */
+/* by_tile: see split_item (never for grey transfer); ring: k_chain's outputs go through the ring, kappa among
+ * them (both uniform, so not worth code of their own: a process pays for loading each variant at its
+ * first solve). */
 template <int FORM, bool GREY>
 __global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tiles, bool by_tile, bool ring,
                                                  const ChunkInit init) {
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tile
   const int nz = a.nz, z0 = (int)(w - t * nch) * RZ, z1 = min(z0 + RZ, nz);
   int64_t cl;
   int iw;
-  const bool active = split_item(a, by_tile, t, cl, iw);
+  const bool active = split_item(a, !GREY && by_tile, t, cl, iw);
   const BlockItem it{a, cl, iw};
   const LamR L(it, nullptr, !GREY);
   TCacheR tc;
@@ -155,16 +156,16 @@ __global__ void __launch_bounds__(128, 4) k_rows(const SolveArgs a, int64_t tile
   }
 }
 
-/* One warp per block, so that the tiles spread over the SMs.  ROWS: the ring's rows are one column's
- * (by_tile). */
-template <int FORM, bool RING, bool ROWS>
-__global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, bool by_tile) {
+/* One warp per block, so that the tiles spread over the SMs.  TILE: by_tile of k_rows (as an argument it
+ * costs the shortest solves 2 of 45 us: 4 columns x 16 levels x 32 wavelengths). */
+template <int FORM, bool RING, bool TILE>
+__global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles) {
   __shared__ RingSmem<double> s_ring[1];
   const int64_t t = blockIdx.x;
   const int nz = a.nz;
   int64_t cl;
   int iw;
-  const bool active = split_item(a, by_tile, t, cl, iw);
+  const bool active = split_item(a, TILE, t, cl, iw);
   const BlockItem it{a, cl, iw};
   const SplitRows S(a, tiles, t, 0);
   bool bad = false;
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, 
     atomicMin(&it.status()[1], it.id());
   }
   __syncwarp();
-  auto st = make_stores<RING ? ST_RING : ST_LANE, ROWS, false>(out_ptrs(it), active, s_ring);
+  auto st = make_stores<RING ? ST_RING : ST_LANE, TILE, false>(out_ptrs(it), active, s_ring);
   solve_reverse<FORM, RG_ALONE>(it, active, e.u, S.aa, S.dd, S.kap, S.xx, st);
 }
 
@@ -227,14 +228,12 @@ __global__ void __launch_bounds__(32) k_chain(const SolveArgs a, int64_t tiles, 
  * 1189, and 1880 x 5 x 2048, 462 MB, 2227 / 1852. */
 constexpr int64_t SPLIT_RING_BYTES = 256ll << 20;
 
-template <int FORM>
-static cudaError_t launch_chain(const SolveArgs &a, int64_t tiles, bool by_tile, bool ring, cudaStream_t s) {
-  if (!ring)
-    k_chain<FORM, false, false><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, by_tile);
-  else if (by_tile)
-    k_chain<FORM, true, true><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, true);
+template <int FORM, bool TILE>
+static cudaError_t launch_chain(const SolveArgs &a, int64_t tiles, bool ring, cudaStream_t s) {
+  if (ring)
+    k_chain<FORM, true, TILE><<<(unsigned)tiles, 32, 0, s>>>(a, tiles);
   else
-    k_chain<FORM, true, false><<<(unsigned)tiles, 32, 0, s>>>(a, tiles, false);
+    k_chain<FORM, false, TILE><<<(unsigned)tiles, 32, 0, s>>>(a, tiles);
   return cudaGetLastError();
 }
 /* init: set up by k_rows where no record kernel comes before it (grey). */
@@ -249,7 +248,8 @@ static cudaError_t split_launch(const SolveArgs &a, int grey, const ChunkInit &i
   else
     k_rows<FORM, false><<<blocks, 128, 0, s>>>(a, tiles, by_tile, ring, init);
   const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? launch_chain<FORM>(a, tiles, by_tile, ring, s) : e;
+  if (e != cudaSuccess) return e;
+  return by_tile ? launch_chain<FORM, true>(a, tiles, ring, s) : launch_chain<FORM, false>(a, tiles, ring, s);
 }
 cudaError_t launch_solve_split(const SolveArgs &a, int form, int grey, const ChunkInit &init, cudaStream_t s) {
   return form == 0 ? split_launch<0>(a, grey, init, s) : split_launch<1>(a, grey, init, s);
