@@ -11,3 +11,11 @@ extern "C" int64_t split_grid(int64_t ncol, int nw, int nz) {
   const int64_t tiles = oco::split_tiles(ncol, nw);
   return std::max(tiles, oco::split_row_blocks(tiles, nz));
 }
+// The other rules by size of the block solves.
+extern "C" int items_few(int mixed, int64_t items, int num_sms) {
+  return mixed ? oco::mixed_items_few(items, num_sms) : oco::solve_items_few(items, num_sms);
+}
+extern "C" int mixed_mode(int arrays, int layout, int64_t items, int nz) {
+  const void *p = &items;
+  return oco::mixed_store_mode(arrays > 0 ? p : nullptr, arrays > 1 ? p : nullptr, arrays > 2 ? p : nullptr, layout, items, nz);
+}

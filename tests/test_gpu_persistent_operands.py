@@ -29,7 +29,7 @@ def _reference(oracle, rho, T, wa, dz, form):
                               form=oracle.FORM_STABLE if form == "stable" else oracle.FORM_REFERENCE, backend="ocomath")
 
 
-def _check(engine, oracle, rho, T, dz, nw, form):
+def _check(engine, oracle, rho, T, dz, nw, form, items=0):
     import torch
 
     from ocotillo_b200 import workloads
@@ -37,7 +37,7 @@ def _check(engine, oracle, rho, T, dz, nw, form):
     wa = workloads.log_wavelengths(nw)
     ref = _reference(oracle, rho, T, wa, dz, form)
     tiles = (nw + 31) // 32 if nw >= 64 or nw % 32 == 0 else nw / 32
-    rep = int(297 / tiles / 8) + 1  # copies of the 8 columns
+    rep = max(int(297 / tiles / 8), items // (8 * nw)) + 1  # copies of the 8 columns
     r, t = (torch.from_numpy(x.reshape(1, 8, nz)).cuda().repeat(1, rep, 1) for x in (rho, T))
     engine.set_wavelengths(wa)
     for layout in (0, 1):
@@ -73,6 +73,14 @@ def test_plateaus(engine, oracle, form, nz, nw):
 def test_operands_out_of_range(engine, oracle, form, nw, scale, dz):
     rho, T = _columns(20)
     _check(engine, oracle, rho * scale, T, dz, nw, form)
+
+
+@pytest.mark.parametrize("form", ["plain", "stable"])
+@pytest.mark.parametrize("nz,nw", [(4, 40), (13, 33), (60, 40)])
+def test_more_warps_than_two_blocks_per_sm_hold(engine, oracle, form, nz, nw):
+    """The by-item kernel's variant for many warps (three blocks per SM)."""
+    rho, T = _columns(nz)
+    _check(engine, oracle, rho, T, 1e16 / (nz - 1), nw, form, items=148 * 2 * 128)
 
 
 @pytest.mark.parametrize("form", ["plain", "stable"])

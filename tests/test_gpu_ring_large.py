@@ -53,7 +53,8 @@ def _pivots(engine, form):
 
 
 @pytest.mark.parametrize("form", ["plain", "stable"])
-@pytest.mark.parametrize("nw,ncol", [(3, 3200), (33, 300), (64, 150), (70, 101)])  # by item, by item, staged, staged
+# by item with few and with many warps, staged
+@pytest.mark.parametrize("nw,ncol", [(3, 3200), (33, 300), (5, 8000), (64, 150), (70, 101)])
 def test_persistent(engine, form, nw, ncol):
     for nz in list(range(2, 36)) + [63, 64, 65, 100]:
         _check(engine, ncol, nz, nw, form)

@@ -1,5 +1,6 @@
-"""Which chunks take the split block solve (oco_internal.h), compiled for the host: few tiles and grey
-transfer, and never with grids beyond the caller's cap, by which a server shares the GPU between jobs."""
+"""The block solves' rules by size (oco_internal.h), compiled for the host.  The split solve takes few tiles
+and grey transfer, and never grids beyond the caller's cap, by which a server shares the GPU between jobs;
+by-item chunks count as few while their warps fit; the mixed form's ring takes z-fastest outputs above 56 MiB."""
 import ctypes
 import os
 import subprocess
@@ -22,6 +23,8 @@ def h():
     lib.split_rule.argtypes = [ctypes.c_int, ctypes.c_int64] + [ctypes.c_int] * 4
     lib.split_grid.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int]
     lib.split_grid.restype = ctypes.c_int64
+    lib.items_few.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int]
+    lib.mixed_mode.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
     return lib
 
 
@@ -37,3 +40,19 @@ def test_the_split_grids_fit_the_cap(h, cap, ncol, nw, nz):
 def test_two_tiles_per_sm(h, ncol, nw, split):
     assert h.split_rule(0, ncol, nw, 100, SMS, 0) == split
     assert h.split_rule(1, ncol, 1, 100, SMS, 0) == 1
+
+
+@pytest.mark.parametrize("mixed,blocks", [(0, 2), (1, 4)])
+def test_few_items(h, mixed, blocks):
+    n = SMS * blocks * 128
+    assert [h.items_few(mixed, i, SMS) for i in (1, n, n + 1, 1 << 40)] == [1, 1, 0, 0]
+
+
+def test_mixed_ring_from_a_size_on(h):
+    lane, ring, planes = 0, 1, 2
+    for arrays in (1, 2, 3):
+        points = (56 << 20) // 8 // arrays
+        assert h.mixed_mode(arrays, 0, points, 1) == lane and h.mixed_mode(arrays, 0, points + 1, 1) == ring
+        assert h.mixed_mode(arrays, 0, points // 7, 7) == lane and h.mixed_mode(arrays, 0, points // 7 + 1, 7) == ring
+        assert h.mixed_mode(arrays, 1, 1 << 40, 100) == lane
+    assert h.mixed_mode(0, 0, 1 << 40, 100) == planes and h.mixed_mode(0, 1, 1, 1) == planes
