@@ -12,8 +12,9 @@ namespace oco {
  * those 16 columns.  That moves ~180 B per point instead of ~75, so it is taken while there are at
  * most two tiles per SM (solve_is_split; a full wave of the persistent kernel holds 16).  Split and
  * persistent solve, plain, tiles of 32 wavelengths x levels: 64 x 512 0.17 and 0.36 ms, 296 x 512 0.35 and
- * 0.41 ms, 592 x 512 0.55 and 0.45 ms; 64 x 128 83 and 110 us, 296 x 128 112 and 110 us.  With 48
- * levels and fewer nothing is gained (64 x 48 62 and 58 us, 64 x 16 52 and 44 us); the rule leaves that out.
+ * 0.41 ms, 592 x 512 0.55 and 0.45 ms; 64 x 128 83 and 110 us, 296 x 128 112 and 110 us.  Columns
+ * of 12 to 48 levels gain little or nothing (64 x 48 56 and 52-64 us, 64 x 16 48 and 32-43 us), shorter ones
+ * lose (SPLIT_MIN_NZ).
  * Grey transfer takes it always: it has one wavelength per column (few items) and no opacity sums, and
  * reads rho and T directly instead of a 208-byte record per cell (16,384 columns x 512: 1.08 -> 0.41 ms).
  * Per point the operations are solve_item's, so the same bits. */

@@ -169,10 +169,15 @@ inline int64_t split_tiles(int64_t ncol, int nw) {
 }
 /* Blocks of k_rows (four warps each); k_chain has a one-warp block per tile. */
 inline int64_t split_row_blocks(int64_t tiles, int nz) { return (tiles * ((nz + RZ - 1) / RZ) + 3) / 4; }
+/* Shorter columns have nothing to split, and the persistent solve is a launch less (992 columns x 4 levels x 5
+ * wavelengths, split and persistent: 30.6 and 22.2 us with lambda fastest, 30.8 and 28.8 us with z fastest;
+ * x 8 levels 43.0 and 32.5, 45.0 and 42.0 us; 33 columns x 12 x 11 45.2 and 36.9, 47.2 and 49.3 us). */
+constexpr int SPLIT_MIN_NZ = 12;
 /* max_blocks: the caller's cap on the grid (0: none), which the split solve's grids must fit. */
 inline bool solve_is_split(int grey, int64_t ncol, int nw, int nz, int num_sms, int max_blocks) {
   const int64_t tiles = split_tiles(ncol, nw);
   if (grey) return true;
+  if (nz < SPLIT_MIN_NZ) return false;
   if (max_blocks > 0 && (tiles > max_blocks || split_row_blocks(tiles, nz) > max_blocks)) return false;
   return tiles <= 2 * (int64_t)num_sms;
 }

@@ -30,7 +30,7 @@ def test_split_scratch_does_not_fit(form):
     # the kernels of both solves loaded, so that the free memory is what the scratch gets
     for ncol in (1, 40):
         e.set_wavelengths(workloads.log_wavelengths(NW))
-        a, b, d = workloads.agn_block(1, ncol, 8, seed=2)
+        a, b, d = workloads.agn_block(1, ncol, 16, seed=2)
         small = {k: torch.empty((NW, 1, ncol), dtype=torch.float64, device="cuda") for k in ("Vtop", "Vbot")}
         e.solve_block_device(torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda(), d, small, form=form)
     torch.cuda.synchronize()

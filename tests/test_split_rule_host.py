@@ -29,7 +29,7 @@ def h():
 
 
 @pytest.mark.parametrize("cap", [1, 7, 74, 148, 592])
-@pytest.mark.parametrize("ncol,nw,nz", [(1, 64, 2), (1, 64, 512), (16, 250, 500), (148, 64, 33), (992, 5, 33), (40, 33, 9)])
+@pytest.mark.parametrize("ncol,nw,nz", [(1, 64, 12), (1, 64, 512), (16, 250, 500), (148, 64, 33), (992, 5, 33), (40, 33, 17)])
 def test_the_split_grids_fit_the_cap(h, cap, ncol, nw, nz):
     grid = h.split_grid(ncol, nw, nz)
     assert h.split_rule(0, ncol, nw, nz, SMS, cap) == (grid <= cap)
@@ -56,3 +56,8 @@ def test_mixed_ring_from_a_size_on(h):
         assert h.mixed_mode(arrays, 0, points // 7, 7) == lane and h.mixed_mode(arrays, 0, points // 7 + 1, 7) == ring
         assert h.mixed_mode(arrays, 1, 1 << 40, 100) == lane
     assert h.mixed_mode(0, 0, 1 << 40, 100) == planes and h.mixed_mode(0, 1, 1, 1) == planes
+
+
+def test_short_columns_are_not_split(h):
+    assert [h.split_rule(0, 4, 64, nz, SMS, 0) for nz in (2, 11, 12, 13)] == [0, 0, 1, 1]
+    assert h.split_rule(1, 4, 1, 2, SMS, 0) == 1
